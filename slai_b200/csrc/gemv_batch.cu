@@ -3,8 +3,9 @@
 //
 // The single-vector kernel (gemv.cu) spends the eight columns of the integer MMA on one vector (four digit planes x two
 // sub-blocks); looping it over a batch streams the matrix once per vector.  Here the packed weights of a tile-step block
-// are loaded and unpacked into MMA operands once and every vector of the batch adds its own MMAs
-// (`compute_batch`, gemv_formats.cuh: per vector the same integer arithmetic as the single-vector code).
+// are loaded and unpacked into MMA operands once and every pair of vectors adds its own MMAs (`compute_pairs`,
+// gemv_formats.cuh; Q6_K, whose sub-blocks of 16 fill half an MMA's depth, one vector at a time): the same integer sums as
+// the single-vector code.
 //
 // Shape.  The digit planes of 8 vectors over the whole of K do not fit in shared memory, so K is cut into chunks of
 // `ch` tile-steps (<= 8) and a unit of work is (chunk, group of 16 row tiles): the 16 warps of a block stage the chunk's
@@ -60,9 +61,7 @@ __device__ __forceinline__ void stage_request(const uint8_t* src, uint32_t dst, 
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// NV vectors are staged; a tile-step block is taken against NC of them at a time (NV / NC passes over the block in shared
-// memory: fewer accumulators live at once).
-template <class F, int NV, int NC = NV>
+template <class F, int NV>
 __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -160,48 +159,24 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
                     tab[(2 * q + 1) * 16 + (sv_j & 7)] = (unsigned char)lo;
                 }
                 *reinterpret_cast<uint2*>(tab + (sv_j & 7) * 16 + 8) = make_uint2(0u, 0u);
-            } else if (F::SV_GRAN == 16) {
-                // Q6_K: 4 x s32 per sub-block of 16 elements
-                int4* sv = reinterpret_cast<int4*>(svb);
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    int sd[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        sd[q] = 0;
-#pragma unroll
-                        for (int e = 0; e < 4; e++) sd[q] = __dp4a((int)pw[4 * half + e][q], 0x01010101, sd[q]);
-                    }
-                    sv[2 * sv_j + half] = make_int4(sd[0], sd[1], sd[2], sd[3]);
-                }
             }
         }
         __syncthreads();
         if (tid < NV) smax[tid] = 0u;  // read by everyone before the barrier above; next written after the next unit's first barrier
 
         // ---- this warp's tile: `nst` blocks against all vectors ----
-        float accA[NV], accB[NV];
+        constexpr int NA = F::PAIRED ? NV / 2 : NV;
+        float accA[NA], accB[NA];
 #pragma unroll
-        for (int v = 0; v < NV; v++) accA[v] = accB[v] = 0.f;
+        for (int v = 0; v < NA; v++) accA[v] = accB[v] = 0.f;
         if (active) {
 #pragma unroll 1
             for (int s = 0; s < nst; s++) {
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest request have landed: block s is here
                 __syncwarp();
                 const uint32_t blk = wb + (uint32_t)(s & 1) * BatchGeom<F>::STRIDE;
-                if (NC == NV) {
-                    F::template compute_batch<NV>(blk, s, L, S, bvs, P.vstride, accA, accB);
-                } else {
-#pragma unroll
-                    for (int pass = 0; pass < NV / NC; pass++) {
-                        LaneCtx L2 = L;
-                        L2.bbase += (uint32_t)(pass * NC) * bvs;
-                        Smem S2 = S;
-                        S2.sv += (uint32_t)(pass * NC) * P.vstride;
-                        F::template compute_batch<NC>(blk, s, L2, S2, bvs, P.vstride, reinterpret_cast<float(&)[NC]>(accA[pass * NC]),
-                                                      reinterpret_cast<float(&)[NC]>(accB[pass * NC]));
-                    }
-                }
+                if constexpr (F::PAIRED) F::template compute_pairs<NV>(blk, s, L, S, P.vstride, accA, accB);
+                else F::template compute_batch<NV>(blk, s, L, S, bvs, P.vstride, accA, accB);
                 __syncwarp();
                 if (s + 2 < nst) stage_request<F>(src + (size_t)(s + 2) * BatchGeom<F>::STEP, blk, lane);
                 stage_commit();
@@ -209,21 +184,26 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
+        for (int v = 0; v < NA; v++) {
             accA[v] += __shfl_xor_sync(0xffffffffu, accA[v], 1);
-            accA[v] += __shfl_xor_sync(0xffffffffu, accA[v], 2);
             accB[v] += __shfl_xor_sync(0xffffffffu, accB[v], 1);
-            accB[v] += __shfl_xor_sync(0xffffffffu, accB[v], 2);
+            if (!F::PAIRED) {
+                accA[v] += __shfl_xor_sync(0xffffffffu, accA[v], 2);
+                accB[v] += __shfl_xor_sync(0xffffffffu, accB[v], 2);
+            }
         }
         if (active) {
+            float* dst = P.part + (size_t)c * NV * P.mp + (size_t)tile * 16;
 #pragma unroll
-            for (int v = 0; v < NV; v++)
-                if ((v & 3) == L.t) {  // the four lanes of a row hold the same sums: lane t stores vectors t and t + 4
-                    const float inv = sinv[v];
-                    float* dst = P.part + ((size_t)c * NV + v) * P.mp + (size_t)tile * 16;
-                    dst[L.g] = accA[v] * inv;
-                    dst[L.g + 8] = accB[v] * inv;
+            for (int v = 0; v < NA; v++) {
+                if (F::PAIRED) {  // lanes t and t ^ 1 hold vector 2v + (t >> 1): the even one stores row g, the odd one row g + 8
+                    const int vec = 2 * v + (L.t >> 1);
+                    dst[(size_t)vec * P.mp + L.g + 8 * (L.t & 1)] = ((L.t & 1) ? accB[v] : accA[v]) * sinv[vec];
+                } else if ((v & 3) == L.t) {  // the four lanes of a row hold the same sums: lane t stores vectors t and t + 4
+                    dst[(size_t)v * P.mp + L.g] = accA[v] * sinv[v];
+                    dst[(size_t)v * P.mp + L.g + 8] = accB[v] * sinv[v];
                 }
+            }
         }
     }
 }
@@ -257,7 +237,7 @@ template <class F>
 size_t batch_smem(int nv, int ch, uint32_t* plane_out, uint32_t* vstride_out) {
     const uint32_t ce = (uint32_t)ch * F::STEP;
     const uint32_t plane = ce + 32;
-    const uint32_t svbytes = F::SV_GRAN == 32 ? 128u * ch : F::SV_GRAN == 16 ? ce : 0u;
+    const uint32_t svbytes = F::SV_GRAN == 32 ? 128u * ch : 0u;  // (the batched Q6_K code has no digit sums)
     const uint32_t vstride = (4 * plane + svbytes + 15) & ~15u;
     *plane_out = plane;
     *vstride_out = vstride;
@@ -265,7 +245,7 @@ size_t batch_smem(int nv, int ch, uint32_t* plane_out, uint32_t* vstride_out) {
     return (size_t)ring_off + (size_t)BWARPS * 2 * BatchGeom<F>::STRIDE;
 }
 
-template <class F, int NV, int NC = NV>
+template <class F, int NV>
 int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate) {
     // Steps per chunk: the fewest rounds of (staging + ch steps) over the SMs; staging a chunk costs about three steps.
     const int G = ctx->sm_count > 0 ? ctx->sm_count : 148;
@@ -288,7 +268,7 @@ int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo
     int rc = ensure_scratch(ctx, part_bytes);
     if (rc) return rc;
     P.part = reinterpret_cast<float*>(ctx->d_scratch);
-    auto kern = gemv_batch_kernel<F, NV, NC>;
+    auto kern = gemv_batch_kernel<F, NV>;
     static PerDeviceOnce attr;  // per instantiation
     if (attr.need(ctx->device)) {
         SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BSMEM_LIMIT));
@@ -308,11 +288,7 @@ template <class F>
 int launch_batch_fmt(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate) {
     if (P.n_batch <= 2) return launch_batch_inst<F, 2>(ctx, P, d_out, ldo, M, epi, gate);
     if (P.n_batch <= 4) return launch_batch_inst<F, 4>(ctx, P, d_out, ldo, M, epi, gate);
-    // Eight vectors: a block is taken against four of them at a time (two passes over it in shared memory) -- with all
-    // eight at once the accumulators leave the compiler no registers to overlap loads and MMAs (measured 7 % slower on
-    // the 11008-wide shapes).  SLAI_BATCH_PASSES=1 selects the one-pass kernel.
-    static const int passes = [] { const char* e = getenv("SLAI_BATCH_PASSES"); return e ? atoi(e) : 2; }();
-    if (passes != 1) return launch_batch_inst<F, 8, 4>(ctx, P, d_out, ldo, M, epi, gate);
+    if (P.n_batch <= 6) return launch_batch_inst<F, 6>(ctx, P, d_out, ldo, M, epi, gate);
     return launch_batch_inst<F, 8>(ctx, P, d_out, ldo, M, epi, gate);
 }
 

@@ -187,6 +187,21 @@ SLAI_HD uint32_t byte_of(uint32_t w, int i) {
 #endif
 }
 
+// The lanes' shares of a pair of vectors (`compute_pairs`) added to one accumulator per vector (zero in the lanes of the other).
+template <class F, int NV>
+SLAI_HD void batch_from_pairs(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t vs, float (&accA)[NV], float (&accB)[NV]) {
+    float a[NV / 2], b[NV / 2];
+    for (int p = 0; p < NV / 2; p++) a[p] = b[p] = 0.f;
+    F::template compute_pairs<NV>(blk, step, L, S, vs, a, b);
+    for (int p = 0; p < NV / 2; p++) {
+        const bool second = (L.t >> 1) != 0;
+        accA[2 * p] += second ? 0.f : a[p];
+        accA[2 * p + 1] += second ? a[p] : 0.f;
+        accB[2 * p] += second ? 0.f : b[p];
+        accB[2 * p + 1] += second ? b[p] : 0.f;
+    }
+}
+
 // Every format provides
 //   STEP      elements of K per tile-step block          SV_GRAN  elements per digit-sum entry (0: none)
 //   compute   one tile-step block at shared address `blk` (K step number `step`): accumulates rows g and g+8
@@ -257,71 +272,91 @@ struct K45 {
         accB = prim::fma(dB, combine(PB0, PB1, L), accB);
         accB = prim::fma(-mnB, (float)(cq[2] * 128 + cq[3]) * L.wq, accB);
     }
-    // The same step against NV staged vectors at once (vector v's digits `bvs` bytes after vector v-1's for the lanes that
-    // read digits, its sum table `svs` bytes after): the packed weights are loaded and masked once, every vector adds its
-    // own MMAs.  Per vector the arithmetic, and its order, is that of `compute`.
+    // The same step against NV staged vectors, two vectors to an MMA: the eight columns hold the four digit planes of both
+    // vectors of a pair, and every lane feeds the same sub-block (8 bytes of the row's 32-byte group), so no column carries
+    // zeros.  Lane t collects digits 2(t & 1), 2(t & 1) + 1 of vector 2p + (t >> 1) for rows g and g + 8: accA[p] / accB[p]
+    // are that lane's share, the sum over lanes t, t ^ 1 is the vector's.  Against one vector per MMA (columns = digits x two
+    // sub-blocks, half of B zero) this halves the MMAs, the loads of B and the integer scale multiplies: they are what bounds the
+    // batched kernel (Q5_K 4096 x 11008, 8 vectors: 24.6 -> 20.5 us).  Vector v's digits are at S.dig + v * vs, its sum table
+    // at S.sv + v * vs.
+    static constexpr bool PAIRED = true;
     template <int NV>
-    SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
-                                      float (&accB)[NV]) {
+    SLAI_HD static void compute_pairs(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t vs, float (&accA)[NV / 2], float (&accB)[NV / 2]) {
+        constexpr int NP = NV / 2;
         const uint32_t hA = blk + 20 * L.g, hB = hA + 160;
         const uint32_t ddA = prim::lds32(hA), ddB = prim::lds32(hB);
-        const uint32_t scA = prim::lds32(hA + 4 + 4 * (L.t >> 1)), scB = prim::lds32(hB + 4 + 4 * (L.t >> 1));
+        const uint32_t scA[2] = {prim::lds32(hA + 4), prim::lds32(hA + 8)}, scB[2] = {prim::lds32(hB + 4), prim::lds32(hB + 8)};
         const uint32_t mA = prim::lds32(hA + 12 + 4 * (L.t & 1)), mB = prim::lds32(hB + 12 + 4 * (L.t & 1));
-        uint4 hqA = make_uint4(0u, 0u, 0u, 0u), hqB = hqA;
+        uint2 hqA = make_uint2(0u, 0u), hqB = hqA;
         if (FIVE) {
-            hqA = prim::lds16(blk + 320 + 32 * L.g + 16 * (L.t & 1));
-            hqB = prim::lds16(blk + 320 + 32 * (L.g + 8) + 16 * (L.t & 1));
+            hqA = prim::lds8(blk + 320 + 32 * L.g + 8 * L.t);
+            hqB = prim::lds8(blk + 320 + 32 * (L.g + 8) + 8 * L.t);
         }
-        const uint32_t q0 = blk + QOFF + 16 * L.lane;
-        const uint32_t ba = L.bbase + (uint32_t)step * L.bmul;
-        int PA0[NV], PA1[NV], PB0[NV], PB1[NV];
+        // Rows are 64 bytes apart, so lanes of rows g and g + 2 would meet in the same banks: half of the rows read the
+        // chunk's second group first.
+        const uint32_t flip = 32u * ((L.g >> 1) & 1);
+        const uint32_t q0 = blk + QOFF + 64 * L.g + 8 * L.t;
+        const uint32_t vb = (uint32_t)(L.g >> 2) * vs;  // second vector of the pair in columns 4..7
+        const uint32_t ba = S.dig + (L.g & 3) * S.plane + vb + (uint32_t)step * STEP + 8 * L.t;
+        int PA0[NP], PA1[NP], PB0[NP], PB1[NP];
 #pragma unroll
-        for (int v = 0; v < NV; v++) PA0[v] = PA1[v] = PB0[v] = PB1[v] = 0;
+        for (int p = 0; p < NP; p++) PA0[p] = PA1[p] = PB0[p] = PB1[p] = 0;
 #pragma unroll
         for (int ci = 0; ci < 2; ci++) {
-            const uint4 qA = prim::lds16(q0 + (ci * 2) * 512), qB = prim::lds16(q0 + (ci * 2 + 1) * 512);
-            const int hsh = 2 * ((L.t >> 1) + 2 * ci);
-            const uint32_t hAx = hqA.x >> hsh, hAy = hqA.y >> hsh, hAz = hqA.z >> hsh, hAw = hqA.w >> hsh;
-            const uint32_t hBx = hqB.x >> hsh, hBy = hqB.y >> hsh, hBz = hqB.z >> hsh, hBw = hqB.w >> hsh;
+            const uint32_t qa = q0 + (ci * 2) * 512, qb = qa + 512;
+            const uint2 fA = prim::lds8(qa + flip), sA2 = prim::lds8(qa + (flip ^ 32u));
+            const uint2 fB = prim::lds8(qb + flip), sB2 = prim::lds8(qb + (flip ^ 32u));
 #pragma unroll
-            for (int nib = 0; nib < 2; nib++) {
-                uint32_t sA = byte_of(scA, 2 * ci + nib), sB = byte_of(scB, 2 * ci + nib);
-                uint32_t a[8];
-                if (FIVE) {
-                    a[0] = q5_nibs(qA.x, hAx, nib); a[1] = q5_nibs(qB.x, hBx, nib); a[2] = q5_nibs(qA.y, hAy, nib); a[3] = q5_nibs(qB.y, hBy, nib);
-                    a[4] = q5_nibs(qA.z, hAz, nib); a[5] = q5_nibs(qB.z, hBz, nib); a[6] = q5_nibs(qA.w, hAw, nib); a[7] = q5_nibs(qB.w, hBw, nib);
-                } else {
-                    const uint32_t mk = nib ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
-                    a[0] = qA.x & mk; a[1] = qB.x & mk; a[2] = qA.y & mk; a[3] = qB.y & mk;
-                    a[4] = qA.z & mk; a[5] = qB.z & mk; a[6] = qA.w & mk; a[7] = qB.w & mk;
-                    if (nib == 0) {
-                        sA <<= 4;
-                        sB <<= 4;
+            for (int h = 0; h < 2; h++) {
+                const int G = 2 * ci + h;  // 64-element group: sub-blocks 2G (low nibbles), 2G + 1 (high nibbles)
+                const bool first = (h == 0) == (flip == 0);
+                const uint32_t ax = first ? fA.x : sA2.x, ay = first ? fA.y : sA2.y, bx = first ? fB.x : sB2.x, by = first ? fB.y : sB2.y;
+#pragma unroll
+                for (int nib = 0; nib < 2; nib++) {
+                    uint32_t sA = byte_of(scA[h], 2 * ci + nib), sB = byte_of(scB[h], 2 * ci + nib);
+                    uint32_t a[4];
+                    if (FIVE) {
+                        a[0] = q5_nibs(ax, hqA.x >> (2 * G), nib); a[1] = q5_nibs(bx, hqB.x >> (2 * G), nib);
+                        a[2] = q5_nibs(ay, hqA.y >> (2 * G), nib); a[3] = q5_nibs(by, hqB.y >> (2 * G), nib);
+                    } else {
+                        const uint32_t mk = nib ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
+                        a[0] = ax & mk; a[1] = bx & mk; a[2] = ay & mk; a[3] = by & mk;
+                        if (nib == 0) {
+                            sA <<= 4;
+                            sB <<= 4;
+                        }
                     }
-                }
 #pragma unroll
-                for (int v = 0; v < NV; v++) {
-                    const uint4 bv = prim::lds16(ba + (uint32_t)v * bvs + 128 * ci + 32 * nib);
-                    int c[4];
-                    prim::mma_i8<true, true>(c, a[0], a[1], a[2], a[3], bv.x, bv.y);
-                    prim::mma_i8<true, false>(c, a[4], a[5], a[6], a[7], bv.z, bv.w);
-                    PA0[v] += (int)sA * c[0]; PA1[v] += (int)sA * c[1];
-                    PB0[v] += (int)sB * c[2]; PB1[v] += (int)sB * c[3];
+                    for (int p = 0; p < NP; p++) {
+                        const uint2 bv = prim::lds8(ba + (uint32_t)(2 * p) * vs + 64 * G + 32 * nib);
+                        int c[4];
+                        prim::mma_i8<true, true>(c, a[0], a[1], a[2], a[3], bv.x, bv.y);
+                        PA0[p] += (int)sA * c[0]; PA1[p] += (int)sA * c[1];
+                        PB0[p] += (int)sB * c[2]; PB1[p] += (int)sB * c[3];
+                    }
                 }
             }
         }
-        const float dA = prim::h2f(ddA & 0xFFFF), mnA = prim::h2f(ddA >> 16);
-        const float dB = prim::h2f(ddB & 0xFFFF), mnB = prim::h2f(ddB >> 16);
+        const float dA = prim::h2f(ddA & 0xFFFF), mnA = prim::h2f(ddA >> 16) * (1.0f / PRESCALE);  // (the digit weights carry PRESCALE)
+        const float dB = prim::h2f(ddB & 0xFFFF), mnB = prim::h2f(ddB >> 16) * (1.0f / PRESCALE);
+        const uint32_t sb = S.sv + vb + 128 * step + 32 * (L.g & 3) + 4 * L.t;
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-            const uint32_t bq = prim::lds32(S.sv + (uint32_t)v * svs + 128 * step + 16 * L.g + 4 * L.t);
-            int cq[4];
-            prim::mma_i8<true, true>(cq, mA, mB, 0u, 0u, bq, 0u);
-            accA[v] = prim::fma(dA, combine(PA0[v], PA1[v], L), accA[v]);
-            accA[v] = prim::fma(-mnA, (float)(cq[0] * 128 + cq[1]) * L.wq, accA[v]);
-            accB[v] = prim::fma(dB, combine(PB0[v], PB1[v], L), accB[v]);
-            accB[v] = prim::fma(-mnB, (float)(cq[2] * 128 + cq[3]) * L.wq, accB[v]);
+        for (int p = 0; p < NP; p++) {
+            const uint32_t bh = prim::lds32(sb + (uint32_t)(2 * p) * vs), bl = prim::lds32(sb + (uint32_t)(2 * p) * vs + 16);
+            int ch[4], cl[4];
+            prim::mma_i8<true, true>(ch, mA, mB, 0u, 0u, bh, 0u);
+            prim::mma_i8<true, true>(cl, mA, mB, 0u, 0u, bl, 0u);
+            accA[p] = prim::fma(dA, combine(PA0[p], PA1[p], L), accA[p]);
+            accA[p] = prim::fma(-mnA, combine(ch[0] * 128 + cl[0], ch[1] * 128 + cl[1], L), accA[p]);
+            accB[p] = prim::fma(dB, combine(PB0[p], PB1[p], L), accB[p]);
+            accB[p] = prim::fma(-mnB, combine(ch[2] * 128 + cl[2], ch[3] * 128 + cl[3], L), accB[p]);
         }
+    }
+    template <int NV>
+    SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
+                                      float (&accB)[NV]) {
+        (void)bvs;
+        batch_from_pairs<K45, NV>(blk, step, L, S, svs, accA, accB);
     }
 };
 using Q4K = K45<false>;
@@ -368,9 +403,11 @@ struct Q6K {
         accA = prim::fma(dA, combine(PA0, PA1, L), accA);
         accB = prim::fma(dB, combine(PB0, PB1, L), accB);
     }
+    static constexpr bool PAIRED = false;  // sub-blocks of 16 elements: one vector per MMA, columns = digits x two sub-blocks
     template <int NV>
     SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
                                       float (&accB)[NV]) {
+        (void)svs;
         int PA0[NV], PA1[NV], PB0[NV], PB1[NV];
 #pragma unroll
         for (int v = 0; v < NV; v++) PA0[v] = PA1[v] = PB0[v] = PB1[v] = 0;
@@ -387,9 +424,8 @@ struct Q6K {
                 for (int nib = 0; nib < 2; nib++) {
                     const int sh = 2 * pair + 4 * nib;
                     const int j8 = 4 * nib + 2 * pair + (L.t >> 1);
-                    const int j = 16 * step + 8 * h + j8;
-                    const uint32_t a0 = q6_nibs(qlA.x, qhA.x >> sh, nib), a1 = q6_nibs(qlB.x, qhB.x >> sh, nib);
-                    const uint32_t a2 = q6_nibs(qlA.y, qhA.y >> sh, nib), a3 = q6_nibs(qlB.y, qhB.y >> sh, nib);
+                    const uint32_t a0 = q6_signed(q6_nibs(qlA.x, qhA.x >> sh, nib)), a1 = q6_signed(q6_nibs(qlB.x, qhB.x >> sh, nib));
+                    const uint32_t a2 = q6_signed(q6_nibs(qlA.y, qhA.y >> sh, nib)), a3 = q6_signed(q6_nibs(qlB.y, qhB.y >> sh, nib));
                     const uint32_t wsA = j8 < 4 ? scwA.x : scwA.y, wsB = j8 < 4 ? scwB.x : scwB.y;
                     const int scA = (int)(signed char)((wsA >> (8 * (j8 & 3))) & 0xFF), scB = (int)(signed char)((wsB >> (8 * (j8 & 3))) & 0xFF);
 #pragma unroll
@@ -397,9 +433,8 @@ struct Q6K {
                         const uint2 bv = prim::lds8(ba + (uint32_t)v * bvs + 128 * h + 64 * nib + 32 * pair);
                         int c[4];
                         prim::mma_i8<false, true>(c, a0, a1, a2, a3, bv.x, bv.y);
-                        const uint2 sv = prim::lds8(S.sv + (uint32_t)v * svs + 16 * j + 8 * (L.t & 1));
-                        PA0[v] += scA * (c[0] - 32 * (int)sv.x); PA1[v] += scA * (c[1] - 32 * (int)sv.y);
-                        PB0[v] += scB * (c[2] - 32 * (int)sv.x); PB1[v] += scB * (c[3] - 32 * (int)sv.y);
+                        PA0[v] += scA * c[0]; PA1[v] += scA * c[1];
+                        PB0[v] += scB * c[2]; PB1[v] += scB * c[3];
                     }
                 }
             }
@@ -436,26 +471,40 @@ struct Q80 {
             accB = prim::fma(sB, combine(c[2], c[3], L), accB);
         }
     }
+    static constexpr bool PAIRED = true;  // two vectors to an MMA, as in K45::compute_pairs
+    template <int NV>
+    SLAI_HD static void compute_pairs(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t vs, float (&accA)[NV / 2], float (&accB)[NV / 2]) {
+        const uint32_t flip = 32u * ((L.g >> 1) & 1);
+        const uint32_t q0 = blk + 128 + 64 * L.g + 8 * L.t;
+        const uint32_t ba = S.dig + (L.g & 3) * S.plane + (uint32_t)(L.g >> 2) * vs + (uint32_t)step * STEP + 8 * L.t;
+        const uint2 sdA = prim::lds8(blk + 8 * L.g), sdB = prim::lds8(blk + 8 * (L.g + 8));
+#pragma unroll
+        for (int ci = 0; ci < 2; ci++) {
+            const uint32_t qa = q0 + (ci * 2) * 512, qb = qa + 512;
+            const uint2 fA = prim::lds8(qa + flip), sA2 = prim::lds8(qa + (flip ^ 32u));
+            const uint2 fB = prim::lds8(qb + flip), sB2 = prim::lds8(qb + (flip ^ 32u));
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int b = 2 * ci + h;  // GGUF block inside the step
+                const bool first = (h == 0) == (flip == 0);
+                const uint32_t ax = first ? fA.x : sA2.x, ay = first ? fA.y : sA2.y, bx = first ? fB.x : sB2.x, by = first ? fB.y : sB2.y;
+                const float sA = prim::h2f(((ci ? sdA.y : sdA.x) >> (16 * h)) & 0xFFFF), sB = prim::h2f(((ci ? sdB.y : sdB.x) >> (16 * h)) & 0xFFFF);
+#pragma unroll
+                for (int p = 0; p < NV / 2; p++) {
+                    const uint2 bv = prim::lds8(ba + (uint32_t)(2 * p) * vs + 32 * b);
+                    int c[4];
+                    prim::mma_i8<false, true>(c, ax, bx, ay, by, bv.x, bv.y);
+                    accA[p] = prim::fma(sA, combine(c[0], c[1], L), accA[p]);
+                    accB[p] = prim::fma(sB, combine(c[2], c[3], L), accB[p]);
+                }
+            }
+        }
+    }
     template <int NV>
     SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
                                       float (&accB)[NV]) {
-        (void)S; (void)svs;
-        const uint32_t ba = L.bbase + (uint32_t)step * L.bmul;
-#pragma unroll
-        for (int ci = 0; ci < 2; ci++) {
-            const int b = 2 * ci + (L.t >> 1);
-            const uint4 qA = prim::lds16(blk + 128 + (ci * 2) * 512 + 16 * L.lane), qB = prim::lds16(blk + 128 + (ci * 2 + 1) * 512 + 16 * L.lane);
-            const float sA = prim::h2f(prim::lds_u16(blk + 8 * L.g + 2 * b)), sB = prim::h2f(prim::lds_u16(blk + 8 * (L.g + 8) + 2 * b));
-#pragma unroll
-            for (int v = 0; v < NV; v++) {
-                const uint4 bv = prim::lds16(ba + (uint32_t)v * bvs + 64 * ci);
-                int c[4];
-                prim::mma_i8<false, true>(c, qA.x, qB.x, qA.y, qB.y, bv.x, bv.y);
-                prim::mma_i8<false, false>(c, qA.z, qB.z, qA.w, qB.w, bv.z, bv.w);
-                accA[v] = prim::fma(sA, combine(c[0], c[1], L), accA[v]);
-                accB[v] = prim::fma(sB, combine(c[2], c[3], L), accB[v]);
-            }
-        }
+        (void)bvs;
+        batch_from_pairs<Q80, NV>(blk, step, L, S, svs, accA, accB);
     }
 };
 

@@ -39,6 +39,9 @@ SLAI_HD uint32_t q6_nibs(uint32_t x, uint32_t hs, int nib) {
     return (nib ? ((x >> 4) & M4) : (x & M4)) | ((hs & 0x03030303u) << 4);
 }
 
+// q - 32 of four 6-bit quants as signed bytes (per byte: the top bit keeps the borrow inside the byte, then flips back).
+SLAI_HD uint32_t q6_signed(uint32_t q) { return ((q | 0x80808080u) - 0x20202020u) ^ 0x80808080u; }
+
 // ---- K-quant 6-bit scale / min of sub-block j from the 12 packed bytes (three words s0,s1,s2),
 // quantization.rs:381-389.
 SLAI_HD void scale_min_k4(int j, uint32_t s0, uint32_t s1, uint32_t s2, uint32_t& sc, uint32_t& m) {
