@@ -283,9 +283,9 @@ bool gemv_batch_supported(const slai_qmatrix* w);
 enum { BATCH_STORE = 0, BATCH_ADD = 1, BATCH_SILU = 2, BATCH_PAIR_SILU = 3 };
 // the same for the concatenation by rows of up to three matrices that share the input (see gemv_batch.cu)
 int gemv_batch_launch_multi(slai_ctx* ctx, float* d_out, const slai_qmatrix* const* ws, int nw, const float* d_v, int n_batch, long long ldo,
-                            int epi, const float* d_gate);
+                            int epi, const float* d_gate, const float* d_norm_w = nullptr, float eps = 0.f, bool pdl = false);
 int gemv_batch_launch(slai_ctx* ctx, float* d_out, const slai_qmatrix* w, const float* d_v, int n_batch, long long ldo = 0, int epi = BATCH_STORE,
-                      const float* d_gate = nullptr);
+                      const float* d_gate = nullptr, const float* d_norm_w = nullptr, float eps = 0.f, bool pdl = false);
 
 // attention.cu
 struct AttnLaunch {
@@ -366,6 +366,25 @@ __device__ __forceinline__ void slai_tl_append(unsigned long long* tl, unsigned 
 }
 #endif
 
+#ifdef __CUDACC__
+// Launch behind the predecessor's start (the kernels wait for its end themselves, before they touch anything it wrote).
+template <class... KArgs, class... Args>
+inline int launch_dependent(slai_ctx* ctx, void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, bool pdl, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, KArgs(args)...));
+    return SLAI_OK;
+}
+#endif
+
 // prefill.cu: prompt processing as GEMMs on the tcgen05 tensor cores
 struct PrefillGemm {
     const slai_qmatrix* w = nullptr;  // quantised matrix [rows_total x K]; the first `rows` rows are used
@@ -392,7 +411,7 @@ int prefill_embed_launch(slai_ctx* ctx, float* x, int dim, const int* d_tokens, 
 // q rotated into q_out ([B][q_dim]), k and v into the caches of sequence b, `seq_stride` bytes after those of sequence b - 1.
 int rope_kv_store_seqs_launch(slai_ctx* ctx, const float* qkv, int ld, int q_dim, int kv_dim, int head_size, const int* d_pos, int B,
                               const float* theta, int neox, float* q_out, void* kcache, void* vcache, int kv_f16, long long kv_head_stride,
-                              long long seq_stride);
+                              long long seq_stride, bool pdl);
 int rope_kv_store_launch(slai_ctx* ctx, float* q, const float* k, const float* v, int q_dim, int kv_dim, int head_size, const int* d_pos,
                          const float* theta, int neox, void* kcache, void* vcache, int kv_f16, long long kv_head_stride, bool pdl);
 bool prefill_attention_supported(int head_size, int kv_f16, const void* kc, const void* vc, long long head_stride);

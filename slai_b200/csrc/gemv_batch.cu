@@ -7,11 +7,15 @@
 // gemv_formats.cuh; Q6_K, whose sub-blocks of 16 fill half an MMA's depth, one vector at a time): the same integer sums as
 // the single-vector code.
 //
-// Shape.  The digit planes of 8 vectors over the whole of K do not fit in shared memory, so K is cut into chunks of
-// `ch` tile-steps (<= 8) and a unit of work is (chunk, group of 16 row tiles): the 16 warps of a block stage the chunk's
-// slice of all vectors once (each vector with its own power-of-two scale for the chunk), then every warp walks its own
-// tile's `ch` blocks, double-buffered with cp.async.  Partial sums per chunk go to a scratch array and a second small
-// kernel adds them in chunk order (deterministic; no atomics).
+// Shape, three launches (dependent launches: each one's start overlaps its predecessor's end):
+//   digits   every vector's 256-element (Q8_0: 128) steps are turned once into digit planes, digit sums and a power-of-two
+//            scale of their own, records of `BatchGeom::REC` bytes per (step, vector); with an RmsNorm in front when asked.
+//            (Staged by every block of the product instead, this was half of its time: 16 row groups redid the same chunk.)
+//   product  the digit planes of 8 vectors over the whole of K do not fit in shared memory, so K is cut into chunks of `ch`
+//            steps and a unit of work is (chunk, group of 16 row tiles).  A block keeps the records of its current and its next
+//            unit (one bulk copy each); each of its 16 warps walks its own tile's blocks through a ring of three stages
+//            that runs on across units and starts before the predecessor has finished (weights do not depend on it).
+//   reduce   adds the chunks' partial sums in order (deterministic; no atomics) and stores.
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -26,7 +30,8 @@ using namespace frag;
 constexpr int BWARPS = 16;
 constexpr int BTHREADS = 32 * BWARPS;
 constexpr int MAX_CH = 8;
-constexpr int BSMEM_LIMIT = 227 * 1024;
+constexpr int BSTAGES = 3;  // weight blocks a warp has in flight
+constexpr int BSMEM_LIMIT = 227 * 1024 - 256;  // the barriers are static
 
 struct BatchParams {
     const uint8_t* w[3];   // up to three matrices of the same format and K that share the input (q / k / v, gate / up): their
@@ -37,152 +42,241 @@ struct BatchParams {
     int ch, nch, ngroups;  // steps per chunk, chunks, groups of 16 tiles
     int n_batch;           // vectors that exist (the others of the instantiation's NV are zero)
     const float* v;        // [n_batch][K]
+    const float* norm_w;   // optional RmsNorm of the vectors
+    float eps;
+    unsigned char* rec;    // [nsteps][NV][REC] digit records
     float* part;           // [nch][NV][mp] partial sums
     int mp;                // ntiles * 16
-    uint32_t plane;        // bytes between the digit planes of a staged vector (chunk elements + 32)
-    uint32_t vstride;      // bytes between the staged vectors (digit planes, then the digit sums)
+    unsigned int* err_flag;
+    unsigned int wait_limit;
 };
 
 template <class F>
 struct BatchGeom {
     static constexpr uint32_t STEP = F::STEP_BYTES;
     static constexpr uint32_t STRIDE = (STEP + 127) & ~127u;
+    static constexpr uint32_t PLANE = F::STEP + 32;  // planes 32 bytes apart modulo 128: the four digit columns hit different banks
+    static constexpr uint32_t SUMS = 4 * PLANE;      // byte table of the digit sums (Q4_K / Q5_K)
+    static constexpr uint32_t REC = SUMS + (F::PAIRED && F::SV_GRAN == 32 ? 128 : 0);
+    static constexpr uint32_t INV = F::STEP;         // 1 / scale, in the gap after the first plane
 };
 
 __device__ __forceinline__ float bmax4(const float4& x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); }
+
+// One warp per (vector, step); block (x, y): vector y, steps x * 16 + warp, onwards by the grid's width.  With a norm one
+// block serves the whole vector.
+template <class F>
+__global__ void __launch_bounds__(BTHREADS) batch_digits_kernel(const __grid_constant__ BatchParams P, int nv) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    using G = BatchGeom<F>;
+    constexpr int PER = F::STEP / 128;  // float4 per lane
+    const int v = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool have = v < P.n_batch;
+    const float* x = P.v + (size_t)(have ? v : 0) * P.K;
+    float mul = 1.f;
+    if (P.norm_w && have) {  // ops/rms_norm.rs:68-77
+        __shared__ float sh[BWARPS];
+        float s = 0.f;
+        for (int i = threadIdx.x; i < P.K / 4; i += BTHREADS) {
+            const float4 q = __ldcg(reinterpret_cast<const float4*>(x) + i);
+            s += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sh[warp] = s;
+        __syncthreads();
+        s = 0.f;
+        for (int w = 0; w < BWARPS; w++) s += sh[w];
+        mul = 1.0f / sqrtf(s / (float)P.K + P.eps);
+    }
+    for (int step = blockIdx.x * BWARPS + warp; step < P.nsteps; step += gridDim.x * BWARPS) {
+        float4 q[PER];
+        float mx = 0.f;
+#pragma unroll
+        for (int e = 0; e < PER; e++) {
+            const int k = step * F::STEP + (PER * lane + e) * 4;
+            q[e] = have && k < P.K ? __ldcg(reinterpret_cast<const float4*>(x + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (P.norm_w && have && k < P.K) {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(P.norm_w + k));
+                q[e].x = (q[e].x * mul) * w.x; q[e].y = (q[e].y * mul) * w.y; q[e].z = (q[e].z * mul) * w.z; q[e].w = (q[e].w * mul) * w.w;
+            }
+            mx = fmaxf(mx, bmax4(q[e]));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float scale = 1.f;
+        if (mx > 0.f && mx < 3.0e38f) {
+            int e = (int)((__float_as_uint(mx) >> 23) & 0xffu) - 126;  // mx = f * 2^e with f in [0.5, 1) (normal numbers)
+            if ((__float_as_uint(mx) >> 23) == 0u) e = -126;
+            e = e < -90 ? -90 : e;
+            scale = __uint_as_float((uint32_t)(127 + 26 - e) << 23);  // 2^(26 - e), exact
+        }
+        unsigned char* rec = P.rec + ((size_t)step * nv + v) * G::REC;
+        uint32_t pw[PER][4];
+#pragma unroll
+        for (int e = 0; e < PER; e++)
+            digit_planes(digits_word(__float2int_rn(q[e].x * scale)), digits_word(__float2int_rn(q[e].y * scale)), digits_word(__float2int_rn(q[e].z * scale)),
+                         digits_word(__float2int_rn(q[e].w * scale)), pw[e]);
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+#pragma unroll
+            for (int e = 0; e < PER; e++) *reinterpret_cast<uint32_t*>(rec + p * G::PLANE + (PER * lane + e) * 4) = pw[e][p];
+        if (lane == 0) *reinterpret_cast<float*>(rec + G::INV) = 1.0f / scale;
+        if (F::PAIRED && F::SV_GRAN == 32) {
+            // Q4_K / Q5_K: sum of a sub-block's digits (four lanes of eight elements) per plane, as two base-128 digits in the byte
+            // table of the step: row 2p the high, row 2p + 1 the low digit of plane p, byte j of a row = sub-block j, bytes 8..15 zero
+            const int j = lane >> 2;
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                int sd = 0;
+#pragma unroll
+                for (int e = 0; e < PER; e++) sd = __dp4a((int)pw[e][p], 0x01010101, sd);
+                sd += __shfl_xor_sync(0xffffffffu, sd, 1);
+                sd += __shfl_xor_sync(0xffffffffu, sd, 2);
+                const int hi = (sd + 64) >> 7, lo = sd - (hi << 7);
+                if ((lane & 3) == 0) {
+                    rec[G::SUMS + (2 * p) * 16 + j] = (unsigned char)hi;
+                    rec[G::SUMS + (2 * p + 1) * 16 + j] = (unsigned char)lo;
+                }
+            }
+            if (lane < 8) *reinterpret_cast<uint2*>(rec + G::SUMS + lane * 16 + 8) = make_uint2(0u, 0u);
+        }
+    }
+}
 
 // One tile-step block, global -> this warp's stage: 16 bytes per lane and round.
 template <class F>
 __device__ __forceinline__ void stage_request(const uint8_t* src, uint32_t dst, int lane) {
     const size_t gsrc = __cvta_generic_to_global(src);
-#pragma unroll 1
-    for (uint32_t off = 16u * lane; off < BatchGeom<F>::STEP; off += 512u)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + off), "l"(gsrc + off) : "memory");
+#pragma unroll
+    for (uint32_t r = 0; r < BatchGeom<F>::STEP; r += 512u) {
+        const uint32_t off = r + 16u * lane;
+        if (off < BatchGeom<F>::STEP) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + off), "l"(gsrc + off) : "memory");
+    }
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// A warp's walk over its blocks: unit by unit, `nst` steps of one tile each.
+struct BatchWalk {
+    int unit, step, nst;
+    const uint8_t* src;  // the unit's first block of this warp's tile (null: the group has no tile for this warp)
+};
+template <class F>
+__device__ __forceinline__ void walk_open(BatchWalk& W, const BatchParams& P, int warp) {
+    W.step = 0;
+    W.nst = 0;
+    if (W.unit >= P.ngroups * P.nch) return;
+    const int c = W.unit / P.ngroups, tile = (W.unit - c * P.ngroups) * BWARPS + warp;
+    W.nst = min(P.ch, P.nsteps - c * P.ch);
+    const uint8_t* base = P.w[0];
+    int t0 = 0;
+    if (P.nw > 1 && tile >= P.t0[1]) { base = P.w[1]; t0 = P.t0[1]; }
+    if (P.nw > 2 && tile >= P.t0[2]) { base = P.w[2]; t0 = P.t0[2]; }
+    W.src = tile < P.ntiles ? base + (size_t)(tile - t0) * P.tile_bytes + (size_t)c * P.ch * BatchGeom<F>::STEP : nullptr;
+}
 
 template <class F, int NV>
 __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long bars[2];
+    using G = BatchGeom<F>;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem), bar = (uint32_t)__cvta_generic_to_shared(bars);
+    const uint32_t slot_bytes = (uint32_t)P.ch * NV * G::REC;
+    const uint32_t wb = sbase + ZERO_BYTES + 2 * slot_bytes + (uint32_t)warp * BSTAGES * G::STRIDE;
+    const int units = P.ngroups * P.nch, stride = (int)gridDim.x;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid < ZERO_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    BatchWalk W;  // the request cursor, BSTAGES - 1 blocks ahead
+    W.unit = (int)blockIdx.x;
+    walk_open<F>(W, P, warp);
+    auto request = [&](int stage) {
+        if (W.nst > 0) {
+            if (W.src) stage_request<F>(W.src + (size_t)W.step * G::STEP, wb + (uint32_t)stage * G::STRIDE, lane);
+            if (++W.step == W.nst) {
+                W.unit += stride;
+                walk_open<F>(W, P, warp);
+            }
+        }
+        stage_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < BSTAGES - 1; s++) request(s);
+
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __syncthreads();
+    auto fetch_records = [&](int unit, int slot) {  // one thread; the slot has been read by everyone
+        const int c = unit / P.ngroups;
+        const uint32_t bytes = (uint32_t)min(P.ch, P.nsteps - c * P.ch) * NV * G::REC, b = bar + 8 * slot;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sbase + ZERO_BYTES + slot * slot_bytes),
+                     "l"(__cvta_generic_to_global(P.rec + (size_t)c * P.ch * NV * G::REC)), "r"(bytes), "r"(b)
+                     : "memory");
+    };
+    if (tid == 0) {
+        fetch_records((int)blockIdx.x, 0);
+        if ((int)blockIdx.x + stride < units) fetch_records((int)blockIdx.x + stride, 1);
+    }
+
     Smem S;
     S.zero = sbase;
-    S.dig = sbase + ZERO_BYTES;
-    S.plane = P.plane;
-    S.sv = S.dig + 4 * P.plane;
-    const uint32_t misc_off = ZERO_BYTES + NV * P.vstride;
-    float* sinv = reinterpret_cast<float*>(smem + misc_off);                 // 1 / scale of every staged vector
-    unsigned int* smax = reinterpret_cast<unsigned int*>(smem + misc_off + 32);  // max |x| of the chunk per vector, as float bits
-    const uint32_t ring_off = (misc_off + 64 + 127) & ~127u;
-    const uint32_t wb = sbase + ring_off + (uint32_t)warp * 2u * BatchGeom<F>::STRIDE;
-
+    S.plane = G::PLANE;
     LaneCtx L;
-    lane_init<F>(L, lane, S);
-    const uint32_t bvs = L.bmul ? P.vstride : 0u;  // lanes that read the zero page read it for every vector
-
-    if (tid < ZERO_BYTES / 4) reinterpret_cast<uint32_t*>(smem)[tid] = 0u;
-    if (tid < NV) smax[tid] = 0u;
-
-    const int ce = P.ch * F::STEP;  // elements of K per chunk
-    const int per = ce >> 5;        // sub-blocks of 32 elements per vector and chunk (<= 64)
-    const int sv_v = tid / per, sv_j = tid - sv_v * per;  // the (vector, sub-block) this thread stages
-    const bool stager = sv_v < NV;
-
-    const int units = P.ngroups * P.nch;
-    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
-        const int c = unit / P.ngroups, grp = unit - c * P.ngroups;
-        const int s0 = c * P.ch;
-        const int nst = min(P.ch, P.nsteps - s0);
-        const int tile = grp * BWARPS + warp;
-        const bool active = tile < P.ntiles;
-        const uint8_t* wbase = P.w[0];
-        int wt0 = 0;
-        if (P.nw > 1 && tile >= P.t0[1]) { wbase = P.w[1]; wt0 = P.t0[1]; }
-        if (P.nw > 2 && tile >= P.t0[2]) { wbase = P.w[2]; wt0 = P.t0[2]; }
-        const uint8_t* src = wbase + (size_t)(active ? tile - wt0 : 0) * P.tile_bytes + (size_t)s0 * BatchGeom<F>::STEP;
-        // the first two blocks of this warp's tile are on their way while the vectors are staged
-        if (active) stage_request<F>(src, wb, lane);
-        stage_commit();
-        if (active && nst > 1) stage_request<F>(src + BatchGeom<F>::STEP, wb + BatchGeom<F>::STRIDE, lane);
-        stage_commit();
-
-        // ---- stage the chunk's slice of every vector: thread (vector, sub-block of 32 elements) ----
-        float4 x[8];
-        {
-            const int k0 = s0 * F::STEP + 32 * sv_j;
-            const bool have = stager && sv_v < P.n_batch && k0 < P.K;
-            const float4* p = reinterpret_cast<const float4*>(P.v + (size_t)(have ? sv_v : 0) * P.K + (have ? k0 : 0));
-            float mx = 0.f;
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                x[e] = have ? __ldcg(p + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-                mx = fmaxf(mx, bmax4(x[e]));
-            }
-            __syncthreads();  // every warp has finished the previous unit (digits, sums and `smax` are free)
-            if (stager && mx > 0.f) atomicMax(&smax[sv_v], __float_as_uint(mx));
-        }
-        __syncthreads();
-        if (stager) {
-            const float mx = __uint_as_float(smax[sv_v]);
-            float scale = 1.f;
-            if (mx > 0.f && mx < 3.0e38f) {
-                int e = (int)((__float_as_uint(mx) >> 23) & 0xffu) - 126;  // mx = f * 2^e with f in [0.5, 1) (normal numbers)
-                if ((__float_as_uint(mx) >> 23) == 0u) e = -126;
-                e = e < -90 ? -90 : e;
-                scale = __uint_as_float((uint32_t)(127 + 26 - e) << 23);  // 2^(26 - e), exact
-            }
-            if (sv_j == 0) sinv[sv_v] = 1.0f / scale;
-            unsigned char* dig = smem + ZERO_BYTES + (size_t)sv_v * P.vstride;
-            unsigned char* svb = dig + 4 * (size_t)P.plane;
-            uint32_t pw[8][4];
-#pragma unroll
-            for (int e = 0; e < 8; e++)
-                digit_planes(digits_word(__float2int_rn(x[e].x * scale)), digits_word(__float2int_rn(x[e].y * scale)),
-                             digits_word(__float2int_rn(x[e].z * scale)), digits_word(__float2int_rn(x[e].w * scale)), pw[e]);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                uint4* d = reinterpret_cast<uint4*>(dig + (size_t)q * P.plane + 32 * sv_j);
-                d[0] = make_uint4(pw[0][q], pw[1][q], pw[2][q], pw[3][q]);
-                d[1] = make_uint4(pw[4][q], pw[5][q], pw[6][q], pw[7][q]);
-            }
-            if (F::SV_GRAN == 32) {
-                // Q4_K / Q5_K: sum of the sub-block's digits per plane as two base-128 digits in the byte table of its step
-                unsigned char* tab = svb + (sv_j >> 3) * 128;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    int sd = 0;
-#pragma unroll
-                    for (int e = 0; e < 8; e++) sd = __dp4a((int)pw[e][q], 0x01010101, sd);
-                    const int hi = (sd + 64) >> 7, lo = sd - (hi << 7);
-                    tab[(2 * q) * 16 + (sv_j & 7)] = (unsigned char)hi;
-                    tab[(2 * q + 1) * 16 + (sv_j & 7)] = (unsigned char)lo;
-                }
-                *reinterpret_cast<uint2*>(tab + (sv_j & 7) * 16 + 8) = make_uint2(0u, 0u);
+    unsigned int limit = P.wait_limit;
+    int stage = 0, it = 0;
+    for (int unit = (int)blockIdx.x; unit < units; unit += stride, it++) {
+        const int c = unit / P.ngroups, grp = unit - c * P.ngroups, slot = it & 1;
+        const int nst = min(P.ch, P.nsteps - c * P.ch), tile = grp * BWARPS + warp;
+        {   // bounded wait for the unit's records; on expiry the error flag is raised and later waits give up at once
+            uint32_t ok = 0;
+            for (unsigned int i = 0; i < limit && !ok; i++)
+                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(ok)
+                             : "r"(bar + 8 * slot), "r"((uint32_t)(it >> 1) & 1u)
+                             : "memory");
+            if (!ok) {
+                atomicExch(P.err_flag, 6u);
+                limit = 1;
             }
         }
-        __syncthreads();
-        if (tid < NV) smax[tid] = 0u;  // read by everyone before the barrier above; next written after the next unit's first barrier
-
+        S.dig = sbase + ZERO_BYTES + slot * slot_bytes;
         // ---- this warp's tile: `nst` blocks against all vectors ----
         constexpr int NA = F::PAIRED ? NV / 2 : NV;
         float accA[NA], accB[NA];
 #pragma unroll
         for (int v = 0; v < NA; v++) accA[v] = accB[v] = 0.f;
-        if (active) {
 #pragma unroll 1
-            for (int s = 0; s < nst; s++) {
-                asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest request have landed: block s is here
-                __syncwarp();
-                const uint32_t blk = wb + (uint32_t)(s & 1) * BatchGeom<F>::STRIDE;
-                if constexpr (F::PAIRED) F::template compute_pairs<NV>(blk, s, L, S, P.vstride, accA, accB);
-                else F::template compute_batch<NV>(blk, s, L, S, bvs, P.vstride, accA, accB);
-                __syncwarp();
-                if (s + 2 < nst) stage_request<F>(src + (size_t)(s + 2) * BatchGeom<F>::STEP, blk, lane);
-                stage_commit();
+        for (int s = 0; s < nst; s++) {
+            request(stage == 0 ? BSTAGES - 1 : stage - 1);  // into the stage consumed one block ago
+            asm volatile("cp.async.wait_group %0;" ::"n"(BSTAGES - 1) : "memory");  // all but the newest requests have landed: this block is here
+            __syncwarp();
+            S.sv = S.dig + G::SUMS;
+            lane_init<F>(L, lane, S);
+            const uint32_t blk = wb + (uint32_t)stage * G::STRIDE;
+            float a[NA], b[NA];
+#pragma unroll
+            for (int v = 0; v < NA; v++) a[v] = b[v] = 0.f;
+            if constexpr (F::PAIRED) F::template compute_pairs<NV>(blk, 0, L, S, G::REC, a, b);
+            else F::template compute_batch<NV>(blk, 0, L, S, L.bmul ? G::REC : 0u, G::REC, a, b);
+#pragma unroll
+            for (int v = 0; v < NA; v++) {  // every step has its own scale
+                const float inv = __uint_as_float(prim::lds32(S.dig + (F::PAIRED ? 2 * v + (L.t >> 1) : v) * G::REC + G::INV));
+                accA[v] = fmaf(inv, a[v], accA[v]);
+                accB[v] = fmaf(inv, b[v], accB[v]);
             }
+            S.dig += NV * G::REC;
+            __syncwarp();
+            if (++stage == BSTAGES) stage = 0;
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
         for (int v = 0; v < NA; v++) {
             accA[v] += __shfl_xor_sync(0xffffffffu, accA[v], 1);
@@ -192,20 +286,35 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
                 accB[v] += __shfl_xor_sync(0xffffffffu, accB[v], 2);
             }
         }
-        if (active) {
+        if (tile < P.ntiles) {
             float* dst = P.part + (size_t)c * NV * P.mp + (size_t)tile * 16;
 #pragma unroll
             for (int v = 0; v < NA; v++) {
                 if (F::PAIRED) {  // lanes t and t ^ 1 hold vector 2v + (t >> 1): the even one stores row g, the odd one row g + 8
-                    const int vec = 2 * v + (L.t >> 1);
-                    dst[(size_t)vec * P.mp + L.g + 8 * (L.t & 1)] = ((L.t & 1) ? accB[v] : accA[v]) * sinv[vec];
+                    dst[(size_t)(2 * v + (L.t >> 1)) * P.mp + L.g + 8 * (L.t & 1)] = (L.t & 1) ? accB[v] : accA[v];
                 } else if ((v & 3) == L.t) {  // the four lanes of a row hold the same sums: lane t stores vectors t and t + 4
-                    dst[(size_t)v * P.mp + L.g] = accA[v] * sinv[v];
-                    dst[(size_t)v * P.mp + L.g + 8] = accB[v] * sinv[v];
+                    dst[(size_t)v * P.mp + L.g] = accA[v];
+                    dst[(size_t)v * P.mp + L.g + 8] = accB[v];
                 }
             }
         }
+        __syncthreads();  // the unit's records have been read
+        if (tid == 0 && unit + 2 * stride < units) fetch_records(unit + 2 * stride, slot);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Sum of n values `stride` apart, in order; eight loads in flight.
+__device__ __forceinline__ float batch_sum(const float* p, int n, size_t stride) {
+    float s = 0.f;
+    for (int c0 = 0; c0 < n; c0 += 8) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = c0 + i < n ? __ldcg(p + (size_t)(c0 + i) * stride) : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) s += x[i];
+    }
+    return s;
 }
 
 // out[v][m] = sum over the chunks, in order, of the partial sums.
@@ -214,11 +323,12 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
 // launch, gate then up: out = up sum * silu(gate sum)).
 __global__ void gemv_batch_reduce_kernel(float* out, long long ldo, const float* part, int nch, int nv, int mp, int M, int n_batch, int epi,
                                          const float* gate) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)n_batch * M) return;
     const int v = (int)(idx / M), m = (int)(idx - (long long)v * M);
-    float s = 0.f;
-    for (int c = 0; c < nch; c++) s += part[((size_t)c * nv + v) * mp + m];
+    float s = batch_sum(part + (size_t)v * mp + m, nch, (size_t)nv * mp);
     const long long o = (long long)v * ldo + m;
     if (epi == BATCH_ADD) {
         s = out[o] + s;
@@ -226,35 +336,27 @@ __global__ void gemv_batch_reduce_kernel(float* out, long long ldo, const float*
         const float g = gate[o];
         s = s * (g / (1.0f + expf(-g)));
     } else if (epi == BATCH_PAIR_SILU) {
-        float u = 0.f;
-        for (int c = 0; c < nch; c++) u += part[((size_t)c * nv + v) * mp + M + m];
+        const float u = batch_sum(part + (size_t)v * mp + M + m, nch, (size_t)nv * mp);
         s = u * (s / (1.0f + expf(-s)));
     }
     out[o] = s;
 }
 
 template <class F>
-size_t batch_smem(int nv, int ch, uint32_t* plane_out, uint32_t* vstride_out) {
-    const uint32_t ce = (uint32_t)ch * F::STEP;
-    const uint32_t plane = ce + 32;
-    const uint32_t svbytes = F::SV_GRAN == 32 ? 128u * ch : 0u;  // (the batched Q6_K code has no digit sums)
-    const uint32_t vstride = (4 * plane + svbytes + 15) & ~15u;
-    *plane_out = plane;
-    *vstride_out = vstride;
-    const uint32_t ring_off = (ZERO_BYTES + nv * vstride + 64 + 127) & ~127u;
-    return (size_t)ring_off + (size_t)BWARPS * 2 * BatchGeom<F>::STRIDE;
+size_t batch_smem(int nv, int ch) {
+    return ZERO_BYTES + 2 * (size_t)ch * nv * BatchGeom<F>::REC + (size_t)BWARPS * BSTAGES * BatchGeom<F>::STRIDE;
 }
 
 template <class F, int NV>
-int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate) {
-    // Steps per chunk: the fewest rounds of (staging + ch steps) over the SMs; staging a chunk costs about three steps.
+int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate, bool pdl) {
+    // Steps per chunk: the fewest rounds of (start of a unit + ch steps) over the SMs; a unit's start costs about one step.
     const int G = ctx->sm_count > 0 ? ctx->sm_count : 148;
     int best_ch = 1;
     long long best_cost = -1;
-    for (int ch = 1; ch <= MAX_CH; ch++) {
+    for (int ch = 1; ch <= MAX_CH && batch_smem<F>(NV, ch) <= (size_t)BSMEM_LIMIT; ch++) {
         const long long nch = (P.nsteps + ch - 1) / ch;
         const long long rounds = (nch * P.ngroups + G - 1) / G;
-        const long long cost = rounds * (3 + ch);
+        const long long cost = rounds * (1 + ch);
         if (best_cost < 0 || cost <= best_cost) {
             best_cost = cost;
             best_ch = ch;
@@ -262,34 +364,34 @@ int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo
     }
     P.ch = best_ch;
     P.nch = (P.nsteps + P.ch - 1) / P.ch;
-    const size_t smem = batch_smem<F>(NV, P.ch, &P.plane, &P.vstride);
+    const size_t smem = batch_smem<F>(NV, P.ch);
     SLAI_REQUIRE(ctx, smem <= (size_t)BSMEM_LIMIT, SLAI_ERR_SHAPE, "gemv: the batched kernel needs %zu bytes of shared memory", smem);
-    const size_t part_bytes = (size_t)P.nch * NV * P.mp * sizeof(float);
-    int rc = ensure_scratch(ctx, part_bytes);
+    const size_t rec_bytes = ((size_t)P.nsteps * NV * BatchGeom<F>::REC + 255) & ~(size_t)255;
+    int rc = ensure_scratch(ctx, rec_bytes + (size_t)P.nch * NV * P.mp * sizeof(float));
     if (rc) return rc;
-    P.part = reinterpret_cast<float*>(ctx->d_scratch);
+    P.rec = reinterpret_cast<unsigned char*>(ctx->d_scratch);
+    P.part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(ctx->d_scratch) + rec_bytes);
     auto kern = gemv_batch_kernel<F, NV>;
     static PerDeviceOnce attr;  // per instantiation
     if (attr.need(ctx->device)) {
         SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BSMEM_LIMIT));
         attr.set(ctx->device);
     }
+    const int dblocks = P.norm_w ? 1 : (P.nsteps + BWARPS - 1) / BWARPS;
+    if ((rc = launch_dependent(ctx, batch_digits_kernel<F>, dim3((unsigned)dblocks, NV), BTHREADS, 0, pdl, P, NV))) return rc;
     const long long units = (long long)P.ngroups * P.nch;
-    const int grid = (int)(units < G ? units : G);
-    kern<<<grid, BTHREADS, smem, ctx->stream>>>(P);
-    SLAI_CHECK_CUDA(ctx, cudaGetLastError());
+    if ((rc = launch_dependent(ctx, kern, dim3((unsigned)(units < G ? units : G)), BTHREADS, smem, true, P))) return rc;
     const long long total = (long long)P.n_batch * M;
-    gemv_batch_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(d_out, ldo, P.part, P.nch, NV, P.mp, M, P.n_batch, epi, gate);
-    SLAI_CHECK_CUDA(ctx, cudaGetLastError());
-    return SLAI_OK;
+    return launch_dependent(ctx, gemv_batch_reduce_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, true, d_out, ldo, P.part, P.nch, NV, P.mp, M,
+                            P.n_batch, epi, gate);
 }
 
 template <class F>
-int launch_batch_fmt(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate) {
-    if (P.n_batch <= 2) return launch_batch_inst<F, 2>(ctx, P, d_out, ldo, M, epi, gate);
-    if (P.n_batch <= 4) return launch_batch_inst<F, 4>(ctx, P, d_out, ldo, M, epi, gate);
-    if (P.n_batch <= 6) return launch_batch_inst<F, 6>(ctx, P, d_out, ldo, M, epi, gate);
-    return launch_batch_inst<F, 8>(ctx, P, d_out, ldo, M, epi, gate);
+int launch_batch_fmt(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo, int M, int epi, const float* gate, bool pdl) {
+    if (P.n_batch <= 2) return launch_batch_inst<F, 2>(ctx, P, d_out, ldo, M, epi, gate, pdl);
+    if (P.n_batch <= 4) return launch_batch_inst<F, 4>(ctx, P, d_out, ldo, M, epi, gate, pdl);
+    if (P.n_batch <= 6) return launch_batch_inst<F, 6>(ctx, P, d_out, ldo, M, epi, gate, pdl);
+    return launch_batch_inst<F, 8>(ctx, P, d_out, ldo, M, epi, gate, pdl);
 }
 
 }  // namespace
@@ -299,11 +401,12 @@ bool gemv_batch_supported(const slai_qmatrix* w) {
 }
 
 // out[b * ldo + m] = sum_k W[m][k] v[b][k] for b < n_batch (2..8), one pass over W (ldo 0: the rows of `out` are M apart);
-// `epi` folds a residual add or the SiLU gate into the store.  W is the concatenation by rows of `nw` (1..3) matrices of the
+// `d_norm_w` puts an RmsNorm of the vectors in front; `pdl`: the first launch may begin before its predecessor in the stream has
+// ended (it waits for it itself); `epi` folds a residual add or the SiLU gate into the store.  W is the concatenation by rows of `nw` (1..3) matrices of the
 // same format and width (all but the last with a multiple of 16 rows); with BATCH_PAIR_SILU the two matrices are gate and up
 // of equal height M and out[b * ldo + m], m < M, receives up * silu(gate).
 int gemv_batch_launch_multi(slai_ctx* ctx, float* d_out, const slai_qmatrix* const* ws, int nw, const float* d_v, int n_batch, long long ldo,
-                            int epi, const float* d_gate) {
+                            int epi, const float* d_gate, const float* d_norm_w, float eps, bool pdl) {
     SLAI_REQUIRE(ctx, nw >= 1 && nw <= 3 && ws && ws[0], SLAI_ERR_INVALID_ARG, "gemv: %d matrices in one batched launch", nw);
     const slai_qmatrix* w = ws[0];
     SLAI_REQUIRE(ctx, gemv_batch_supported(w), SLAI_ERR_UNSUPPORTED_FORMAT, "gemv: format %d has no batched kernel", w->fmt);
@@ -331,6 +434,10 @@ int gemv_batch_launch_multi(slai_ctx* ctx, float* d_out, const slai_qmatrix* con
     P.ngroups = (P.ntiles + BWARPS - 1) / BWARPS;
     P.n_batch = n_batch;
     P.v = d_v;
+    P.norm_w = d_norm_w;
+    P.eps = eps;
+    P.err_flag = ctx->d_counters + CNT_ERR_FLAG;
+    P.wait_limit = ctx->wait_limit;
     P.mp = P.ntiles * 16;
     int M = rows_total;
     if (epi == BATCH_PAIR_SILU) {
@@ -342,15 +449,15 @@ int gemv_batch_launch_multi(slai_ctx* ctx, float* d_out, const slai_qmatrix* con
     SLAI_REQUIRE(ctx, epi == BATCH_STORE || epi == BATCH_ADD || epi == BATCH_PAIR_SILU || (epi == BATCH_SILU && d_gate), SLAI_ERR_INVALID_ARG,
                  "gemv: batch epilogue %d", epi);
     switch (w->fmt) {
-        case SLAI_FMT_Q8_0: return launch_batch_fmt<Q80>(ctx, P, d_out, ldo, M, epi, d_gate);
-        case SLAI_FMT_Q4_K: return launch_batch_fmt<Q4K>(ctx, P, d_out, ldo, M, epi, d_gate);
-        case SLAI_FMT_Q5_K: return launch_batch_fmt<Q5K>(ctx, P, d_out, ldo, M, epi, d_gate);
-        case SLAI_FMT_Q6_K: return launch_batch_fmt<Q6K>(ctx, P, d_out, ldo, M, epi, d_gate);
+        case SLAI_FMT_Q8_0: return launch_batch_fmt<Q80>(ctx, P, d_out, ldo, M, epi, d_gate, pdl);
+        case SLAI_FMT_Q4_K: return launch_batch_fmt<Q4K>(ctx, P, d_out, ldo, M, epi, d_gate, pdl);
+        case SLAI_FMT_Q5_K: return launch_batch_fmt<Q5K>(ctx, P, d_out, ldo, M, epi, d_gate, pdl);
+        case SLAI_FMT_Q6_K: return launch_batch_fmt<Q6K>(ctx, P, d_out, ldo, M, epi, d_gate, pdl);
     }
     return SLAI_ERR_UNSUPPORTED_FORMAT;
 }
 
 int gemv_batch_launch(slai_ctx* ctx, float* d_out, const slai_qmatrix* w, const float* d_v, int n_batch, long long ldo, int epi,
-                      const float* d_gate) {
-    return gemv_batch_launch_multi(ctx, d_out, &w, 1, d_v, n_batch, ldo, epi, d_gate);
+                      const float* d_gate, const float* d_norm_w, float eps, bool pdl) {
+    return gemv_batch_launch_multi(ctx, d_out, &w, 1, d_v, n_batch, ldo, epi, d_gate, d_norm_w, eps, pdl);
 }

@@ -607,10 +607,17 @@ static int llama_batch_record(slai_llama* m, int B, int cap_pos) {
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     const long long kv_head_stride = (long long)c.seq_len * m->head_size;
     const int qkv_ld = m->q_dim + 2 * m->kv_dim;
-    // out[b * ldo + r] (=, +=) (W in[b])[r]: one pass over a quantised matrix for all sequences (the residual add or the SiLU
-    // gate folded into its store), else vector by vector and the operators after it
-    auto product = [&](const slai_qmatrix* wm, const float* in, float* out, long long ldo, int epi = BATCH_STORE, float* gate = nullptr) -> int {
-        if (B > 1 && gemv_batch_supported(wm)) return gemv_batch_launch(ctx, out, wm, in, B, ldo, epi, gate);
+    const bool pdl = ctx->use_pdl;
+    // out[b * ldo + r] (=, +=) (W n(in[b]))[r], n = RmsNorm with `norm` (null: none): one pass over a quantised matrix for all
+    // sequences (the norm in front and the residual add or the SiLU gate folded in), else vector by vector and the operators around it
+    auto product = [&](const slai_qmatrix* wm, const float* norm, const float* in, float* out, long long ldo, int epi = BATCH_STORE,
+                       float* gate = nullptr) -> int {
+        if (B > 1 && gemv_batch_supported(wm)) return gemv_batch_launch(ctx, out, wm, in, B, ldo, epi, gate, norm, c.rms_norm_eps, pdl);
+        if (norm) {
+            const int r = rms_norm_rows_launch(ctx, m->bt_xn, in, norm, c.dim, B, c.rms_norm_eps);
+            if (r) return r;
+            in = m->bt_xn;
+        }
         float* dst = epi == BATCH_ADD ? m->bt_t : out;  // (the residual streams are dense: ldo == rows)
         for (int b = 0; b < B; b++) {
             const int r = slai_gemv_quant(ctx, dst + (size_t)b * ldo, wm, in + (size_t)b * wm->ncols, 1);
@@ -628,46 +635,43 @@ static int llama_batch_record(slai_llama* m, int B, int cap_pos) {
         const LlamaLayer& w = m->layers[l];
         void* kc = (char*)m->bt_k + (size_t)l * m->kv_layer_elems * esz;  // layer l of sequence 0; sequence b is bt_cache_bytes further
         void* vc = (char*)m->bt_v + (size_t)l * m->kv_layer_elems * esz;
-        if ((rc = rms_norm_rows_launch(ctx, m->bt_xn, m->bt_x, w.attn_norm, c.dim, B, c.rms_norm_eps))) return rc;
         // q, k, v in one launch where the three matrices can be walked as one (same format, heights multiples of 16)
         const bool qkv_one = B > 1 && gemv_batch_supported(w.wq) && w.wk->fmt == w.wq->fmt && w.wv->fmt == w.wq->fmt && m->q_dim % 16 == 0 &&
                              m->kv_dim % 16 == 0;
         if (qkv_one) {
             const slai_qmatrix* ws[3] = {w.wq, w.wk, w.wv};
-            if ((rc = gemv_batch_launch_multi(ctx, m->bt_qkv, ws, 3, m->bt_xn, B, qkv_ld, BATCH_STORE, nullptr))) return rc;
+            if ((rc = gemv_batch_launch_multi(ctx, m->bt_qkv, ws, 3, m->bt_x, B, qkv_ld, BATCH_STORE, nullptr, w.attn_norm, c.rms_norm_eps, pdl))) return rc;
         } else {
-            if ((rc = product(w.wq, m->bt_xn, m->bt_qkv, qkv_ld))) return rc;
-            if ((rc = product(w.wk, m->bt_xn, m->bt_qkv + m->q_dim, qkv_ld))) return rc;
-            if ((rc = product(w.wv, m->bt_xn, m->bt_qkv + m->q_dim + m->kv_dim, qkv_ld))) return rc;
+            if ((rc = product(w.wq, w.attn_norm, m->bt_x, m->bt_qkv, qkv_ld))) return rc;
+            if ((rc = product(w.wk, w.attn_norm, m->bt_x, m->bt_qkv + m->q_dim, qkv_ld))) return rc;
+            if ((rc = product(w.wv, w.attn_norm, m->bt_x, m->bt_qkv + m->q_dim + m->kv_dim, qkv_ld))) return rc;
         }
         if ((rc = rope_kv_store_seqs_launch(ctx, m->bt_qkv, qkv_ld, m->q_dim, m->kv_dim, m->head_size, d_pos, B, m->rope_theta, c.rope_variant != 0,
-                                            m->bt_q, kc, vc, c.kv_dtype == SLAI_KV_F16, kv_head_stride, (long long)m->bt_cache_bytes)))
+                                            m->bt_q, kc, vc, c.kv_dtype == SLAI_KV_F16, kv_head_stride, (long long)m->bt_cache_bytes, pdl)))
             return rc;
         {
             AttnLaunch A = {};
             A.q = m->bt_q; A.kcache = kc; A.vcache = vc; A.kv_dtype = c.kv_dtype;
             A.pos_stride = m->head_size; A.head_stride = kv_head_stride;
             A.n_heads = m->n_q_local; A.kv_mul = m->kv_mul; A.head_size = m->head_size;
-            A.d_pos = nullptr; A.max_pos = cap_pos; A.out = m->bt_xb; A.pdl = false;
+            A.d_pos = nullptr; A.max_pos = cap_pos; A.out = m->bt_xb; A.pdl = pdl;
             A.scratch = m->bt_attn; A.scratch_bytes = (size_t)m->bt_n * m->attn_scratch_bytes;
             A.batch = B; A.pos0 = 0; A.q_batch_stride = m->q_dim; A.out_batch_stride = m->q_dim; A.batch_counters = m->bt_tickets;
             A.cache_batch_stride = (long long)m->bt_cache_bytes; A.d_pos_batch = d_pos;
             if ((rc = attention_launch(ctx, A))) return rc;
         }
-        if ((rc = product(w.wo, m->bt_xb, m->bt_x, c.dim, BATCH_ADD))) return rc;
-        if ((rc = rms_norm_rows_launch(ctx, m->bt_xn, m->bt_x, w.ffn_norm, c.dim, B, c.rms_norm_eps))) return rc;
+        if ((rc = product(w.wo, nullptr, m->bt_xb, m->bt_x, c.dim, BATCH_ADD))) return rc;
         if (B > 1 && gemv_batch_supported(w.wgate) && w.wup->fmt == w.wgate->fmt && m->hidden % 16 == 0) {
             const slai_qmatrix* ws[2] = {w.wgate, w.wup};  // gate and up in one launch, SiLU in its store
-            if ((rc = gemv_batch_launch_multi(ctx, m->bt_u, ws, 2, m->bt_xn, B, m->hidden, BATCH_PAIR_SILU, nullptr))) return rc;
+            if ((rc = gemv_batch_launch_multi(ctx, m->bt_u, ws, 2, m->bt_x, B, m->hidden, BATCH_PAIR_SILU, nullptr, w.ffn_norm, c.rms_norm_eps, pdl))) return rc;
         } else {
-            if ((rc = product(w.wgate, m->bt_xn, m->bt_g, m->hidden))) return rc;
-            if ((rc = product(w.wup, m->bt_xn, m->bt_u, m->hidden, BATCH_SILU, m->bt_g))) return rc;
+            if ((rc = product(w.wgate, w.ffn_norm, m->bt_x, m->bt_g, m->hidden))) return rc;
+            if ((rc = product(w.wup, w.ffn_norm, m->bt_x, m->bt_u, m->hidden, BATCH_SILU, m->bt_g))) return rc;
         }
-        if ((rc = product(w.wdown, m->bt_u, m->bt_x, c.dim, BATCH_ADD))) return rc;
+        if ((rc = product(w.wdown, nullptr, m->bt_u, m->bt_x, c.dim, BATCH_ADD))) return rc;
     }
     const slai_qmatrix* wout = m->output ? m->output : (m->embd_q ? m->embd_q : &m->embd_as_matrix);
-    if ((rc = rms_norm_rows_launch(ctx, m->bt_xn, m->bt_x, m->out_norm, c.dim, B, c.rms_norm_eps))) return rc;
-    if ((rc = product(wout, m->bt_xn, m->bt_logits, c.vocab_size))) return rc;
+    if ((rc = product(wout, m->out_norm, m->bt_x, m->bt_logits, c.vocab_size))) return rc;
     for (int b = 0; b < B; b++)
         if ((rc = launch_argmax(ctx, m->bt_logits + (size_t)b * c.vocab_size, c.vocab_size, d_next + b, false))) return rc;
     return SLAI_OK;

@@ -598,6 +598,8 @@ __global__ void rope_kv_store_kernel(const float* __restrict__ q_src, const floa
                                      int ld, int q_dim, int kv_dim, int head_size, int pos0, const int* __restrict__ d_pos,
                                      const float* __restrict__ theta, int neox, float* __restrict__ q_out, int ldq, void* kcache, void* vcache,
                                      int kv_f16, long long kv_head_stride, long long seq_stride) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.y;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;  // pair index over q then k; then plain copies of v
     // seq_stride > 0: row t is a sequence of its own, at position d_pos[t] of caches seq_stride bytes after row t - 1's
@@ -789,12 +791,19 @@ int rope_kv_store_launch(slai_ctx* ctx, float* q, const float* k, const float* v
 }
 int rope_kv_store_seqs_launch(slai_ctx* ctx, const float* qkv, int ld, int q_dim, int kv_dim, int head_size, const int* d_pos, int B,
                               const float* theta, int neox, float* q_out, void* kcache, void* vcache, int kv_f16, long long kv_head_stride,
-                              long long seq_stride) {
+                              long long seq_stride, bool pdl) {
     SLAI_REQUIRE(ctx, seq_stride > 0 && d_pos && B >= 1, SLAI_ERR_INVALID_ARG, "rope: a batch of sequences needs positions and a cache stride");
     const int work = q_dim / 2 + kv_dim / 2 + kv_dim;
-    rope_kv_store_kernel<<<dim3((work + 255) / 256, B), 256, 0, ctx->stream>>>(qkv, qkv + q_dim, qkv + q_dim + kv_dim, ld, q_dim, kv_dim, head_size,
-                                                                              0, d_pos, theta, neox, q_out, q_dim, kcache, vcache, kv_f16,
-                                                                              kv_head_stride, seq_stride);
-    SLAI_CHECK_CUDA(ctx, cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((work + 255) / 256, B);
+    cfg.blockDim = dim3(256);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, rope_kv_store_kernel, qkv, qkv + q_dim, qkv + q_dim + kv_dim, ld, q_dim, kv_dim, head_size, 0, d_pos, theta,
+                                            neox, q_out, q_dim, kcache, vcache, kv_f16, kv_head_stride, seq_stride));
     return SLAI_OK;
 }
