@@ -385,26 +385,31 @@ inline int launch_dependent(slai_ctx* ctx, void (*kern)(KArgs...), dim3 grid, in
 }
 #endif
 
-// prefill.cu: prompt processing as GEMMs on the tcgen05 tensor cores
-struct PrefillGemm {
-    const slai_qmatrix* w = nullptr;  // quantised matrix [rows_total x K]; the first `rows` rows are used
-    int rows = 0;
-    const __half* x_hi = nullptr;     // activations as fp16 pairs (x = hi + lo), planes of [t_pad][K]
-    const __half* x_lo = nullptr;
-    int T = 0, t_pad = 0, NT = 0;     // valid tokens, allocated rows (multiple of NT), tokens per CTA tile
-    float* out = nullptr;             // [T][ldo], row m of the product at column out_off + m
-    int ldo = 0, out_off = 0;
-    const float* resid = nullptr;     // optional [T][ldr]: out = resid + product (may alias out)
-    int ldr = 0;
-    const float* bias = nullptr;      // optional [rows]
+// prefill_gemm.cu: a prompt through quantised matrices on the tcgen05 tensor cores
+struct PrefillOperands {
+    __half *hi = nullptr, *lo = nullptr;  // activations as fp16 pairs (x = hi + lo), planes of [t_pad][K]
+    __half* sum = nullptr;                // their sub-blocks' sums, [t_pad][K / 16] (written where K is a multiple of 256)
 };
-size_t prefill_gemm_smem(int NT);
+struct PrefillGemm {
+    int n = 1;                            // matrices of one format and width that share the activations
+    const slai_qmatrix* w[3] = {};
+    int rows[3] = {};                     // the first `rows` rows of each are used
+    float* out[3] = {};                   // row m of the product of token t at out[t * ldo + m]
+    const float* bias[3] = {};            // optional [rows]
+    const __half *x_hi = nullptr, *x_lo = nullptr, *x_sum = nullptr;
+    int T = 0, t_pad = 0;                 // valid tokens, allocated rows (a multiple of prefill_gemm_nt(T))
+    int ldo = 0;
+    const float* resid = nullptr;         // optional [T][ldr]: out = resid + product (may alias out)
+    int ldr = 0;
+};
+int prefill_gemm_nt(int T);
 int prefill_gemm_launch(slai_ctx* ctx, const PrefillGemm& G);
-int prefill_split_launch(slai_ctx* ctx, const float* x, int ldx, const float* norm_w, float eps, int T, int K, __half* hi, __half* lo);
-int prefill_silu_split_launch(slai_ctx* ctx, const float* gate, const float* up, int T, int H, __half* hi, __half* lo);
-int prefill_split_ln_launch(slai_ctx* ctx, const float* x, int ldx, const float* gamma, const float* beta, float eps, int T, int K, __half* hi,
-                            __half* lo);
-int prefill_gelu_split_launch(slai_ctx* ctx, const float* g, int T, int H, __half* hi, __half* lo);
+// prefill.cu: the kernels around the GEMMs
+int prefill_split_launch(slai_ctx* ctx, const float* x, int ldx, const float* norm_w, float eps, int T, int K, const PrefillOperands& o);
+int prefill_silu_split_launch(slai_ctx* ctx, const float* gate, const float* up, int T, int H, const PrefillOperands& o);
+int prefill_split_ln_launch(slai_ctx* ctx, const float* x, int ldx, const float* gamma, const float* beta, float eps, int T, int K,
+                            const PrefillOperands& o);
+int prefill_gelu_split_launch(slai_ctx* ctx, const float* g, int T, int H, const PrefillOperands& o);
 int prefill_add_rows_launch(slai_ctx* ctx, float* x, int dim, const float* table, int pos0, int T);
 int prefill_embed_launch(slai_ctx* ctx, float* x, int dim, const int* d_tokens, int T, const float* table, const slai_qmatrix* qtable);
 // One token of each of `B` sequences: row b of qkv ([B][ld]: q, k, v side by side) at position d_pos[b] (negative: skipped),

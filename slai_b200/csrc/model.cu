@@ -133,7 +133,7 @@ struct slai_llama {
     int pf_cap = 0, pf_attn_batch = 0;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_q = nullptr, *pf_xb = nullptr, *pf_g = nullptr, *pf_u = nullptr;
     float* pf_part = nullptr;  // sharded models: this rank's partial of a row-parallel product, [tokens][dim]
-    __half *pf_hi = nullptr, *pf_lo = nullptr;
+    PrefillOperands pf_op;
     int* pf_tokens = nullptr;
     void* pf_attn_scratch = nullptr;
     size_t pf_attn_scratch_bytes = 0;
@@ -178,10 +178,10 @@ static void llama_drop_batch(slai_llama* m) {
 static void llama_drop_prefill(slai_llama* m) {
     if (m->pf_cap) cudaStreamSynchronize(m->ctx->stream);
     cudaFree(m->pf_x); cudaFree(m->pf_qkv); cudaFree(m->pf_q); cudaFree(m->pf_xb); cudaFree(m->pf_g); cudaFree(m->pf_u);
-    cudaFree(m->pf_hi); cudaFree(m->pf_lo); cudaFree(m->pf_tokens); cudaFree(m->pf_attn_scratch); cudaFree(m->pf_tickets);
+    cudaFree(m->pf_op.hi); cudaFree(m->pf_op.lo); cudaFree(m->pf_op.sum); cudaFree(m->pf_tokens); cudaFree(m->pf_attn_scratch); cudaFree(m->pf_tickets);
     cudaFree(m->pf_part);
     m->pf_x = m->pf_qkv = m->pf_q = m->pf_xb = m->pf_g = m->pf_u = m->pf_part = nullptr;
-    m->pf_hi = m->pf_lo = nullptr;
+    m->pf_op = PrefillOperands();
     m->pf_tokens = nullptr;
     m->pf_attn_scratch = nullptr;
     m->pf_attn_scratch_bytes = 0;
@@ -919,6 +919,13 @@ static int prefill_impl(M* m, RecordFn record, int vocab, int seq_len, const int
 // norm + logits GEMV (+ greedy choice) run on it.  Sharded models run the same sequence on their shards; the two
 // row-parallel products of a layer (output and down projection) leave a partial [tokens][dim] on every rank, summed with
 // one all-reduce each and added to the residual stream, which stays identical on all ranks.
+struct PrefillGemmPart {  // one of several matrices that share their input
+    const slai_qmatrix* w;
+    int rows;
+    float* out;
+    const float* bias;
+};
+
 static bool llama_prefill_eligible(const slai_llama* m, int n) {
     const char* e = getenv("SLAI_PREFILL_SEQUENTIAL");
     if (e && e[0] == '1') return false;
@@ -945,7 +952,8 @@ static int llama_prefill_reserve(slai_llama* m, int t_pad, int attn_batch, size_
                   cudaMalloc(&m->pf_q, T * m->q_dim * 4) == cudaSuccess && cudaMalloc(&m->pf_xb, T * m->q_dim * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_g, T * m->hidden * 4) == cudaSuccess && cudaMalloc(&m->pf_u, T * m->hidden * 4) == cudaSuccess &&
                   (m->tp == 1 || cudaMalloc(&m->pf_part, T * c.dim * 4) == cudaSuccess) &&
-                  cudaMalloc(&m->pf_hi, T * kmax * 2) == cudaSuccess && cudaMalloc(&m->pf_lo, T * kmax * 2) == cudaSuccess &&
+                  cudaMalloc(&m->pf_op.hi, T * kmax * 2) == cudaSuccess &&
+                  cudaMalloc(&m->pf_op.lo, T * kmax * 2) == cudaSuccess && cudaMalloc(&m->pf_op.sum, T * kmax / 8) == cudaSuccess &&
                   cudaMalloc(&m->pf_tokens, T * 4) == cudaSuccess && cudaMalloc(&m->pf_tickets, (size_t)attn_batch * n_kv * 4) == cudaSuccess &&
                   cudaMemsetAsync(m->pf_tickets, 0, (size_t)attn_batch * n_kv * 4, ctx->stream) == cudaSuccess;
         if (!ok) {
@@ -976,8 +984,7 @@ static int llama_prefill_reserve(slai_llama* m, int t_pad, int attn_batch, size_
 static int llama_prefill_batched(slai_llama* m, const int32_t* h_tokens, int n, int pos0, float* h_last_logits) {
     slai_ctx* ctx = m->ctx;
     const slai_llama_config& c = m->cfg;
-    const int NT = std::min(256, (n + 15) / 16 * 16);
-    const int t_pad = (n + NT - 1) / NT * NT;
+    const int NT = prefill_gemm_nt(n), t_pad = (n + NT - 1) / NT * NT;
     const int AB = 64;  // query tokens per attention launch
     const int n_kv = attention_tickets(m->n_q_local, m->kv_mul);  // tickets per query token (virtual heads of the attention kernel)
     const size_t attn_per_token = attention_scratch_bytes(ctx, m->n_q_local, m->kv_mul, m->head_size, pos0 + n - 1);
@@ -986,25 +993,41 @@ static int llama_prefill_batched(slai_llama* m, const int32_t* h_tokens, int n, 
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     const size_t kmax = (size_t)std::max(std::max(c.dim, m->hidden), m->q_dim);
     SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->pf_tokens, h_tokens, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SLAI_CHECK_CUDA(ctx, cudaMemsetAsync(m->pf_hi, 0, (size_t)m->pf_cap * kmax * 2, ctx->stream));  // rows beyond the prompt stay zero
-    SLAI_CHECK_CUDA(ctx, cudaMemsetAsync(m->pf_lo, 0, (size_t)m->pf_cap * kmax * 2, ctx->stream));
     if ((rc = prefill_embed_launch(ctx, m->pf_x, c.dim, m->pf_tokens, n, m->embd_q ? nullptr : m->token_embd, m->embd_q))) return rc;
     const int qkv_ld = m->q_dim + 2 * m->kv_dim;
-    auto gemm = [&](const slai_qmatrix* w, int rows, float* out, int ldo, int off, const float* resid, int ldr, const float* bias) {
+    auto operands = [&](PrefillGemm& G) {
+        G.x_hi = m->pf_op.hi; G.x_lo = m->pf_op.lo; G.x_sum = m->pf_op.sum; G.T = n; G.t_pad = t_pad;
+    };
+    // one product; matrices of one format that share their input go through one launch
+    auto gemm = [&](const slai_qmatrix* w, int rows, float* out, int ldo, const float* resid, int ldr, const float* bias) {
         PrefillGemm G;
-        // Fewer tokens per CTA tile while the grid would leave half of the SMs without a tile (4096-row matrices at 512 tokens:
-        // 64 CTAs of 256 tokens become 128 CTAs of 128); every CTA dequantises its weight rows itself, so no further.
-        int nt = NT;
-        const int m_tiles = (rows + 127) / 128;
-        while (nt > 64 && (nt / 2) % 16 == 0 && t_pad % (nt / 2) == 0 && m_tiles * (t_pad / nt) * 2 <= ctx->sm_count) nt /= 2;
-        G.w = w; G.rows = rows; G.x_hi = m->pf_hi; G.x_lo = m->pf_lo; G.T = n; G.t_pad = t_pad; G.NT = nt;
-        G.out = out; G.ldo = ldo; G.out_off = off; G.resid = resid; G.ldr = ldr; G.bias = bias;
+        operands(G);
+        G.w[0] = w; G.rows[0] = rows; G.out[0] = out; G.bias[0] = bias; G.ldo = ldo; G.resid = resid; G.ldr = ldr;
         return prefill_gemm_launch(ctx, G);
     };
-    // x += W * (the activations in pf_hi / pf_lo), W split by columns over the ranks of a sharded model
+    auto gemms = [&](std::initializer_list<PrefillGemmPart> parts, int ldo) -> int {
+        const slai_qmatrix* w0 = parts.begin()->w;
+        bool same = true;
+        for (auto& p : parts) same = same && p.w->fmt == w0->fmt && p.w->ncols == w0->ncols;
+        PrefillGemm G;
+        operands(G);
+        G.n = 0;
+        G.ldo = ldo;
+        for (auto& p : parts) {
+            if (!same) {
+                const int r = gemm(p.w, p.rows, p.out, ldo, nullptr, 0, p.bias);
+                if (r) return r;
+                continue;
+            }
+            G.w[G.n] = p.w; G.rows[G.n] = p.rows; G.out[G.n] = p.out; G.bias[G.n] = p.bias;
+            G.n++;
+        }
+        return same ? prefill_gemm_launch(ctx, G) : SLAI_OK;
+    };
+    // x += W * (the activations in pf_op), W split by columns over the ranks of a sharded model
     auto row_parallel = [&](const slai_qmatrix* w) -> int {
-        if (m->tp == 1) return gemm(w, c.dim, m->pf_x, c.dim, 0, m->pf_x, c.dim, nullptr);
-        int r = gemm(w, c.dim, m->pf_part, c.dim, 0, nullptr, 0, nullptr);
+        if (m->tp == 1) return gemm(w, c.dim, m->pf_x, c.dim, m->pf_x, c.dim, nullptr);
+        int r = gemm(w, c.dim, m->pf_part, c.dim, nullptr, 0, nullptr);
         if (!r) r = tp_all_reduce_sum(ctx, m->pf_part, m->pf_part, (int64_t)n * c.dim);
         if (!r) r = slai_add_assign(ctx, m->pf_x, m->pf_part, (int64_t)n * c.dim);
         return r;
@@ -1014,10 +1037,10 @@ static int llama_prefill_batched(slai_llama* m, const int32_t* h_tokens, int n, 
         void* kc = (char*)m->kcache + (size_t)l * m->kv_layer_elems * esz;
         void* vc = (char*)m->vcache + (size_t)l * m->kv_layer_elems * esz;
         // q, k, v                                                              transformer.rs:327-347
-        if ((rc = prefill_split_launch(ctx, m->pf_x, c.dim, w.attn_norm, c.rms_norm_eps, n, c.dim, m->pf_hi, m->pf_lo))) return rc;
-        if ((rc = gemm(w.wq, m->q_dim, m->pf_qkv, qkv_ld, 0, nullptr, 0, w.bq))) return rc;
-        if ((rc = gemm(w.wk, m->kv_dim, m->pf_qkv, qkv_ld, m->q_dim, nullptr, 0, w.bk))) return rc;
-        if ((rc = gemm(w.wv, m->kv_dim, m->pf_qkv, qkv_ld, m->q_dim + m->kv_dim, nullptr, 0, w.bv))) return rc;
+        if ((rc = prefill_split_launch(ctx, m->pf_x, c.dim, w.attn_norm, c.rms_norm_eps, n, c.dim, m->pf_op))) return rc;
+        if ((rc = gemms({{w.wq, m->q_dim, m->pf_qkv, w.bq}, {w.wk, m->kv_dim, m->pf_qkv + m->q_dim, w.bk},
+                         {w.wv, m->kv_dim, m->pf_qkv + m->q_dim + m->kv_dim, w.bv}}, qkv_ld)))
+            return rc;
         if ((rc = prefill_rope_kv_launch(ctx, m->pf_qkv, qkv_ld, m->q_dim, m->kv_dim, m->head_size, pos0, n, m->rope_theta, c.rope_variant != 0,
                                          m->pf_q, kc, vc, c.kv_dtype == SLAI_KV_F16, (long long)c.seq_len * m->head_size)))
             return rc;
@@ -1040,13 +1063,12 @@ static int llama_prefill_batched(slai_llama* m, const int32_t* h_tokens, int n, 
             if ((rc = attention_launch(ctx, A))) return rc;
         }
         // x += Wo xb                                                           transformer.rs:352-355
-        if ((rc = prefill_split_launch(ctx, m->pf_xb, m->q_dim, nullptr, 0.f, n, m->q_dim, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_split_launch(ctx, m->pf_xb, m->q_dim, nullptr, 0.f, n, m->q_dim, m->pf_op))) return rc;
         if ((rc = row_parallel(w.wo))) return rc;
         // FFN                                                                  transformer.rs:356-365
-        if ((rc = prefill_split_launch(ctx, m->pf_x, c.dim, w.ffn_norm, c.rms_norm_eps, n, c.dim, m->pf_hi, m->pf_lo))) return rc;
-        if ((rc = gemm(w.wgate, m->hidden, m->pf_g, m->hidden, 0, nullptr, 0, nullptr))) return rc;
-        if ((rc = gemm(w.wup, m->hidden, m->pf_u, m->hidden, 0, nullptr, 0, nullptr))) return rc;
-        if ((rc = prefill_silu_split_launch(ctx, m->pf_g, m->pf_u, n, m->hidden, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_split_launch(ctx, m->pf_x, c.dim, w.ffn_norm, c.rms_norm_eps, n, c.dim, m->pf_op))) return rc;
+        if ((rc = gemms({{w.wgate, m->hidden, m->pf_g, nullptr}, {w.wup, m->hidden, m->pf_u, nullptr}}, m->hidden))) return rc;
+        if ((rc = prefill_silu_split_launch(ctx, m->pf_g, m->pf_u, n, m->hidden, m->pf_op))) return rc;
         if ((rc = row_parallel(w.wdown))) return rc;
     }
     // the last token's state goes back to the decode step's vectors; final norm, logits and the greedy choice as there
@@ -1217,16 +1239,16 @@ struct slai_gpt2 {
     // prompt processing as GEMMs (prefill.cu): buffers for `pf_cap` tokens, grown on demand
     int pf_cap = 0;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_q = nullptr, *pf_xb = nullptr, *pf_ff = nullptr, *pf_theta0 = nullptr;
-    __half *pf_hi = nullptr, *pf_lo = nullptr;
+    PrefillOperands pf_op;
     int* pf_tokens = nullptr;
 };
 
 static void gpt2_drop_prefill(slai_gpt2* m) {
     if (m->pf_cap) cudaStreamSynchronize(m->ctx->stream);
     cudaFree(m->pf_x); cudaFree(m->pf_qkv); cudaFree(m->pf_q); cudaFree(m->pf_xb); cudaFree(m->pf_ff); cudaFree(m->pf_theta0);
-    cudaFree(m->pf_hi); cudaFree(m->pf_lo); cudaFree(m->pf_tokens);
+    cudaFree(m->pf_op.hi); cudaFree(m->pf_op.lo); cudaFree(m->pf_op.sum); cudaFree(m->pf_tokens);
     m->pf_x = m->pf_qkv = m->pf_q = m->pf_xb = m->pf_ff = m->pf_theta0 = nullptr;
-    m->pf_hi = m->pf_lo = nullptr;
+    m->pf_op = PrefillOperands();
     m->pf_tokens = nullptr;
     m->pf_cap = 0;
 }
@@ -1469,16 +1491,15 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
     slai_ctx* ctx = m->ctx;
     const slai_gpt2_config& c = m->cfg;
     const int E = c.n_embd, F = c.ff_len;
-    const int NT = std::min(256, (n + 15) / 16 * 16);
-    const int t_pad = (n + NT - 1) / NT * NT;
+    const int NT = prefill_gemm_nt(n), t_pad = (n + NT - 1) / NT * NT;
     const size_t kmax = (size_t)std::max(E, F);
     if (t_pad > m->pf_cap) gpt2_drop_prefill(m);
     if (!m->pf_cap) {
         const size_t T = (size_t)t_pad;
         bool ok = cudaMalloc(&m->pf_x, T * E * 4) == cudaSuccess && cudaMalloc(&m->pf_qkv, T * 3 * E * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_q, T * E * 4) == cudaSuccess && cudaMalloc(&m->pf_xb, T * E * 4) == cudaSuccess &&
-                  cudaMalloc(&m->pf_ff, T * F * 4) == cudaSuccess && cudaMalloc(&m->pf_hi, T * kmax * 2) == cudaSuccess &&
-                  cudaMalloc(&m->pf_lo, T * kmax * 2) == cudaSuccess && cudaMalloc(&m->pf_tokens, T * 4) == cudaSuccess &&
+                  cudaMalloc(&m->pf_ff, T * F * 4) == cudaSuccess && cudaMalloc(&m->pf_op.hi, T * kmax * 2) == cudaSuccess &&
+                  cudaMalloc(&m->pf_op.lo, T * kmax * 2) == cudaSuccess && cudaMalloc(&m->pf_op.sum, T * kmax / 8) == cudaSuccess && cudaMalloc(&m->pf_tokens, T * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_theta0, (size_t)m->head_size * 4) == cudaSuccess &&
                   cudaMemsetAsync(m->pf_theta0, 0, (size_t)m->head_size * 4, ctx->stream) == cudaSuccess;
         if (!ok) {
@@ -1491,18 +1512,13 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
     int rc;
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->pf_tokens, h_tokens, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SLAI_CHECK_CUDA(ctx, cudaMemsetAsync(m->pf_hi, 0, (size_t)m->pf_cap * kmax * 2, ctx->stream));  // rows beyond the prompt stay zero
-    SLAI_CHECK_CUDA(ctx, cudaMemsetAsync(m->pf_lo, 0, (size_t)m->pf_cap * kmax * 2, ctx->stream));
     // x = wte[:,tok] + wpe[:,pos]                                              gpt2/cpu.rs:227-228
     if ((rc = prefill_embed_launch(ctx, m->pf_x, E, m->pf_tokens, n, nullptr, m->wte))) return rc;
     if ((rc = prefill_add_rows_launch(ctx, m->pf_x, E, m->wpe, pos0, n))) return rc;
     auto gemm = [&](const slai_qmatrix* w, int rows, float* out, int ldo, const float* resid, int ldr, const float* bias) {
         PrefillGemm G;
-        int nt = NT;
-        const int m_tiles = (rows + 127) / 128;
-        while (nt > 64 && (nt / 2) % 16 == 0 && t_pad % (nt / 2) == 0 && m_tiles * (t_pad / nt) * 2 <= ctx->sm_count) nt /= 2;
-        G.w = w; G.rows = rows; G.x_hi = m->pf_hi; G.x_lo = m->pf_lo; G.T = n; G.t_pad = t_pad; G.NT = nt;
-        G.out = out; G.ldo = ldo; G.out_off = 0; G.resid = resid; G.ldr = ldr; G.bias = bias;
+        G.x_hi = m->pf_op.hi; G.x_lo = m->pf_op.lo; G.x_sum = m->pf_op.sum; G.T = n; G.t_pad = t_pad;
+        G.w[0] = w; G.rows[0] = rows; G.out[0] = out; G.bias[0] = bias; G.ldo = ldo; G.resid = resid; G.ldr = ldr;
         return prefill_gemm_launch(ctx, G);
     };
     const long long kv_head_stride = (long long)c.n_seq * m->head_size;
@@ -1510,7 +1526,7 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
         const Gpt2Layer& w = m->layers[l];
         void* kc = (char*)m->kcache + (size_t)l * m->kv_layer_elems * esz;
         void* vc = (char*)m->vcache + (size_t)l * m->kv_layer_elems * esz;
-        if ((rc = prefill_split_ln_launch(ctx, m->pf_x, E, w.ln1_g, w.ln1_b, c.layernorm_eps, n, E, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_split_ln_launch(ctx, m->pf_x, E, w.ln1_g, w.ln1_b, c.layernorm_eps, n, E, m->pf_op))) return rc;
         if ((rc = gemm(w.w_qkv, 3 * E, m->pf_qkv, 3 * E, nullptr, 0, w.b_qkv))) return rc;
         if ((rc = prefill_rope_kv_launch(ctx, m->pf_qkv, 3 * E, E, E, m->head_size, pos0, n, m->pf_theta0, 0, m->pf_q, kc, vc,
                                          c.kv_dtype == SLAI_KV_F16, kv_head_stride)))
@@ -1518,11 +1534,11 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
         if ((rc = prefill_attention_launch(ctx, m->pf_q, E, kc, vc, c.kv_dtype == SLAI_KV_F16, kv_head_stride, m->head_size, c.n_head, 1, pos0, n,
                                            m->pf_xb, E)))
             return rc;
-        if ((rc = prefill_split_launch(ctx, m->pf_xb, E, nullptr, 0.f, n, E, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_split_launch(ctx, m->pf_xb, E, nullptr, 0.f, n, E, m->pf_op))) return rc;
         if ((rc = gemm(w.w_proj, E, m->pf_x, E, m->pf_x, E, w.b_proj))) return rc;
-        if ((rc = prefill_split_ln_launch(ctx, m->pf_x, E, w.ln2_g, w.ln2_b, c.layernorm_eps, n, E, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_split_ln_launch(ctx, m->pf_x, E, w.ln2_g, w.ln2_b, c.layernorm_eps, n, E, m->pf_op))) return rc;
         if ((rc = gemm(w.w_fc, F, m->pf_ff, F, nullptr, 0, w.b_fc))) return rc;
-        if ((rc = prefill_gelu_split_launch(ctx, m->pf_ff, n, F, m->pf_hi, m->pf_lo))) return rc;
+        if ((rc = prefill_gelu_split_launch(ctx, m->pf_ff, n, F, m->pf_op))) return rc;
         if ((rc = gemm(w.w_fcproj, E, m->pf_x, E, m->pf_x, E, w.b_fcproj))) return rc;
     }
     // the last token's state goes back to the decode step's vector; final norm, logits and the greedy choice as there

@@ -1,0 +1,640 @@
+// Y[T x M] = X[T x K] W^T for a prompt of T tokens on the 5th-generation tensor cores, W quantised (tile-major, layout.cuh).
+//
+// Numerics.  Parity with the sequential path is the contract, and a single fp16 rounding of both operands (4e-4 per GEMM)
+// would spend its budget.  The activations are fp16 pairs v = hi + lo (22 bits).  The weights of Q4_K / Q5_K go in as the
+// exact integers sc * q, so two products per 16 columns suffice (hi, lo); the super-block scale d multiplies the f32 sums
+// of each 256 columns, in registers, and the minimum term is one more product per super-block with its own sums and scale
+// dmin.  Q6_K (integers beyond fp16's 11 bits) and Q8_0 (a scale every 32 columns) carry the weights as pairs too: three
+// products (hi hi, hi lo, lo hi), about 2^-21 each.
+//
+// One CTA computes 128 weight rows x NT tokens (<= 128) over its share of K:
+//   warp 0      TMA: the activations' hi and lo planes, 64 columns per stage; the sums plane, 16 columns per super-block
+//   warp 1      issues tcgen05.mma (kind::f16, M = 128, N = NT, K = 16), commits stages and super-blocks to mbarriers
+//   warp 2      bulk copies of the packed tile-step blocks (8 row tiles x one super-block), two or three super-blocks ahead: a
+//               few tokens read the matrix from HBM, which takes some 40 KB in flight per SM
+//   warps 4-11  packed bytes -> operand rows (prefill_dequant.cuh), one 16-row tile each
+//   warps 12-19 sums of a super-block out of tensor memory (two buffers) into registers, times d (and dmin), while the tensor
+//               cores work on the next one.  (Done by warps 4-11 between two stages, this put a super-block's drain and the
+//               next stages' operands one after the other: 1000 cycles per stage whatever the number of tokens.)
+// CTAs are persistent: a tile's sums are stored by warps 12-19 while the other warps are in the next tile.  (One CTA per tile:
+// each wave paid its start, its residual loads and its stores on top of 30 us of products: 7B, 511 tokens, output
+// projection 70 us, q/k/v 124 us.)
+// Few tokens leave most SMs without a tile (4096 rows x 37 tokens: 32 tiles), so K is split over a cluster of up to 8
+// CTAs, whose sums meet through distributed shared memory in rank order (deterministic, no second launch).
+//
+// What bounds it: with 128 tokens per tile the shared-memory traffic of the operands (A and B are read for every product,
+// 128 B per cycle at the tensor cores' full rate) and the L2 reads of the activations; with few tokens HBM and the
+// latency of a super-block's round through the stages.
+// Every mbarrier wait is bounded: on expiry the error flag is raised, later waits of the thread give up at once and the
+// kernel runs to its end.
+#include <algorithm>
+
+#include <cuda.h>
+
+#include "common.cuh"
+#include "prefill_dequant.cuh"
+
+namespace {
+
+constexpr int PG_THREADS = 640;
+constexpr int PG_BM = 128, PG_BK = 64;          // weight rows per CTA, columns per stage (one 128-byte swizzle row of fp16)
+constexpr int PG_MAX_NT = 128;
+constexpr int PG_MAX_STAGES = 6, PG_MAX_PACK = 3, PG_MAX_KS = 8;
+constexpr int PG_A_BYTES = PG_BM * PG_BK * 2;   // one operand plane of a stage
+constexpr int PG_SMEM_LIMIT = 227 * 1024 - 512; // the barriers are static
+
+struct PgSeg {
+    const uint8_t* w;
+    float* out;
+    const float* bias;
+    int rows, tile0;  // logical rows; first 128-row tile in the launch's tile space
+};
+struct PgParams {
+    PgSeg seg[3];
+    int nseg;
+    long long tile_bytes;  // bytes of one 16-row tile (all K steps)
+    int nch;               // packed blocks (super-blocks) along K
+    int T, NT, NTP;        // tokens, tokens per tile, the same rounded up to a power of two (tensor-memory columns)
+    int ldo;
+    const float* resid;    // optional [T][ldr]: out = resid + y (may alias out)
+    int ldr;
+    int n_tiles, tiles;    // token tiles, all tiles (token tiles fastest: neighbours share the weights in L2)
+    int ks;                // CTAs of a cluster that share K
+    int stages, packs;     // operand stages, packed blocks in flight
+    unsigned int* err_flag;
+    unsigned int wait_limit;
+};
+
+// ---- PTX wrappers ---------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t a) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(a), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Bounded wait.  On expiry the error flag is raised and `limit` drops to one poll.
+__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
+    for (unsigned int i = 0; i < limit; i++) {
+        if (mbar_try(a, parity)) return true;
+        if (i > 64) __nanosleep(40);
+    }
+    atomicExch(err_flag, 5u);
+    limit = 1;
+    return false;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"(map), "r"(mbar), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Shared-memory matrix descriptor of a K-major operand tile: start address / 16 in bits 0-13, leading offset (unused with a
+// swizzle of the row length) 1 in bits 16-29, stride between 8-row groups / 16 in bits 32-45, descriptor version 1 in bits
+// 46-47, swizzle mode in bits 61-63 (2: rows of 128 bytes, 6: rows of 32 bytes).
+__device__ __forceinline__ uint64_t desc128(uint32_t a) {
+    return (uint64_t)((a >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t desc32(uint32_t a) {
+    return (uint64_t)((a >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
+}
+// Instruction descriptor, kind::f16: f32 accumulator (bits 4-5 = 1), A and B fp16 (0), both K-major (bits 15, 16 = 0),
+// N / 8 in bits 17-22, M / 16 in bits 24-28.
+__device__ __forceinline__ uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PG_BM >> 4) << 24); }
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t mbar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Dynamic shared memory, from a 1024-byte boundary: operand planes of the weights, of the activations, the operands of the
+// minimum term (two super-blocks), row scales (four super-blocks), packed blocks.
+struct PgLayout {
+    uint32_t a, b, amin, bmin, scale, pack, total;
+};
+template <int FMT>
+__host__ __device__ inline PgLayout pg_layout(int NT, int stages, int packs) {
+    using F = pfq::Fmt<FMT>;
+    PgLayout L;
+    L.a = 0;
+    L.b = L.a + (uint32_t)stages * F::PLANES * PG_A_BYTES;
+    L.amin = L.b + (uint32_t)stages * 2 * NT * PG_BK * 2;
+    L.bmin = L.amin + (F::MIN ? 2 * PG_BM * 32 : 0);
+    L.scale = L.bmin + (F::MIN ? 2 * (uint32_t)NT * 32 : 0);
+    L.pack = L.scale + 4 * PG_BM * 4;
+    L.total = L.pack + (uint32_t)packs * 8 * F::STEP;
+    return L;
+}
+
+template <int FMT>
+__global__ void __launch_bounds__(PG_THREADS, 1)
+prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                    const __grid_constant__ CUtensorMap map_sum) {
+    using F = pfq::Fmt<FMT>;
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    const PgLayout L = pg_layout<FMT>(P.NT, P.stages, P.packs);
+    const int NT = P.NT, S = P.stages, PK = P.packs;
+    const uint32_t b_bytes = (uint32_t)NT * PG_BK * 2;  // one activation plane of a stage
+    __shared__ __align__(8) unsigned long long bars[3 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 10];
+    __shared__ uint32_t tmem_slot;
+    const uint32_t sb = smem_u32(smem);
+    const uint32_t full_a = smem_u32(bars), full_b = full_a + 8 * PG_MAX_STAGES, empty = full_b + 8 * PG_MAX_STAGES,
+                   pk_full = empty + 8 * PG_MAX_STAGES, pk_empty = pk_full + 8 * PG_MAX_PACK, dfull = pk_empty + 8 * PG_MAX_PACK,
+                   dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16;
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform for the compiler too)
+    const int rank = P.ks > 1 ? (int)(blockIdx.x % P.ks) : 0;
+    const int tile0 = (int)blockIdx.x / P.ks, tile_step = (int)gridDim.x / P.ks;
+    const int c0 = (int)((long long)P.nch * rank / P.ks), nc = (int)((long long)P.nch * (rank + 1) / P.ks) - c0;  // super-blocks of this CTA
+    // a tile's matrix, first row in it and first token
+    auto tile_of = [&](int tile, PgSeg& sg, int& m0, int& n0) {
+        const int mt = tile / P.n_tiles;
+        n0 = (tile - mt * P.n_tiles) * NT;
+        sg = P.seg[0];
+        if (P.nseg > 1 && mt >= P.seg[1].tile0) sg = P.seg[1];
+        if (P.nseg > 2 && mt >= P.seg[2].tile0) sg = P.seg[2];
+        m0 = (mt - sg.tile0) * PG_BM;
+    };
+
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(full_a + 8 * s, 8);
+            mbar_init(full_b + 8 * s, 1);
+            mbar_init(empty + 8 * s, 1);
+        }
+        for (int s = 0; s < PK; s++) {
+            mbar_init(pk_full + 8 * s, 1);
+            mbar_init(pk_empty + 8 * s, 8);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(dfull + 8 * s, 1);
+            mbar_init(dempty + 8 * s, 8);
+            mbar_init(bmin_full + 8 * s, 1);
+        }
+        for (int s = 0; s < 4; s++) mbar_init(sc_full + 8 * s, 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async();
+    }
+    int ncols = 32;
+    while (ncols < (F::MIN ? 4 : 2) * P.NTP) ncols <<= 1;
+    if (warp == 1) {  // the MMA warp owns the tensor-memory allocation
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    unsigned int limit = P.wait_limit;
+    // Dependent launch: the weights' warps need not wait for the kernel before this one, everything else does.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp < 2 || warp >= 12) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // readers of the sums (warps 12-19): 32 rows each, every other group of 16 tokens
+    float acc[4][16];
+    const int quad = warp & 3, half = (warp - 12) >> 2;
+
+    if (warp == 0) {
+        // ---- activations ----
+        if (lane == 0) {
+            int slot = 0, issued = 0, gc = 0;  // gc: super-blocks so far
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < P.tiles && ok; tile += tile_step) {
+                PgSeg sg;
+                int m0, n0;
+                tile_of(tile, sg, m0, n0);
+                for (int c = 0; c < nc && ok; c++, gc++) {
+                    if (F::MIN) {
+                        const int buf = gc & 1;
+                        if (gc >= 2 && !(ok = mbar_wait(dfull + 8 * buf, ((gc >> 1) - 1) & 1, limit, P.err_flag))) break;
+                        mbar_expect_tx(bmin_full + 8 * buf, (uint32_t)NT * 32);
+                        tma_load_2d(sb + L.bmin + buf * NT * 32, &map_sum, 16 * (c0 + c), n0, bmin_full + 8 * buf);
+                    }
+                    for (int st = 0; st < F::STAGES; st++) {
+                        if (!(ok = mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
+                        const int x = ((c0 + c) * F::STAGES + st) * PG_BK;
+                        mbar_expect_tx(full_b + 8 * slot, 2 * b_bytes);
+                        tma_load_2d(sb + L.b + slot * 2 * b_bytes, &map_hi, x, n0, full_b + 8 * slot);
+                        tma_load_2d(sb + L.b + slot * 2 * b_bytes + b_bytes, &map_lo, x, n0, full_b + 8 * slot);
+                        issued++;
+                        if (++slot == S) {
+                            slot = 0;
+                            ph ^= 1;
+                        }
+                    }
+                }
+            }
+            if (!ok) {  // a wait ran out: this thread's own copies in flight land before the CTA may end
+                for (int i = max(0, issued - S); i < issued; i++) {
+                    limit = P.wait_limit;
+                    mbar_wait(full_b + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- tensor cores: the whole warp walks the loop, so that descriptors live in uniform registers, one lane issues ----
+        const uint32_t idesc = umma_idesc(NT);
+        const uint64_t da0 = desc128(sb + L.a), db0 = desc128(sb + L.b);
+        int slot = 0, u = 0;  // u: sums so far (of a super-block; Q8_0: of a whole tile), alternately in two buffers
+        uint32_t ph = 0;
+        for (int tile = tile0; tile < P.tiles; tile += tile_step)
+        for (int c = 0; c < nc; c++) {
+            const int buf = u & 1;
+            const uint32_t d = tmem + buf * P.NTP;
+            if ((F::SCALED || c == 0) && u >= 2) mbar_wait(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
+            for (int st = 0; st < F::STAGES; st++) {
+                mbar_wait(full_a + 8 * slot, ph, limit, P.err_flag);
+                mbar_wait(full_b + 8 * slot, ph, limit, P.err_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                __syncwarp();
+                // 16 elements = 32 bytes further along the swizzled row: 2 in the descriptor's units of 16 bytes
+                const uint64_t dah = da0 + (uint64_t)(slot * F::PLANES * (PG_A_BYTES >> 4)), dbh = db0 + (uint64_t)(slot * 2 * (b_bytes >> 4));
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < PG_BK / 16; kk++) {
+                        const bool first = kk == 0 && st == 0 && (F::SCALED || c == 0);
+                        umma_f16(d, dah + 2 * kk, dbh + 2 * kk, idesc, first ? 0u : 1u);
+                        umma_f16(d, dah + 2 * kk, dbh + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                        if (F::PLANES == 2) umma_f16(d, dah + (PG_A_BYTES >> 4) + 2 * kk, dbh + 2 * kk, idesc, 1u);
+                    }
+                    umma_commit(empty + 8 * slot);
+                }
+                __syncwarp();
+                if (++slot == S) {
+                    slot = 0;
+                    ph ^= 1;
+                }
+            }
+            if (F::MIN) {
+                mbar_wait(bmin_full + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                __syncwarp();
+            }
+            if (elect_one()) {
+                if (F::MIN)
+                    umma_f16(tmem + (2 + buf) * P.NTP, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NT * 32), idesc, 0u);
+                if (F::SCALED || c == nc - 1) umma_commit(dfull + 8 * buf);
+            }
+            if (F::SCALED || c == nc - 1) u++;
+            __syncwarp();
+        }
+    } else if (warp == 2) {
+        // ---- packed weights ----
+        if (lane == 0) {
+            int slot = 0, issued = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < P.tiles && ok; tile += tile_step) {
+                PgSeg sg;
+                int m0, n0;
+                tile_of(tile, sg, m0, n0);
+                const int nt = min(8, (sg.rows - m0 + 15) >> 4);  // 16-row tiles that exist
+                const uint8_t* src = sg.w + (long long)(m0 >> 4) * P.tile_bytes + (long long)c0 * F::STEP;
+                for (int c = 0; c < nc; c++) {
+                    if (!(ok = mbar_wait(pk_empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
+                    fence_async();  // the warps' reads of the block before come before the copy's writes
+                    mbar_expect_tx(pk_full + 8 * slot, (uint32_t)nt * F::STEP);
+                    for (int i = 0; i < nt; i++)
+                        bulk_load(sb + L.pack + (slot * 8 + i) * F::STEP, src + i * P.tile_bytes + (long long)c * F::STEP, F::STEP, pk_full + 8 * slot);
+                    issued++;
+                    if (++slot == PK) {
+                        slot = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            if (!ok) {
+                for (int i = max(0, issued - PK); i < issued; i++) {
+                    limit = P.wait_limit;
+                    mbar_wait(pk_full + 8 * (i % PK), (i / PK) & 1, limit, P.err_flag);
+                }
+            }
+        }
+    } else if (warp >= 4 && warp < 12) {
+        // ---- weights into operand rows ----
+        const int w8 = warp - 4, r16 = lane & 15, part = lane >> 4, r = 16 * w8 + r16;
+        uint32_t* scales = reinterpret_cast<uint32_t*>(smem + L.scale);
+        int slot = 0, ps = 0, c = 0;  // c: super-blocks so far
+        uint32_t ph = 0, pph = 0;
+        for (int tile = tile0; tile < P.tiles; tile += tile_step)
+        for (int i = 0; i < nc; i++, c++) {
+            mbar_wait(pk_full + 8 * ps, pph, limit, P.err_flag);
+            const unsigned char* blk = smem + L.pack + (ps * 8 + w8) * F::STEP;
+            if (F::MIN) {
+                if (c >= 2) mbar_wait(dfull + 8 * (c & 1), ((c >> 1) - 1) & 1, limit, P.err_flag);  // c - 2's product has read its operand
+                pfq::min_row(blk, r16, r, part, smem + L.amin + (c & 1) * PG_BM * 32);
+            }
+            if (F::SCALED) {
+                // (four super-blocks of scales: stages run at most one and a half ahead of the products, those at most two ahead of
+                // the readers)
+                if (part == 0) scales[(c & 3) * PG_BM + r] = pfq::row_scale<FMT>(blk, r16);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sc_full + 8 * (c & 3));
+            }
+#pragma unroll
+            for (int st = 0; st < F::STAGES; st++) {
+                pfq::Packed pk;
+                pfq::fetch<FMT>(blk, r16, part, st, pk);
+                mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag);
+                unsigned char* a = smem + L.a + slot * F::PLANES * PG_A_BYTES;
+                pfq::emit<FMT>(pk, r, part, st, a, a + PG_A_BYTES);
+                fence_async();  // these stores come before the tensor core's reads
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(full_a + 8 * slot);
+                    if (st == F::STAGES - 1) mbar_arrive(pk_empty + 8 * ps);
+                }
+                if (++slot == S) {
+                    slot = 0;
+                    ph ^= 1;
+                }
+            }
+            if (++ps == PK) {
+                ps = 0;
+                pph ^= 1;
+            }
+        }
+    } else if (warp >= 12) {
+        // ---- sums out of tensor memory ----
+        const uint32_t* scales = reinterpret_cast<const uint32_t*>(smem + L.scale);
+        int u = 0;
+        for (int tile = tile0; tile < P.tiles; tile += tile_step) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 16; j++) acc[i][j] = 0.f;
+            for (int c = F::SCALED ? 0 : nc - 1; c < nc; c++, u++) {
+                const int buf = u & 1;
+                float d = 1.f, mn = 0.f;
+                if (F::SCALED) {
+                    mbar_wait(sc_full + 8 * (u & 3), (u >> 2) & 1, limit, P.err_flag);
+                    const uint32_t dd = scales[(u & 3) * PG_BM + 32 * quad + lane];
+                    d = __half2float(__ushort_as_half((unsigned short)(dd & 0xFFFFu)));
+                    if (F::MIN) mn = -32.f * __half2float(__ushort_as_half((unsigned short)(dd >> 16)));  // the sums plane holds sums / 32
+                }
+                mbar_wait(dfull + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t t0 = tmem + ((uint32_t)(32 * quad) << 16) + buf * P.NTP;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int col = 16 * (2 * i + half);
+                    if (col < NT) {
+                        uint32_t v[16];
+                        tmem_ld16(t0 + col, v);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : __uint_as_float(v[j]);
+                        if (F::MIN) {
+                            tmem_ld16(t0 + 2 * P.NTP + col, v);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 16; j++) acc[i][j] = fmaf(mn, __uint_as_float(v[j]), acc[i][j]);
+                        }
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(dempty + 8 * buf);
+            }
+            if (P.ks > 1) break;  // one tile per cluster, stored below
+            PgSeg sg;
+            int m0, n0;
+            tile_of(tile, sg, m0, n0);
+            const int row = m0 + 32 * quad + lane;
+            if (row < sg.rows) {
+                const float bias = sg.bias ? sg.bias[row] : 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int t0 = n0 + 16 * (2 * i + half);
+                    if (16 * (2 * i + half) < NT && t0 < P.T) {
+                        float res[16];  // all residuals on their way before the first store (the output may be the residual)
+#pragma unroll
+                        for (int j = 0; j < 16; j++) res[j] = P.resid && t0 + j < P.T ? __ldcg(P.resid + (size_t)(t0 + j) * P.ldr + row) : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (t0 + j < P.T) sg.out[(size_t)(t0 + j) * P.ldo + row] = P.resid ? res[j] + (acc[i][j] + bias) : acc[i][j] + bias;
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- K split over a cluster ----
+    __syncwarp();
+    if (P.ks > 1) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        PgSeg sg;
+        int m0, n0;
+        tile_of(tile0, sg, m0, n0);
+        // every CTA leaves its sums [token][row] in its own shared memory (the operand planes are free: all products are done)
+        float* red = reinterpret_cast<float*>(smem);
+        if (warp >= 12) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int col = 16 * (2 * i + half) + j;
+                    if (col < NT) red[col * PG_BM + 32 * quad + lane] = acc[i][j];
+                }
+        }
+        cluster_sync();
+        const int lo = NT * rank / P.ks * PG_BM, hi = NT * (rank + 1) / P.ks * PG_BM;  // this CTA adds and stores a share of the tokens
+        for (int i = lo + tid; i < hi; i += PG_THREADS) {
+            const int t = n0 + i / PG_BM, m = m0 + i % PG_BM;
+            float y = 0.f;
+            for (int z = 0; z < P.ks; z++) y += ld_cluster(sb + 4 * i, z);
+            if (m < sg.rows && t < P.T) {
+                if (sg.bias) y += sg.bias[m];
+                if (P.resid) y = P.resid[(size_t)t * P.ldr + m] + y;
+                sg.out[(size_t)t * P.ldo + m] = y;
+            }
+        }
+        cluster_sync();  // no CTA leaves while another reads its sums
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+}
+
+// ---- host side ------------------------------------------------------------------------------------------------------
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// fp16 plane [rows][cols] row-major -> boxes of `box_cols` x `box_rows`, swizzled over rows of 128 (64 columns) or 32 bytes (16).
+int make_plane_map(slai_ctx* ctx, CUtensorMap* map, const __half* base, int rows, int cols, int box_cols, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    SLAI_REQUIRE(ctx, enc, SLAI_ERR_CUDA, "prefill: the driver does not provide cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(base), dims, strides, box, elem,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    SLAI_REQUIRE(ctx, r == CUDA_SUCCESS, SLAI_ERR_CUDA, "prefill: cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return SLAI_OK;
+}
+
+template <int FMT>
+int launch_fmt(slai_ctx* ctx, PgParams& P, int m_tiles, int n_tiles, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& sum) {
+    // K is split while that shortens the longest SM: its tiles one after the other, or one share of a tile plus about two
+    // super-blocks for its start and end in every round.
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    P.n_tiles = n_tiles;
+    P.tiles = m_tiles * n_tiles;
+    long long best = -1;
+    P.ks = 1;
+    for (int ks = 1; ks <= PG_MAX_KS && ks <= P.nch; ks *= 2) {
+        const long long rounds = ((long long)P.tiles * ks + sms - 1) / sms;
+        const long long cost = ks == 1 ? rounds * P.nch + 2 : rounds * ((P.nch + ks - 1) / ks + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            P.ks = ks;
+        }
+    }
+    // Packed blocks in flight first (three if two stages still fit beside them), then as many operand stages as fit.
+    P.packs = pg_layout<FMT>(P.NT, 3, 3).total <= PG_SMEM_LIMIT - 1024 ? 3 : 2;
+    P.stages = 2;
+    while (P.stages < PG_MAX_STAGES && pg_layout<FMT>(P.NT, P.stages + 1, P.packs).total <= PG_SMEM_LIMIT - 1024) P.stages++;
+    const size_t smem = pg_layout<FMT>(P.NT, P.stages, P.packs).total + 1024;
+    auto kern = prefill_gemm_kernel<FMT>;
+    static PerDeviceOnce attr;  // per instantiation
+    if (attr.need(ctx->device)) {
+        SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM_LIMIT));
+        attr.set(ctx->device);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(P.ks == 1 ? std::min(P.tiles, sms) : P.tiles * P.ks));
+    cfg.blockDim = dim3(PG_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (P.ks > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)P.ks;
+        at[n].val.clusterDim.y = 1;
+        at[n++].val.clusterDim.z = 1;
+    }
+    if (ctx->use_pdl) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, P, hi, lo, sum));
+    return SLAI_OK;
+}
+
+}  // namespace
+
+// Tokens per CTA tile of a prompt of T tokens: as few tiles as 128 tokens allow, of equal size (a multiple of 16).
+int prefill_gemm_nt(int T) {
+    const int tiles = (T + PG_MAX_NT - 1) / PG_MAX_NT;
+    return ((T + tiles - 1) / tiles + 15) / 16 * 16;
+}
+
+// out_i[t][m] = (resid[t][m] +) sum_k W_i[m][k] X[t][k] (+ bias_i[m]) for t < T and up to three matrices W_i of one format and
+// width that share the activations, given as hi / lo planes (and the sub-blocks' sums, see PrefillGemm) of `t_pad` rows.
+// Rows T .. t_pad - 1 of the planes may hold anything: a token's sums depend on its own row alone.
+int prefill_gemm_launch(slai_ctx* ctx, const PrefillGemm& G) {
+    SLAI_REQUIRE(ctx, G.n >= 1 && G.n <= 3 && G.w[0], SLAI_ERR_INVALID_ARG, "prefill: %d matrices in one launch", G.n);
+    const slai_qmatrix* w = G.w[0];
+    SLAI_REQUIRE(ctx, w->fmt == SLAI_FMT_Q4_K || w->fmt == SLAI_FMT_Q5_K || w->fmt == SLAI_FMT_Q6_K || w->fmt == SLAI_FMT_Q8_0,
+                 SLAI_ERR_UNSUPPORTED_FORMAT, "prefill: format %d has no GEMM path", w->fmt);
+    const int NT = prefill_gemm_nt(G.T), K = (int)w->ncols;
+    SLAI_REQUIRE(ctx, K % PG_BK == 0 && G.T >= 1 && G.t_pad % NT == 0 && G.T <= G.t_pad && (w->fmt == SLAI_FMT_Q8_0 || K % 256 == 0), SLAI_ERR_SHAPE,
+                 "prefill: K=%d / %d tokens not supported", K, G.T);
+    SLAI_REQUIRE(ctx, (w->fmt != SLAI_FMT_Q4_K && w->fmt != SLAI_FMT_Q5_K) || G.x_sum, SLAI_ERR_INVALID_ARG, "prefill: the minimum term needs the sub-block sums");
+    PgParams P = {};
+    int tiles = 0;
+    for (int i = 0; i < G.n; i++) {
+        SLAI_REQUIRE(ctx, G.w[i] && G.w[i]->fmt == w->fmt && G.w[i]->ncols == w->ncols && G.w[i]->tile_bytes == w->tile_bytes && G.rows[i] > 0 &&
+                              G.rows[i] <= G.w[i]->nrows,
+                     SLAI_ERR_SHAPE, "prefill: matrices of one launch must share format and width");
+        SLAI_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(G.w[i]->data) & 15) == 0 && w->tile_bytes % 16 == 0, SLAI_ERR_INVALID_ARG,
+                     "prefill: matrix data must be 16-byte aligned");
+        P.seg[i].w = G.w[i]->data;
+        P.seg[i].out = G.out[i];
+        P.seg[i].bias = G.bias[i];
+        P.seg[i].rows = G.rows[i];
+        P.seg[i].tile0 = tiles;
+        tiles += (G.rows[i] + PG_BM - 1) / PG_BM;
+    }
+    P.nseg = G.n;
+    P.tile_bytes = w->tile_bytes;
+    P.nch = (int)layout::num_steps(w->fmt, K);
+    P.T = G.T; P.NT = NT; P.ldo = G.ldo; P.resid = G.resid; P.ldr = G.ldr;
+    P.NTP = 16;
+    while (P.NTP < NT) P.NTP <<= 1;
+    P.err_flag = ctx->d_counters + CNT_ERR_FLAG;
+    P.wait_limit = ctx->wait_limit;
+    CUtensorMap hi, lo, sum;
+    int rc = make_plane_map(ctx, &hi, G.x_hi, G.t_pad, K, PG_BK, NT);
+    if (rc) return rc;
+    if ((rc = make_plane_map(ctx, &lo, G.x_lo, G.t_pad, K, PG_BK, NT))) return rc;
+    sum = hi;
+    if ((w->fmt == SLAI_FMT_Q4_K || w->fmt == SLAI_FMT_Q5_K) && (rc = make_plane_map(ctx, &sum, G.x_sum, G.t_pad, K / 16, 16, NT))) return rc;
+    switch (w->fmt) {
+        case SLAI_FMT_Q4_K: return launch_fmt<SLAI_FMT_Q4_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
+        case SLAI_FMT_Q5_K: return launch_fmt<SLAI_FMT_Q5_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
+        case SLAI_FMT_Q6_K: return launch_fmt<SLAI_FMT_Q6_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
+        default: return launch_fmt<SLAI_FMT_Q8_0>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
+    }
+}
