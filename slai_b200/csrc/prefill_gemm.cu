@@ -84,20 +84,50 @@ __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
                  : "memory");
     return ok != 0;
 }
+// The same for a barrier that the other CTA of a pair arrives on too.
+__device__ __forceinline__ bool mbar_try_cluster(uint32_t a, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(a), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
 // Bounded wait.  On expiry the error flag is raised and `limit` drops to one poll.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
     for (unsigned int i = 0; i < limit; i++) {
-        if (mbar_try(a, parity)) return true;
+        if (CLUSTER ? mbar_try_cluster(a, parity) : mbar_try(a, parity)) return true;
         if (i > 64) __nanosleep(40);
     }
     atomicExch(err_flag, 5u);
     limit = 1;
     return false;
 }
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {  // the same shared-memory address in another CTA of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+// Arrive on the barrier of the CTA that issues the products (a pair's first).  Default semantics (release at CTA scope): what the
+// arrival announces is read by the tensor core out of the writer's own shared memory, and the writer's proxy fence comes first; a
+// release at cluster scope held every operand writer for some 600 cycles per arrival.
+template <bool PAIR>
+__device__ __forceinline__ void arrive_issuer(uint32_t a) {
+    if (PAIR) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(map_rank(a, 0)) : "memory");
+    else mbar_arrive(a);
+}
+// Box at (x, y) into this CTA's shared memory; the bytes count on the issuing CTA's barrier.
+template <bool PAIR>
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-                 "l"(map), "r"(mbar), "r"(x), "r"(y)
-                 : "memory");
+    if (PAIR)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                     "l"(map), "r"(map_rank(mbar, 0)), "r"(x), "r"(y)
+                     : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                     "l"(map), "r"(mbar), "r"(x), "r"(y)
+                     : "memory");
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -116,15 +146,28 @@ __device__ __forceinline__ uint64_t desc32(uint32_t a) {
 }
 // Instruction descriptor, kind::f16: f32 accumulator (bits 4-5 = 1), A and B fp16 (0), both K-major (bits 15, 16 = 0),
 // N / 8 in bits 17-22, M / 16 in bits 24-28.
-__device__ __forceinline__ uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PG_BM >> 4) << 24); }
+__device__ __forceinline__ uint32_t umma_idesc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
+// Arrives on the barrier (a pair: on both CTAs') when everything issued so far has completed.
+template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+    if (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(mbar), "h"((unsigned short)3)
+                     : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
@@ -156,29 +199,36 @@ struct PgLayout {
     uint32_t a, b, amin, bmin, scale, pack, total;
 };
 template <int FMT>
-__host__ __device__ inline PgLayout pg_layout(int NT, int stages, int packs) {
+__host__ __device__ inline PgLayout pg_layout(int NB, int stages, int packs) {
     using F = pfq::Fmt<FMT>;
     PgLayout L;
     L.a = 0;
     L.b = L.a + (uint32_t)stages * F::PLANES * PG_A_BYTES;
-    L.amin = L.b + (uint32_t)stages * 2 * NT * PG_BK * 2;
+    L.amin = L.b + (uint32_t)stages * 2 * NB * PG_BK * 2;
     L.bmin = L.amin + (F::MIN ? 2 * PG_BM * 32 : 0);
-    L.scale = L.bmin + (F::MIN ? 2 * (uint32_t)NT * 32 : 0);
+    L.scale = L.bmin + (F::MIN ? 2 * (uint32_t)NB * 32 : 0);
     L.pack = L.scale + 4 * PG_BM * 4;
     L.total = L.pack + (uint32_t)packs * 8 * F::STEP;
     return L;
 }
 
-template <int FMT>
+// PG_PLAIN: one CTA, a product with each of the two activation planes.  PG_MERGED (at most 64 tokens): the planes lie one behind the
+// other and are one operand of twice the width, with sums of their own.  PG_PAIR: two CTAs of a cluster hold 128 rows each and
+// half of the tokens' operands each, one of them issues products of 256 rows (cta_group::2).
+enum { PG_PLAIN = 0, PG_MERGED = 1, PG_PAIR = 2 };
+
+template <int FMT, int MODE>
 __global__ void __launch_bounds__(PG_THREADS, 1)
 prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                     const __grid_constant__ CUtensorMap map_sum) {
     using F = pfq::Fmt<FMT>;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    const PgLayout L = pg_layout<FMT>(P.NT, P.stages, P.packs);
+    constexpr bool PAIR = MODE == PG_PAIR, MERGED = MODE == PG_MERGED;
+    const int NB = PAIR ? P.NT / 2 : P.NT;  // tokens whose operands this CTA holds
+    const PgLayout L = pg_layout<FMT>(NB, P.stages, P.packs);
     const int NT = P.NT, S = P.stages, PK = P.packs;
-    const uint32_t b_bytes = (uint32_t)NT * PG_BK * 2;  // one activation plane of a stage
+    const uint32_t b_bytes = (uint32_t)NB * PG_BK * 2;  // one activation plane of a stage
     __shared__ __align__(8) unsigned long long bars[3 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 10];
     __shared__ uint32_t tmem_slot;
     const uint32_t sb = smem_u32(smem);
@@ -187,8 +237,9 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                    dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform for the compiler too)
-    const int rank = P.ks > 1 ? (int)(blockIdx.x % P.ks) : 0;
-    const int tile0 = (int)blockIdx.x / P.ks, tile_step = (int)gridDim.x / P.ks;
+    const int pr = PAIR ? (int)(blockIdx.x & 1) : 0;  // rank in the pair
+    const int rank = !PAIR && P.ks > 1 ? (int)(blockIdx.x % P.ks) : 0;
+    const int tile0 = (int)blockIdx.x / (PAIR ? 2 : P.ks), tile_step = (int)gridDim.x / (PAIR ? 2 : P.ks);
     const int c0 = (int)((long long)P.nch * rank / P.ks), nc = (int)((long long)P.nch * (rank + 1) / P.ks) - c0;  // super-blocks of this CTA
     // a tile's matrix, first row in it and first token
     auto tile_of = [&](int tile, PgSeg& sg, int& m0, int& n0) {
@@ -197,12 +248,12 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         sg = P.seg[0];
         if (P.nseg > 1 && mt >= P.seg[1].tile0) sg = P.seg[1];
         if (P.nseg > 2 && mt >= P.seg[2].tile0) sg = P.seg[2];
-        m0 = (mt - sg.tile0) * PG_BM;
+        m0 = PAIR ? (mt - sg.tile0) * 2 * PG_BM + pr * PG_BM : (mt - sg.tile0) * PG_BM;
     };
 
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
-            mbar_init(full_a + 8 * s, 8);
+            mbar_init(full_a + 8 * s, PAIR ? 16 : 8);
             mbar_init(full_b + 8 * s, 1);
             mbar_init(empty + 8 * s, 1);
         }
@@ -212,21 +263,29 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         }
         for (int s = 0; s < 2; s++) {
             mbar_init(dfull + 8 * s, 1);
-            mbar_init(dempty + 8 * s, 8);
+            mbar_init(dempty + 8 * s, PAIR ? 16 : 8);
             mbar_init(bmin_full + 8 * s, 1);
         }
         for (int s = 0; s < 4; s++) mbar_init(sc_full + 8 * s, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async();
     }
+    // tensor memory: two buffers of sums, then two of the minimum term
+    const int DS = MERGED ? 2 * P.NTP : P.NTP;
     int ncols = 32;
-    while (ncols < (F::MIN ? 4 : 2) * P.NTP) ncols <<= 1;
+    while (ncols < 2 * DS + (F::MIN ? 2 * P.NTP : 0)) ncols <<= 1;
     if (warp == 1) {  // the MMA warp owns the tensor-memory allocation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(ncols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(ncols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(ncols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync();  // the other CTA's barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     unsigned int limit = P.wait_limit;
@@ -234,7 +293,8 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp < 2 || warp >= 12) asm volatile("griddepcontrol.wait;" ::: "memory");
     // readers of the sums (warps 12-19): 32 rows each, every other group of 16 tokens
-    float acc[4][16];
+    constexpr int NG = MERGED ? 2 : 4;
+    float acc[NG][16];
     const int quad = warp & 3, half = (warp - 12) >> 2;
 
     if (warp == 0) {
@@ -251,15 +311,15 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                     if (F::MIN) {
                         const int buf = gc & 1;
                         if (gc >= 2 && !(ok = mbar_wait(dfull + 8 * buf, ((gc >> 1) - 1) & 1, limit, P.err_flag))) break;
-                        mbar_expect_tx(bmin_full + 8 * buf, (uint32_t)NT * 32);
-                        tma_load_2d(sb + L.bmin + buf * NT * 32, &map_sum, 16 * (c0 + c), n0, bmin_full + 8 * buf);
+                        if (pr == 0) mbar_expect_tx(bmin_full + 8 * buf, (uint32_t)NT * 32);
+                        tma_load_2d<PAIR>(sb + L.bmin + buf * NB * 32, &map_sum, 16 * (c0 + c), n0 + pr * NB, bmin_full + 8 * buf);
                     }
                     for (int st = 0; st < F::STAGES; st++) {
                         if (!(ok = mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
                         const int x = ((c0 + c) * F::STAGES + st) * PG_BK;
-                        mbar_expect_tx(full_b + 8 * slot, 2 * b_bytes);
-                        tma_load_2d(sb + L.b + slot * 2 * b_bytes, &map_hi, x, n0, full_b + 8 * slot);
-                        tma_load_2d(sb + L.b + slot * 2 * b_bytes + b_bytes, &map_lo, x, n0, full_b + 8 * slot);
+                        if (pr == 0) mbar_expect_tx(full_b + 8 * slot, (PAIR ? 4 : 2) * b_bytes);
+                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes, &map_hi, x, n0 + pr * NB, full_b + 8 * slot);
+                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes + b_bytes, &map_lo, x, n0 + pr * NB, full_b + 8 * slot);
                         issued++;
                         if (++slot == S) {
                             slot = 0;
@@ -268,7 +328,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                     }
                 }
             }
-            if (!ok) {  // a wait ran out: this thread's own copies in flight land before the CTA may end
+            if (!ok && pr == 0) {  // a wait ran out: the copies in flight land before the CTA (the pair) may end
                 for (int i = max(0, issued - S); i < issued; i++) {
                     limit = P.wait_limit;
                     mbar_wait(full_b + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
@@ -276,19 +336,20 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
+        if (pr == 0) {
         // ---- tensor cores: the whole warp walks the loop, so that descriptors live in uniform registers, one lane issues ----
-        const uint32_t idesc = umma_idesc(NT);
+        const uint32_t idesc = umma_idesc(PAIR ? 2 * PG_BM : PG_BM, NT), idesc2 = umma_idesc(PG_BM, 2 * NT);
         const uint64_t da0 = desc128(sb + L.a), db0 = desc128(sb + L.b);
         int slot = 0, u = 0;  // u: sums so far (of a super-block; Q8_0: of a whole tile), alternately in two buffers
         uint32_t ph = 0;
         for (int tile = tile0; tile < P.tiles; tile += tile_step)
         for (int c = 0; c < nc; c++) {
             const int buf = u & 1;
-            const uint32_t d = tmem + buf * P.NTP;
-            if ((F::SCALED || c == 0) && u >= 2) mbar_wait(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
+            const uint32_t d = tmem + buf * DS;
+            if ((F::SCALED || c == 0) && u >= 2) mbar_wait<PAIR>(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
             for (int st = 0; st < F::STAGES; st++) {
-                mbar_wait(full_a + 8 * slot, ph, limit, P.err_flag);
-                mbar_wait(full_b + 8 * slot, ph, limit, P.err_flag);
+                mbar_wait<PAIR>(full_a + 8 * slot, ph, limit, P.err_flag);
+                mbar_wait<PAIR>(full_b + 8 * slot, ph, limit, P.err_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 __syncwarp();
                 // 16 elements = 32 bytes further along the swizzled row: 2 in the descriptor's units of 16 bytes
@@ -297,11 +358,15 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
 #pragma unroll
                     for (int kk = 0; kk < PG_BK / 16; kk++) {
                         const bool first = kk == 0 && st == 0 && (F::SCALED || c == 0);
-                        umma_f16(d, dah + 2 * kk, dbh + 2 * kk, idesc, first ? 0u : 1u);
-                        umma_f16(d, dah + 2 * kk, dbh + (b_bytes >> 4) + 2 * kk, idesc, 1u);
-                        if (F::PLANES == 2) umma_f16(d, dah + (PG_A_BYTES >> 4) + 2 * kk, dbh + 2 * kk, idesc, 1u);
+                        if (MERGED) {
+                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + 2 * kk, idesc2, first ? 0u : 1u);
+                        } else {
+                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + 2 * kk, idesc, first ? 0u : 1u);
+                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                        }
+                        if (F::PLANES == 2) umma_f16<PAIR>(d, dah + (PG_A_BYTES >> 4) + 2 * kk, dbh + 2 * kk, idesc, 1u);
                     }
-                    umma_commit(empty + 8 * slot);
+                    umma_commit<PAIR>(empty + 8 * slot);
                 }
                 __syncwarp();
                 if (++slot == S) {
@@ -310,17 +375,18 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
             }
             if (F::MIN) {
-                mbar_wait(bmin_full + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
+                mbar_wait<PAIR>(bmin_full + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 __syncwarp();
             }
             if (elect_one()) {
                 if (F::MIN)
-                    umma_f16(tmem + (2 + buf) * P.NTP, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NT * 32), idesc, 0u);
-                if (F::SCALED || c == nc - 1) umma_commit(dfull + 8 * buf);
+                    umma_f16<PAIR>(tmem + 2 * DS + buf * P.NTP, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NB * 32), idesc, 0u);
+                if (F::SCALED || c == nc - 1) umma_commit<PAIR>(dfull + 8 * buf);
             }
             if (F::SCALED || c == nc - 1) u++;
             __syncwarp();
+        }
         }
     } else if (warp == 2) {
         // ---- packed weights ----
@@ -332,7 +398,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 PgSeg sg;
                 int m0, n0;
                 tile_of(tile, sg, m0, n0);
-                const int nt = min(8, (sg.rows - m0 + 15) >> 4);  // 16-row tiles that exist
+                const int nt = max(0, min(8, (sg.rows - m0 + 15) >> 4));  // 16-row tiles that exist
                 const uint8_t* src = sg.w + (long long)(m0 >> 4) * P.tile_bytes + (long long)c0 * F::STEP;
                 for (int c = 0; c < nc; c++) {
                     if (!(ok = mbar_wait(pk_empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
@@ -375,18 +441,29 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sc_full + 8 * (c & 3));
             }
+            // two stages at a time: a warp's way through one is a chain of latencies (load, arithmetic, store, fence, arrive)
 #pragma unroll
-            for (int st = 0; st < F::STAGES; st++) {
-                pfq::Packed pk;
-                pfq::fetch<FMT>(blk, r16, part, st, pk);
-                mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag);
-                unsigned char* a = smem + L.a + slot * F::PLANES * PG_A_BYTES;
-                pfq::emit<FMT>(pk, r, part, st, a, a + PG_A_BYTES);
+            for (int st = 0; st < F::STAGES; st += 2) {
+                pfq::Packed pk[2];
+                pfq::fetch<FMT>(blk, r16, part, st, pk[0]);
+                pfq::fetch<FMT>(blk, r16, part, st + 1, pk[1]);
+                const int slot0 = slot;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag);
+                    unsigned char* a = smem + L.a + slot * F::PLANES * PG_A_BYTES;
+                    pfq::emit<FMT>(pk[k], r, part, st + k, a, a + PG_A_BYTES);
+                    if (k == 0 && ++slot == S) {
+                        slot = 0;
+                        ph ^= 1;
+                    }
+                }
                 fence_async();  // these stores come before the tensor core's reads
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(full_a + 8 * slot);
-                    if (st == F::STAGES - 1) mbar_arrive(pk_empty + 8 * ps);
+                    arrive_issuer<PAIR>(full_a + 8 * slot0);
+                    arrive_issuer<PAIR>(full_a + 8 * slot);
+                    if (st == F::STAGES - 2) mbar_arrive(pk_empty + 8 * ps);
                 }
                 if (++slot == S) {
                     slot = 0;
@@ -404,7 +481,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         int u = 0;
         for (int tile = tile0; tile < P.tiles; tile += tile_step) {
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < NG; i++)
 #pragma unroll
                 for (int j = 0; j < 16; j++) acc[i][j] = 0.f;
             for (int c = F::SCALED ? 0 : nc - 1; c < nc; c++, u++) {
@@ -419,9 +496,9 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 mbar_wait(dfull + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
                 __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t t0 = tmem + ((uint32_t)(32 * quad) << 16) + buf * P.NTP;
+                const uint32_t tq = tmem + ((uint32_t)(32 * quad) << 16), t0 = tq + buf * DS;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
+                for (int i = 0; i < NG; i++) {
                     const int col = 16 * (2 * i + half);
                     if (col < NT) {
                         uint32_t v[16];
@@ -429,8 +506,14 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : __uint_as_float(v[j]);
+                        if (MERGED) {
+                            tmem_ld16(t0 + NT + col, v);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : acc[i][j] + __uint_as_float(v[j]);
+                        }
                         if (F::MIN) {
-                            tmem_ld16(t0 + 2 * P.NTP + col, v);
+                            tmem_ld16(tq + 2 * DS + buf * P.NTP + col, v);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                             for (int j = 0; j < 16; j++) acc[i][j] = fmaf(mn, __uint_as_float(v[j]), acc[i][j]);
@@ -439,9 +522,9 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(dempty + 8 * buf);
+                if (lane == 0) arrive_issuer<PAIR>(dempty + 8 * buf);
             }
-            if (P.ks > 1) break;  // one tile per cluster, stored below
+            if (!PAIR && P.ks > 1) break;  // one tile per cluster, stored below
             PgSeg sg;
             int m0, n0;
             tile_of(tile, sg, m0, n0);
@@ -449,7 +532,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             if (row < sg.rows) {
                 const float bias = sg.bias ? sg.bias[row] : 0.f;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
+                for (int i = 0; i < NG; i++) {
                     const int t0 = n0 + 16 * (2 * i + half);
                     if (16 * (2 * i + half) < NT && t0 < P.T) {
                         float res[16];  // all residuals on their way before the first store (the output may be the residual)
@@ -466,7 +549,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
 
     // ---- K split over a cluster ----
     __syncwarp();
-    if (P.ks > 1) {
+    if (!PAIR && P.ks > 1) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         PgSeg sg;
         int m0, n0;
@@ -475,7 +558,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         float* red = reinterpret_cast<float*>(smem);
         if (warp >= 12) {
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < NG; i++)
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const int col = 16 * (2 * i + half) + j;
@@ -498,7 +581,11 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+    if (PAIR) cluster_sync();  // neither CTA leaves while the other reads its operands or arrives on its barriers
+    if (warp == 1) {
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+    }
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------
@@ -531,44 +618,38 @@ int make_plane_map(slai_ctx* ctx, CUtensorMap* map, const __half* base, int rows
     return SLAI_OK;
 }
 
-template <int FMT>
-int launch_fmt(slai_ctx* ctx, PgParams& P, int m_tiles, int n_tiles, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& sum) {
-    // K is split while that shortens the longest SM: its tiles one after the other, or one share of a tile plus about two
-    // super-blocks for its start and end in every round.
-    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    P.n_tiles = n_tiles;
-    P.tiles = m_tiles * n_tiles;
-    long long best = -1;
-    P.ks = 1;
-    for (int ks = 1; ks <= PG_MAX_KS && ks <= P.nch; ks *= 2) {
-        const long long rounds = ((long long)P.tiles * ks + sms - 1) / sms;
-        const long long cost = ks == 1 ? rounds * P.nch + 2 : rounds * ((P.nch + ks - 1) / ks + 2);
-        if (best < 0 || cost < best) {
-            best = cost;
-            P.ks = ks;
-        }
+template <int FMT, int MODE>
+int launch_mode(slai_ctx* ctx, PgParams& P, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& sum) {
+    const int NB = MODE == PG_PAIR ? P.NT / 2 : P.NT;
+    const int cluster = MODE == PG_PAIR ? 2 : P.ks, rows = MODE == PG_PAIR ? 2 * PG_BM : PG_BM;
+    int tiles = 0;
+    for (int i = 0; i < P.nseg; i++) {
+        P.seg[i].tile0 = tiles;
+        tiles += (P.seg[i].rows + rows - 1) / rows;
     }
+    P.tiles = tiles * P.n_tiles;
     // Packed blocks in flight first (three if two stages still fit beside them), then as many operand stages as fit.
-    P.packs = pg_layout<FMT>(P.NT, 3, 3).total <= PG_SMEM_LIMIT - 1024 ? 3 : 2;
+    P.packs = pg_layout<FMT>(NB, 3, 3).total <= PG_SMEM_LIMIT - 1024 ? 3 : 2;
     P.stages = 2;
-    while (P.stages < PG_MAX_STAGES && pg_layout<FMT>(P.NT, P.stages + 1, P.packs).total <= PG_SMEM_LIMIT - 1024) P.stages++;
-    const size_t smem = pg_layout<FMT>(P.NT, P.stages, P.packs).total + 1024;
-    auto kern = prefill_gemm_kernel<FMT>;
+    while (P.stages < PG_MAX_STAGES && pg_layout<FMT>(NB, P.stages + 1, P.packs).total <= PG_SMEM_LIMIT - 1024) P.stages++;
+    const size_t smem = pg_layout<FMT>(NB, P.stages, P.packs).total + 1024;
+    auto kern = prefill_gemm_kernel<FMT, MODE>;
     static PerDeviceOnce attr;  // per instantiation
     if (attr.need(ctx->device)) {
         SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM_LIMIT));
         attr.set(ctx->device);
     }
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(P.ks == 1 ? std::min(P.tiles, sms) : P.tiles * P.ks));
+    cfg.gridDim = dim3((unsigned)(MODE != PG_PAIR && P.ks > 1 ? P.tiles * P.ks : std::min(P.tiles, sms / cluster) * cluster));
     cfg.blockDim = dim3(PG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at[2];
     int n = 0;
-    if (P.ks > 1) {
+    if (cluster > 1) {
         at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = (unsigned)P.ks;
+        at[n].val.clusterDim.x = (unsigned)cluster;
         at[n].val.clusterDim.y = 1;
         at[n++].val.clusterDim.z = 1;
     }
@@ -580,6 +661,43 @@ int launch_fmt(slai_ctx* ctx, PgParams& P, int m_tiles, int n_tiles, const CUten
     cfg.numAttrs = n;
     SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, P, hi, lo, sum));
     return SLAI_OK;
+}
+
+template <int FMT>
+int launch_fmt(slai_ctx* ctx, PgParams& P, const PrefillGemm& G) {
+    // What the longest SM has to do, in units of a plain super-block: its tiles one after the other, alone or as one of a pair
+    // (a pair's super-block takes about two thirds of the time, measured at 128 tokens: half the activations' L2 and shared-
+    // memory traffic per SM), or a share of K of one tile, plus about two for its start and end, in every round.
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    auto m_tiles = [&](int rows) {
+        int t = 0;
+        for (int i = 0; i < P.nseg; i++) t += (P.seg[i].rows + rows - 1) / rows;
+        return t;
+    };
+    const long long tiles = (long long)m_tiles(PG_BM) * P.n_tiles, pairs = (long long)m_tiles(2 * PG_BM) * P.n_tiles;
+    double best = -1;
+    P.ks = 1;
+    for (int ks = 1; ks <= PG_MAX_KS && ks <= P.nch; ks *= 2) {
+        const long long rounds = (tiles * ks + sms - 1) / sms;
+        const double cost = ks == 1 ? (double)rounds * P.nch + 2 : (double)rounds * ((P.nch + ks - 1) / ks + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            P.ks = ks;
+        }
+    }
+    const bool merged = P.NT <= 64;
+    const bool pair = !merged && (double)((pairs + sms / 2 - 1) / (sms / 2)) * P.nch * 0.65 + 2 < best;
+    if (pair) P.ks = 1;
+    const int NB = pair ? P.NT / 2 : P.NT, K = (int)G.w[0]->ncols;
+    CUtensorMap hi, lo, sum;
+    int rc = make_plane_map(ctx, &hi, G.x_hi, G.t_pad, K, PG_BK, NB);
+    if (rc) return rc;
+    if ((rc = make_plane_map(ctx, &lo, G.x_lo, G.t_pad, K, PG_BK, NB))) return rc;
+    sum = hi;
+    if (pfq::Fmt<FMT>::MIN && (rc = make_plane_map(ctx, &sum, G.x_sum, G.t_pad, K / 16, 16, NB))) return rc;
+    if (pair) return launch_mode<FMT, PG_PAIR>(ctx, P, hi, lo, sum);
+    if (merged) return launch_mode<FMT, PG_MERGED>(ctx, P, hi, lo, sum);
+    return launch_mode<FMT, PG_PLAIN>(ctx, P, hi, lo, sum);
 }
 
 }  // namespace
@@ -603,7 +721,6 @@ int prefill_gemm_launch(slai_ctx* ctx, const PrefillGemm& G) {
                  "prefill: K=%d / %d tokens not supported", K, G.T);
     SLAI_REQUIRE(ctx, (w->fmt != SLAI_FMT_Q4_K && w->fmt != SLAI_FMT_Q5_K) || G.x_sum, SLAI_ERR_INVALID_ARG, "prefill: the minimum term needs the sub-block sums");
     PgParams P = {};
-    int tiles = 0;
     for (int i = 0; i < G.n; i++) {
         SLAI_REQUIRE(ctx, G.w[i] && G.w[i]->fmt == w->fmt && G.w[i]->ncols == w->ncols && G.w[i]->tile_bytes == w->tile_bytes && G.rows[i] > 0 &&
                               G.rows[i] <= G.w[i]->nrows,
@@ -614,27 +731,19 @@ int prefill_gemm_launch(slai_ctx* ctx, const PrefillGemm& G) {
         P.seg[i].out = G.out[i];
         P.seg[i].bias = G.bias[i];
         P.seg[i].rows = G.rows[i];
-        P.seg[i].tile0 = tiles;
-        tiles += (G.rows[i] + PG_BM - 1) / PG_BM;
     }
     P.nseg = G.n;
     P.tile_bytes = w->tile_bytes;
     P.nch = (int)layout::num_steps(w->fmt, K);
-    P.T = G.T; P.NT = NT; P.ldo = G.ldo; P.resid = G.resid; P.ldr = G.ldr;
+    P.T = G.T; P.NT = NT; P.n_tiles = G.t_pad / NT; P.ldo = G.ldo; P.resid = G.resid; P.ldr = G.ldr;
     P.NTP = 16;
     while (P.NTP < NT) P.NTP <<= 1;
     P.err_flag = ctx->d_counters + CNT_ERR_FLAG;
     P.wait_limit = ctx->wait_limit;
-    CUtensorMap hi, lo, sum;
-    int rc = make_plane_map(ctx, &hi, G.x_hi, G.t_pad, K, PG_BK, NT);
-    if (rc) return rc;
-    if ((rc = make_plane_map(ctx, &lo, G.x_lo, G.t_pad, K, PG_BK, NT))) return rc;
-    sum = hi;
-    if ((w->fmt == SLAI_FMT_Q4_K || w->fmt == SLAI_FMT_Q5_K) && (rc = make_plane_map(ctx, &sum, G.x_sum, G.t_pad, K / 16, 16, NT))) return rc;
     switch (w->fmt) {
-        case SLAI_FMT_Q4_K: return launch_fmt<SLAI_FMT_Q4_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
-        case SLAI_FMT_Q5_K: return launch_fmt<SLAI_FMT_Q5_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
-        case SLAI_FMT_Q6_K: return launch_fmt<SLAI_FMT_Q6_K>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
-        default: return launch_fmt<SLAI_FMT_Q8_0>(ctx, P, tiles, G.t_pad / NT, hi, lo, sum);
+        case SLAI_FMT_Q4_K: return launch_fmt<SLAI_FMT_Q4_K>(ctx, P, G);
+        case SLAI_FMT_Q5_K: return launch_fmt<SLAI_FMT_Q5_K>(ctx, P, G);
+        case SLAI_FMT_Q6_K: return launch_fmt<SLAI_FMT_Q6_K>(ctx, P, G);
+        default: return launch_fmt<SLAI_FMT_Q8_0>(ctx, P, G);
     }
 }
