@@ -18,7 +18,7 @@ using namespace attn;
 
 namespace {
 
-template <typename T, int MAXQ>
+template <typename T, int MAXQ, int HSF>
 __global__ void __launch_bounds__(ATT_THREADS, SLAI_ATT_MINB) attn_kernel(const AttnParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
 #ifdef SLAI_TRACE
@@ -45,11 +45,11 @@ __global__ void __launch_bounds__(ATT_THREADS, SLAI_ATT_MINB) attn_kernel(const 
         Q.vc = reinterpret_cast<const char*>(P.vc) + (size_t)b * P.cache_bs;
         const int n = (P.seq_pos ? __ldcg(P.seq_pos + b) : P.pos0 + b) + 1;
         const int ns = n > 0 ? attn_splits(Q, n) : 0;  // a sequence left out of the step (negative position): nothing to do
-        if ((int)blockIdx.y < ns) attn_item<T, MAXQ>(Q, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
+        if ((int)blockIdx.y < ns) attn_item<T, MAXQ, HSF>(Q, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
     } else {
         const int n = __ldcg(P.d_pos) + 1;
         const int ns = attn_splits(P, n);
-        if ((int)blockIdx.y < ns) attn_item<T, MAXQ>(P, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
+        if ((int)blockIdx.y < ns) attn_item<T, MAXQ, HSF>(P, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
     }
 #ifdef SLAI_TRACE
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && P.tl) {
@@ -62,9 +62,9 @@ __global__ void __launch_bounds__(ATT_THREADS, SLAI_ATT_MINB) attn_kernel(const 
 #endif
 }
 
-template <typename T, int MAXQ>
-int launch_t(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pdl) {
-    auto kern = attn_kernel<T, MAXQ>;
+template <typename T, int MAXQ, int HSF>
+int launch_hs(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pdl) {
+    auto kern = attn_kernel<T, MAXQ, HSF>;
     static PerDeviceOnce attr;
     if (attr.need(ctx->device)) {
         SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
@@ -86,6 +86,17 @@ int launch_t(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pdl
     cfg.numAttrs = pdl ? 1 : 0;
     SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, P));
     return SLAI_OK;
+}
+
+// Heads of 128 with 16-byte aligned rows keep keys and values in registers (attn_item); at most two query heads each.  Heads of 64
+// do not: twice as many lane groups share a split, each with half as much to do (GPT-2 XL, position 127: 1548 against 1516 us
+// per token).
+template <typename T, int MAXQ>
+int launch_t(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pdl) {
+    if constexpr (MAXQ <= 2) {
+        if (P.vec16 && P.hs == 128) return launch_hs<T, MAXQ, 128>(ctx, P, n_kv, smem, pdl);
+    }
+    return launch_hs<T, MAXQ, 0>(ctx, P, n_kv, smem, pdl);
 }
 
 }  // namespace
@@ -129,6 +140,9 @@ static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, 
                            (uintptr_t)(P.head_stride * esz) | (uintptr_t)(P.hs * esz);
     SLAI_REQUIRE(ctx, (bits & 3) == 0, SLAI_ERR_INVALID_ARG, "attention: caches and strides must be 4-byte aligned");
     P.vec16 = (bits & 15) == 0;
+    // The register path of f32 caches: splits of 32 positions, not of one staged tile (16) -- at position 515 that is one round of
+    // blocks instead of two, and half of the partial outputs to merge.
+    if (P.vec16 && P.hs == 128 && P.kv_mul <= 2 && esz == 4) P.tile_pos = 32;
     *smem = attn_item_bytes(P.kv_mul, P.hs, esz, P.tile_pos, P.n_splits);
     SLAI_REQUIRE(ctx, *smem <= 160 * 1024, SLAI_ERR_SHAPE, "attention: shared memory %zu too large", *smem);
     return SLAI_OK;

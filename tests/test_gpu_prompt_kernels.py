@@ -1,0 +1,89 @@
+"""The prompt pass's GEMM variants and its tensor-core attention at the edges of their tiles, and the decode attention whose keys and
+values stay in registers: against the sequential pass and against 64-bit arithmetic."""
+import numpy as np
+import pytest
+
+from slai_b200 import synth, _lib
+from slai_b200.models import Llama2Config, llama_from_host, synthetic_llama_host
+from slai_b200.ops import BatchedMultiqueryAttentionParams, GpuQuantMatrix
+from helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+# Tokens: up to 64 the two planes of the activations are one operand, above two CTAs share a tile or K is split over a cluster; one
+# past a tile, ragged last tiles, several tiles per CTA.  768 columns and 192 rows (k, v): a matrix that ends inside a CTA's rows.
+@pytest.mark.parametrize("fmt", [synth.FMT_Q4_K, synth.FMT_Q5_K, synth.FMT_Q6_K, synth.FMT_Q8_0])
+@pytest.mark.parametrize("T", [16, 17, 64, 65, 129, 300, 1200])
+def test_prompt_pass_at_the_edges_of_its_tiles(backend, monkeypatch, fmt, T):
+    cfg = Llama2Config(dim=768, hidden_dim=1280, n_layers=1, n_q_heads=12, n_kv_heads=3, vocab_size=300, seq_len=1240, kv_dtype=_lib.KV_F32)
+    w = synthetic_llama_host(cfg, fmt, fmt, seed=T, std=0.05, embd_std=1.0)
+    batched, seq = llama_from_host(backend, cfg, w, fmt, fmt), llama_from_host(backend, cfg, w, fmt, fmt)
+    prompt = np.random.default_rng(T).integers(0, cfg.vocab_size, size=T).astype(np.int32)
+    got = batched.prefill(prompt, 0, want_logits=True)
+    monkeypatch.setenv("SLAI_PREFILL_SEQUENTIAL", "1")
+    want = seq.prefill(prompt, 0, want_logits=True)
+    kb, vb = batched.read_kv(0, T)
+    ks, vs = seq.read_kv(0, T)
+    # operands of 22 bits (2^-22 of each, both planes of both factors at most) and f32 sums of at most 5 blocks of 256: below 1e-5
+    assert rel_l2(kb, ks) < 1e-5 and rel_l2(vb, vs) < 1e-5, (rel_l2(kb, ks), rel_l2(vb, vs))
+    for t in {0, T // 2, T - 1}:  # every token on its own, the last row of every head included
+        assert rel_l2(kb[t], ks[t]) < 2e-5 and rel_l2(vb[t], vs[t]) < 2e-5
+    assert rel_l2(got, want) < 1e-4  # one layer and the logits product
+
+
+# The tensor-core attention (f16 cache, heads of 64 and 128): query tiles of 64, position tiles of 64, a first position inside a tile.
+@pytest.mark.parametrize("heads,kv_heads", [(8, 8), (16, 4)])  # head size 128, 64
+@pytest.mark.parametrize("pos,T", [(0, 16), (0, 63), (0, 65), (48, 17), (64, 64), (5, 200)])
+def test_prompt_attention_on_the_tensor_cores(backend, monkeypatch, heads, kv_heads, pos, T):
+    cfg = Llama2Config(dim=1024, hidden_dim=1024, n_layers=1, n_q_heads=heads, n_kv_heads=kv_heads, vocab_size=300, seq_len=256, kv_dtype=_lib.KV_F16)
+    w = synthetic_llama_host(cfg, synth.FMT_Q8_0, synth.FMT_Q8_0, seed=3, std=0.08, embd_std=1.0)
+    batched, seq = (llama_from_host(backend, cfg, w, synth.FMT_Q8_0, synth.FMT_Q8_0) for _ in range(2))
+    ids = np.random.default_rng(pos + T).integers(0, cfg.vocab_size, size=pos + T).astype(np.int32)
+    monkeypatch.setenv("SLAI_PREFILL_SEQUENTIAL", "1")
+    want = seq.prefill(ids, 0, want_logits=True)
+    if pos:
+        batched.prefill(ids[:pos], 0)
+    monkeypatch.delenv("SLAI_PREFILL_SEQUENTIAL")
+    got = batched.prefill(ids[pos:], pos, want_logits=True)
+    # a cached value may round to the other of two neighbouring halves (2^-11) where the passes differ in the last bits of f32
+    assert rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("hs", [64, 128])
+@pytest.mark.parametrize("kv_dtype", [_lib.KV_F16, _lib.KV_F32])
+@pytest.mark.parametrize("heads,kv_heads", [(4, 4), (4, 2), (6, 2), (8, 1)])
+def test_decode_attention_in_registers(backend, ctx, hs, kv_dtype, heads, kv_heads):
+    """One query token; positions at the edges of a group's share, of a batch of loads and of a split."""
+    n = 2200
+    rng = np.random.default_rng(hs + heads)
+    dt = np.float16 if kv_dtype == _lib.KV_F16 else np.float32
+    k, v = (rng.standard_normal((n, kv_heads, hs)).astype(dt) for _ in range(2))
+    q = (2 * rng.standard_normal((heads, hs))).astype(np.float32)
+    dk, dv, dq, out = backend.vector(k.ravel(), dt), backend.vector(v.ravel(), dt), backend.vector(q.ravel()), backend.zeros(heads * hs)
+    for pos in (0, 1, 7, 8, 15, 16, 31, 32, 33, 64, 515, 2047, 2048, n - 1):
+        p = BatchedMultiqueryAttentionParams(seq_len=n, kv_dim=kv_heads * hs, kv_mul=heads // kv_heads, n_heads=heads, head_size=hs, pos=pos)
+        ctx.attention(p, dq, dk, dv, out, kv_dtype)
+        got = out.to_numpy().reshape(heads, hs)
+        for h in range(heads):
+            K, V = k[:pos + 1, h // (heads // kv_heads)].astype(np.float64), v[:pos + 1, h // (heads // kv_heads)].astype(np.float64)
+            s = K @ q[h].astype(np.float64) / np.sqrt(hs)
+            e = np.exp(s - s.max())
+            # f32 scores of up to ~25 are off by a few 2^-24 of that, the exponentials by as much relative: below 1e-5
+            assert rel_l2(got[h], e @ V / e.sum()) < 1e-5, (pos, h)
+
+
+def test_gemv_right_after_its_matrix_was_uploaded(backend, ctx):
+    """Consecutive products start behind one another's start and request their weights early: not before an upload is done."""
+    rng = np.random.default_rng(2)
+    M = K = 1024
+    x = rng.standard_normal(K).astype(np.float32)
+    for i in range(4):
+        w = synth.normal_matrix(i, M, K)
+        m = GpuQuantMatrix(backend, synth.FMT_Q8_0, M, K, synth.quantize(synth.FMT_Q8_0, w))
+        a, b, c = backend.vector(x), backend.zeros(M), backend.zeros(M)
+        ctx.matmul_quant_assign(b, m, a)
+        ctx.matmul_quant_assign(c, m, b)  # consumes the product before it
+        W = w.reshape(M, K).astype(np.float64)
+        assert rel_l2(b.to_numpy(), W @ x) < 1e-2  # Q8_0's own rounding
+        assert rel_l2(c.to_numpy(), W @ b.to_numpy().astype(np.float64)) < 1e-2
