@@ -17,6 +17,7 @@
 namespace {
 
 constexpr int ST = 1024;
+constexpr int REGS = 32;         // values per thread kept in registers between the passes
 constexpr int SORT_SMEM = 4096;  // candidates sorted in shared memory; more go through the global scratch
 
 struct SampleParams {  // device-resident (the generate graph reads them from memory)
@@ -71,23 +72,37 @@ __device__ __forceinline__ float block_max(float v, float* sh) {
     return m;
 }
 
-// ascending bitonic sort of `n2` (a power of two) 64-bit keys
+// Ascending bitonic sort of `n2` (a power of two) 64-bit keys.  Exchanges across 128 keys or more are the block's; nearer ones stay
+// inside segments of 128 keys, one warp each, without a block barrier: 21 barriers instead of 78 for 4096 keys.
+__device__ __forceinline__ void exchange(unsigned long long* keys, int i, int p, int k) {
+    const unsigned long long a = keys[i], b = keys[p];
+    if ((a > b) == ((i & k) == 0)) {
+        keys[i] = b;
+        keys[p] = a;
+    }
+}
 __device__ void bitonic_sort(unsigned long long* keys, int n2) {
-    for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n2; i += ST) {
-                const int p = i ^ j;
-                if (p > i) {
-                    const unsigned long long a = keys[i], b = keys[p];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        keys[i] = b;
-                        keys[p] = a;
-                    }
-                }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seg = min(n2, 128);
+    for (int k = 2; k <= n2; k <<= 1) {
+        int j = k >> 1;
+        for (; j >= 128; j >>= 1) {
+            for (int q = threadIdx.x; q < n2 / 2; q += ST) {
+                const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
+                exchange(keys, i, i | j, k);
             }
             __syncthreads();
         }
+        for (int s0 = warp * seg; s0 < n2; s0 += (ST / 32) * seg)
+            for (int jj = j; jj > 0; jj >>= 1) {
+                for (int q = lane; q < seg / 2; q += 32) {
+                    const int i = s0 + (((q & ~(jj - 1)) << 1) | (q & (jj - 1)));
+                    exchange(keys, i, i | jj, k);
+                }
+                __syncwarp();
+            }
+        if (k >= 128) __syncthreads();  // the next round reaches across segments
+    }
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(ST) sample_kernel(float* logits, int n, const SampleParams* sp, const int* d_step, float host_coin,
@@ -124,39 +139,75 @@ __global__ void __launch_bounds__(ST) sample_kernel(float* logits, int n, const 
         const unsigned long long h = mix64(sp->seed + (unsigned long long)(d_step ? *d_step : 0));
         coin = (float)((h >> 40) & 0xFFFFFFull) * (1.0f / 16777216.0f);
     }
+    // Up to 32 values per thread (32768 entries) stay in registers between the passes: read from memory in every one of them, each
+    // pass was a chain of 32 dependent trips (32000 entries, top-p: 157 us).
+    const bool reg = C <= REGS;
+    float x[REGS];
+    const bool quads = reg && i1 - i0 == REGS && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+    if (quads) {
+#pragma unroll
+        for (int k = 0; k < REGS; k += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(logits + i0 + k);
+            x[k] = v.x; x[k + 1] = v.y; x[k + 2] = v.z; x[k + 3] = v.w;
+        }
+    } else if (reg) {
+#pragma unroll
+        for (int k = 0; k < REGS; k++) x[k] = i0 + k < i1 ? logits[i0 + k] : 0.f;
+    }
+    // f(index, value) over this thread's chunk in index order; a value may be changed
+    auto each = [&](auto f) {
+        if (reg) {
+#pragma unroll
+            for (int k = 0; k < REGS; k++)
+                if (i0 + k < i1) f(i0 + k, x[k]);
+        } else {
+            for (int i = i0; i < i1; i++) {
+                float v = logits[i];
+                const float was = v;
+                f(i, v);
+                if (__float_as_uint(v) != __float_as_uint(was)) logits[i] = v;
+            }
+        }
+    };
     // probabilities (written over the logits, as the reference does)
     float mx = -INFINITY;
-    for (int i = i0; i < i1; i++) {
-        const float x = logits[i] / temperature;
-        logits[i] = x;
-        mx = fmaxf(mx, x);
-    }
+    each([&](int, float& v) {
+        v = v / temperature;
+        mx = fmaxf(mx, v);
+    });
     mx = block_max(mx, shf);
     float local = 0.f;
-    for (int i = i0; i < i1; i++) {
-        const float e = expf(logits[i] - mx);
-        logits[i] = e;
-        local += e;
-    }
+    each([&](int, float& v) {
+        v = expf(v - mx);
+        local += v;
+    });
     float sum;
     block_excl_scan(local, shf, sum);
     local = 0.f;
-    for (int i = i0; i < i1; i++) {
-        const float p = logits[i] / sum;
-        logits[i] = p;
-        local += p;
+    each([&](int, float& v) {
+        v = v / sum;
+        local += v;
+    });
+    if (quads) {
+#pragma unroll
+        for (int k = 0; k < REGS; k += 4) *reinterpret_cast<float4*>(logits + i0 + k) = make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+    } else if (reg) {
+#pragma unroll
+        for (int k = 0; k < REGS; k++)
+            if (i0 + k < i1) logits[i0 + k] = x[k];
     }
     if (tid == 0) s_idx = 0x7fffffff;
     if (topp <= 0.0f || topp >= 1.0f) {  // sample_mult: first index whose inclusive prefix exceeds the coin
         float total;
         float cdf = block_excl_scan(local, shf, total);
-        for (int i = i0; i < i1; i++) {
-            cdf += logits[i];
-            if (coin < cdf) {
+        bool found = false;
+        each([&](int i, float& v) {
+            cdf += v;
+            if (!found && coin < cdf) {
                 atomicMin(&s_idx, i);
-                break;
+                found = true;
             }
-        }
+        });
         __syncthreads();
         if (tid == 0) *out = s_idx == 0x7fffffff ? n - 1 : s_idx;
         return;
@@ -164,7 +215,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(float* logits, int n, const 
     // sample_topp: candidates in index order -> keys (descending probability, ascending index)
     const float cutoff = (1.0f - topp) / ((float)n - 1.0f);
     int cnt = 0;
-    for (int i = i0; i < i1; i++) cnt += logits[i] >= cutoff;
+    each([&](int, float& v) { cnt += v >= cutoff; });
     int n0;
     int off = block_excl_scan(cnt, shi, n0);
     if (n0 == 0) {
@@ -173,11 +224,12 @@ __global__ void __launch_bounds__(ST) sample_kernel(float* logits, int n, const 
         // over the probabilities: first maximal index, 0 if nothing compares.
         float best = -INFINITY;
         int bi = 0x7fffffff;
-        for (int i = i0; i < i1; i++)
-            if (logits[i] > best) {
-                best = logits[i];
+        each([&](int i, float& v) {
+            if (v > best) {
+                best = v;
                 bi = i;
             }
+        });
         const float m = block_max(best, shf);
         if (best == m && bi != 0x7fffffff) atomicMin(&s_idx, bi);
         __syncthreads();
@@ -192,8 +244,9 @@ __global__ void __launch_bounds__(ST) sample_kernel(float* logits, int n, const 
         return;
     }
     unsigned long long* keys = in_smem ? skeys : scratch;
-    for (int i = i0; i < i1; i++)
-        if (logits[i] >= cutoff) keys[off++] = ((unsigned long long)(~__float_as_uint(logits[i])) << 32) | (unsigned int)i;
+    each([&](int i, float& v) {
+        if (v >= cutoff) keys[off++] = ((unsigned long long)(~__float_as_uint(v)) << 32) | (unsigned int)i;
+    });
     for (int i = n0 + tid; i < n2; i += ST) keys[i] = ~0ull;
     __syncthreads();
     bitonic_sort(keys, n2);
