@@ -672,9 +672,7 @@ static int llama_batch_record(slai_llama* m, int B, int cap_pos) {
     }
     const slai_qmatrix* wout = m->output ? m->output : (m->embd_q ? m->embd_q : &m->embd_as_matrix);
     if ((rc = product(wout, m->out_norm, m->bt_x, m->bt_logits, c.vocab_size))) return rc;
-    for (int b = 0; b < B; b++)
-        if ((rc = launch_argmax(ctx, m->bt_logits + (size_t)b * c.vocab_size, c.vocab_size, d_next + b, false))) return rc;
-    return SLAI_OK;
+    return launch_argmax_rows(ctx, m->bt_logits, c.vocab_size, B, d_next, pdl);
 }
 
 // One token of every sequence b < n_seq at position h_pos[b] (a negative position leaves sequence b out of this step: its

@@ -352,6 +352,7 @@ SLAI_API int slai_qmatrix_create_from_device(slai_ctx* ctx, int fmt, int64_t nro
     int rc = qmatrix_alloc(ctx, fmt, nrows, ncols, nbytes, out);
     if (rc) return rc;
     slai_qmatrix* m = *out;
+    ctx->weights_fresh = true;
     const int be = fmt_block_elems(fmt), bb = fmt_block_bytes(fmt);
     const long long nbk = ncols / be;
     if (fmt == SLAI_FMT_F32) {
@@ -441,8 +442,12 @@ SLAI_API int slai_gemv_quant(slai_ctx* ctx, float* d_out, const slai_qmatrix* w,
     if (!ctx || !w || !d_out || !d_v) return SLAI_ERR_INVALID_ARG;
     SLAI_ENTER(ctx);
     SLAI_REQUIRE(ctx, n_batch >= 1 && n_batch <= 8, SLAI_ERR_INVALID_ARG, "gemv: n_batch=%d must be in 1..8", n_batch);
+    // Launched behind the predecessor's start: the product requests its weights while that kernel ends and waits for it before it
+    // touches anything else (4096 x 4096 back to back: see the figures in gemv.cu).  Not behind an upload of weights.
+    const bool pdl = ctx->use_pdl && !ctx->weights_fresh;
+    ctx->weights_fresh = false;
     // A batch streams a quantised matrix once (gemv_batch.cu); dense f32 matrices take the vectors one by one.
-    if (n_batch > 1 && gemv_batch_supported(w)) return gemv_batch_launch(ctx, d_out, w, d_v, n_batch);
+    if (n_batch > 1 && gemv_batch_supported(w)) return gemv_batch_launch(ctx, d_out, w, d_v, n_batch, 0, BATCH_STORE, nullptr, nullptr, 0.f, pdl);
     for (int b = 0; b < n_batch; b++) {
         GemvLaunch L;
         L.fmt = w->fmt;
@@ -453,6 +458,7 @@ SLAI_API int slai_gemv_quant(slai_ctx* ctx, float* d_out, const slai_qmatrix* w,
         L.seg[0].rows = (int)w->nrows;
         L.v = d_v + (size_t)b * w->ncols;
         L.out = d_out + (size_t)b * w->nrows;
+        L.pdl = pdl;
         int rc = gemv_launch(ctx, L);
         if (rc) return rc;
     }
@@ -663,8 +669,11 @@ __global__ void kv_append_kernel<__half>(__half* kc, __half* vc, const float* k,
 // the last one to finish (ticket) combines the per-block results.
 constexpr int ARG_BLOCKS = 32, ARG_THREADS = 256;
 __device__ __forceinline__ bool arg_better(float a, int ai, float b, int bi) { return a > b || (a == b && ai < bi); }
-__global__ void __launch_bounds__(ARG_THREADS) argmax_kernel(const float* v, long long n, int* out, unsigned int* work /* ticket, then ARG_BLOCKS x (value, index) */) {
+__global__ void __launch_bounds__(ARG_THREADS) argmax_kernel(const float* v, long long n, int* out, unsigned int* work /* per row: ticket, then ARG_BLOCKS x (value, index) */) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    v += (size_t)blockIdx.y * n;  // row of a batch
+    out += blockIdx.y;
+    work += blockIdx.y * (1 + 2 * ARG_BLOCKS);
     __shared__ float sv[ARG_THREADS / 32];
     __shared__ int si[ARG_THREADS / 32];
     __shared__ int s_last;
@@ -927,6 +936,10 @@ SLAI_API int slai_argmax(slai_ctx* ctx, const float* d_v, int64_t n, int32_t* d_
 
 int launch_argmax(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, bool pdl) {
     return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX);
+}
+int launch_argmax_rows(slai_ctx* ctx, const float* v, int64_t n, int rows, int32_t* d_out, bool pdl) {
+    SLAI_REQUIRE(ctx, rows >= 1 && CNT_ARGMAX + rows * (1 + 2 * ARG_BLOCKS) <= CNT_ATTN_POS, SLAI_ERR_INVALID_ARG, "argmax: %d rows", rows);
+    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS, rows), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX);
 }
 int launch_embed_f32(slai_ctx* ctx, float* x, const float* table, int dim, const int* d_token, const float* wpe,
                      const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half) {
