@@ -132,7 +132,8 @@ size_t attention_scratch_bytes(slai_ctx* ctx, int n_heads, int kv_mul, int head_
 }
 
 // Tile size, split count, copy width and shared memory of a launch.
-static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, size_t* smem) {
+// `regs`: the launch takes the register path where the shape allows it (at most two query heads an item).
+static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, bool regs, size_t* smem) {
     const int esz = kv_dtype == SLAI_KV_F16 ? 2 : 4;
     P.tile_pos = attn_tile_pos(P.hs, esz);
     P.n_splits = pick_splits(P.hs, esz, n_max);
@@ -142,7 +143,7 @@ static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, 
     P.vec16 = (bits & 15) == 0;
     // The register path of f32 caches: splits of 32 positions, not of one staged tile (16) -- at position 515 that is one round of
     // blocks instead of two, and half of the partial outputs to merge.
-    if (P.vec16 && P.hs == 128 && P.kv_mul <= 2 && esz == 4) P.tile_pos = 32;
+    if (regs && P.vec16 && P.hs == 128 && esz == 4) P.tile_pos = 32;
     *smem = attn_item_bytes(P.kv_mul, P.hs, esz, P.tile_pos, P.n_splits);
     SLAI_REQUIRE(ctx, *smem <= 160 * 1024, SLAI_ERR_SHAPE, "attention: shared memory %zu too large", *smem);
     return SLAI_OK;
@@ -172,7 +173,7 @@ static int attention_launch_inner(slai_ctx* ctx, const AttnLaunch& A) {
     P.n_heads = A.n_heads; P.kv_mul = kv_mul; P.kv_share = share; P.hs = A.head_size;
     size_t smem = 0;
     {
-        int rc = attn_geometry(ctx, P, A.kv_dtype, n_max, &smem);
+        int rc = attn_geometry(ctx, P, A.kv_dtype, n_max, A.cache_batch_stride % 16 == 0, &smem);
         if (rc) return rc;
     }
     const size_t po = (size_t)A.n_heads * P.n_splits * A.head_size * 4;
@@ -259,7 +260,7 @@ SLAI_API int slai_attention_static(slai_ctx* ctx, const slai_attn_params* p, con
     P.n_heads = n_heads; P.kv_mul = kv_mul; P.hs = hs;
     size_t smem = 0;
     {
-        int rc = attn_geometry(ctx, P, kv_dtype, pos + 1, &smem);
+        int rc = attn_geometry(ctx, P, kv_dtype, pos + 1, kv_mul == 1, &smem);
         if (rc) return rc;
     }
     const size_t po = (size_t)n_heads * P.n_splits * hs * 4;

@@ -52,7 +52,7 @@ __host__ __device__ inline size_t attn_item_bytes(int kv_mul, int hs, int esz, i
     size_t tile = tile_pos * attn_k_stride(hs, esz);
     const size_t merge = (size_t)kv_mul * n_splits * 4 * 4 + 4 * ATT_THREADS * 4;  // (max, sum) pairs of all splits, their weights, the groups' sums of the merge
     if (merge > tile) tile = merge;
-    const size_t groups = (size_t)kv_mul * (8192 / esz);  // the lane groups' outputs (register path)
+    const size_t groups = hs == 128 && kv_mul <= 2 ? (size_t)kv_mul * (8192 / esz) : 0;  // the lane groups' outputs (register path)
     if (groups > tile) tile = groups;
     return attn_head_bytes(kv_mul, hs, tile_pos) + ((tile + 15) & ~(size_t)15);
 }

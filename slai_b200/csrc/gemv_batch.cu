@@ -302,6 +302,16 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
         if (tid == 0 && unit + 2 * stride < units) fetch_records(unit + 2 * stride, slot);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (limit != P.wait_limit && tid == 0) {  // a wait ran out: the records still on their way land before the block ends
+        for (int f = max(0, it - 1); f <= it; f++) {
+            uint32_t ok = 0;
+            for (unsigned int i = 0; i < P.wait_limit && !ok; i++)
+                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(ok)
+                             : "r"(bar + 8 * ((f + 1) & 1)), "r"((uint32_t)((f - 1) >> 1) & 1u)
+                             : "memory");
+        }
+    }
 }
 
 // Sum of n values `stride` apart, in order; eight loads in flight.
@@ -380,9 +390,9 @@ int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo
     const int dblocks = P.norm_w ? 1 : (P.nsteps + BWARPS - 1) / BWARPS;
     if ((rc = launch_dependent(ctx, batch_digits_kernel<F>, dim3((unsigned)dblocks, NV), BTHREADS, 0, pdl, P, NV))) return rc;
     const long long units = (long long)P.ngroups * P.nch;
-    if ((rc = launch_dependent(ctx, kern, dim3((unsigned)(units < G ? units : G)), BTHREADS, smem, true, P))) return rc;
+    if ((rc = launch_dependent(ctx, kern, dim3((unsigned)(units < G ? units : G)), BTHREADS, smem, ctx->use_pdl, P))) return rc;
     const long long total = (long long)P.n_batch * M;
-    return launch_dependent(ctx, gemv_batch_reduce_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, true, d_out, ldo, P.part, P.nch, NV, P.mp, M,
+    return launch_dependent(ctx, gemv_batch_reduce_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, ctx->use_pdl, d_out, ldo, P.part, P.nch, NV, P.mp, M,
                             P.n_batch, epi, gate);
 }
 

@@ -443,7 +443,7 @@ SLAI_API int slai_gemv_quant(slai_ctx* ctx, float* d_out, const slai_qmatrix* w,
     SLAI_ENTER(ctx);
     SLAI_REQUIRE(ctx, n_batch >= 1 && n_batch <= 8, SLAI_ERR_INVALID_ARG, "gemv: n_batch=%d must be in 1..8", n_batch);
     // Launched behind the predecessor's start: the product requests its weights while that kernel ends and waits for it before it
-    // touches anything else (4096 x 4096 back to back: see the figures in gemv.cu).  Not behind an upload of weights.
+    // touches anything else (Q4_K 4096 x 4096 back to back: 8.19 -> 4.96 us).  Not behind an upload of weights.
     const bool pdl = ctx->use_pdl && !ctx->weights_fresh;
     ctx->weights_fresh = false;
     // A batch streams a quantised matrix once (gemv_batch.cu); dense f32 matrices take the vectors one by one.

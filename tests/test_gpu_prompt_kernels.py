@@ -1,5 +1,7 @@
 """The prompt pass's GEMM variants and its tensor-core attention at the edges of their tiles, and the decode attention whose keys and
 values stay in registers: against the sequential pass and against 64-bit arithmetic."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -65,6 +67,10 @@ def test_decode_attention_in_registers(backend, ctx, hs, kv_dtype, heads, kv_hea
         p = BatchedMultiqueryAttentionParams(seq_len=n, kv_dim=kv_heads * hs, kv_mul=heads // kv_heads, n_heads=heads, head_size=hs, pos=pos)
         ctx.attention(p, dq, dk, dv, out, kv_dtype)
         got = out.to_numpy().reshape(heads, hs)
+        # the entry point that allocates nothing serves more query heads per item: the staged path beside the register path
+        backend.check(backend.lib.slai_attention_static(backend.h, C.byref(p.to_c()), C.c_void_p(dq.ptr), C.c_void_p(dk.ptr), C.c_void_p(dv.ptr), kv_dtype,
+                                                        C.c_void_p(out.ptr)))
+        assert rel_l2(out.to_numpy().reshape(heads, hs), got) < 1e-5, pos
         for h in range(heads):
             K, V = k[:pos + 1, h // (heads // kv_heads)].astype(np.float64), v[:pos + 1, h // (heads // kv_heads)].astype(np.float64)
             s = K @ q[h].astype(np.float64) / np.sqrt(hs)
