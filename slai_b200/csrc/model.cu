@@ -442,10 +442,11 @@ static int llama_record(slai_llama* m, int kind) {
         }
     }
     if (kind == G_SAMPLED) rc = launch_sample(ctx, m->logits, c.vocab_size, m->d_samp, m->sc.d + 2, 0.f, false, m->d_samp_scratch, m->sc.d + 3, pdl);
+    else if (kind == G_GENERATE) rc = launch_argmax_advance(ctx, m->logits, c.vocab_size, m->sc.d + 3, d_token, d_pos, m->d_history, pdl);
     else rc = launch_argmax(ctx, m->logits, c.vocab_size, m->sc.d + 3, pdl);
     if (rc) return rc;
     n++;
-    if (kind == G_GENERATE || kind == G_SAMPLED) {
+    if (kind == G_SAMPLED) {
         if ((rc = launch_advance(ctx, d_token, d_pos, m->sc.d + 3, m->d_history, c.vocab_size, pdl))) return rc;
         n++;
     } else if (kind == G_FORCED) {
@@ -1323,12 +1324,11 @@ static int gpt2_record(slai_gpt2* m, int kind) {
         if ((rc = gemv_launch(ctx, L))) return rc;
         n++;
     }
-    if ((rc = launch_argmax(ctx, m->logits, c.n_vocab, m->sc.d + 3, pdl))) return rc;
+    if (kind == G_GENERATE) rc = launch_argmax_advance(ctx, m->logits, c.n_vocab, m->sc.d + 3, d_token, d_pos, m->d_history, pdl);
+    else rc = launch_argmax(ctx, m->logits, c.n_vocab, m->sc.d + 3, pdl);
+    if (rc) return rc;
     n++;
-    if (kind == G_GENERATE) {
-        if ((rc = launch_advance(ctx, d_token, d_pos, m->sc.d + 3, m->d_history, c.n_vocab, pdl))) return rc;
-        n++;
-    } else if (kind == G_FORCED) {
+    if (kind == G_FORCED) {
         if ((rc = launch_advance(ctx, d_token, d_pos, nullptr, m->d_history, c.n_vocab, pdl))) return rc;
         n++;
     }

@@ -667,9 +667,22 @@ __global__ void kv_append_kernel<__half>(__half* kc, __half* vc, const float* k,
 
 // first maximal index (nalgebra `imax`): ties resolve to the smaller index.  ARG_BLOCKS blocks scan a slice each;
 // the last one to finish (ticket) combines the per-block results.
+// The device-side loop's scalars: the next token, the position with the step counter behind it, the tokens so far.
+struct LoopState {
+    int *token, *pos, *history;  // (token null: no loop)
+    int vocab;
+};
+__device__ __forceinline__ void loop_advance(const LoopState& s, int next, bool record) {
+    const int step = s.pos[1];
+    if (record) s.history[step] = next;
+    *s.token = next < 0 ? 0 : (next >= s.vocab ? s.vocab - 1 : next);  // whatever a kernel produced, the embedding lookup stays inside its table
+    s.pos[0] = s.pos[0] + 1;
+    s.pos[1] = step + 1;
+}
 constexpr int ARG_BLOCKS = 32, ARG_THREADS = 256;
 __device__ __forceinline__ bool arg_better(float a, int ai, float b, int bi) { return a > b || (a == b && ai < bi); }
-__global__ void __launch_bounds__(ARG_THREADS) argmax_kernel(const float* v, long long n, int* out, unsigned int* work /* per row: ticket, then ARG_BLOCKS x (value, index) */) {
+__global__ void __launch_bounds__(ARG_THREADS) argmax_kernel(const float* v, long long n, int* out, unsigned int* work /* per row: ticket, then ARG_BLOCKS x (value, index) */,
+                                                             LoopState loop) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     v += (size_t)blockIdx.y * n;  // row of a batch
     out += blockIdx.y;
@@ -724,7 +737,9 @@ __global__ void __launch_bounds__(ARG_THREADS) argmax_kernel(const float* v, lon
                     bi = oi;
                 }
             }
-            *out = bi == 0x7fffffff ? 0 : bi;
+            const int best_index = bi == 0x7fffffff ? 0 : bi;
+            *out = best_index;
+            if (loop.token) loop_advance(loop, best_index, true);
         }
     }
 }
@@ -763,20 +778,9 @@ __global__ void embed_q_kernel(float* x, int fmt, const uint8_t* data, int dim, 
 // Advance the device-side loop state without a host round trip: pos <- pos + 1, step <- step + 1 and
 //   greedy (d_next != NULL): token <- *d_next, history[step] <- *d_next
 //   forced (d_next == NULL): token <- history[step]   (prompt processing)
-__global__ void advance_kernel(int* d_token, int* d_pos, const int* d_next, int* d_history, int* d_step, int vocab) {
+__global__ void advance_kernel(LoopState s, const int* d_next) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int step = *d_step;
-    int nx;
-    if (d_next) {
-        nx = *d_next;
-        d_history[step] = nx;
-    } else {
-        nx = d_history[step];
-    }
-    nx = nx < 0 ? 0 : (nx >= vocab ? vocab - 1 : nx);  // whatever a kernel produced, the embedding lookup stays inside its table
-    *d_token = nx;
-    *d_pos = *d_pos + 1;
-    *d_step = step + 1;
+    loop_advance(s, d_next ? *d_next : s.history[s.pos[1]], d_next != nullptr);
 }
 
 template <typename... Args>
@@ -935,11 +939,18 @@ SLAI_API int slai_argmax(slai_ctx* ctx, const float* d_v, int64_t n, int32_t* d_
 }
 
 int launch_argmax(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, bool pdl) {
-    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX);
+    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX,
+                      LoopState{});
+}
+// The greedy choice and, in the same launch, the loop's advance (a launch less per token; tiny model, 64 tokens: 7.93 -> 7.80 ms).
+int launch_argmax_advance(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, int* d_token, int* d_pos, int32_t* d_history, bool pdl) {
+    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX,
+                      LoopState{d_token, d_pos, (int*)d_history, (int)n});
 }
 int launch_argmax_rows(slai_ctx* ctx, const float* v, int64_t n, int rows, int32_t* d_out, bool pdl) {
     SLAI_REQUIRE(ctx, rows >= 1 && CNT_ARGMAX + rows * (1 + 2 * ARG_BLOCKS) <= CNT_ATTN_POS, SLAI_ERR_INVALID_ARG, "argmax: %d rows", rows);
-    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS, rows), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX);
+    return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS, rows), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX,
+                      LoopState{});
 }
 int launch_embed_f32(slai_ctx* ctx, float* x, const float* table, int dim, const int* d_token, const float* wpe,
                      const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half) {
@@ -954,8 +965,7 @@ int launch_embed_q8(slai_ctx* ctx, float* x, const slai_qmatrix* wte, const int*
 }
 int launch_advance(slai_ctx* ctx, int* d_token, int* d_pos, const int32_t* d_next, int32_t* d_history, int vocab, bool pdl) {
     // d_history[-1] is not used; the step counter lives right after the position scalar (see models)
-    return launch_pdl(ctx, advance_kernel, dim3(1), dim3(1), pdl, d_token, d_pos, (const int*)d_next, (int*)d_history,
-                      d_pos + 1, vocab);
+    return launch_pdl(ctx, advance_kernel, dim3(1), dim3(1), pdl, LoopState{d_token, d_pos, (int*)d_history, vocab}, (const int*)d_next);
 }
 
 // ------------------------------------------------------------------------------------------------
