@@ -9,6 +9,9 @@
 #include "common.cuh"
 #include "dequant.cuh"
 
+// All of these launch behind their predecessor's start.  What a kernel in front of them wrote (activations, q / k / v, caches) is
+// read with __ldcg and without __restrict__: the read-only path asks for memory that is constant as long as the kernel runs, and
+// a load marked so may move in front of griddepcontrol.wait.  Weights and tables may use both.
 namespace {
 
 // ---- causal attention of a block of prompt tokens ---------------------------------------------------------------------
@@ -22,14 +25,14 @@ namespace {
 constexpr int PA_QT = 16, PA_KT = 32, PA_THREADS = 128, PA_MAXC = 2;  // head_size <= 128 * PA_MAXC
 
 template <typename T>
-__device__ __forceinline__ void pa_load_rows(const T* __restrict__ g, long long row_stride, int rows, int hs, float* s, int s_stride, int tid) {
+__device__ __forceinline__ void pa_load_rows(const T* g, long long row_stride, int rows, int hs, float* s, int s_stride, int tid) {
     constexpr int VEC = 16 / (int)sizeof(T);  // elements per 16-byte piece
     const int ppr = hs / VEC;
     for (int idx = tid; idx < PA_KT * ppr; idx += PA_THREADS) {
         const int r = idx / ppr, c = idx - r * ppr;
         float v[VEC];
         if (r < rows) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(g + (long long)r * row_stride) + c);
+            const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(g + (long long)r * row_stride) + c);
             if (sizeof(T) == 2) {
                 const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
@@ -55,8 +58,8 @@ __device__ __forceinline__ void pa_load_rows(const T* __restrict__ g, long long 
 
 template <typename T>
 __global__ void __launch_bounds__(PA_THREADS)
-prefill_attn_kernel(const float* __restrict__ q, int q_ld, const T* __restrict__ kc, const T* __restrict__ vc, long long head_stride, int hs, int kv_mul,
-                    int pos0, int n_tokens, float* __restrict__ out, int out_ld) {
+prefill_attn_kernel(const float* q, int q_ld, const T* kc, const T* vc, long long head_stride, int hs, int kv_mul, int pos0, int n_tokens, float* out,
+                    int out_ld) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ __align__(16) float pa_sm[];
@@ -74,7 +77,7 @@ prefill_attn_kernel(const float* __restrict__ q, int q_ld, const T* __restrict__
     const float inv = 1.0f / sqrtf((float)hs);
     for (int i = tid; i < PA_QT * hs; i += PA_THREADS) {
         const int tq = i / hs, d = i - tq * hs;
-        q_s[i] = tq < nq ? q[(size_t)(t0 + tq) * q_ld + (size_t)head * hs + d] * inv : 0.f;
+        q_s[i] = tq < nq ? __ldcg(q + (size_t)(t0 + tq) * q_ld + (size_t)head * hs + d) * inv : 0.f;
     }
     float m[4], l[4], acc[4][PA_MAXC][4];
 #pragma unroll
@@ -201,8 +204,8 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
 
 template <int HS>
 __global__ void __launch_bounds__(PM_THREADS, 2)
-prefill_attn_mma_kernel(const float* __restrict__ q, int q_ld, const __half* __restrict__ kc, const __half* __restrict__ vc, long long head_stride,
-                        int kv_mul, int pos0, int n_tokens, float* __restrict__ out, int out_ld) {
+prefill_attn_mma_kernel(const float* q, int q_ld, const __half* kc, const __half* vc, long long head_stride, int kv_mul, int pos0, int n_tokens, float* out,
+                        int out_ld) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int ROW = HS * 2, CH = HS / 8, TILE = PM_KT * ROW;  // bytes of a cached row, its 16-byte chunks, bytes of a tile
@@ -244,7 +247,7 @@ prefill_attn_mma_kernel(const float* __restrict__ q, int q_ld, const __half* __r
         for (int i = 0; i < 4; i++) {
             const int row = row0 + 8 * (i & 1), d = 16 * k + 2 * t + 8 * (i >> 1);
             float2 v = make_float2(0.f, 0.f);
-            if (row < n_tokens) v = *reinterpret_cast<const float2*>(q + (size_t)row * q_ld + (size_t)head * HS + d);
+            if (row < n_tokens) v = __ldcg(reinterpret_cast<const float2*>(q + (size_t)row * q_ld + (size_t)head * HS + d));
             split2(v.x * inv, v.y * inv, qh[k][i], ql[k][i]);
         }
     float acc[NT8][4];
@@ -370,8 +373,7 @@ __device__ __forceinline__ float block_sum256(float x, float* sh) {
 // that it stays inside fp16's range whenever the activations do), as 16 columns per super-block of 256: eight fp16 sums,
 // then 2048 times their rounding errors (the minimum term of Q4_K / Q5_K, prefill_dequant.cuh).  Eight lanes hold a sub-block;
 // whole warps call this (`on`: the group exists).
-__device__ __forceinline__ void store_operands(__half* __restrict__ hi, __half* __restrict__ lo, __half* __restrict__ sum, int t, int K, int i, bool on,
-                                               float4 y) {
+__device__ __forceinline__ void store_operands(__half* hi, __half* lo, __half* sum, int t, int K, int i, bool on, float4 y) {
     const float v[4] = {y.x, y.y, y.z, y.w};
     __half h[4], l[4];
     float s = 0.f;
@@ -400,8 +402,7 @@ __device__ __forceinline__ void store_operands(__half* __restrict__ hi, __half* 
 }
 
 // Row t of X (optionally RmsNorm'd: ops/rms_norm.rs:68-77) as GEMM operands.
-__global__ void prefill_split_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ norm_w, float eps, int K,
-                                     __half* __restrict__ hi, __half* __restrict__ lo, __half* __restrict__ sum) {
+__global__ void prefill_split_kernel(const float* x, int ldx, const float* __restrict__ norm_w, float eps, int K, __half* hi, __half* lo, __half* sum) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float sh[32];
@@ -412,7 +413,7 @@ __global__ void prefill_split_kernel(const float* __restrict__ x, int ldx, const
     if (norm_w) {
         float s = 0.f;
         for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-            const float4 v = xr[i];
+            const float4 v = __ldcg(xr + i);
             s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
         s = block_sum256(s, sh);
@@ -422,7 +423,7 @@ __global__ void prefill_split_kernel(const float* __restrict__ x, int ldx, const
         const int i = i0 + threadIdx.x;
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < n4) {
-            y = xr[i];
+            y = __ldcg(xr + i);
             if (norm_w) {
                 const float4 w = w4[i];
                 y.x = __fmul_rn(__fmul_rn(y.x, mul), w.x); y.y = __fmul_rn(__fmul_rn(y.y, mul), w.y);
@@ -435,8 +436,8 @@ __global__ void prefill_split_kernel(const float* __restrict__ x, int ldx, const
 
 // Row t of X after LayerNorm with gamma / beta (ops/layernorm.rs:104-111 and the caller's scale and shift,
 // models/gpt2/cpu.rs:239-240) as GEMM operands; same arithmetic as the decode step's fused prologue.
-__global__ void prefill_split_ln_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
-                                        int K, __half* __restrict__ hi, __half* __restrict__ lo, __half* __restrict__ sum) {
+__global__ void prefill_split_ln_kernel(const float* x, int ldx, const float* __restrict__ gamma, const float* __restrict__ beta, float eps, int K, __half* hi,
+                                        __half* lo, __half* sum) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float sh[32];
@@ -445,13 +446,13 @@ __global__ void prefill_split_ln_kernel(const float* __restrict__ x, int ldx, co
     const float4 *g4 = reinterpret_cast<const float4*>(gamma), *b4 = reinterpret_cast<const float4*>(beta);
     float s = 0.f;
     for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 v = xr[i];
+        const float4 v = __ldcg(xr + i);
         s += (v.x + v.y) + (v.z + v.w);
     }
     const float mean = block_sum256(s, sh) / (float)K;
     float v = 0.f;
     for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-        float4 d = xr[i];
+        float4 d = __ldcg(xr + i);
         d.x -= mean; d.y -= mean; d.z -= mean; d.w -= mean;
         v += d.x * d.x + d.y * d.y + d.z * d.z + d.w * d.w;
     }
@@ -461,7 +462,7 @@ __global__ void prefill_split_ln_kernel(const float* __restrict__ x, int ldx, co
         const int i = i0 + threadIdx.x;
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < n4) {
-            y = xr[i];
+            y = __ldcg(xr + i);
             const float4 g = g4[i], b = beta ? b4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
             y.x = __fmul_rn(__fmul_rn(y.x - mean, mul), g.x) + b.x; y.y = __fmul_rn(__fmul_rn(y.y - mean, mul), g.y) + b.y;
             y.z = __fmul_rn(__fmul_rn(y.z - mean, mul), g.z) + b.z; y.w = __fmul_rn(__fmul_rn(y.w - mean, mul), g.w) + b.w;
@@ -475,36 +476,35 @@ __device__ __forceinline__ float gelu1(float x) {
     const float A = 0.044715f, Sq = 0.7978846f;
     return 0.5f * x * (1.0f + tanhf(Sq * x * (1.0f + A * x * x)));
 }
-__global__ void prefill_gelu_split_kernel(const float* __restrict__ g, int H, __half* __restrict__ hi, __half* __restrict__ lo, __half* __restrict__ sum) {
+__global__ void prefill_gelu_split_kernel(const float* g, int H, __half* hi, __half* lo, __half* sum) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = i < (H >> 2);
-    float4 y = on ? reinterpret_cast<const float4*>(g + (size_t)t * H)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 y = on ? __ldcg(reinterpret_cast<const float4*>(g + (size_t)t * H) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     y.x = gelu1(y.x); y.y = gelu1(y.y); y.z = gelu1(y.z); y.w = gelu1(y.w);
     store_operands(hi, lo, sum, t, H, i, on, y);
 }
 
 // x[t] += row (pos0 + t) of a table of position vectors (models/gpt2/cpu.rs:227-228).
-__global__ void prefill_add_rows_kernel(float* __restrict__ x, int dim, const float* __restrict__ table, int pos0) {
+__global__ void prefill_add_rows_kernel(float* x, int dim, const float* __restrict__ table, int pos0) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < dim) x[(size_t)t * dim + i] += table[(size_t)(pos0 + t) * dim + i];
+    if (i < dim) x[(size_t)t * dim + i] = __ldcg(x + (size_t)t * dim + i) + table[(size_t)(pos0 + t) * dim + i];
 }
 
 // hb = up * gate / (1 + exp(-gate)) (ops/silu.rs:50-58) straight into the operands of the down projection.
 __device__ __forceinline__ float silu1(float g, float u) { return u * (g / (1.0f + expf(-g))); }
-__global__ void prefill_silu_split_kernel(const float* __restrict__ gate, const float* __restrict__ up, int H, __half* __restrict__ hi,
-                                          __half* __restrict__ lo, __half* __restrict__ sum) {
+__global__ void prefill_silu_split_kernel(const float* gate, const float* up, int H, __half* hi, __half* lo, __half* sum) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = i < (H >> 2);
     float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
     if (on) {
-        const float4 g = reinterpret_cast<const float4*>(gate + (size_t)t * H)[i], u = reinterpret_cast<const float4*>(up + (size_t)t * H)[i];
+        const float4 g = __ldcg(reinterpret_cast<const float4*>(gate + (size_t)t * H) + i), u = __ldcg(reinterpret_cast<const float4*>(up + (size_t)t * H) + i);
         y = make_float4(silu1(g.x, u.x), silu1(g.y, u.y), silu1(g.z, u.z), silu1(g.w, u.w));
     }
     store_operands(hi, lo, sum, t, H, i, on, y);
@@ -524,16 +524,15 @@ __global__ void prefill_embed_kernel(float* __restrict__ x, int dim, const int* 
 // (may be its source), k and, when given, v into the cache ([kv_head][position][head_size], f16 or f32): the q/k/v
 // epilogue of the decode step for T tokens at once, and the decode step's own RoPE stage where the fused epilogue
 // cannot serve (pairs half a head apart, dense f32 matrices).
-__global__ void rope_kv_store_kernel(const float* __restrict__ q_src, const float* __restrict__ k_src, const float* __restrict__ v_src,
-                                     int ld, int q_dim, int kv_dim, int head_size, int pos0, const int* __restrict__ d_pos,
-                                     const float* __restrict__ theta, int neox, float* __restrict__ q_out, int ldq, void* kcache, void* vcache,
+__global__ void rope_kv_store_kernel(const float* q_src, const float* k_src, const float* v_src, int ld, int q_dim, int kv_dim, int head_size, int pos0,
+                                     const int* d_pos, const float* __restrict__ theta, int neox, float* q_out, int ldq, void* kcache, void* vcache,
                                      int kv_f16, long long kv_head_stride, long long seq_stride) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.y;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;  // pair index over q then k; then plain copies of v
     // seq_stride > 0: row t is a sequence of its own, at position d_pos[t] of caches seq_stride bytes after row t - 1's
-    const int pos = seq_stride > 0 ? d_pos[t] : (d_pos ? *d_pos : pos0) + t;
+    const int pos = seq_stride > 0 ? __ldcg(d_pos + t) : (d_pos ? __ldcg(d_pos) : pos0) + t;
     if (pos < 0) return;
     kcache = reinterpret_cast<char*>(kcache) + (size_t)t * seq_stride;
     vcache = reinterpret_cast<char*>(vcache) + (size_t)t * seq_stride;
@@ -553,7 +552,7 @@ __global__ void rope_kv_store_kernel(const float* __restrict__ q_src, const floa
         }
         float sn, cs;
         sincosf((float)pos * theta[fi], &sn, &cs);
-        const float xa = src[a], xb = src[b];
+        const float xa = __ldcg(src + a), xb = __ldcg(src + b);
         const float ya = cs * xa - sn * xb, yb = sn * xa + cs * xb;
         if (!is_k) {
             q_out[(size_t)t * ldq + a] = ya;
@@ -571,7 +570,7 @@ __global__ void rope_kv_store_kernel(const float* __restrict__ q_src, const floa
         }
     } else if (v_src && p < nq + nk + kv_dim) {
         const int e = p - nq - nk;
-        const float y = v_src[(size_t)t * ld + e];
+        const float y = __ldcg(v_src + (size_t)t * ld + e);
         const long long o = (long long)pos * head_size + (e / head_size) * kv_head_stride + e % head_size;
         if (kv_f16) reinterpret_cast<__half*>(vcache)[o] = __float2half_rn(y);
         else reinterpret_cast<float*>(vcache)[o] = y;
@@ -580,8 +579,8 @@ __global__ void rope_kv_store_kernel(const float* __restrict__ q_src, const floa
 
 // The q/k/v epilogue of a prompt: as rope_kv_store_kernel, one block per token, the angles' sines and cosines once per
 // token instead of once per head (they were most of that kernel's time: 511 tokens x 32 heads 23.7 us).
-__global__ void prefill_rope_kv_kernel(const float* __restrict__ qkv, int ld, int q_dim, int kv_dim, int head_size, int pos0, const float* __restrict__ theta,
-                                       int neox, float* __restrict__ q_out, int ldq, void* kcache, void* vcache, int kv_f16, long long kv_head_stride) {
+__global__ void prefill_rope_kv_kernel(const float* qkv, int ld, int q_dim, int kv_dim, int head_size, int pos0, const float* __restrict__ theta,
+                                       int neox, float* q_out, int ldq, void* kcache, void* vcache, int kv_f16, long long kv_head_stride) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ float2 rope_cs[];  // [head_size / 2] (cos, sin)
@@ -602,8 +601,8 @@ __global__ void prefill_rope_kv_kernel(const float* __restrict__ qkv, int ld, in
         const int da = halves ? fi : 2 * fi, db = halves ? fi + hh : 2 * fi + 1;
         const float* src = row + (part == 0 ? 0 : part == 1 ? q_dim : q_dim + kv_dim) + head * head_size;
         float2 y;
-        if (halves) y = make_float2(src[da], src[db]);
-        else y = *reinterpret_cast<const float2*>(src + da);  // neighbours travel together
+        if (halves) y = make_float2(__ldcg(src + da), __ldcg(src + db));
+        else y = __ldcg(reinterpret_cast<const float2*>(src + da));  // neighbours travel together
         if (part < 2) {
             const float2 w = rope_cs[fi];
             y = make_float2(w.x * y.x - w.y * y.y, w.y * y.x + w.x * y.y);
