@@ -39,7 +39,6 @@ struct slai_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::string last_error;
     bool use_pdl = true;            // programmatic dependent launch between decode kernels
-    bool weights_fresh = false;     // a matrix was uploaded without a wait: the next product must not request weights early
     void* d_scratch = nullptr;      // attention split partials etc.
     size_t scratch_bytes = 0;
     std::vector<void*> retired_scratch;  // outgrown scratch buffers: recorded passes may still point at them, freed with the context

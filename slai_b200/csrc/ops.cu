@@ -271,6 +271,11 @@ __global__ void place_kernel(int fmt, const uint8_t* __restrict__ raw, uint8_t* 
     layout::place_block(fmt, raw + (size_t)i * bb, dst, i / nbk, i % nbk, K);
 }
 
+// Ends every upload.  A product may be a dependent launch that reads its weights before it waits for the kernel in front of it,
+// so that kernel must not be the one that writes them.  This one is launched plainly: it starts when the upload is complete and
+// visible, and only after its start can a dependent launch behind it begin.
+__global__ void upload_end_kernel() {}
+
 __global__ void dequant_kernel(int fmt, const uint8_t* __restrict__ data, long long row0, long long nrows, long long K,
                                float* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -352,7 +357,6 @@ SLAI_API int slai_qmatrix_create_from_device(slai_ctx* ctx, int fmt, int64_t nro
     int rc = qmatrix_alloc(ctx, fmt, nrows, ncols, nbytes, out);
     if (rc) return rc;
     slai_qmatrix* m = *out;
-    ctx->weights_fresh = true;
     const int be = fmt_block_elems(fmt), bb = fmt_block_bytes(fmt);
     const long long nbk = ncols / be;
     if (fmt == SLAI_FMT_F32) {
@@ -378,6 +382,8 @@ SLAI_API int slai_qmatrix_create_from_device(slai_ctx* ctx, int fmt, int64_t nro
         place_kernel<<<(unsigned)((total + 127) / 128), 128, 0, ctx->stream>>>(fmt, (const uint8_t*)d_blocks, m->data, nrows, nbk, ncols, bb);
         SLAI_CHECK_CUDA(ctx, cudaGetLastError());
     }
+    upload_end_kernel<<<1, 1, 0, ctx->stream>>>();
+    SLAI_CHECK_CUDA(ctx, cudaGetLastError());
     return SLAI_OK;
 }
 
@@ -443,9 +449,8 @@ SLAI_API int slai_gemv_quant(slai_ctx* ctx, float* d_out, const slai_qmatrix* w,
     SLAI_ENTER(ctx);
     SLAI_REQUIRE(ctx, n_batch >= 1 && n_batch <= 8, SLAI_ERR_INVALID_ARG, "gemv: n_batch=%d must be in 1..8", n_batch);
     // Launched behind the predecessor's start: the product requests its weights while that kernel ends and waits for it before it
-    // touches anything else (Q4_K 4096 x 4096 back to back: 8.19 -> 4.96 us).  Not behind an upload of weights.
-    const bool pdl = ctx->use_pdl && !ctx->weights_fresh;
-    ctx->weights_fresh = false;
+    // touches anything else (Q4_K 4096 x 4096 back to back: 8.19 -> 4.96 us).  Weights are complete by then: see upload_end_kernel.
+    const bool pdl = ctx->use_pdl;
     // A batch streams a quantised matrix once (gemv_batch.cu); dense f32 matrices take the vectors one by one.
     if (n_batch > 1 && gemv_batch_supported(w)) return gemv_batch_launch(ctx, d_out, w, d_v, n_batch, 0, BATCH_STORE, nullptr, nullptr, 0.f, pdl);
     for (int b = 0; b < n_batch; b++) {

@@ -7,7 +7,7 @@ import pytest
 
 from slai_b200 import synth, _lib
 from slai_b200.models import Llama2Config, llama_from_host, synthetic_llama_host
-from slai_b200.ops import BatchedMultiqueryAttentionParams, GpuQuantMatrix
+from slai_b200.ops import BatchedMultiqueryAttentionParams
 from helpers import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -77,19 +77,3 @@ def test_decode_attention_in_registers(backend, ctx, hs, kv_dtype, heads, kv_hea
             e = np.exp(s - s.max())
             # f32 scores of up to ~25 are off by a few 2^-24 of that, the exponentials by as much relative: below 1e-5
             assert rel_l2(got[h], e @ V / e.sum()) < 1e-5, (pos, h)
-
-
-def test_gemv_right_after_its_matrix_was_uploaded(backend, ctx):
-    """Consecutive products start behind one another's start and request their weights early: not before an upload is done."""
-    rng = np.random.default_rng(2)
-    M = K = 1024
-    x = rng.standard_normal(K).astype(np.float32)
-    for i in range(4):
-        w = synth.normal_matrix(i, M, K)
-        m = GpuQuantMatrix(backend, synth.FMT_Q8_0, M, K, synth.quantize(synth.FMT_Q8_0, w))
-        a, b, c = backend.vector(x), backend.zeros(M), backend.zeros(M)
-        ctx.matmul_quant_assign(b, m, a)
-        ctx.matmul_quant_assign(c, m, b)  # consumes the product before it
-        W = w.reshape(M, K).astype(np.float64)
-        assert rel_l2(b.to_numpy(), W @ x) < 1e-2  # Q8_0's own rounding
-        assert rel_l2(c.to_numpy(), W @ b.to_numpy().astype(np.float64)) < 1e-2
