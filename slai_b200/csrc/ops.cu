@@ -101,7 +101,7 @@ int slai_check_wait_flag(slai_ctx* ctx) {
     if (flag) {
         cudaMemset(ctx->d_counters + CNT_ERR_FLAG, 0, sizeof(flag));
         return slai_set_error(ctx, SLAI_ERR_TIMEOUT, "a bounded wait inside a kernel ran out (%s); results of the last launches are invalid",
-                              flag == 1 ? "weight ring" : flag == 2 ? "grid barrier" : "tensor-parallel peer");
+                              flag == 1 ? "weight ring" : flag == 5 ? "prompt product" : flag == 6 ? "batched product" : "tensor-parallel peer");
     }
     return SLAI_OK;
 }

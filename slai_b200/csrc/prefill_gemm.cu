@@ -134,6 +134,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(mbar)
                  : "memory");
 }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // Shared-memory matrix descriptor of a K-major operand tile: start address / 16 in bits 0-13, leading offset (unused with a
 // swizzle of the row length) 1 in bits 16-29, stride between 8-row groups / 16 in bits 32-45, descriptor version 1 in bits
@@ -289,9 +290,11 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     unsigned int limit = P.wait_limit;
-    // Dependent launch: the weights' warps need not wait for the kernel before this one, everything else does.
+    // Dependent launch: the weights' warps fill their rings while the kernel before this one ends, and wait for its end before their first
+    // wait on a slot that has been used: its consumers cannot start sooner, and that time is not this kernel's to count (a
+    // bounded wait in its place gave up on a healthy predecessor at up to 1024 rounds, where 96 are enough now).  Everything else waits here.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (warp < 2 || warp >= 12) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp < 2 || warp >= 12) griddep_wait();
     // readers of the sums (warps 12-19): 32 rows each, every other group of 16 tokens
     constexpr int NG = MERGED ? 2 : 4;
     float acc[NG][16];
@@ -401,6 +404,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 const int nt = max(0, min(8, (sg.rows - m0 + 15) >> 4));  // 16-row tiles that exist
                 const uint8_t* src = sg.w + (long long)(m0 >> 4) * P.tile_bytes + (long long)c0 * F::STEP;
                 for (int c = 0; c < nc; c++) {
+                    if (issued == PK) griddep_wait();
                     if (!(ok = mbar_wait(pk_empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
                     fence_async();  // the warps' reads of the block before come before the copy's writes
                     mbar_expect_tx(pk_full + 8 * slot, (uint32_t)nt * F::STEP);
@@ -426,6 +430,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         uint32_t* scales = reinterpret_cast<uint32_t*>(smem + L.scale);
         int slot = 0, ps = 0, c = 0;  // c: super-blocks so far
         uint32_t ph = 0, pph = 0;
+        bool behind = false;
         for (int tile = tile0; tile < P.tiles; tile += tile_step)
         for (int i = 0; i < nc; i++, c++) {
             mbar_wait(pk_full + 8 * ps, pph, limit, P.err_flag);
@@ -450,6 +455,10 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 const int slot0 = slot;
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
+                    if (ph && !behind) {
+                        griddep_wait();
+                        behind = true;
+                    }
                     mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag);
                     unsigned char* a = smem + L.a + slot * F::PLANES * PG_A_BYTES;
                     pfq::emit<FMT>(pk[k], r, part, st + k, a, a + PG_A_BYTES);
@@ -550,7 +559,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     // ---- K split over a cluster ----
     __syncwarp();
     if (!PAIR && P.ks > 1) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        griddep_wait();
         PgSeg sg;
         int m0, n0;
         tile_of(tile0, sg, m0, n0);

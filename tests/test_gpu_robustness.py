@@ -9,6 +9,7 @@ import pytest
 from oracle import oracle as O
 from slai_b200 import synth, _lib
 from slai_b200._lib import SlaiError
+from slai_b200.models import Llama2Config, synthetic_llama_device
 from slai_b200.ops import Backend, BatchedMultiqueryAttentionParams, GpuQuantMatrix, LlmContext
 from helpers import rel_l2
 
@@ -167,3 +168,23 @@ def test_recorded_pass_with_attention_replays(backend, ctx):
     ref, _ = O.attention(q, kc_h, vc_h, seq_len=seq, kv_dim=kvd, kv_mul=kvm, n_heads=nh, head_size=hs, pos=pos)
     assert rel_l2(want, ref) < 2e-5
     rec.close()
+
+
+def test_prompt_products_do_not_count_the_time_of_the_kernel_before_them():
+    """The prompt's GEMMs start while their predecessor still runs and fill their rings with weights.  Their bounded waits must count from
+    the predecessor's end: with a limit that is enough for the GEMM itself (96 rounds measured at this shape) nothing may run out."""
+    backend = Backend(0)
+    cfg = Llama2Config(dim=8192, hidden_dim=28672, n_layers=2, n_q_heads=64, n_kv_heads=8, vocab_size=512, seq_len=320, kv_dtype=_lib.KV_F16)
+    m = synthetic_llama_device(backend, cfg, synth.FMT_Q4_K, synth.FMT_Q4_K, seed=1, std=0.02)
+    prompt = (np.arange(300) % cfg.vocab_size).astype(np.int32)
+    m.prefill(prompt, 0)
+    backend.synchronize()
+    want = m.read_kv(1, 300)
+    backend.set_wait_limit(256)
+    for _ in range(4):
+        m.prefill(prompt, 0)
+        backend.synchronize()  # reports a wait that ran out
+    for got, ref in zip(m.read_kv(1, 300), want):
+        assert np.array_equal(got, ref)
+    m.close()
+    backend.close()
