@@ -405,6 +405,7 @@ struct PrefillGemm {
     int ldr = 0;
 };
 int prefill_gemm_nt(int T);
+int prefill_buffer_rows(int t_pad);
 int prefill_gemm_launch(slai_ctx* ctx, const PrefillGemm& G);
 // prefill.cu: the kernels around the GEMMs
 int prefill_split_launch(slai_ctx* ctx, const float* x, int ldx, const float* norm_w, float eps, int T, int K, const PrefillOperands& o);

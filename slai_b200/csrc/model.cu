@@ -945,7 +945,7 @@ static int llama_prefill_reserve(slai_llama* m, int t_pad, int attn_batch, size_
     const slai_llama_config& c = m->cfg;
     if (t_pad > m->pf_cap || attn_batch > m->pf_attn_batch) llama_drop_prefill(m);
     if (!m->pf_cap) {
-        const size_t T = (size_t)t_pad;
+        const size_t T = (size_t)prefill_buffer_rows(t_pad);
         const size_t kmax = (size_t)std::max(std::max(c.dim, m->hidden), m->q_dim);
         bool ok = cudaMalloc(&m->pf_x, T * c.dim * 4) == cudaSuccess && cudaMalloc(&m->pf_qkv, T * (m->q_dim + 2 * m->kv_dim) * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_q, T * m->q_dim * 4) == cudaSuccess && cudaMalloc(&m->pf_xb, T * m->q_dim * 4) == cudaSuccess &&
@@ -960,7 +960,7 @@ static int llama_prefill_reserve(slai_llama* m, int t_pad, int attn_batch, size_
             llama_drop_prefill(m);
             return slai_set_error(ctx, SLAI_ERR_OOM, "prefill: cannot allocate buffers for %d tokens", t_pad);
         }
-        m->pf_cap = t_pad;
+        m->pf_cap = (int)T;
         m->pf_attn_batch = attn_batch;
     }
     // attention partials of one batch of query tokens: sized by the last position of this prompt
@@ -1493,7 +1493,7 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
     const size_t kmax = (size_t)std::max(E, F);
     if (t_pad > m->pf_cap) gpt2_drop_prefill(m);
     if (!m->pf_cap) {
-        const size_t T = (size_t)t_pad;
+        const size_t T = (size_t)prefill_buffer_rows(t_pad);
         bool ok = cudaMalloc(&m->pf_x, T * E * 4) == cudaSuccess && cudaMalloc(&m->pf_qkv, T * 3 * E * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_q, T * E * 4) == cudaSuccess && cudaMalloc(&m->pf_xb, T * E * 4) == cudaSuccess &&
                   cudaMalloc(&m->pf_ff, T * F * 4) == cudaSuccess && cudaMalloc(&m->pf_op.hi, T * kmax * 2) == cudaSuccess &&
@@ -1505,7 +1505,7 @@ static int gpt2_prefill_batched(slai_gpt2* m, const int32_t* h_tokens, int n, in
             gpt2_drop_prefill(m);
             return slai_set_error(ctx, SLAI_ERR_OOM, "prefill: cannot allocate buffers for %d tokens", t_pad);
         }
-        m->pf_cap = t_pad;
+        m->pf_cap = (int)T;
     }
     int rc;
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;

@@ -717,6 +717,10 @@ int prefill_gemm_nt(int T) {
     return ((T + tiles - 1) / tiles + 15) / 16 * 16;
 }
 
+// Rows that the buffers of a pass with `t_pad` rows get: in steps of 256 above 256, so that a conversation whose turns grow does not
+// allocate anew on each (7B shape, 511 tokens after 300: 8.0 ms, of which 6 are the allocation).
+int prefill_buffer_rows(int t_pad) { return t_pad <= 256 ? t_pad : (t_pad + 255) / 256 * 256; }
+
 // out_i[t][m] = (resid[t][m] +) sum_k W_i[m][k] X[t][k] (+ bias_i[m]) for t < T and up to three matrices W_i of one format and
 // width that share the activations, given as hi / lo planes (and the sub-blocks' sums, see PrefillGemm) of `t_pad` rows.
 // Rows T .. t_pad - 1 of the planes may hold anything: a token's sums depend on its own row alone.

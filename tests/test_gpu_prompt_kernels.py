@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from slai_b200 import synth, _lib
-from slai_b200.models import Llama2Config, llama_from_host, synthetic_llama_host
+from slai_b200.models import Gpt2Params, Llama2Config, llama_from_host, synthetic_gpt2_device, synthetic_llama_host
 from slai_b200.ops import BatchedMultiqueryAttentionParams
 from helpers import rel_l2
 
@@ -77,3 +77,16 @@ def test_decode_attention_in_registers(backend, ctx, hs, kv_dtype, heads, kv_hea
             e = np.exp(s - s.max())
             # f32 scores of up to ~25 are off by a few 2^-24 of that, the exponentials by as much relative: below 1e-5
             assert rel_l2(got[h], e @ V / e.sum()) < 1e-5, (pos, h)
+
+
+def test_longer_prompts_do_not_allocate_anew(backend):
+    """Above 256 tokens the buffers of a pass grow in steps of 256 rows (GPT-2: its pass holds nothing that grows with the position)."""
+    p = Gpt2Params(n_vocab=300, n_seq=1024, n_embd=1024, n_head=16, n_layer=1, ff_len=4096, kv_dtype=_lib.KV_F16)
+    m = synthetic_gpt2_device(backend, p, synth.FMT_Q8_0, seed=1, std=0.02)
+    ids = np.random.default_rng(1).integers(0, p.n_vocab, size=1024).astype(np.int32)
+    for first, longer in ((257, (300, 400, 512)), (513, (600, 768))):
+        m.prefill(ids[:first], 0)
+        free = backend.mem_info()[0]
+        for n in longer:
+            m.prefill(ids[:n], 0)
+            assert backend.mem_info()[0] == free, n
