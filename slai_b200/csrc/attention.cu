@@ -88,13 +88,22 @@ int launch_hs(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pd
     return SLAI_OK;
 }
 
-// Heads of 128 with 16-byte aligned rows keep keys and values in registers (attn_item); at most two query heads each.  Heads of 64
-// do not: twice as many lane groups share a split, each with half as much to do (GPT-2 XL, position 127: 1548 against 1516 us
-// per token).
+// Which launches keep keys and values in registers (attn_item) instead of staging tiles: 16-byte aligned heads of 128, with room for
+// one query head an item, or two where the cache is f32 (`max_q`: what the launch's kernel has room for).  us per token and layer,
+// staged / registers:
+//   f16, one:  32 heads  46.9 / 46.4 at position 150, 65.3 / 63.6 at 2000, 72.9 / 69.8 at 3500
+//   f16, two:  32 heads on 16  48.1 / 52.2 at 150, 66.3 / 70.2 at 3500; 16 on 4  42.2 / 45.2 at 3500 (twice the products a lane for
+//              the same loads): staged
+//   f32, one:  32 heads  55.0 / 49.4 at 515, 87.3 / 80.2 at 3500
+//   f32, two:  64 heads on 8  128.8 / 124.0 at 515, 170.6 / 157.9 at 3500; 32 on 16  51.9 / 53.1 at 515, 59.3 / 53.7 at 900
+// Heads of 64 are staged: twice as many lane groups share a split, each with half as much to do (GPT-2 XL, position 127: 1516
+// against 1548 us per token).
+bool attn_in_registers(const AttnParams& P, int esz, int max_q) { return P.vec16 && P.hs == 128 && max_q <= (esz == 4 ? 2 : 1); }
+
 template <typename T, int MAXQ>
 int launch_t(slai_ctx* ctx, const AttnParams& P, int n_kv, size_t smem, bool pdl) {
-    if constexpr (MAXQ <= 2) {
-        if (P.vec16 && P.hs == 128) return launch_hs<T, MAXQ, 128>(ctx, P, n_kv, smem, pdl);
+    if constexpr (MAXQ <= (sizeof(T) == 4 ? 2 : 1)) {  // (the others are never asked for)
+        if (P.regs) return launch_hs<T, MAXQ, 128>(ctx, P, n_kv, smem, pdl);
     }
     return launch_hs<T, MAXQ, 0>(ctx, P, n_kv, smem, pdl);
 }
@@ -132,18 +141,21 @@ size_t attention_scratch_bytes(slai_ctx* ctx, int n_heads, int kv_mul, int head_
 }
 
 // Tile size, split count, copy width and shared memory of a launch.
-// `regs`: the launch takes the register path where the shape allows it (at most two query heads an item).
-static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, bool regs, size_t* smem) {
+// `max_q`: query heads an item of the launch's kernel has room for; `seq_stride`: bytes between the caches of a batch of sequences.
+static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, int max_q, long long seq_stride, size_t* smem) {
     const int esz = kv_dtype == SLAI_KV_F16 ? 2 : 4;
     P.tile_pos = attn_tile_pos(P.hs, esz);
     P.n_splits = pick_splits(P.hs, esz, n_max);
     const uintptr_t bits = reinterpret_cast<uintptr_t>(P.kc) | reinterpret_cast<uintptr_t>(P.vc) | (uintptr_t)(P.pos_stride * esz) |
                            (uintptr_t)(P.head_stride * esz) | (uintptr_t)(P.hs * esz);
     SLAI_REQUIRE(ctx, (bits & 3) == 0, SLAI_ERR_INVALID_ARG, "attention: caches and strides must be 4-byte aligned");
-    P.vec16 = (bits & 15) == 0;
+    P.vec16 = ((bits | (uintptr_t)seq_stride) & 15) == 0;
+    P.regs = attn_in_registers(P, esz, max_q);
     // The register path of f32 caches: splits of 32 positions, not of one staged tile (16) -- at position 515 that is one round of
-    // blocks instead of two, and half of the partial outputs to merge.
-    if (regs && P.vec16 && P.hs == 128 && esz == 4) P.tile_pos = 32;
+    // blocks instead of two, and half of the partial outputs to merge.  A short context has too few blocks for that and keeps
+    // splits of 16 (32 query heads on 16, position 150: 50.5 -> 49.0 us per token and layer, 48.5 staged).
+    P.split_short = P.tile_pos;
+    if (P.regs && esz == 4) P.tile_pos = 32;
     *smem = attn_item_bytes(P.kv_mul, P.hs, esz, P.tile_pos, P.n_splits);
     SLAI_REQUIRE(ctx, *smem <= 160 * 1024, SLAI_ERR_SHAPE, "attention: shared memory %zu too large", *smem);
     return SLAI_OK;
@@ -173,7 +185,7 @@ static int attention_launch_inner(slai_ctx* ctx, const AttnLaunch& A) {
     P.n_heads = A.n_heads; P.kv_mul = kv_mul; P.kv_share = share; P.hs = A.head_size;
     size_t smem = 0;
     {
-        int rc = attn_geometry(ctx, P, A.kv_dtype, n_max, A.cache_batch_stride % 16 == 0, &smem);
+        int rc = attn_geometry(ctx, P, A.kv_dtype, n_max, kv_mul == 1 ? 1 : 2, A.cache_batch_stride, &smem);
         if (rc) return rc;
     }
     const size_t po = (size_t)A.n_heads * P.n_splits * A.head_size * 4;
@@ -203,7 +215,6 @@ static int attention_launch_inner(slai_ctx* ctx, const AttnLaunch& A) {
     SLAI_REQUIRE(ctx, (A.cache_batch_stride == 0 && !A.d_pos_batch) || (A.batch > 0 && A.cache_batch_stride > 0 && A.d_pos_batch &&
                           A.cache_batch_stride % 4 == 0), SLAI_ERR_INVALID_ARG, "attention: a batch of sequences needs positions and a cache stride");
     P.cache_bs = A.cache_batch_stride; P.seq_pos = A.d_pos_batch;
-    if (A.cache_batch_stride & 15) P.vec16 = 0;
     P.po_bs = (long long)(per_token / 4); P.pml_bs = (long long)(per_token / 4);  // every token's partials in its own slice of the scratch
     const bool f16 = A.kv_dtype == SLAI_KV_F16;
     if (kv_mul == 1) return f16 ? launch_t<__half, 1>(ctx, P, n_kv, smem, A.pdl) : launch_t<float, 1>(ctx, P, n_kv, smem, A.pdl);
@@ -260,7 +271,7 @@ SLAI_API int slai_attention_static(slai_ctx* ctx, const slai_attn_params* p, con
     P.n_heads = n_heads; P.kv_mul = kv_mul; P.hs = hs;
     size_t smem = 0;
     {
-        int rc = attn_geometry(ctx, P, kv_dtype, pos + 1, kv_mul == 1, &smem);
+        int rc = attn_geometry(ctx, P, kv_dtype, pos + 1, kv_mul == 1 ? 1 : kv_mul <= 4 ? 4 : 8, 0, &smem);
         if (rc) return rc;
     }
     const size_t po = (size_t)n_heads * P.n_splits * hs * 4;

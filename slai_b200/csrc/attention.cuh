@@ -19,7 +19,9 @@ struct AttnParams {
     int early = 0;  // the position scalar is final before this kernel's blocks can start (AttnLaunch::pos_stable): read it before the wait
     int n_splits;   // most splits a KV head is cut into (stride of the partial buffers)
     int tile_pos;   // positions staged in shared memory at a time
+    int split_short;  // positions of a split while the context is at most 256 positions
     int vec16;      // rows can be copied in 16-byte pieces (alignment of bases, strides and row length)
+    int regs = 0;   // keys and values stay in registers (attn_in_registers)
     float* out;
     float* part_o;   // [n_heads][n_splits][hs]
     float* part_ml;  // [n_heads][n_splits][2]
@@ -68,7 +70,8 @@ __host__ __device__ inline int attn_tile_pos(int hs, int esz) {
 }
 // Splits actually used at `n` positions: one per tile, up to the maximum.
 __device__ __forceinline__ int attn_splits(const AttnParams& P, int n) {
-    const int want = (n + P.tile_pos - 1) / P.tile_pos;
+    const int per = n <= 256 ? P.split_short : P.tile_pos;
+    const int want = (n + per - 1) / per;
     return want < 1 ? 1 : want > P.n_splits ? P.n_splits : want;
 }
 
@@ -141,7 +144,7 @@ __device__ __forceinline__ void copy_rows_u32(const unsigned char* g, size_t row
 // index `tid`, shared memory `smb` (attn_item_bytes) and barrier `bar_id`.  The split's positions are walked in
 // tiles with a running (max, sum) per query head (the usual streaming softmax); the partial output of the split is
 // the un-normalised weighted sum of V relative to the final max.
-// HSF: the head size where it is 128 and everything is 16-byte aligned (0: any).  Then keys and values never enter shared
+// HSF: the head size on the register path (attn_in_registers), which is 128 with everything 16-byte aligned (0: any, staged).  Then keys and values never enter shared
 // memory: a group of lanes holds one cached row (16 bytes per lane), takes every GB-th position of the split, four at a time
 // with the next four on their way, and keeps its own running softmax; the groups meet once at the end.  The staged
 // path below costs four block barriers and about 1700 warp instructions per tile of 32 positions; at position 515 the f32
@@ -477,8 +480,10 @@ __device__ __forceinline__ void attn_item(const AttnParams& P, int kvh, int spli
         w_all[2 * i + 1] = w * l;
     }
     att_sync(bar_id);
-    if (ns > 32 && (hs & 3) == 0 && (hs >> 2) <= ATT_THREADS / 2) {
-        // Many splits (measured: pays from three rounds of sixteen loads on; with fewer the plain loop below is quicker).
+    if (ns > (HSF > 0 && ESZ == 4 ? 16 : 32) && (hs & 3) == 0 && (hs >> 2) <= ATT_THREADS / 2) {
+        // Many splits (measured: pays from three rounds of sixteen loads on; with fewer the plain loop below is quicker.  The
+        // register path of f32 caches has half as many, larger splits, and gains from the second round on: 16 query heads on 4,
+        // position 700: 38.7 -> 36.7 us per token and layer, 36.8 staged).
         // Threads as (group g, 16-byte chunk c of the head's output): group g adds the splits s = g, g + G, ... of its chunk
         // (all of a thread's loads are independent: one trip to memory for up to 16 splits per group), the groups' sums
         // meet in shared memory and are added in group order.  Fixed order throughout.

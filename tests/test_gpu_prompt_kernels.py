@@ -79,6 +79,27 @@ def test_decode_attention_in_registers(backend, ctx, hs, kv_dtype, heads, kv_hea
             assert rel_l2(got[h], e @ V / e.sum()) < 1e-5, (pos, h)
 
 
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (4, 2), (3, 1)])  # one and two query heads an item; three: one each
+@pytest.mark.parametrize("kv_dtype", [_lib.KV_F16, _lib.KV_F32])
+def test_decode_attention_where_its_splits_change(backend, ctx, kv_dtype, heads, kv_heads):
+    """f32 caches of 128-wide heads: 16 positions a split up to 256 positions, 32 beyond; more than 16 splits are merged by groups."""
+    hs, n = 128, 1100
+    rng = np.random.default_rng(heads)
+    dt = np.float16 if kv_dtype == _lib.KV_F16 else np.float32
+    k, v = (rng.standard_normal((n, kv_heads, hs)).astype(dt) for _ in range(2))
+    q = (2 * rng.standard_normal((heads, hs))).astype(np.float32)
+    dk, dv, dq, out = backend.vector(k.ravel(), dt), backend.vector(v.ravel(), dt), backend.vector(q.ravel()), backend.zeros(heads * hs)
+    for pos in (239, 240, 254, 255, 256, 287, 511, 512, 543, 544, 1023, 1024, n - 1):
+        p = BatchedMultiqueryAttentionParams(seq_len=n, kv_dim=kv_heads * hs, kv_mul=heads // kv_heads, n_heads=heads, head_size=hs, pos=pos)
+        ctx.attention(p, dq, dk, dv, out, kv_dtype)
+        got = out.to_numpy().reshape(heads, hs)
+        for h in range(heads):
+            K, V = k[:pos + 1, h // (heads // kv_heads)].astype(np.float64), v[:pos + 1, h // (heads // kv_heads)].astype(np.float64)
+            s = K @ q[h].astype(np.float64) / np.sqrt(hs)
+            e = np.exp(s - s.max())
+            assert rel_l2(got[h], e @ V / e.sum()) < 1e-5, (pos, h)  # f32 scores of up to ~25, as above
+
+
 def test_longer_prompts_do_not_allocate_anew(backend):
     """Above 256 tokens the buffers of a pass grow in steps of 256 rows (GPT-2: its pass holds nothing that grows with the position)."""
     p = Gpt2Params(n_vocab=300, n_seq=1024, n_embd=1024, n_head=16, n_layer=1, ff_len=4096, kv_dtype=_lib.KV_F16)
