@@ -314,15 +314,16 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
     }
 }
 
-// Sum of n values `stride` apart, in order; eight loads in flight.
+// Sum of n values `stride` apart, in order; U loads in flight.
+template <int U>
 __device__ __forceinline__ float batch_sum(const float* p, int n, size_t stride) {
     float s = 0.f;
-    for (int c0 = 0; c0 < n; c0 += 8) {
-        float x[8];
+    for (int c0 = 0; c0 < n; c0 += U) {
+        float x[U];
 #pragma unroll
-        for (int i = 0; i < 8; i++) x[i] = c0 + i < n ? __ldcg(p + (size_t)(c0 + i) * stride) : 0.f;
+        for (int i = 0; i < U; i++) x[i] = c0 + i < n ? __ldcg(p + (size_t)(c0 + i) * stride) : 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; i++) s += x[i];
+        for (int i = 0; i < U; i++) s += x[i];
     }
     return s;
 }
@@ -331,6 +332,7 @@ __device__ __forceinline__ float batch_sum(const float* p, int n, size_t stride)
 // epi: BATCH_STORE, BATCH_ADD (out += sum: the residual streams of the batch), BATCH_SILU (out = sum * silu(gate), gate laid
 // out like out: ops/silu.rs:50-58 with the sum as h2 and gate as h1), BATCH_PAIR_SILU (two matrices of M rows each in one
 // launch, gate then up: out = up sum * silu(gate sum)).
+template <int U>
 __global__ void gemv_batch_reduce_kernel(float* out, long long ldo, const float* part, int nch, int nv, int mp, int M, int n_batch, int epi,
                                          const float* gate) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -338,7 +340,7 @@ __global__ void gemv_batch_reduce_kernel(float* out, long long ldo, const float*
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)n_batch * M) return;
     const int v = (int)(idx / M), m = (int)(idx - (long long)v * M);
-    float s = batch_sum(part + (size_t)v * mp + m, nch, (size_t)nv * mp);
+    float s = batch_sum<U>(part + (size_t)v * mp + m, nch, (size_t)nv * mp);
     const long long o = (long long)v * ldo + m;
     if (epi == BATCH_ADD) {
         s = out[o] + s;
@@ -346,7 +348,7 @@ __global__ void gemv_batch_reduce_kernel(float* out, long long ldo, const float*
         const float g = gate[o];
         s = s * (g / (1.0f + expf(-g)));
     } else if (epi == BATCH_PAIR_SILU) {
-        const float u = batch_sum(part + (size_t)v * mp + M + m, nch, (size_t)nv * mp);
+        const float u = batch_sum<U>(part + (size_t)v * mp + M + m, nch, (size_t)nv * mp);
         s = u * (s / (1.0f + expf(-s)));
     }
     out[o] = s;
@@ -392,7 +394,12 @@ int launch_batch_inst(slai_ctx* ctx, BatchParams& P, float* d_out, long long ldo
     const long long units = (long long)P.ngroups * P.nch;
     if ((rc = launch_dependent(ctx, kern, dim3((unsigned)(units < G ? units : G)), BTHREADS, smem, ctx->use_pdl, P))) return rc;
     const long long total = (long long)P.n_batch * M;
-    return launch_dependent(ctx, gemv_batch_reduce_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, ctx->use_pdl, d_out, ldo, P.part, P.nch, NV, P.mp, M,
+    // More than eight chunks: 32 loads in flight.  Eight at a time, the 32 chunks of a short wide matrix were four trips to memory one
+    // after the other: Q8_0 1000 x 4096, 2 vectors 12.0 -> 8.3 us, 8 vectors 13.5 -> 8.4; Q5_K 4096 x 11008, 8 vectors 21.9 -> 20.3.
+    // (Summed by the last block of a row group inside the product instead, one launch less, 32000 x 4096 Q4_K with 8 vectors took
+    // 43.8 us for 35.6, and 2048 x 2048 10.6 for 8.6: every unit pays the fence and the ticket.)
+    auto reduce = P.nch <= 8 ? gemv_batch_reduce_kernel<8> : gemv_batch_reduce_kernel<32>;
+    return launch_dependent(ctx, reduce, dim3((unsigned)((total + 255) / 256)), 256, 0, ctx->use_pdl, d_out, ldo, P.part, P.nch, NV, P.mp, M,
                             P.n_batch, epi, gate);
 }
 

@@ -24,8 +24,8 @@ def run_batch(backend, ctx, m, v):
 SHAPES = [(16, 256), (5, 512), (300, 2816), (1000, 4096), (4096, 4096), (512, 11008), (272, 28672)]
 
 
-# all shapes with a full batch; the smaller instantiations (2 and 4 vectors, partly filled) on two of them
-CASES = [(s, 8) for s in SHAPES] + [(s, nb) for s in ((300, 2816), (1000, 4096)) for nb in (2, 3, 5)]
+# all shapes with a full batch; the instantiations of 2, 4, 6 and 8 vectors, full and partly filled, on two of them
+CASES = [(s, 8) for s in SHAPES] + [(s, nb) for s in ((300, 2816), (1000, 4096)) for nb in range(2, 8)]
 
 
 @pytest.mark.parametrize("fmt", FMTS)
