@@ -187,21 +187,6 @@ SLAI_HD uint32_t byte_of(uint32_t w, int i) {
 #endif
 }
 
-// The lanes' shares of a pair of vectors (`compute_pairs`) added to one accumulator per vector (zero in the lanes of the other).
-template <class F, int NV>
-SLAI_HD void batch_from_pairs(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t vs, float (&accA)[NV], float (&accB)[NV]) {
-    float a[NV / 2], b[NV / 2];
-    for (int p = 0; p < NV / 2; p++) a[p] = b[p] = 0.f;
-    F::template compute_pairs<NV>(blk, step, L, S, vs, a, b);
-    for (int p = 0; p < NV / 2; p++) {
-        const bool second = (L.t >> 1) != 0;
-        accA[2 * p] += second ? 0.f : a[p];
-        accA[2 * p + 1] += second ? a[p] : 0.f;
-        accB[2 * p] += second ? 0.f : b[p];
-        accB[2 * p + 1] += second ? b[p] : 0.f;
-    }
-}
-
 // Every format provides
 //   STEP      elements of K per tile-step block          SV_GRAN  elements per digit-sum entry (0: none)
 //   compute   one tile-step block at shared address `blk` (K step number `step`): accumulates rows g and g+8
@@ -352,12 +337,6 @@ struct K45 {
             accB[p] = prim::fma(-mnB, combine(ch[2] * 128 + cl[2], ch[3] * 128 + cl[3], L), accB[p]);
         }
     }
-    template <int NV>
-    SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
-                                      float (&accB)[NV]) {
-        (void)bvs;
-        batch_from_pairs<K45, NV>(blk, step, L, S, svs, accA, accB);
-    }
 };
 using Q4K = K45<false>;
 using Q5K = K45<true>;
@@ -499,12 +478,6 @@ struct Q80 {
                 }
             }
         }
-    }
-    template <int NV>
-    SLAI_HD static void compute_batch(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t bvs, uint32_t svs, float (&accA)[NV],
-                                      float (&accB)[NV]) {
-        (void)bvs;
-        batch_from_pairs<Q80, NV>(blk, step, L, S, svs, accA, accB);
     }
 };
 

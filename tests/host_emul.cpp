@@ -1,7 +1,7 @@
 // CPU emulation of one warp of the dequant-GEMV kernel: 32 host threads play the lanes, the MMA and the
 // shared-memory loads are emulated (slai_b200/csrc/gemv_formats.cuh), everything else is the kernel's own
 // source.  Usage: host_emul <fmt> <K> <blocks.bin (16 rows, GGUF order)> <v.bin (K f32)>  -> prints 16 floats;
-// with a fifth argument NV (2, 4 or 8) v.bin holds NV vectors, the batched per-lane code runs and NV x 16 floats are printed.
+// with a fifth argument NV (2, 4, 6 or 8) v.bin holds NV vectors, the batched per-lane code runs and NV x 16 floats are printed.
 // Compiled for the host only; it never touches a GPU.
 #include <cmath>
 #include <cstdio>
@@ -47,10 +47,20 @@ template <class F, int NV>
 static void lane_body_batch(Job* J, int lane) {
     LaneCtx L;
     lane_init<F>(L, lane, J->S);
-    const uint32_t bvs = L.bmul ? J->vstride : 0u;
     float a[NV], b[NV];
     for (int v = 0; v < NV; v++) a[v] = b[v] = 0.f;
-    for (int s = 0; s < J->nsteps; s++) F::template compute_batch<NV>(J->tile0 + (uint32_t)s * J->step_bytes, s, L, J->S, bvs, J->vstride, a, b);
+    if constexpr (F::PAIRED) {  // a lane's share of a pair belongs to one of its two vectors
+        float pa[NV / 2], pb[NV / 2];
+        for (int p = 0; p < NV / 2; p++) pa[p] = pb[p] = 0.f;
+        for (int s = 0; s < J->nsteps; s++) F::template compute_pairs<NV>(J->tile0 + (uint32_t)s * J->step_bytes, s, L, J->S, J->vstride, pa, pb);
+        for (int p = 0; p < NV / 2; p++) {
+            a[2 * p + (L.t >> 1)] = pa[p];
+            b[2 * p + (L.t >> 1)] = pb[p];
+        }
+    } else {
+        const uint32_t bvs = L.bmul ? J->vstride : 0u;
+        for (int s = 0; s < J->nsteps; s++) F::template compute_batch<NV>(J->tile0 + (uint32_t)s * J->step_bytes, s, L, J->S, bvs, J->vstride, a, b);
+    }
     for (int v = 0; v < NV; v++) {
         J->bacc[lane][v][0] = a[v];
         J->bacc[lane][v][1] = b[v];
@@ -62,6 +72,7 @@ static void lane_dispatch(Job* J, int lane) {
         case 0: lane_body<F>(J, lane); break;
         case 2: lane_body_batch<F, 2>(J, lane); break;
         case 4: lane_body_batch<F, 4>(J, lane); break;
+        case 6: lane_body_batch<F, 6>(J, lane); break;
         case 8: lane_body_batch<F, 8>(J, lane); break;
     }
 }
@@ -100,7 +111,7 @@ int main(int argc, char** argv) {
     const float* vall = (const float*)vb.data();
     const int nv = argc > 5 ? atoi(argv[5]) : 0;
     const int nvec = nv > 0 ? nv : 1;
-    if (nv != 0 && nv != 2 && nv != 4 && nv != 8) return 2;
+    if (nv != 0 && nv != 2 && nv != 4 && nv != 6 && nv != 8) return 2;
     const int be = fmt == 8 ? 32 : 256, bb = fmt == 8 ? 34 : fmt == 12 ? 144 : fmt == 13 ? 176 : 210;
     const int nbk = K / be;
     if ((int)raw.size() != 16 * nbk * bb || (int)vb.size() != 4 * K * nvec) { fprintf(stderr, "size mismatch\n"); return 2; }

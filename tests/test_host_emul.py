@@ -43,7 +43,8 @@ def test_emulated_warp_matches_oracle(emul, tmp_path, fmt, K, kind):
 
 
 BATCH_CASES = [(synth.FMT_Q4_K, 512, 8), (synth.FMT_Q4_K, 2816, 4), (synth.FMT_Q5_K, 768, 8), (synth.FMT_Q5_K, 256, 2), (synth.FMT_Q6_K, 512, 8),
-               (synth.FMT_Q6_K, 2816, 2), (synth.FMT_Q8_0, 288, 8), (synth.FMT_Q8_0, 1600, 4)]
+               (synth.FMT_Q6_K, 2816, 2), (synth.FMT_Q8_0, 288, 8), (synth.FMT_Q8_0, 1600, 4), (synth.FMT_Q4_K, 768, 6), (synth.FMT_Q6_K, 256, 6),
+               (synth.FMT_Q8_0, 288, 6)]
 
 
 @pytest.mark.parametrize("fmt,K,nv", BATCH_CASES)
