@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(ATT_THREADS, SLAI_ATT_MINB) attn_kernel(const 
 #endif
     // The grid is sized for the longest context; the blocks of splits the current context does not use leave at once,
     // while the predecessor still runs, when the position is known not to be written by it.
-    if (P.early && P.batch == 0 && (int)blockIdx.y >= attn_splits(P, __ldcg(P.d_pos) + 1)) return;
+    if (P.early && P.batch == 0 && (int)blockIdx.y >= attn_splits<HSF, (int)sizeof(T)>(P, __ldcg(P.d_pos) + 1)) return;
     prefetch_plan_issue(P.ahead, (int)(blockIdx.x + gridDim.x * blockIdx.y), (int)(gridDim.x * gridDim.y), (int)threadIdx.x, ATT_THREADS);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next kernel may start fetching its weights
@@ -44,11 +44,11 @@ __global__ void __launch_bounds__(ATT_THREADS, SLAI_ATT_MINB) attn_kernel(const 
         Q.kc = reinterpret_cast<const char*>(P.kc) + (size_t)b * P.cache_bs;
         Q.vc = reinterpret_cast<const char*>(P.vc) + (size_t)b * P.cache_bs;
         const int n = (P.seq_pos ? __ldcg(P.seq_pos + b) : P.pos0 + b) + 1;
-        const int ns = n > 0 ? attn_splits(Q, n) : 0;  // a sequence left out of the step (negative position): nothing to do
+        const int ns = n > 0 ? attn_splits<HSF, (int)sizeof(T)>(Q, n) : 0;  // a sequence left out of the step (negative position): nothing to do
         if ((int)blockIdx.y < ns) attn_item<T, MAXQ, HSF>(Q, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
     } else {
         const int n = __ldcg(P.d_pos) + 1;
-        const int ns = attn_splits(P, n);
+        const int ns = attn_splits<HSF, (int)sizeof(T)>(P, n);
         if ((int)blockIdx.y < ns) attn_item<T, MAXQ, HSF>(P, blockIdx.x, blockIdx.y, ns, n, threadIdx.x, sm, 0);
     }
 #ifdef SLAI_TRACE
@@ -151,11 +151,6 @@ static int attn_geometry(slai_ctx* ctx, AttnParams& P, int kv_dtype, int n_max, 
     SLAI_REQUIRE(ctx, (bits & 3) == 0, SLAI_ERR_INVALID_ARG, "attention: caches and strides must be 4-byte aligned");
     P.vec16 = ((bits | (uintptr_t)seq_stride) & 15) == 0;
     P.regs = attn_in_registers(P, esz, max_q);
-    // The register path of f32 caches: splits of 32 positions, not of one staged tile (16) -- at position 515 that is one round of
-    // blocks instead of two, and half of the partial outputs to merge.  A short context has too few blocks for that and keeps
-    // splits of 16 (32 query heads on 16, position 150: 50.5 -> 49.0 us per token and layer, 48.5 staged).
-    P.split_short = P.tile_pos;
-    if (P.regs && esz == 4) P.tile_pos = 32;
     *smem = attn_item_bytes(P.kv_mul, P.hs, esz, P.tile_pos, P.n_splits);
     SLAI_REQUIRE(ctx, *smem <= 160 * 1024, SLAI_ERR_SHAPE, "attention: shared memory %zu too large", *smem);
     return SLAI_OK;

@@ -19,7 +19,6 @@ struct AttnParams {
     int early = 0;  // the position scalar is final before this kernel's blocks can start (AttnLaunch::pos_stable): read it before the wait
     int n_splits;   // most splits a KV head is cut into (stride of the partial buffers)
     int tile_pos;   // positions staged in shared memory at a time
-    int split_short;  // positions of a split while the context is at most 256 positions
     int vec16;      // rows can be copied in 16-byte pieces (alignment of bases, strides and row length)
     int regs = 0;   // keys and values stay in registers (attn_in_registers)
     float* out;
@@ -68,9 +67,13 @@ __host__ __device__ inline int attn_tile_pos(int hs, int esz) {
     int t = (8192 / (hs * esz)) & ~7;
     return t < 8 ? 8 : t > 32 ? 32 : t;
 }
-// Splits actually used at `n` positions: one per tile, up to the maximum.
+// Splits actually used at `n` positions: one per tile, up to the maximum.  The register path has no tiles; with f32 caches a staged
+// one would be 16 positions: splits of 32 are one round of blocks instead of two at position 515, and half of the partial outputs
+// to merge, but a short context has too few blocks for that (32 query heads on 16, position 150: 50.5 us per token and layer
+// with splits of 32, 49.0 with 16, 48.5 staged).
+template <int HSF, int ESZ>
 __device__ __forceinline__ int attn_splits(const AttnParams& P, int n) {
-    const int per = n <= 256 ? P.split_short : P.tile_pos;
+    const int per = HSF == 0 ? P.tile_pos : ESZ == 4 && n <= 256 ? 16 : 32;
     const int want = (n + per - 1) / per;
     return want < 1 ? 1 : want > P.n_splits ? P.n_splits : want;
 }
