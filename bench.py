@@ -56,19 +56,23 @@ def measured_tensor_peak():
     return 1400.0, "fallback (1.4 PFLOP/s sustained, earlier measurement on this pool)"
 
 
-def prefill_record(cfg, n_tokens, seconds, sequential_ms_per_token=None, n_gpus=1):
+def prefill_record(cfg, fmt, n_tokens, seconds, sequential_ms_per_token=None, n_gpus=1):
     """Prompt processing of `n_tokens` through the tensor-core GEMM path: model FLOPs = 2 x layer weights x tokens (the
-    logits matrix is applied to the last token only).  Every model product is issued as three fp16 products
-    (hi*hi, hi*lo, lo*hi of fp16 operand pairs, f32 accumulation), so the tensor cores execute three times the model
-    FLOPs; both figures are given against the measured dense bf16 peak (of all `n_gpus` GPUs for a sharded model, whose
-    ranks each run their shard of every GEMM and sum the row-parallel products with an all-reduce)."""
+    logits matrix is applied to the last token only).  Activations are fp16 pairs (hi + lo): Q4_K and Q5_K weights go in
+    as exact integers, two fp16 products per model product; Q6_K and Q8_0 as pairs too, three (hi*hi, hi*lo, lo*hi).  The
+    tensor cores execute that many times the model FLOPs; both figures are given against the measured dense bf16 peak (of
+    all `n_gpus` GPUs for a sharded model, whose ranks each run their shard of every GEMM and sum the row-parallel
+    products with an all-reduce)."""
+    from slai_b200 import synth
+    products = 2 if fmt in (synth.FMT_Q4_K, synth.FMT_Q5_K) else 3
     peak, src = measured_tensor_peak()
     peak *= n_gpus
     layer_params = sum(r * c for r, c in cfg.matrix_shapes().values())
     flops = 2.0 * cfg.n_layers * layer_params * n_tokens
     rec = {"tokens": n_tokens, "seconds": seconds, "tok_s": n_tokens / seconds, "model_tflops": flops / seconds / 1e12,
-           "tensor_tflops_executed": 3 * flops / seconds / 1e12, "operands": "fp16 pairs (hi + lo) for weights and activations, f32 accumulators in TMEM",
-           "peak_tflops": peak, "frac_model": flops / seconds / 1e12 / peak, "frac_executed": 3 * flops / seconds / 1e12 / peak, "peak_source": src}
+           "tensor_tflops_executed": products * flops / seconds / 1e12, "products_per_model_product": products,
+           "operands": "activations as fp16 pairs (hi + lo), weights as " + ("exact fp16 integers" if products == 2 else "fp16 pairs") + ", f32 accumulators in TMEM",
+           "peak_tflops": peak, "frac_model": flops / seconds / 1e12 / peak, "frac_executed": products * flops / seconds / 1e12 / peak, "peak_source": src}
     if sequential_ms_per_token:
         rec["sequential_estimate_s"] = sequential_ms_per_token * 1e-3 * n_tokens
         rec["speedup_vs_sequential"] = rec["sequential_estimate_s"] / seconds
@@ -461,7 +465,7 @@ def measure_tp(args, group, n_layers=0, prompt_len=1024, steps=None, warmup=None
                           "prompt_len": PL, "decode_positions": [pos, pos + K - 1], "parallelism": f"tp{world}", "exchange": exchange,
                           "logits": "output matrix sharded by rows, logits all-gathered" if world > 1 else "whole output matrix"},
                "prefill_s": prefill_s,
-               "prefill": prefill_record(cfg, PL - 1, prefill_s, ms / K, n_gpus=world),
+               "prefill": prefill_record(cfg, synth.FMT_Q4_K, PL - 1, prefill_s, ms / K, n_gpus=world),
                "clocks": clocks, "launches_per_token": m.launches_per_token(), "gpu_launches": m.launches_per_token() * K,
                "ranks_agree": all(r == ids[0] for r in ids), "nccl_and_peer_exchange_bit_identical": identical, "batch8": batch,
                "roofline": {"bound": "hbm", "per_gpu_bytes_per_token": per_rank + kv, "achieved": (per_rank + kv) / t / 1e9, "peak": peak,
@@ -638,7 +642,7 @@ def main():
             "config": workload_config(world, K, W),
             "clocks": clocks,
             "e2e": {"value": e2e, "unit": "tok/s", "h2d_bytes_per_step": 16, "d2h_bytes_per_step": cfg.vocab_size * 4 + 4},
-            "prefill": prefill_record(cfg, PROMPT_LEN - 1, prefill_s, ms / K),
+            "prefill": prefill_record(cfg, synth.FMT_Q4_K, PROMPT_LEN - 1, prefill_s, ms / K),
             "gpu_launches": launches_per_token * K,
             "launches_per_token": launches_per_token,
             "token_roofline": {"bytes_per_token": token_bytes, "roofline_tok_s": peak * 1e9 / token_bytes,
