@@ -151,7 +151,7 @@ __device__ __forceinline__ void copy_rows_u32(const unsigned char* g, size_t row
 // memory: a group of lanes holds one cached row (16 bytes per lane), takes every GB-th position of the split, four at a time
 // with the next four on their way, and keeps its own running softmax; the groups meet once at the end.  The staged
 // path below costs four block barriers and about 1700 warp instructions per tile of 32 positions; at position 515 the f32
-// cache of the 7B shape took 19.3 us per layer, 14.1 this way (f16: 7.5 and 7.5, twice as many rows per load).
+// cache of the 7B shape took 19.3 us per layer, 14.1 this way.  Figures of both paths by shape: attn_in_registers.
 template <typename T, int MAXQ, int HSF>
 __device__ __forceinline__ void attn_item(const AttnParams& P, int kvh, int split, int ns, int n, int tid, unsigned char* smb, int bar_id) {
     constexpr int ESZ = (int)sizeof(T);

@@ -262,8 +262,8 @@ struct K45 {
     // zeros.  Lane t collects digits 2(t & 1), 2(t & 1) + 1 of vector 2p + (t >> 1) for rows g and g + 8: accA[p] / accB[p]
     // are that lane's share, the sum over lanes t, t ^ 1 is the vector's.  Against one vector per MMA (columns = digits x two
     // sub-blocks, half of B zero) this halves the MMAs, the loads of B and the integer scale multiplies: they are what bounds the
-    // batched kernel (Q5_K 4096 x 11008, 8 vectors: 24.6 -> 20.5 us).  Vector v's digits are at S.dig + v * vs, its sum table
-    // at S.sv + v * vs.
+    // batched kernel (Q5_K 4096 x 11008, 8 vectors: 24.6 -> 20.5 us then, 19.8 with what came after).
+    // Vector v's digits are at S.dig + v * vs, its sum table at S.sv + v * vs.
     static constexpr bool PAIRED = true;
     template <int NV>
     SLAI_HD static void compute_pairs(uint32_t blk, int step, const LaneCtx& L, const Smem& S, uint32_t vs, float (&accA)[NV / 2], float (&accB)[NV / 2]) {

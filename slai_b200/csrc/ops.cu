@@ -947,7 +947,8 @@ int launch_argmax(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, bool
     return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX,
                       LoopState{});
 }
-// The greedy choice and, in the same launch, the loop's advance (a launch less per token; tiny model, 64 tokens: 7.93 -> 7.80 ms).
+// The greedy choice and, in the same launch, the loop's advance (a launch less per token;
+// tiny model, 64 tokens: 7.91 -> 7.86 ms, no more than runs differ).
 int launch_argmax_advance(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, int* d_token, int* d_pos, int32_t* d_history, bool pdl) {
     return launch_pdl(ctx, argmax_kernel, dim3(ARG_BLOCKS), dim3(ARG_THREADS), pdl, v, (long long)n, (int*)d_out, ctx->d_counters + CNT_ARGMAX,
                       LoopState{d_token, d_pos, (int*)d_history, (int)n});
