@@ -10,8 +10,8 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libslai_b200.so")
-SOURCES = ["gemv.cu", "gemv_batch.cu", "attention.cu", "ops.cu", "model.cu", "tp.cu", "sampler.cu", "prefill.cu", "prefill_gemm.cu"]
-HEADERS = ["common.cuh", "dequant.cuh", "gemv_frag.cuh", "gemv_formats.cuh", "gemv_kernel.cuh", "attention.cuh", "layout.cuh", "prefill_dequant.cuh", os.path.join("..", "..", "include", "slai_b200.h")]
+SOURCES = ["decode_layers_q5k.cu", "decode_layers_q4k.cu", "decode_layers_q6k.cu", "decode_layers_q80.cu", "decode_layers.cu", "gemv.cu", "gemv_batch.cu", "attention.cu", "ops.cu", "model.cu", "tp.cu", "sampler.cu", "prefill.cu", "prefill_gemm.cu"]
+HEADERS = ["common.cuh", "dequant.cuh", "gemv_frag.cuh", "gemv_formats.cuh", "gemv_kernel.cuh", "decode_layers.cuh", "decode_layers.h", "attention.cuh", "layout.cuh", "prefill_dequant.cuh", os.path.join("..", "..", "include", "slai_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-fvisibility=hidden"]
 

@@ -326,9 +326,9 @@ const float* rope_table(slai_ctx* ctx, int head_size, float base);
 
 // ops.cu helpers used by the models
 int launch_embed_f32(slai_ctx* ctx, float* x, const float* table, int dim, const int* d_token, const float* wpe,
-                     const int* d_pos, bool pdl, const float* rope_theta = nullptr, float* rope_cs = nullptr, int rope_half = 0);
+                     const int* d_pos, bool pdl, const float* rope_theta = nullptr, float* rope_cs = nullptr, int rope_half = 0, unsigned int* zero = nullptr);  // zero: a word to clear
 int launch_embed_q8(slai_ctx* ctx, float* x, const slai_qmatrix* wte, const int* d_token, const float* wpe,
-                    const int* d_pos, bool pdl, const float* rope_theta = nullptr, float* rope_cs = nullptr, int rope_half = 0);
+                    const int* d_pos, bool pdl, const float* rope_theta = nullptr, float* rope_cs = nullptr, int rope_half = 0, unsigned int* zero = nullptr);  // zero: a word to clear
 int launch_argmax(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, bool pdl);
 int launch_argmax_advance(slai_ctx* ctx, const float* v, int64_t n, int32_t* d_out, int* d_token, int* d_pos, int32_t* d_history, bool pdl);
 int launch_argmax_rows(slai_ctx* ctx, const float* v, int64_t n, int rows, int32_t* d_out, bool pdl);  // v [rows][n]

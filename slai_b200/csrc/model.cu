@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "decode_layers.h"
 
 namespace {
 
@@ -127,6 +128,7 @@ struct slai_llama {
     void* attn_scratch = nullptr;
     size_t attn_scratch_bytes = 0;
     const float* rope_theta = nullptr;
+    void* layers_scratch = nullptr;  // all layers in one launch (decode_layers.h): barrier counter, attention partials
     GraphSet graphs;
     int launches = 0;
     // prompt processing as GEMMs (prefill.cu): buffers for `pf_cap` tokens, grown on demand
@@ -189,6 +191,40 @@ static void llama_drop_prefill(slai_llama* m) {
     m->pf_cap = 0;
 }
 
+// The step's layers as one launch (decode_layers.cuh), if these are layers it takes: one format for all their matrices, adjacent-pair
+// RoPE from the table, not sharded, not being timed kernel by kernel.
+static bool llama_one_launch(slai_llama* m, bool table, DecodeLayers& D, std::vector<DecodeLayerPtrs>& layers) {
+    const slai_llama_config& c = m->cfg;
+    if (m->tp != 1 || m->ctx->stats_on || !table) return false;
+    layers.resize(c.n_layers);
+    const int fmt = m->layers[0].wq ? m->layers[0].wq->fmt : -1;
+    for (int l = 0; l < c.n_layers; l++) {
+        const LlamaLayer& w = m->layers[l];
+        const slai_qmatrix* ws[7] = {w.wq, w.wk, w.wv, w.wo, w.wgate, w.wup, w.wdown};
+        DecodeLayerPtrs& d = layers[l];
+        d = DecodeLayerPtrs();
+        for (int i = 0; i < 7; i++) {
+            if (!ws[i] || ws[i]->fmt != fmt) return false;
+            d.w[i] = ws[i]->data;
+        }
+        if (!w.attn_norm || !w.ffn_norm) return false;
+        d.norm_w[0] = w.attn_norm; d.norm_w[1] = w.ffn_norm;
+        d.bias[0] = w.bq; d.bias[1] = w.bk; d.bias[2] = w.bv;
+    }
+    D.arch = 0; D.fmt = fmt; D.kv_f16 = c.kv_dtype == SLAI_KV_F16;
+    D.n_layers = c.n_layers; D.dim = c.dim; D.q_dim = m->q_dim; D.kv_dim = m->kv_dim; D.hidden = m->hidden;
+    D.head_size = m->head_size; D.n_heads = m->n_q_local; D.kv_mul = m->kv_mul; D.seq_len = c.seq_len; D.eps = c.rms_norm_eps;
+    D.x = m->x; D.q = m->q; D.xb = m->xb; D.hb = m->hb; D.rope_cs = m->rope_cs; D.d_pos = m->sc.d + 1;
+    D.kcache = m->kcache; D.vcache = m->vcache; D.layer_bytes = m->kv_layer_elems * (D.kv_f16 ? 2 : 4);
+    return decode_layers_supported(m->ctx, D);
+}
+
+// The scratch of the one-launch layers, made by the first step that takes them (never inside a capture: a step's first run is eager).
+static int layers_scratch_reserve(slai_ctx* ctx, const DecodeLayers& D, void** scratch) {
+    if (!*scratch) SLAI_CHECK_CUDA(ctx, cudaMalloc(scratch, decode_layers_scratch_bytes(D)));
+    return SLAI_OK;
+}
+
 static int llama_record(slai_llama* m, int kind) {
     slai_ctx* ctx = m->ctx;
     const slai_llama_config& c = m->cfg;
@@ -199,10 +235,19 @@ static int llama_record(slai_llama* m, int kind) {
     int rc;
     SLAI_REQUIRE(ctx, m->out_norm && (m->token_embd || m->embd_q), SLAI_ERR_INVALID_ARG, "llama: embedding / output norm not set");
     const bool table = c.rope_variant == 0 && m->head_size / 2 <= 256;
-    if (m->embd_q) rc = launch_embed_q8(ctx, m->x, m->embd_q, d_token, nullptr, d_pos, false, m->rope_theta, table ? m->rope_cs : nullptr, m->head_size / 2);
-    else rc = launch_embed_f32(ctx, m->x, m->token_embd, c.dim, d_token, nullptr, d_pos, false, m->rope_theta, table ? m->rope_cs : nullptr, m->head_size / 2);
+    DecodeLayers D;
+    std::vector<DecodeLayerPtrs> dl;
+    const bool one_launch = llama_one_launch(m, table, D, dl);
+    if (one_launch && (rc = layers_scratch_reserve(ctx, D, &m->layers_scratch))) return rc;
+    unsigned int* zero = one_launch ? decode_layers_counter(m->layers_scratch) : nullptr;
+    if (m->embd_q) rc = launch_embed_q8(ctx, m->x, m->embd_q, d_token, nullptr, d_pos, false, m->rope_theta, table ? m->rope_cs : nullptr, m->head_size / 2, zero);
+    else rc = launch_embed_f32(ctx, m->x, m->token_embd, c.dim, d_token, nullptr, d_pos, false, m->rope_theta, table ? m->rope_cs : nullptr, m->head_size / 2, zero);
     if (rc) return rc;
     n++;
+    if (one_launch) {
+        if ((rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch))) return rc;
+        n++;
+    }
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     // A row-parallel GEMV (each rank holds a K range of every row): x += W v.  Sharded: the partial goes to xpart
     // (rank 0 adds the residual), then one sum over the ranks writes x on every rank.
@@ -256,7 +301,7 @@ static int llama_record(slai_llama* m, int kind) {
         n += 2;
         return SLAI_OK;
     };
-    for (int l = 0; l < c.n_layers; l++) {
+    for (int l = one_launch ? c.n_layers : 0; l < c.n_layers; l++) {
         const LlamaLayer& w = m->layers[l];
         SLAI_REQUIRE(ctx, w.wq && w.wk && w.wv && w.wo && w.wgate && w.wup && w.wdown && w.attn_norm && w.ffn_norm,
                      SLAI_ERR_INVALID_ARG, "llama: layer %d has unset weights", l);
@@ -760,7 +805,7 @@ SLAI_API int slai_llama_destroy(slai_llama* m) {
     cudaFree(m->token_embd); cudaFree(m->out_norm);
     cudaFree(m->x); cudaFree(m->xb); cudaFree(m->xpart); cudaFree(m->q); cudaFree(m->hb); cudaFree(m->hb2); cudaFree(m->logits);
     cudaFree(m->logits_part); cudaFree(m->ktmp); cudaFree(m->vtmp);
-    cudaFree(m->kcache); cudaFree(m->vcache); cudaFree(m->sc.d); cudaFree(m->d_history); cudaFree(m->attn_scratch);
+    cudaFree(m->kcache); cudaFree(m->vcache); cudaFree(m->sc.d); cudaFree(m->d_history); cudaFree(m->layers_scratch); cudaFree(m->attn_scratch);
     cudaFree(m->d_samp); cudaFree(m->d_samp_scratch); cudaFree(m->rope_cs);
     delete m;
     return SLAI_OK;
@@ -1166,6 +1211,10 @@ SLAI_API int slai_llama_stats(slai_llama* m, int32_t token, int32_t pos, slai_ll
     ctx->stats_cls.clear();
     if (rc) return rc;
     if (e != cudaSuccess) return slai_set_error(ctx, SLAI_ERR_CUDA, "stats: %s", cudaGetErrorString(e));
+    // What is left behind (cache row, logits) is a plain step's, whose layers may be one launch with sums in another order.
+    if ((rc = set_scalars(m, token, pos, 0))) return rc;
+    if ((rc = llama_record(m, G_DECODE))) return rc;
+    SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return slai_check_wait_flag(ctx);
 }
 
@@ -1233,6 +1282,7 @@ struct slai_gpt2 {
     int history_cap = 0;
     void* attn_scratch = nullptr;
     size_t attn_scratch_bytes = 0;
+    void* layers_scratch = nullptr;  // as slai_llama's
     GraphSet graphs;
     int launches = 0;
     // prompt processing as GEMMs (prefill.cu): buffers for `pf_cap` tokens, grown on demand
@@ -1252,6 +1302,37 @@ static void gpt2_drop_prefill(slai_gpt2* m) {
     m->pf_cap = 0;
 }
 
+static bool gpt2_one_launch(slai_gpt2* m, DecodeLayers& D, std::vector<DecodeLayerPtrs>& layers) {
+    const slai_gpt2_config& c = m->cfg;
+    if (m->ctx->stats_on || c.n_embd % 16) return false;
+    layers.resize(c.n_layer);
+    const int fmt = m->layers[0].w_qkv ? m->layers[0].w_qkv->fmt : -1;
+    if (fmt == SLAI_FMT_F32) return false;
+    for (int l = 0; l < c.n_layer; l++) {
+        const Gpt2Layer& w = m->layers[l];
+        const slai_qmatrix* ws[4] = {w.w_qkv, w.w_proj, w.w_fc, w.w_fcproj};
+        for (const slai_qmatrix* q : ws)
+            if (!q || q->fmt != fmt) return false;
+        if (!w.ln1_g || !w.ln1_b || !w.ln2_g || !w.ln2_b || !w.b_qkv || !w.b_proj || !w.b_fc || !w.b_fcproj) return false;
+        DecodeLayerPtrs& d = layers[l];
+        d = DecodeLayerPtrs();
+        const int E = c.n_embd;
+        for (int i = 0; i < 3; i++) {
+            d.w[i] = w.w_qkv->data + (size_t)(i * E / 16) * w.w_qkv->tile_bytes;
+            d.bias[i] = w.b_qkv + i * E;
+        }
+        d.w[3] = w.w_proj->data; d.w[4] = d.w[5] = w.w_fc->data; d.w[6] = w.w_fcproj->data;
+        d.bias[3] = w.b_proj; d.bias[4] = w.b_fc; d.bias[5] = w.b_fcproj;
+        d.norm_w[0] = w.ln1_g; d.norm_b[0] = w.ln1_b; d.norm_w[1] = w.ln2_g; d.norm_b[1] = w.ln2_b;
+    }
+    D.arch = 1; D.fmt = fmt; D.kv_f16 = c.kv_dtype == SLAI_KV_F16;
+    D.n_layers = c.n_layer; D.dim = D.q_dim = D.kv_dim = c.n_embd; D.hidden = c.ff_len;
+    D.head_size = m->head_size; D.n_heads = c.n_head; D.kv_mul = 1; D.seq_len = c.n_seq; D.eps = c.layernorm_eps;
+    D.x = m->x; D.q = m->q; D.xb = m->xb; D.hb = m->ff; D.d_pos = m->sc.d + 1;
+    D.kcache = m->kcache; D.vcache = m->vcache; D.layer_bytes = m->kv_layer_elems * (D.kv_f16 ? 2 : 4);
+    return decode_layers_supported(m->ctx, D);
+}
+
 static int gpt2_record(slai_gpt2* m, int kind) {
     slai_ctx* ctx = m->ctx;
     const slai_gpt2_config& c = m->cfg;
@@ -1262,10 +1343,20 @@ static int gpt2_record(slai_gpt2* m, int kind) {
     int* d_pos = m->sc.d + 1;
     SLAI_REQUIRE(ctx, m->wte && m->wpe && m->lnf_g && m->lnf_b, SLAI_ERR_INVALID_ARG, "gpt2: embeddings / final norm not set");
     // x = wte[:,tok] + wpe[:,pos]                                              gpt2/cpu.rs:227-228
-    if ((rc = launch_embed_q8(ctx, m->x, m->wte, d_token, m->wpe, d_pos, false))) return rc;
+    DecodeLayers D;
+    std::vector<DecodeLayerPtrs> dl;
+    const bool one_launch = gpt2_one_launch(m, D, dl);
+    if (one_launch && (rc = layers_scratch_reserve(ctx, D, &m->layers_scratch))) return rc;
+    if ((rc = launch_embed_q8(ctx, m->x, m->wte, d_token, m->wpe, d_pos, false, nullptr, nullptr, 0,
+                              one_launch ? decode_layers_counter(m->layers_scratch) : nullptr)))
+        return rc;
     n++;
+    if (one_launch) {
+        if ((rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch))) return rc;
+        n++;
+    }
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
-    for (int l = 0; l < c.n_layer; l++) {
+    for (int l = one_launch ? c.n_layer : 0; l < c.n_layer; l++) {
         const Gpt2Layer& w = m->layers[l];
         SLAI_REQUIRE(ctx, w.w_qkv && w.w_proj && w.w_fc && w.w_fcproj && w.ln1_g && w.ln1_b && w.ln2_g && w.ln2_b && w.b_qkv &&
                               w.b_proj && w.b_fc && w.b_fcproj, SLAI_ERR_INVALID_ARG, "gpt2: layer %d has unset weights", l);
@@ -1388,7 +1479,7 @@ SLAI_API int slai_gpt2_destroy(slai_gpt2* m) {
     }
     cudaFree(m->wpe); cudaFree(m->lnf_g); cudaFree(m->lnf_b);
     cudaFree(m->x); cudaFree(m->xb); cudaFree(m->q); cudaFree(m->ff); cudaFree(m->logits);
-    cudaFree(m->kcache); cudaFree(m->vcache); cudaFree(m->sc.d); cudaFree(m->d_history); cudaFree(m->attn_scratch);
+    cudaFree(m->kcache); cudaFree(m->vcache); cudaFree(m->sc.d); cudaFree(m->d_history); cudaFree(m->layers_scratch); cudaFree(m->attn_scratch);
     gpt2_drop_prefill(m);
     delete m;
     return SLAI_OK;

@@ -101,7 +101,7 @@ int slai_check_wait_flag(slai_ctx* ctx) {
     if (flag) {
         cudaMemset(ctx->d_counters + CNT_ERR_FLAG, 0, sizeof(flag));
         return slai_set_error(ctx, SLAI_ERR_TIMEOUT, "a bounded wait inside a kernel ran out (%s); results of the last launches are invalid",
-                              flag == 1 ? "weight ring" : flag == 5 ? "prompt product" : flag == 6 ? "batched product" : "tensor-parallel peer");
+                              flag == 1 ? "weight ring" : flag == 2 ? "barrier of a decode step" : flag == 5 ? "prompt product" : flag == 6 ? "batched product" : "tensor-parallel peer");
     }
     return SLAI_OK;
 }
@@ -760,8 +760,9 @@ __device__ __forceinline__ void rope_pairs(const float* theta, float* cs, int ha
     }
 }
 __global__ void embed_f32_kernel(float* x, const float* table, int dim, const int* d_token, const float* wpe, const int* d_pos,
-                                 const float* theta, float* cs, int half) {
+                                 const float* theta, float* cs, int half, unsigned int* zero) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;
     rope_pairs(theta, cs, half, d_pos);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= dim) return;
@@ -770,8 +771,9 @@ __global__ void embed_f32_kernel(float* x, const float* table, int dim, const in
     x[i] = y;
 }
 __global__ void embed_q_kernel(float* x, int fmt, const uint8_t* data, int dim, const int* d_token, const float* wpe,
-                               const int* d_pos, const float* theta, float* cs, int half) {
+                               const int* d_pos, const float* theta, float* cs, int half, unsigned int* zero) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;
     rope_pairs(theta, cs, half, d_pos);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= dim) return;
@@ -959,15 +961,15 @@ int launch_argmax_rows(slai_ctx* ctx, const float* v, int64_t n, int rows, int32
                       LoopState{});
 }
 int launch_embed_f32(slai_ctx* ctx, float* x, const float* table, int dim, const int* d_token, const float* wpe,
-                     const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half) {
+                     const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half, unsigned int* zero) {
     return launch_pdl(ctx, embed_f32_kernel, dim3((dim + NT - 1) / NT), dim3(NT), pdl, x, table, dim, d_token, wpe, d_pos, rope_theta,
-                      rope_cs, rope_half);
+                      rope_cs, rope_half, zero);
 }
 int launch_embed_q8(slai_ctx* ctx, float* x, const slai_qmatrix* wte, const int* d_token, const float* wpe,
-                    const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half) {
+                    const int* d_pos, bool pdl, const float* rope_theta, float* rope_cs, int rope_half, unsigned int* zero) {
     const int dim = (int)wte->ncols;
     return launch_pdl(ctx, embed_q_kernel, dim3((dim + NT - 1) / NT), dim3(NT), pdl, x, wte->fmt, (const uint8_t*)wte->data, dim,
-                      d_token, wpe, d_pos, rope_theta, rope_cs, rope_half);
+                      d_token, wpe, d_pos, rope_theta, rope_cs, rope_half, zero);
 }
 int launch_advance(slai_ctx* ctx, int* d_token, int* d_pos, const int32_t* d_next, int32_t* d_history, int vocab, bool pdl) {
     // d_history[-1] is not used; the step counter lives right after the position scalar (see models)

@@ -1,0 +1,80 @@
+"""The layers of a decode step in one launch (decode_layers.cuh) against the oracle, at the edges of its dispatch: one cluster of blocks or the whole chip,
+splits of the positions (more positions than a round of lane groups holds), one or two query heads an item, widths that are not multiples of a digit step,
+both cache types, every format.  Bars as in test_gpu_models.py: 1e-3 relative L2 of the logits, two orders above what is measured."""
+import threading
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from slai_b200 import _lib, synth
+from slai_b200.models import Gpt2Params, Llama2Config, gpt2_from_host, llama_from_host, synthetic_gpt2_host, synthetic_llama_device, synthetic_llama_host
+from slai_b200.ops import Backend
+from helpers import oracle_gpt2, oracle_llama, rel_l2
+
+pytestmark = pytest.mark.gpu
+F16, F32 = _lib.KV_F16, _lib.KV_F32
+
+
+@pytest.mark.parametrize("dim,hidden,hq,hkv,fmt,kv,n", [
+    (256, 512, 4, 4, synth.FMT_Q4_K, F16, 70),      # one cluster
+    (288, 768, 6, 6, synth.FMT_Q8_0, F32, 40),      # 48-wide heads, half-empty steps
+    (512, 1280, 4, 4, synth.FMT_Q6_K, F32, 200),    # one cluster, up to four splits of 64 positions
+    (512, 1280, 8, 2, synth.FMT_Q5_K, F16, 140),    # two query heads an item
+    (1024, 2816, 8, 8, synth.FMT_Q4_K, F16, 140),   # the whole chip, 128 positions to a round
+    (1024, 2816, 16, 4, synth.FMT_Q8_0, F32, 140),  # two query heads an item, blocks without items
+])
+def test_decode_against_the_oracle(backend, dim, hidden, hq, hkv, fmt, kv, n):
+    cfg = Llama2Config(dim=dim, hidden_dim=hidden, n_layers=2, n_q_heads=hq, n_kv_heads=hkv, vocab_size=400, seq_len=n, kv_dtype=kv)
+    w = synthetic_llama_host(cfg, fmt, seed=11, std=0.05, embd_std=1.0)
+    m = llama_from_host(backend, cfg, w, fmt)
+    ref = oracle_llama(cfg, w, fmt, kv_f16=kv == F16)
+    toks = np.random.default_rng(2).integers(0, cfg.vocab_size, size=n)
+    for pos, tok in enumerate(toks):
+        got = m.forward_logits(pos, int(tok))[0]
+        want = ref.forward(int(tok), pos)
+        if pos < 3 or pos % 16 < 2 or pos == n - 1:
+            assert rel_l2(got, want) < 1e-3, pos
+            assert rel_l2(m.read_state("x"), ref.x()) < 1e-3, pos
+    assert m.launches_per_token() == 4  # embedding, layers, logits, greedy choice
+    m.close()
+
+
+def test_gpt2_decode_against_the_oracle(backend):
+    p = Gpt2Params(n_vocab=300, n_seq=300, n_embd=960, n_head=15, n_layer=2, ff_len=3840, kv_dtype=F16)
+    w = synthetic_gpt2_host(p, synth.FMT_Q8_0, seed=4, std=0.05)
+    m = gpt2_from_host(backend, p, w, synth.FMT_Q8_0)
+    ref = oracle_gpt2(p, w, kv_f16=True)
+    toks = np.random.default_rng(3).integers(0, p.n_vocab, size=p.n_seq)
+    for pos, tok in enumerate(toks):  # 256 positions to a round: the last 44 tokens have two splits
+        got = m.forward(int(tok), pos)[0]
+        want = ref.forward(int(tok), pos)
+        if pos < 3 or pos % 32 < 2 or pos == p.n_seq - 1:
+            assert rel_l2(got, want) < 1e-3, pos
+    m.close()
+
+
+def test_two_contexts_decode_at_the_same_time():
+    """Two threads, two streams: launches whose blocks wait on one another share the chip (one after the other, or side by side where both fit)."""
+    shapes = [dict(dim=1024, hidden_dim=2816, n_q_heads=8, n_kv_heads=8), dict(dim=256, hidden_dim=768, n_q_heads=4, n_kv_heads=4)]
+    models = []
+    for i, sh in enumerate(shapes * 2):
+        be = Backend(0)
+        cfg = Llama2Config(n_layers=4, vocab_size=500, seq_len=80, kv_dtype=F16, **sh)
+        models.append((be, synthetic_llama_device(be, cfg, synth.FMT_Q4_K, synth.FMT_Q4_K, seed=1 + i, std=0.05)))
+    alone = [list(m.generate(3, 0, 64)) for _, m in models]
+    got = [None] * len(models)
+
+    def work(i):
+        for _ in range(3):
+            got[i] = list(models[i][1].generate(3, 0, 64))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(models))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got == alone
+    for be, m in models:
+        m.close()
+        be.close()
