@@ -47,6 +47,7 @@ struct slai_ctx {
     unsigned long long trace_launches = 0;
     unsigned long long* tl = nullptr;         // trace build only: the launch timeline
     unsigned int* d_counters = nullptr;  // CNT_WORDS zeroed words, see the map below
+    unsigned int prompt_seq = 0;         // prompt GEMM launches so far
     unsigned int wait_limit = 1u << 20;  // rounds a bounded device-side wait polls before it gives up (slai_ctx_set_wait_limit)
     // tensor-parallel group (tp.cu): NCCL communicator of this context's rank, null when not sharded
     void* tp_comm = nullptr;
@@ -77,6 +78,8 @@ constexpr int CNT_ATTN_TICKETS = 0;    // one ticket per KV head (<= 1024): last
 constexpr int CNT_ARGMAX = 1100;       // ticket, then per-block (value, index) pairs of the multi-block argmax
 constexpr int CNT_ATTN_POS = 2048;     // position scalar of the stand-alone slai_attention
 constexpr int CNT_ERR_FLAG = 3000;     // raised by a bounded wait that ran out (1 weight ring, 2 grid barrier, 3 peer exchange)
+constexpr int CNT_PROMPT_FLAGS = 3072;  // one word per CTA of a prompt GEMM: the launch whose partial sums it has left (PgParams::seq)
+constexpr int CNT_PROMPT_FLAG_WORDS = 512;
 constexpr int CNT_WORDS = 4096;
 
 int slai_set_error(slai_ctx* ctx, int code, const char* fmt, ...);

@@ -14,8 +14,7 @@
 //                 d as above.
 //   Q8_0          d * q: fp16 pair hi + lo, the same two halves as rounding the f32 product and its remainder.
 //
-// Thread (row r16 of a 16-row tile, part) serves 32 of the 64 columns of a stage and writes 16-byte chunks of 8 halves;
-// chunk c of row r sits at chunk position c ^ (r & 7) of the row's 128 bytes (the 128-byte swizzle of the tensor core).
+// Thread (row r16 of a 16-row tile, part) serves 32 of the 64 columns of a stage.
 #pragma once
 #include <cuda_fp16.h>
 #include <stdint.h>
@@ -84,9 +83,10 @@ SLAI_HD void put(unsigned char* plane, int r, int c, const uint32_t (&v)[4]) {
     *reinterpret_cast<uint4*>(plane + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-// Row r (of the 128 of the CTA) of the stage's operand planes.
+// A row's 32 of the 64 columns of a stage as pairs of halves, hi (and lo) plane: words 0-7 and 8-15 are columns 16 part .. and 32 + 16 part ..
+// (Q8_0: all sixteen are columns 32 part ..).
 template <int FMT>
-SLAI_HD void emit(const Packed& P, int r, int part, int st, unsigned char* hi, unsigned char* lo) {
+SLAI_HD void make(const Packed& P, int st, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
     const uint32_t w0[4] = {P.q[0].x, P.q[0].y, P.q[0].z, P.q[0].w};
     const uint32_t w1[4] = {P.q[1].x, P.q[1].y, P.q[1].z, P.q[1].w};
     if (FMT == 12 || FMT == 13) {
@@ -95,23 +95,16 @@ SLAI_HD void emit(const Packed& P, int r, int part, int st, unsigned char* hi, u
         const __half2 sh16 = FMT == 12 ? __hmul2(sh, h2(0x2C002C00u)) : sh;                       // sc / 16 (the high nibble goes in as 16 q)
         const __half2 oh = __hmul2(sh16, h2(0xE400E400u));
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-            uint32_t lw[4], hw[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t w = w0[2 * c + (i >> 1)];
-                const uint32_t p = frag::perm_bytes(w, 0u, (i & 1) ? 0x4342 : 0x4140);  // two bytes, one per half
-                if (FMT == 12) {
-                    lw[i] = bits(fma2(h2((p & 0x000F000Fu) | 0x64006400u), sl, ol));
-                    hw[i] = bits(fma2(h2((p & 0x00F000F0u) | 0x64006400u), sh16, oh));
-                } else {
-                    const uint32_t h = frag::perm_bytes(w1[2 * c + (i >> 1)], 0u, (i & 1) ? 0x4342 : 0x4140) >> (2 * st);
-                    lw[i] = bits(fma2(h2((p & 0x000F000Fu) | ((h & 0x00010001u) << 4) | 0x64006400u), sl, ol));
-                    hw[i] = bits(fma2(h2(((p >> 4) & 0x000F000Fu) | ((h & 0x00020002u) << 3) | 0x64006400u), sh16, oh));
-                }
+        for (int i = 0; i < 8; i++) {
+            const uint32_t p = frag::perm_bytes(w0[i >> 1], 0u, (i & 1) ? 0x4342 : 0x4140);  // two bytes, one per half
+            if (FMT == 12) {
+                hi[i] = bits(fma2(h2((p & 0x000F000Fu) | 0x64006400u), sl, ol));
+                hi[8 + i] = bits(fma2(h2((p & 0x00F000F0u) | 0x64006400u), sh16, oh));
+            } else {
+                const uint32_t h = frag::perm_bytes(w1[i >> 1], 0u, (i & 1) ? 0x4342 : 0x4140) >> (2 * st);
+                hi[i] = bits(fma2(h2((p & 0x000F000Fu) | ((h & 0x00010001u) << 4) | 0x64006400u), sl, ol));
+                hi[8 + i] = bits(fma2(h2(((p >> 4) & 0x000F000Fu) | ((h & 0x00020002u) << 3) | 0x64006400u), sh16, oh));
             }
-            put(hi, r, 2 * part + c, lw);
-            put(hi, r, 4 + 2 * part + c, hw);
         }
     } else if (FMT == 14) {
         const uint32_t h4[4] = {P.qh.x, P.qh.y, P.qh.z, P.qh.w};
@@ -119,38 +112,42 @@ SLAI_HD void emit(const Packed& P, int r, int part, int st, unsigned char* hi, u
         for (int u = 0; u < 2; u++) {  // quarter 2 (st & 1) + u of the half super-block
             const __half2 s = __half2half2(__short2half_rn((short)(signed char)((P.sc >> (8 * u)) & 0xFFu)));
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t hw[4], lw[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const uint32_t w = u ? w1[2 * c + (i >> 1)] : w0[2 * c + (i >> 1)];
-                    const uint32_t sel = (i & 1) ? 0x4342 : 0x4140;
-                    const uint32_t p = frag::perm_bytes(w, 0u, sel) >> (4 * (st & 1));
-                    const uint32_t h = frag::perm_bytes(h4[2 * c + (i >> 1)], 0u, sel) >> (4 * (st & 1) + 2 * u);
-                    const __half2 q = __hsub2(h2((p & 0x000F000Fu) | ((h & 0x00030003u) << 4) | 0x64006400u), h2(0x64206420u));  // q - 32
-                    const __half2 v = __hmul2(q, s);
-                    hw[i] = bits(v);
-                    lw[i] = bits(fma2(q, s, __hneg2(v)));
-                }
-                put(hi, r, 4 * u + 2 * part + c, hw);
-                put(lo, r, 4 * u + 2 * part + c, lw);
+            for (int i = 0; i < 8; i++) {
+                const uint32_t w = u ? w1[i >> 1] : w0[i >> 1];
+                const uint32_t sel = (i & 1) ? 0x4342 : 0x4140;
+                const uint32_t p = frag::perm_bytes(w, 0u, sel) >> (4 * (st & 1));
+                const uint32_t h = frag::perm_bytes(h4[i >> 1], 0u, sel) >> (4 * (st & 1) + 2 * u);
+                const __half2 q = __hsub2(h2((p & 0x000F000Fu) | ((h & 0x00030003u) << 4) | 0x64006400u), h2(0x64206420u));  // q - 32
+                const __half2 v = __hmul2(q, s);
+                hi[8 * u + i] = bits(v);
+                lo[8 * u + i] = bits(fma2(q, s, __hneg2(v)));
             }
         }
     } else {
         const __half2 d = both(P.sc);
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            uint32_t hw[4], lw[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t w = (c < 2 ? w0[2 * c + (i >> 1)] : w1[2 * (c - 2) + (i >> 1)]) ^ 0x80808080u;
-                const __half2 q = __hsub2(h2(frag::perm_bytes(w, 0x64646464u, (i & 1) ? 0x4342 : 0x4140)), h2(0x64806480u));  // 1024 + 128 + q
-                const __half2 v = __hmul2(q, d);
-                hw[i] = bits(v);
-                lw[i] = bits(fma2(q, d, __hneg2(v)));
-            }
-            put(hi, r, 4 * part + c, hw);
-            put(lo, r, 4 * part + c, lw);
+        for (int i = 0; i < 16; i++) {
+            const uint32_t w = (i < 8 ? w0[i >> 1] : w1[(i - 8) >> 1]) ^ 0x80808080u;
+            const __half2 q = __hsub2(h2(frag::perm_bytes(w, 0x64646464u, (i & 1) ? 0x4342 : 0x4140)), h2(0x64806480u));  // 1024 + 128 + q
+            const __half2 v = __hmul2(q, d);
+            hi[i] = bits(v);
+            lo[i] = bits(fma2(q, d, __hneg2(v)));
+        }
+    }
+}
+
+// The same words as row r of operand planes in memory, in 128-byte swizzled chunks (what the CPU test looks at).
+template <int FMT>
+SLAI_HD void emit(const Packed& P, int r, int part, int st, unsigned char* hi, unsigned char* lo) {
+    uint32_t h[16], l[16];
+    make<FMT>(P, st, h, l);
+    for (int c = 0; c < 4; c++) {
+        const int chunk = FMT == 8 ? 4 * part + c : 4 * (c >> 1) + 2 * part + (c & 1);
+        const uint32_t vh[4] = {h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]};
+        put(hi, r, chunk, vh);
+        if (Fmt<FMT>::PLANES == 2) {
+            const uint32_t vl[4] = {l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]};
+            put(lo, r, chunk, vl);
         }
     }
 }

@@ -12,21 +12,24 @@
 //   warp 1      issues tcgen05.mma (kind::f16, M = 128, N = NT, K = 16), commits stages and super-blocks to mbarriers
 //   warp 2      bulk copies of the packed tile-step blocks (8 row tiles x one super-block), two or three super-blocks ahead: a
 //               few tokens read the matrix from HBM, which takes some 40 KB in flight per SM
-//   warps 4-11  packed bytes -> operand rows (prefill_dequant.cuh), one 16-row tile each
+//   warps 4-11  packed bytes -> operand rows in tensor memory (prefill_dequant.cuh), one row a thread
 //   warps 12-19 sums of a super-block out of tensor memory (two buffers) into registers, times d (and dmin), while the tensor
 //               cores work on the next one.  (Done by warps 4-11 between two stages, this put a super-block's drain and the
 //               next stages' operands one after the other: 1000 cycles per stage whatever the number of tokens.)
-// CTAs are persistent: a tile's sums are stored by warps 12-19 while the other warps are in the next tile.  (One CTA per tile:
-// each wave paid its start, its residual loads and its stores on top of 30 us of products: 7B, 511 tokens, output
-// projection 70 us, q/k/v 124 us.)
-// Few tokens leave most SMs without a tile (4096 rows x 37 tokens: 32 tiles), so K is split over a cluster of up to 8
+// CTAs are persistent: a tile's sums are stored by warps 12-19 while the other warps are in the next tile.  A CTA (pair) takes whole tiles, or an equal share
+// of the launch's super-blocks that begins and ends inside tiles: the CTA with a tile's first super-blocks adds the sums that the ones behind it
+// left in memory, which was the first thing they did.  (It waits for CTAs of its own launch, all of which start without waiting for any other; the wait is bounded.)
+// Few tokens leave most SMs without a tile (4096 rows x 37 tokens: 32 tiles): there K is split over a cluster of up to 8
 // CTAs, whose sums meet through distributed shared memory in rank order (deterministic, no second launch).
 //
-// What bounds it: with 128 tokens per tile the shared-memory traffic of the operands (A and B are read for every product,
-// 128 B per cycle at the tensor cores' full rate) and the L2 reads of the activations; with few tokens HBM and the
-// latency of a super-block's round through the stages.
+// What bounds it: from some 200 tokens on power (the clock falls to 1.6 GHz with the tensor cores 63 % busy; 511 tokens, gate and up: 1180 TFLOP/s
+// executed, where cuBLAS keeps 1375); with few tokens the chain of a stage through operand writer, product and commit (some 620 cycles for products of
+// 200), and 8 us of start and end a launch.  us per product of the 7B shape, weights' operands in shared memory and whole tiles / now: 511 tokens q/k/v 89.5 / 82, gate
+// and up 145 / 135, down 77 / 72; 37 tokens gate and up 57 / 34.
 // Every mbarrier wait is bounded: on expiry the error flag is raised, later waits of the thread give up at once and the
 // kernel runs to its end.
+#include <math.h>
+
 #include <algorithm>
 
 #include <cuda.h>
@@ -39,8 +42,9 @@ namespace {
 constexpr int PG_THREADS = 640;
 constexpr int PG_BM = 128, PG_BK = 64;          // weight rows per CTA, columns per stage (one 128-byte swizzle row of fp16)
 constexpr int PG_MAX_NT = 128;
+constexpr int PG_MAX_CTAS = CNT_PROMPT_FLAG_WORDS;
 constexpr int PG_MAX_STAGES = 6, PG_MAX_PACK = 3, PG_MAX_KS = 8;
-constexpr int PG_A_BYTES = PG_BM * PG_BK * 2;   // one operand plane of a stage
+constexpr int PG_A_COLS = PG_BK / 2;            // tensor-memory columns of one operand plane of a stage
 constexpr int PG_SMEM_LIMIT = 227 * 1024 - 512; // the barriers are static
 
 struct PgSeg {
@@ -60,6 +64,10 @@ struct PgParams {
     int ldr;
     int n_tiles, tiles;    // token tiles, all tiles (token tiles fastest: neighbours share the weights in L2)
     int ks;                // CTAs of a cluster that share K
+    int shared;            // CTAs have equal shares of the super-blocks (else whole tiles)
+    float* part;           // [CTA][tokens of a tile][128]: sums of a tile that another CTA finishes
+    unsigned int* flags;   // [CTA]: `seq` when they are there
+    unsigned int seq;      // of this launch
     int stages, packs;     // operand stages, packed blocks in flight
     unsigned int* err_flag;
     unsigned int wait_limit;
@@ -161,6 +169,20 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b
             "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
             : "memory");
 }
+// The same with A in tensor memory: row = lane, two columns of the operand to a word.
+template <bool PAIR>
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    if (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
+}
 // Arrives on the barrier (a pair: on both CTAs') when everything issued so far has completed.
 template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
@@ -183,6 +205,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
 __device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {
     uint32_t a;
     float v;
@@ -194,17 +221,16 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Dynamic shared memory, from a 1024-byte boundary: operand planes of the weights, of the activations, the operands of the
+// Dynamic shared memory, from a 1024-byte boundary: operand planes of the activations, the operands of the
 // minimum term (two super-blocks), row scales (four super-blocks), packed blocks.
 struct PgLayout {
-    uint32_t a, b, amin, bmin, scale, pack, total;
+    uint32_t b, amin, bmin, scale, pack, total;
 };
 template <int FMT>
 __host__ __device__ inline PgLayout pg_layout(int NB, int stages, int packs) {
     using F = pfq::Fmt<FMT>;
     PgLayout L;
-    L.a = 0;
-    L.b = L.a + (uint32_t)stages * F::PLANES * PG_A_BYTES;
+    L.b = 0;
     L.amin = L.b + (uint32_t)stages * 2 * NB * PG_BK * 2;
     L.bmin = L.amin + (F::MIN ? 2 * PG_BM * 32 : 0);
     L.scale = L.bmin + (F::MIN ? 2 * (uint32_t)NB * 32 : 0);
@@ -230,18 +256,32 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     const PgLayout L = pg_layout<FMT>(NB, P.stages, P.packs);
     const int NT = P.NT, S = P.stages, PK = P.packs;
     const uint32_t b_bytes = (uint32_t)NB * PG_BK * 2;  // one activation plane of a stage
-    __shared__ __align__(8) unsigned long long bars[3 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 10];
+    __shared__ __align__(8) unsigned long long bars[2 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 11];
     __shared__ uint32_t tmem_slot;
     const uint32_t sb = smem_u32(smem);
-    const uint32_t full_a = smem_u32(bars), full_b = full_a + 8 * PG_MAX_STAGES, empty = full_b + 8 * PG_MAX_STAGES,
+    const uint32_t full = smem_u32(bars), empty = full + 8 * PG_MAX_STAGES,
                    pk_full = empty + 8 * PG_MAX_STAGES, pk_empty = pk_full + 8 * PG_MAX_PACK, dfull = pk_empty + 8 * PG_MAX_PACK,
-                   dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16;
+                   dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16, mempty = sc_full + 32;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform for the compiler too)
     const int pr = PAIR ? (int)(blockIdx.x & 1) : 0;  // rank in the pair
-    const int rank = !PAIR && P.ks > 1 ? (int)(blockIdx.x % P.ks) : 0;
-    const int tile0 = (int)blockIdx.x / (PAIR ? 2 : P.ks), tile_step = (int)gridDim.x / (PAIR ? 2 : P.ks);
-    const int c0 = (int)((long long)P.nch * rank / P.ks), nc = (int)((long long)P.nch * (rank + 1) / P.ks) - c0;  // super-blocks of this CTA
+    // This CTA's (pair's) super-blocks of the launch, in order of tiles: whole tiles, or an equal share of all of them, from
+    // somewhere in a tile to somewhere in another.
+    const int rank = !PAIR && P.ks > 1 ? (int)(blockIdx.x % P.ks) : 0, me = (int)blockIdx.x / (PAIR ? 2 : P.ks), many = (int)gridDim.x / (PAIR ? 2 : P.ks);
+    auto share = [&](int i) { return P.shared ? (int)((long long)P.tiles * P.nch * i / many) : (int)((long long)P.tiles * i / many) * P.nch; };
+    const int u_lo = P.ks > 1 ? me * P.nch + (int)((long long)P.nch * rank / P.ks) : share(me);
+    const int u_hi = P.ks > 1 ? me * P.nch + (int)((long long)P.nch * (rank + 1) / P.ks) : share(me + 1);
+    // ... and the part of them that is of one tile: super-blocks c0 .. c0 + nc - 1 of it
+    struct Part {
+        int tile, c0, nc;
+    };
+    auto part_at = [&](int un) {
+        Part q;
+        q.tile = un / P.nch;
+        q.c0 = un - q.tile * P.nch;
+        q.nc = min(P.nch - q.c0, u_hi - un);
+        return q;
+    };
     // a tile's matrix, first row in it and first token
     auto tile_of = [&](int tile, PgSeg& sg, int& m0, int& n0) {
         const int mt = tile / P.n_tiles;
@@ -254,8 +294,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
 
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
-            mbar_init(full_a + 8 * s, PAIR ? 16 : 8);
-            mbar_init(full_b + 8 * s, 1);
+            mbar_init(full + 8 * s, (PAIR ? 16 : 8) + 1);  // the operand-writing warps and the activations' request (and its bytes)
             mbar_init(empty + 8 * s, 1);
         }
         for (int s = 0; s < PK; s++) {
@@ -268,13 +307,15 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             mbar_init(bmin_full + 8 * s, 1);
         }
         for (int s = 0; s < 4; s++) mbar_init(sc_full + 8 * s, 8);
+        mbar_init(mempty, PAIR ? 16 : 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async();
     }
-    // tensor memory: two buffers of sums, then two of the minimum term
+    // tensor memory: two buffers of sums, the minimum term, the weights' operand planes of all stages
     const int DS = MERGED ? 2 * P.NTP : P.NTP;
+    const uint32_t TA = 2 * DS + (F::MIN ? P.NTP : 0);
     int ncols = 32;
-    while (ncols < 2 * DS + (F::MIN ? 2 * P.NTP : 0)) ncols <<= 1;
+    while (ncols < (int)TA + S * F::PLANES * PG_A_COLS) ncols <<= 1;
     if (warp == 1) {  // the MMA warp owns the tensor-memory allocation
         if (PAIR) {
             asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(ncols) : "memory");
@@ -301,73 +342,82 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     const int quad = warp & 3, half = (warp - 12) >> 2;
 
     if (warp == 0) {
-        // ---- activations ----
-        if (lane == 0) {
-            int slot = 0, issued = 0, gc = 0;  // gc: super-blocks so far
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = tile0; tile < P.tiles && ok; tile += tile_step) {
-                PgSeg sg;
-                int m0, n0;
-                tile_of(tile, sg, m0, n0);
-                for (int c = 0; c < nc && ok; c++, gc++) {
-                    if (F::MIN) {
-                        const int buf = gc & 1;
-                        if (gc >= 2 && !(ok = mbar_wait(dfull + 8 * buf, ((gc >> 1) - 1) & 1, limit, P.err_flag))) break;
+        // ---- activations: the whole warp walks the loop and one elected lane issues, as for the products (issued by lane 0 of a diverged warp, a
+        // copy took some 200 cycles: more than half of the tensor cores' waiting was for them) ----
+        int slot = 0, issued = 0, gc = 0;  // gc: super-blocks so far
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int un = u_lo; un < u_hi && ok;) {
+            const Part q = part_at(un);
+            const int c0 = q.c0, nc = q.nc;
+            un += nc;
+            PgSeg sg;
+            int m0, n0;
+            tile_of(q.tile, sg, m0, n0);
+            for (int c = 0; c < nc && ok; c++, gc++) {
+                if (F::MIN) {
+                    const int buf = gc & 1;
+                    if (gc >= 2 && !(ok = __all_sync(0xffffffffu, mbar_wait(dfull + 8 * buf, ((gc >> 1) - 1) & 1, limit, P.err_flag)))) break;
+                    if (elect_one()) {
                         if (pr == 0) mbar_expect_tx(bmin_full + 8 * buf, (uint32_t)NT * 32);
                         tma_load_2d<PAIR>(sb + L.bmin + buf * NB * 32, &map_sum, 16 * (c0 + c), n0 + pr * NB, bmin_full + 8 * buf);
                     }
-                    for (int st = 0; st < F::STAGES; st++) {
-                        if (!(ok = mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
-                        const int x = ((c0 + c) * F::STAGES + st) * PG_BK;
-                        if (pr == 0) mbar_expect_tx(full_b + 8 * slot, (PAIR ? 4 : 2) * b_bytes);
-                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes, &map_hi, x, n0 + pr * NB, full_b + 8 * slot);
-                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes + b_bytes, &map_lo, x, n0 + pr * NB, full_b + 8 * slot);
-                        issued++;
-                        if (++slot == S) {
-                            slot = 0;
-                            ph ^= 1;
-                        }
+                    __syncwarp();
+                }
+                for (int st = 0; st < F::STAGES; st++) {
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag)))) break;
+                    const int x = ((c0 + c) * F::STAGES + st) * PG_BK;
+                    if (elect_one()) {
+                        if (pr == 0) mbar_expect_tx(full + 8 * slot, (PAIR ? 4 : 2) * b_bytes);
+                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes, &map_hi, x, n0 + pr * NB, full + 8 * slot);
+                        tma_load_2d<PAIR>(sb + L.b + slot * 2 * b_bytes + b_bytes, &map_lo, x, n0 + pr * NB, full + 8 * slot);
+                    }
+                    __syncwarp();
+                    issued++;
+                    if (++slot == S) {
+                        slot = 0;
+                        ph ^= 1;
                     }
                 }
             }
-            if (!ok && pr == 0) {  // a wait ran out: the copies in flight land before the CTA (the pair) may end
-                for (int i = max(0, issued - S); i < issued; i++) {
-                    limit = P.wait_limit;
-                    mbar_wait(full_b + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
-                }
+        }
+        if (!ok && pr == 0) {  // a wait ran out: the copies in flight land before the CTA (the pair) may end
+            for (int i = max(0, issued - S); i < issued; i++) {
+                limit = P.wait_limit;
+                mbar_wait(full + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
             }
         }
     } else if (warp == 1) {
         if (pr == 0) {
         // ---- tensor cores: the whole warp walks the loop, so that descriptors live in uniform registers, one lane issues ----
         const uint32_t idesc = umma_idesc(PAIR ? 2 * PG_BM : PG_BM, NT), idesc2 = umma_idesc(PG_BM, 2 * NT);
-        const uint64_t da0 = desc128(sb + L.a), db0 = desc128(sb + L.b);
-        int slot = 0, u = 0;  // u: sums so far (of a super-block; Q8_0: of a whole tile), alternately in two buffers
+        const uint64_t db0 = desc128(sb + L.b);
+        int slot = 0, u = 0;  // u: sums so far (of a super-block; Q8_0: of a tile's part), alternately in two buffers
         uint32_t ph = 0;
-        for (int tile = tile0; tile < P.tiles; tile += tile_step)
+        for (int un = u_lo, nc; un < u_hi; un += nc) {
+        nc = part_at(un).nc;
         for (int c = 0; c < nc; c++) {
             const int buf = u & 1;
             const uint32_t d = tmem + buf * DS;
             if ((F::SCALED || c == 0) && u >= 2) mbar_wait<PAIR>(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
             for (int st = 0; st < F::STAGES; st++) {
-                mbar_wait<PAIR>(full_a + 8 * slot, ph, limit, P.err_flag);
-                mbar_wait<PAIR>(full_b + 8 * slot, ph, limit, P.err_flag);
+                mbar_wait<PAIR>(full + 8 * slot, ph, limit, P.err_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 __syncwarp();
                 // 16 elements = 32 bytes further along the swizzled row: 2 in the descriptor's units of 16 bytes
-                const uint64_t dah = da0 + (uint64_t)(slot * F::PLANES * (PG_A_BYTES >> 4)), dbh = db0 + (uint64_t)(slot * 2 * (b_bytes >> 4));
+                const uint32_t ah = tmem + TA + slot * F::PLANES * PG_A_COLS;
+                const uint64_t dbh = db0 + (uint64_t)(slot * 2 * (b_bytes >> 4));
                 if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < PG_BK / 16; kk++) {
                         const bool first = kk == 0 && st == 0 && (F::SCALED || c == 0);
                         if (MERGED) {
-                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + 2 * kk, idesc2, first ? 0u : 1u);
+                            umma_f16_ts<PAIR>(d, ah + 8 * kk, dbh + 2 * kk, idesc2, first ? 0u : 1u);
                         } else {
-                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + 2 * kk, idesc, first ? 0u : 1u);
-                            umma_f16<PAIR>(d, dah + 2 * kk, dbh + (b_bytes >> 4) + 2 * kk, idesc, 1u);
+                            umma_f16_ts<PAIR>(d, ah + 8 * kk, dbh + 2 * kk, idesc, first ? 0u : 1u);
+                            umma_f16_ts<PAIR>(d, ah + 8 * kk, dbh + (b_bytes >> 4) + 2 * kk, idesc, 1u);
                         }
-                        if (F::PLANES == 2) umma_f16<PAIR>(d, dah + (PG_A_BYTES >> 4) + 2 * kk, dbh + 2 * kk, idesc, 1u);
+                        if (F::PLANES == 2) umma_f16_ts<PAIR>(d, ah + PG_A_COLS + 8 * kk, dbh + 2 * kk, idesc, 1u);
                     }
                     umma_commit<PAIR>(empty + 8 * slot);
                 }
@@ -378,61 +428,73 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
             }
             if (F::MIN) {
+                // (one buffer: read out for the super-block before)
+                if (PAIR && u >= 1) mbar_wait<PAIR>(mempty, (u - 1) & 1, limit, P.err_flag);
+                if (!PAIR && u >= 1) mbar_wait<PAIR>(dempty + 8 * (buf ^ 1), ((u - 1) >> 1) & 1, limit, P.err_flag);
                 mbar_wait<PAIR>(bmin_full + 8 * buf, (u >> 1) & 1, limit, P.err_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 __syncwarp();
             }
             if (elect_one()) {
                 if (F::MIN)
-                    umma_f16<PAIR>(tmem + 2 * DS + buf * P.NTP, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NB * 32), idesc, 0u);
+                    umma_f16<PAIR>(tmem + 2 * DS, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NB * 32), idesc, 0u);
                 if (F::SCALED || c == nc - 1) umma_commit<PAIR>(dfull + 8 * buf);
             }
             if (F::SCALED || c == nc - 1) u++;
             __syncwarp();
         }
         }
+        }
     } else if (warp == 2) {
         // ---- packed weights ----
-        if (lane == 0) {
-            int slot = 0, issued = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = tile0; tile < P.tiles && ok; tile += tile_step) {
-                PgSeg sg;
-                int m0, n0;
-                tile_of(tile, sg, m0, n0);
-                const int nt = max(0, min(8, (sg.rows - m0 + 15) >> 4));  // 16-row tiles that exist
-                const uint8_t* src = sg.w + (long long)(m0 >> 4) * P.tile_bytes + (long long)c0 * F::STEP;
-                for (int c = 0; c < nc; c++) {
-                    if (issued == PK) griddep_wait();
-                    if (!(ok = mbar_wait(pk_empty + 8 * slot, ph ^ 1, limit, P.err_flag))) break;
+        int slot = 0, issued = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int un = u_lo; un < u_hi && ok;) {
+            const Part q = part_at(un);
+            const int c0 = q.c0, nc = q.nc;
+            un += nc;
+            PgSeg sg;
+            int m0, n0;
+            tile_of(q.tile, sg, m0, n0);
+            const int nt = max(0, min(8, (sg.rows - m0 + 15) >> 4));  // 16-row tiles that exist
+            const uint8_t* src = sg.w + (long long)(m0 >> 4) * P.tile_bytes + (long long)c0 * F::STEP;
+            for (int c = 0; c < nc; c++) {
+                if (issued == PK) griddep_wait();
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(pk_empty + 8 * slot, ph ^ 1, limit, P.err_flag)))) break;
+                if (elect_one()) {
                     fence_async();  // the warps' reads of the block before come before the copy's writes
                     mbar_expect_tx(pk_full + 8 * slot, (uint32_t)nt * F::STEP);
                     for (int i = 0; i < nt; i++)
                         bulk_load(sb + L.pack + (slot * 8 + i) * F::STEP, src + i * P.tile_bytes + (long long)c * F::STEP, F::STEP, pk_full + 8 * slot);
-                    issued++;
-                    if (++slot == PK) {
-                        slot = 0;
-                        ph ^= 1;
-                    }
                 }
-            }
-            if (!ok) {
-                for (int i = max(0, issued - PK); i < issued; i++) {
-                    limit = P.wait_limit;
-                    mbar_wait(pk_full + 8 * (i % PK), (i / PK) & 1, limit, P.err_flag);
+                __syncwarp();
+                issued++;
+                if (++slot == PK) {
+                    slot = 0;
+                    ph ^= 1;
                 }
             }
         }
+        if (!ok) {
+            for (int i = max(0, issued - PK); i < issued; i++) {
+                limit = P.wait_limit;
+                mbar_wait(pk_full + 8 * (i % PK), (i / PK) & 1, limit, P.err_flag);
+            }
+        }
     } else if (warp >= 4 && warp < 12) {
-        // ---- weights into operand rows ----
-        const int w8 = warp - 4, r16 = lane & 15, part = lane >> 4, r = 16 * w8 + r16;
+        // ---- weights into operand rows in tensor memory ----
+        // Thread = row: a warp reaches the 32 lanes of its quarter; the two warps of a quarter share the columns.  (In shared memory the rows cost, per
+        // stage and SM, 128 cycles to write and 256 to read for the two products, of 820 the stage took.)
+        // (Sixteen of these warps, every other two stages each: no faster at 37 tokens, 35.5 for 34.4 us.)
+        const int q4 = warp & 3, w8 = 2 * q4 + (lane >> 4), r16 = lane & 15, r = 32 * q4 + lane;
+        const int part = (warp - 4) >> 2;
+        const uint32_t mine = tmem + TA + ((uint32_t)(32 * q4) << 16) + (FMT == SLAI_FMT_Q8_0 ? 16 : 8) * part;
         uint32_t* scales = reinterpret_cast<uint32_t*>(smem + L.scale);
-        int slot = 0, ps = 0, c = 0;  // c: super-blocks so far
+        int slot = 0, ps = 0;
         uint32_t ph = 0, pph = 0;
         bool behind = false;
-        for (int tile = tile0; tile < P.tiles; tile += tile_step)
-        for (int i = 0; i < nc; i++, c++) {
+        for (int c = 0; c < u_hi - u_lo; c++) {  // super-blocks
             mbar_wait(pk_full + 8 * ps, pph, limit, P.err_flag);
             const unsigned char* blk = smem + L.pack + (ps * 8 + w8) * F::STEP;
             if (F::MIN) {
@@ -446,37 +508,47 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sc_full + 8 * (c & 3));
             }
-            // two stages at a time: a warp's way through one is a chain of latencies (load, arithmetic, store, fence, arrive)
+            // two stages at a time: a warp's way through one is a chain of latencies (load, arithmetic, store, arrive)
 #pragma unroll
             for (int st = 0; st < F::STAGES; st += 2) {
+                const int slot0 = slot, slot1 = slot + 1 == S ? 0 : slot + 1;
+                const uint32_t ph0 = ph, ph1 = slot + 1 == S ? ph ^ 1 : ph;
+                slot += 2;
+                if (slot >= S) {
+                    slot -= S;
+                    ph ^= 1;
+                }
                 pfq::Packed pk[2];
                 pfq::fetch<FMT>(blk, r16, part, st, pk[0]);
                 pfq::fetch<FMT>(blk, r16, part, st + 1, pk[1]);
-                const int slot0 = slot;
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
-                    if (ph && !behind) {
+                    const uint32_t p = k ? ph1 : ph0;
+                    if (p && !behind) {
                         griddep_wait();
                         behind = true;
                     }
-                    mbar_wait(empty + 8 * slot, ph ^ 1, limit, P.err_flag);
-                    unsigned char* a = smem + L.a + slot * F::PLANES * PG_A_BYTES;
-                    pfq::emit<FMT>(pk[k], r, part, st + k, a, a + PG_A_BYTES);
-                    if (k == 0 && ++slot == S) {
-                        slot = 0;
-                        ph ^= 1;
+                    mbar_wait(empty + 8 * (k ? slot1 : slot0), p ^ 1, limit, P.err_flag);
+                    __syncwarp();
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t hi[16], lo[16];
+                    pfq::make<FMT>(pk[k], st + k, hi, lo);
+                    const uint32_t a = mine + (k ? slot1 : slot0) * F::PLANES * PG_A_COLS;
+                    tmem_st8(a, hi);
+                    tmem_st8(a + (FMT == SLAI_FMT_Q8_0 ? 8 : 16), hi + 8);
+                    if (F::PLANES == 2) {
+                        tmem_st8(a + PG_A_COLS, lo);
+                        tmem_st8(a + PG_A_COLS + (FMT == SLAI_FMT_Q8_0 ? 8 : 16), lo + 8);
                     }
                 }
-                fence_async();  // these stores come before the tensor core's reads
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (F::MIN && st == 0) fence_async();  // the minimum term's operand comes before the tensor core's reads
                 __syncwarp();
                 if (lane == 0) {
-                    arrive_issuer<PAIR>(full_a + 8 * slot0);
-                    arrive_issuer<PAIR>(full_a + 8 * slot);
+                    arrive_issuer<PAIR>(full + 8 * slot0);
+                    arrive_issuer<PAIR>(full + 8 * slot1);
                     if (st == F::STAGES - 2) mbar_arrive(pk_empty + 8 * ps);
-                }
-                if (++slot == S) {
-                    slot = 0;
-                    ph ^= 1;
                 }
             }
             if (++ps == PK) {
@@ -488,7 +560,10 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         // ---- sums out of tensor memory ----
         const uint32_t* scales = reinterpret_cast<const uint32_t*>(smem + L.scale);
         int u = 0;
-        for (int tile = tile0; tile < P.tiles; tile += tile_step) {
+        for (int un = u_lo; un < u_hi;) {
+            const Part q = part_at(un);
+            const int nc = q.nc;
+            un += nc;
 #pragma unroll
             for (int i = 0; i < NG; i++)
 #pragma unroll
@@ -506,26 +581,44 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tq = tmem + ((uint32_t)(32 * quad) << 16), t0 = tq + buf * DS;
+                if (PAIR && F::MIN) {  // first, because it has one buffer (511 tokens, gate and up 156 -> 151 us)
+#pragma unroll
+                    for (int i = 0; i < NG; i++) {
+                        const int col = 16 * (2 * i + half);
+                        if (col < NT) {
+                            uint32_t v[16];
+                            tmem_ld16(tq + 2 * DS + col, v);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 16; j++) acc[i][j] = fmaf(mn, __uint_as_float(v[j]), acc[i][j]);
+                        }
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) arrive_issuer<PAIR>(mempty);
+                }
 #pragma unroll
                 for (int i = 0; i < NG; i++) {
                     const int col = 16 * (2 * i + half);
                     if (col < NT) {
-                        uint32_t v[16];
+                        uint32_t v[16], w[16], z[16];  // (few tokens: all of a group's loads, then one wait)
                         tmem_ld16(t0 + col, v);
+                        if (MERGED) tmem_ld16(t0 + NT + col, w);
+                        if (MERGED && F::MIN) tmem_ld16(tq + 2 * DS + col, z);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : __uint_as_float(v[j]);
                         if (MERGED) {
-                            tmem_ld16(t0 + NT + col, v);
-                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : acc[i][j] + __uint_as_float(v[j]);
+                            for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(w[j]), acc[i][j]) : acc[i][j] + __uint_as_float(w[j]);
                         }
-                        if (F::MIN) {
-                            tmem_ld16(tq + 2 * DS + buf * P.NTP + col, v);
-                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (!PAIR && F::MIN) {
+                            if (!MERGED) {
+                                tmem_ld16(tq + 2 * DS + col, z);
+                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            }
 #pragma unroll
-                            for (int j = 0; j < 16; j++) acc[i][j] = fmaf(mn, __uint_as_float(v[j]), acc[i][j]);
+                            for (int j = 0; j < 16; j++) acc[i][j] = fmaf(mn, __uint_as_float(z[j]), acc[i][j]);
                         }
                     }
                 }
@@ -534,9 +627,48 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 if (lane == 0) arrive_issuer<PAIR>(dempty + 8 * buf);
             }
             if (!PAIR && P.ks > 1) break;  // one tile per cluster, stored below
+            const size_t slot_floats = (size_t)NT * PG_BM;
+            if (q.c0 > 0) {  // the tile's first super-blocks, and its sums, are another CTA's
+                float* dst = P.part + blockIdx.x * slot_floats + 32 * quad + lane;
+#pragma unroll
+                for (int i = 0; i < NG; i++)
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (16 * (2 * i + half) < NT) __stcg(dst + (16 * (2 * i + half) + j) * PG_BM, acc[i][j]);
+                __threadfence();
+                asm volatile("bar.sync 1, 256;" ::: "memory");  // (warps 12-19)
+                if (warp == 12 && lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.flags + blockIdx.x), "r"(P.seq) : "memory");
+                continue;
+            }
+            // The rest of the tile is the first work of the CTAs that follow, and done by now (or they end where this one does): added in order.
+            for (int p = me + 1; q.c0 + nc < P.nch && p < many && share(p) < (q.tile + 1) * P.nch; p++) {
+                const int cta = PAIR ? 2 * p + pr : p;
+                bool there = false;
+                for (unsigned int i = 0; i < limit && !there; i++) {
+                    unsigned int f;
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(P.flags + cta) : "memory");
+                    there = f == P.seq;
+                    if (!there && i > 64) __nanosleep(40);
+                }
+                if (!there) {
+                    atomicExch(P.err_flag, 5u);
+                    limit = 1;
+                }
+                __syncwarp();
+                const float* src = P.part + cta * slot_floats + 32 * quad + lane;
+#pragma unroll
+                for (int i = 0; i < NG; i++)
+                    if (16 * (2 * i + half) < NT) {
+                        float x[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) x[j] = __ldcg(src + (16 * (2 * i + half) + j) * PG_BM);
+#pragma unroll
+                        for (int j = 0; j < 16; j++) acc[i][j] += x[j];
+                    }
+            }
             PgSeg sg;
             int m0, n0;
-            tile_of(tile, sg, m0, n0);
+            tile_of(q.tile, sg, m0, n0);
             const int row = m0 + 32 * quad + lane;
             if (row < sg.rows) {
                 const float bias = sg.bias ? sg.bias[row] : 0.f;
@@ -562,7 +694,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         griddep_wait();
         PgSeg sg;
         int m0, n0;
-        tile_of(tile0, sg, m0, n0);
+        tile_of(me, sg, m0, n0);
         // every CTA leaves its sums [token][row] in its own shared memory (the operand planes are free: all products are done)
         float* red = reinterpret_cast<float*>(smem);
         if (warp >= 12) {
@@ -638,9 +770,12 @@ int launch_mode(slai_ctx* ctx, PgParams& P, const CUtensorMap& hi, const CUtenso
     }
     P.tiles = tiles * P.n_tiles;
     // Packed blocks in flight first (three if two stages still fit beside them), then as many operand stages as fit.
-    P.packs = pg_layout<FMT>(NB, 3, 3).total <= PG_SMEM_LIMIT - 1024 ? 3 : 2;
+    P.packs = pg_layout<FMT>(NB, 4, 3).total <= PG_SMEM_LIMIT - 1024 ? 3 : 2;
     P.stages = 2;
-    while (P.stages < PG_MAX_STAGES && pg_layout<FMT>(NB, P.stages + 1, P.packs).total <= PG_SMEM_LIMIT - 1024) P.stages++;
+    const int sums = (MODE == PG_MERGED ? 4 : 2) * P.NTP + (pfq::Fmt<FMT>::MIN ? P.NTP : 0);  // tensor-memory columns, of 512
+    while (P.stages < PG_MAX_STAGES && pg_layout<FMT>(NB, P.stages + 1, P.packs).total <= PG_SMEM_LIMIT - 1024 &&
+           sums + (P.stages + 1) * pfq::Fmt<FMT>::PLANES * PG_A_COLS <= 512)
+        P.stages++;
     const size_t smem = pg_layout<FMT>(NB, P.stages, P.packs).total + 1024;
     auto kern = prefill_gemm_kernel<FMT, MODE>;
     static PerDeviceOnce attr;  // per instantiation
@@ -648,9 +783,18 @@ int launch_mode(slai_ctx* ctx, PgParams& P, const CUtensorMap& hi, const CUtenso
         SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM_LIMIT));
         attr.set(ctx->device);
     }
-    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    const int sms = std::min(ctx->sm_count > 0 ? ctx->sm_count : 148, PG_MAX_CTAS);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(MODE != PG_PAIR && P.ks > 1 ? P.tiles * P.ks : std::min(P.tiles, sms / cluster) * cluster));
+    const int grid = MODE != PG_PAIR && P.ks > 1 ? P.tiles * P.ks
+                                                 : std::min((int)std::min((long long)P.tiles * (P.shared ? P.nch : 1), 1ll << 20), sms / cluster) * cluster;
+    cfg.gridDim = dim3((unsigned)grid);
+    if (P.shared) {
+        const int rc = ensure_scratch(ctx, (size_t)grid * P.NT * PG_BM * sizeof(float));
+        if (rc) return rc;
+        P.part = reinterpret_cast<float*>(ctx->d_scratch);
+        P.flags = ctx->d_counters + CNT_PROMPT_FLAGS;
+        P.seq = ++ctx->prompt_seq ? ctx->prompt_seq : ++ctx->prompt_seq;  // (0 is what the flags hold at first)
+    }
     cfg.blockDim = dim3(PG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -674,29 +818,46 @@ int launch_mode(slai_ctx* ctx, PgParams& P, const CUtensorMap& hi, const CUtenso
 
 template <int FMT>
 int launch_fmt(slai_ctx* ctx, PgParams& P, const PrefillGemm& G) {
-    // What the longest SM has to do, in units of a plain super-block: its tiles one after the other, alone or as one of a pair
-    // (a pair's super-block takes about two thirds of the time, measured at 128 tokens: half the activations' L2 and shared-
-    // memory traffic per SM), or a share of K of one tile, plus about two for its start and end, in every round.
-    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    // What the longest SM has to do, in units of a plain super-block (some 2400 cycles): whole tiles one after the other; an equal share of all super-blocks,
+    // where every CTA that a tile is spread over beyond its first costs the one that adds the sums about two; or a share of K of one tile in a
+    // cluster, about three and a half for its start and end in every round.  A pair's super-block takes about two thirds of the time (half the
+    // activations' L2 and shared-memory traffic per SM).  us per product, 7B shape, whole tiles or cluster / equal shares: 37 tokens q/k/v 30.1 / 27.7, o
+    // 17 (cluster of 4) / 21, gate and up 57 (2) / 38.6, down 27 (4) / 31; 200 tokens q/k/v 64 / 56, gate and up 95 / 88; 511 tokens (pairs) o 41 / 47.
+    const int sms = std::min(ctx->sm_count > 0 ? ctx->sm_count : 148, PG_MAX_CTAS);
     auto m_tiles = [&](int rows) {
         int t = 0;
         for (int i = 0; i < P.nseg; i++) t += (P.seg[i].rows + rows - 1) / rows;
         return t;
     };
     const long long tiles = (long long)m_tiles(PG_BM) * P.n_tiles, pairs = (long long)m_tiles(2 * PG_BM) * P.n_tiles;
-    double best = -1;
+    auto whole = [&](long long t, int ctas) { return (double)((t + ctas - 1) / ctas) * P.nch; };
+    auto equal = [&](long long t, int ctas, double sb, double& cost) {
+        const double each = (double)t * P.nch / ctas;
+        if (each < 1) return false;
+        const double c = sb * each + 2 * ceil(P.nch / each);
+        if (c >= cost) return false;
+        cost = c;
+        return true;
+    };
+    double best = whole(tiles, sms);
     P.ks = 1;
-    for (int ks = 1; ks <= PG_MAX_KS && ks <= P.nch; ks *= 2) {
-        const long long rounds = (tiles * ks + sms - 1) / sms;
-        const double cost = ks == 1 ? (double)rounds * P.nch + 2 : (double)rounds * ((P.nch + ks - 1) / ks + 2);
-        if (best < 0 || cost < best) {
+    for (int ks = 2; ks <= PG_MAX_KS && ks <= P.nch; ks *= 2) {
+        const double cost = (double)((tiles * ks + sms - 1) / sms) * ((P.nch + ks - 1) / ks + 3.5);
+        if (cost < best) {
             best = cost;
             P.ks = ks;
         }
     }
+    P.shared = equal(tiles, sms, 1.0, best);
+    if (P.shared) P.ks = 1;
     const bool merged = P.NT <= 64;
-    const bool pair = !merged && (double)((pairs + sms / 2 - 1) / (sms / 2)) * P.nch * 0.65 + 2 < best;
-    if (pair) P.ks = 1;
+    double best_pair = 0.65 * whole(pairs, sms / 2);
+    const int shared_pair = equal(pairs, sms / 2, 0.65, best_pair);
+    const bool pair = !merged && best_pair < best;
+    if (pair) {
+        P.ks = 1;
+        P.shared = shared_pair;
+    }
     const int NB = pair ? P.NT / 2 : P.NT, K = (int)G.w[0]->ncols;
     CUtensorMap hi, lo, sum;
     int rc = make_plane_map(ctx, &hi, G.x_hi, G.t_pad, K, PG_BK, NB);
