@@ -186,6 +186,9 @@ prefill_attn_kernel(const float* q, int q_ld, const T* kc, const T* vc, long lon
 // arithmetic (values).  Relative error over the whole output against 64 bits, the f32 kernel's / this one's (heads of 128, 511
 // tokens): normal queries and keys 3.4e-7 / 2.1e-7, queries 30 times that 2.3e-6 / 0.7e-6, a thousandth 1.7e-7 / 1.0e-7, a mean of
 // 3 on both 4.8e-6 / 1.1e-6; no larger at any of 50 settings (heads of 64 and 128, 37 to 3064 positions).
+//
+// A short turn has one CTA per head, which walks the whole conversation tile by tile (5 us a tile): the tiles of a (head, 64 queries) are dealt to the CTAs
+// of a cluster along z, whose outputs and (max, sum) pairs meet through distributed shared memory in rank order.
 constexpr int PM_QT = 64, PM_KT = 64, PM_THREADS = 128;
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -222,7 +225,8 @@ prefill_attn_mma_kernel(const float* q, int q_ld, const __half* kc, const __half
     const __half* kb = kc + (long long)(head / kv_mul) * head_stride;
     const __half* vb = vc + (long long)(head / kv_mul) * head_stride;
     const int last_pos = pos0 + t0 + nq - 1;  // last position any query of this CTA attends to
-    const int tiles = last_pos / PM_KT + 1;
+    const int all_tiles = last_pos / PM_KT + 1, ranks = (int)gridDim.z, rank = (int)blockIdx.z;  // (the grid is one cluster deep)
+    const int tile_lo = all_tiles * rank / ranks, tiles = all_tiles * (rank + 1) / ranks;
 
     auto load_tile = [&](int tile) {
         const int p0 = tile * PM_KT;
@@ -239,7 +243,7 @@ prefill_attn_mma_kernel(const float* q, int q_ld, const __half* kc, const __half
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_tile(0);
+    if (tile_lo < tiles) load_tile(tile_lo);
 
     // Queries of this warp (rows g and g + 8 of its 16), divided by sqrt(head size), each row times a power of two that puts its largest
     // element below 2^15: whatever their size they fit a pair of halves.  `unit` takes the power out of the row's scores again.
@@ -280,7 +284,7 @@ prefill_attn_mma_kernel(const float* q, int q_ld, const __half* kc, const __half
     const int warp_last = pos0 + t0 + 16 * warp + 15;  // last position any query of this warp attends to
     const int qpos[2] = {pos0 + row0, pos0 + row0 + 8};
 
-    for (int tile = 0; tile < tiles; tile++) {
+    for (int tile = tile_lo; tile < tiles; tile++) {
         if (tile + 1 < tiles) load_tile(tile + 1);
         else asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -386,14 +390,65 @@ prefill_attn_mma_kernel(const float* q, int q_ld, const __half* kc, const __half
     for (int h = 0; h < 2; h++) {
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        const int row = row0 + 8 * h;
-        if (row < n_tokens) {
-            const float il = 1.0f / (l[h] * 4096.f);  // position 0 is always attended to: l > 0
-#pragma unroll
-            for (int n = 0; n < NT8; n++)
-                *reinterpret_cast<float2*>(out + (size_t)row * out_ld + (size_t)head * HS + 8 * n + 2 * t) = make_float2(acc[n][2 * h] * il, acc[n][2 * h + 1] * il);
-        }
     }
+    if (ranks == 1) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int row = row0 + 8 * h;
+            if (row < n_tokens) {
+                const float il = 1.0f / (l[h] * 4096.f);  // position 0 is always attended to: l > 0
+#pragma unroll
+                for (int n = 0; n < NT8; n++)
+                    *reinterpret_cast<float2*>(out + (size_t)row * out_ld + (size_t)head * HS + 8 * n + 2 * t) = make_float2(acc[n][2 * h] * il, acc[n][2 * h + 1] * il);
+            }
+        }
+        return;
+    }
+    // [64][HS] outputs, [64][2] (max, sum) where the tiles were (all of them have been read)
+    float* so = reinterpret_cast<float*>(pm_sm);
+    float* sml = so + PM_QT * HS;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int r = 16 * warp + g + 8 * h;
+#pragma unroll
+        for (int n = 0; n < NT8; n++) *reinterpret_cast<float2*>(so + r * HS + 8 * n + 2 * t) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        if (t == 0) *reinterpret_cast<float2*>(sml + 2 * r) = make_float2(m[h], l[h]);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int lo = nq * rank / ranks * (HS / 4), hi = nq * (rank + 1) / ranks * (HS / 4);  // this CTA's share of the rows, four elements a thread
+    for (int i = lo + tid; i < hi; i += PM_THREADS) {
+        const int r = i / (HS / 4), d = 4 * (i - r * (HS / 4));
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+        float M = -INFINITY, den = 0.f;
+        for (int z0 = 0; z0 < ranks; z0 += 4) {
+            float2 ml[4];
+            float4 o[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                ml[u] = make_float2(-INFINITY, 0.f);
+                o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (z0 + u < ranks) {
+                    uint32_t a, b;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sm + 4 * (PM_QT * HS + 2 * r)), "r"(z0 + u));
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(sm + 4 * (r * HS + d)), "r"(z0 + u));
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(ml[u].x), "=f"(ml[u].y) : "r"(a) : "memory");
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o[u].x), "=f"(o[u].y), "=f"(o[u].z), "=f"(o[u].w) : "r"(b) : "memory");
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (ml[u].y > 0.f || ml[u].y != ml[u].y) {  // (a rank without positions of this query has no sum; a NaN stays one)
+                    const float Mn = fmaxf(M, ml[u].x);
+                    const float a = M == -INFINITY ? 0.f : expf(M - Mn), b = expf(ml[u].x - Mn);
+                    num.x = num.x * a + b * o[u].x; num.y = num.y * a + b * o[u].y; num.z = num.z * a + b * o[u].z; num.w = num.w * a + b * o[u].w;
+                    den = den * a + b * ml[u].y;
+                    M = Mn;
+                }
+        }
+        const float il = 1.0f / (den * 4096.f);
+        *reinterpret_cast<float4*>(out + (size_t)(t0 + r) * out_ld + (size_t)head * HS + d) = make_float4(num.x * il, num.y * il, num.z * il, num.w * il);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while another reads
 }
 
 // ---- small kernels around the GEMMs ---------------------------------------------------------------------------------
@@ -721,14 +776,36 @@ int prefill_attention_launch(slai_ctx* ctx, const float* q, int q_ld, const void
     if (kv_f16 && (head_size == 64 || head_size == 128) && q_ld % 2 == 0) {
         // (other heads and f32 caches: the f32 kernel below)
         const size_t sm = (size_t)4 * PM_KT * head_size * 2;
-        const dim3 g((unsigned)n_heads, (unsigned)((T + PM_QT - 1) / PM_QT));
+        const int q_tiles = (T + PM_QT - 1) / PM_QT, tiles = (pos0 + T - 1) / PM_KT + 1;
+        // CTAs that share a (head, 64 queries): while all of them run side by side (two to an SM) and none is left without a tile for long.
+        int ranks = 1;
+        while (ranks < 8 && ranks < tiles && (long long)n_heads * q_tiles * ranks * 2 <= 2 * (ctx->sm_count > 0 ? ctx->sm_count : 148)) ranks *= 2;
         static PerDeviceOnce once;
         if (once.need(ctx->device)) {
             SLAI_CHECK_CUDA(ctx, cudaFuncSetAttribute(prefill_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * PM_KT * 128 * 2));
             once.set(ctx->device);
         }
-        return launch_dependent(ctx, head_size == 64 ? prefill_attn_mma_kernel<64> : prefill_attn_mma_kernel<128>, g, PM_THREADS, sm, ctx->use_pdl, q, q_ld,
-                                (const __half*)kc, (const __half*)vc, head_stride, kv_mul, pos0, T, out, out_ld);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n_heads, (unsigned)q_tiles, (unsigned)ranks);
+        cfg.blockDim = dim3(PM_THREADS);
+        cfg.dynamicSmemBytes = sm;
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute at[2];
+        int n = 0;
+        if (ranks > 1) {
+            at[n].id = cudaLaunchAttributeClusterDimension;
+            at[n].val.clusterDim.x = at[n].val.clusterDim.y = 1;
+            at[n++].val.clusterDim.z = (unsigned)ranks;
+        }
+        if (ctx->use_pdl) {
+            at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[n++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        cfg.attrs = at;
+        cfg.numAttrs = n;
+        SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, head_size == 64 ? prefill_attn_mma_kernel<64> : prefill_attn_mma_kernel<128>, q, q_ld, (const __half*)kc,
+                                                (const __half*)vc, (long long)head_stride, kv_mul, pos0, T, out, out_ld));
+        return SLAI_OK;
     }
     const size_t smem = ((size_t)PA_QT * head_size + (size_t)PA_KT * (head_size + 4) + (size_t)PA_KT * head_size + PA_QT * PA_KT) * 4;
     const dim3 grid((unsigned)n_heads, (unsigned)((T + PA_QT - 1) / PA_QT));
