@@ -31,7 +31,7 @@ struct Plan {
     size_t smem = 0;
 };
 
-bool plan(slai_ctx* ctx, const DecodeLayers& D, LayersParams& P, Plan& pl) {
+bool plan(slai_ctx* ctx, const DecodeLayers& D, bool cluster, LayersParams& P, Plan& pl) {
     const int esz = D.kv_f16 ? 2 : 4, hs = D.head_size;
     if (ctx->sm_count <= 0 || D.n_layers < 1 || D.n_layers > MAX_LAYERS) return false;
     if (hs % 8 || hs * esz < 64 || hs * esz > 512) return false;  // a cached row is 4 to 32 lanes, 16 bytes each; eight elements share a lane's work
@@ -58,7 +58,7 @@ bool plan(slai_ctx* ctx, const DecodeLayers& D, LayersParams& P, Plan& pl) {
     if (P.kvq > 2) return false;
     // No more blocks than some phase has tiles: a barrier of fewer blocks is quicker.
     pl.grid = std::min(ctx->sm_count, *std::max_element(items, items + PH_COUNT));
-    P.cluster = one_cluster(D) ? 1 : 0;
+    P.cluster = cluster && one_cluster(D) ? 1 : 0;
     if (P.cluster) pl.grid = CLUSTER;
 
     size_t dig = 0;
@@ -102,7 +102,7 @@ bool plan(slai_ctx* ctx, const DecodeLayers& D, LayersParams& P, Plan& pl) {
 bool decode_layers_supported(slai_ctx* ctx, const DecodeLayers& D) {
     static thread_local LayersParams P;  // (some 20 KB: not on the caller's stack)
     Plan pl;
-    return plan(ctx, D, P, pl);
+    return plan(ctx, D, false, P, pl);  // (one cluster is only ever taken instead)
 }
 
 size_t decode_layers_scratch_bytes(const DecodeLayers& D) {
@@ -111,11 +111,14 @@ size_t decode_layers_scratch_bytes(const DecodeLayers& D) {
 
 unsigned int* decode_layers_counter(void* scratch) { return reinterpret_cast<unsigned int*>(scratch); }
 
-int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch) {
+static int launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch, bool cluster) {
     static thread_local LayersParams P;
     P = LayersParams{};
     Plan pl;
-    SLAI_REQUIRE(ctx, plan(ctx, D, P, pl), SLAI_ERR_SHAPE, "decode: these layers do not fit one launch");
+    if (!plan(ctx, D, cluster, P, pl)) {
+        if (cluster) return NO_CLUSTER;  // (a few tall matrices: more rows than 16 blocks' epilogues take)
+        return slai_set_error(ctx, SLAI_ERR_SHAPE, "decode: these layers do not fit one launch");
+    }
     P.n_layers = D.n_layers;
     P.eps = D.eps;
     P.x = D.x; P.q = D.q; P.xb = D.xb; P.hb = D.hb;
@@ -151,4 +154,9 @@ int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayer
         case SLAI_FMT_Q8_0: return decode_layers_launch_q80(ctx, P, D.arch, D.kv_f16, pl.grid, pl.smem);
     }
     return slai_set_error(ctx, SLAI_ERR_UNSUPPORTED_FORMAT, "decode: format %d has no kernel", D.fmt);
+}
+
+int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch) {
+    const int rc = launch(ctx, D, layers, scratch, true);
+    return rc == NO_CLUSTER ? launch(ctx, D, layers, scratch, false) : rc;
 }

@@ -33,6 +33,7 @@ enum Phase { PH_QKV = 0, PH_O = 1, PH_FF1 = 2, PH_FF2 = 3, PH_COUNT = 4 };
 enum Arch { ARCH_LLAMA = 0, ARCH_GPT2 = 1 };
 constexpr int MAX_LAYERS = 128;
 constexpr int MAX_SPLITS = 16;
+constexpr int NO_CLUSTER = -1000;  // launch_inst: the cluster does not fit, nothing was launched
 constexpr int MAX_TILES = THREADS / 16;  // row tiles of a block in a phase: its rows are the epilogue's threads
 
 struct LayerPtrs {
@@ -855,16 +856,21 @@ int launch_inst(slai_ctx* ctx, const LayersParams& P, int grid, size_t smem) {
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at[1];  // the blocks wait on one another: all of them resident, or none
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     if (P.cluster) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned int)grid;
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        int clusters = 0;  // (none on a part of a chip without that many neighbouring SMs)
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
+            cudaGetLastError();
+            return NO_CLUSTER;
+        }
     } else {
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
     }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, P));
     return SLAI_OK;
 }

@@ -40,6 +40,24 @@ def test_decode_against_the_oracle(backend, dim, hidden, hq, hkv, fmt, kv, n):
     m.close()
 
 
+def test_biases_and_a_tall_feed_forward_part(backend):
+    """q / k / v biases with adjacent-pair RoPE; few bytes a layer, but more feed-forward rows than one cluster's epilogues take."""
+    cfg = Llama2Config(dim=64, hidden_dim=9216, n_layers=2, n_q_heads=2, n_kv_heads=1, vocab_size=200, seq_len=24, kv_dtype=F32)
+    fmt = synth.FMT_Q8_0
+    w = synthetic_llama_host(cfg, fmt, seed=13, std=0.05, embd_std=1.0)
+    rng = np.random.default_rng(1)
+    for l in range(cfg.n_layers):
+        w[("bq", l)] = (0.1 * rng.standard_normal(64)).astype(np.float32)
+        w[("bk", l)], w[("bv", l)] = ((0.1 * rng.standard_normal(32)).astype(np.float32) for _ in range(2))
+    m = llama_from_host(backend, cfg, w, fmt)
+    ref = oracle_llama(cfg, w, fmt)
+    for pos in range(cfg.seq_len):
+        tok = int(rng.integers(cfg.vocab_size))
+        assert rel_l2(m.forward_logits(pos, tok)[0], ref.forward(tok, pos)) < 1e-3, pos
+    assert m.launches_per_token() == 4
+    m.close()
+
+
 def test_gpt2_decode_against_the_oracle(backend):
     p = Gpt2Params(n_vocab=300, n_seq=300, n_embd=960, n_head=15, n_layer=2, ff_len=3840, kv_dtype=F16)
     w = synthetic_gpt2_host(p, synth.FMT_Q8_0, seed=4, std=0.05)
