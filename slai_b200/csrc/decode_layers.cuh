@@ -206,40 +206,13 @@ __device__ __forceinline__ void merged(const LayersParams& P, int S, int i, floa
     for (int e = 0; e < 2; e++) { q[e].x *= r; q[e].y *= r; q[e].z *= r; q[e].w *= r; }
 }
 
-// ---- the input vector as digit planes --------------------------------------------------------------------------------
-// One pass: a warp turns 256 elements (8 a lane) into digits at a power-of-two scale of their own, so nothing waits for the vector's largest
-// element; the product's sums of a step are multiplied by 1 / scale.  An RmsNorm needs no pass either: the digits are those of x * w, and
-// 1 / rms is a factor of the results (`sq`: this warp's sum of squares).  A LayerNorm does (its mean is subtracted first), for K <= 4096,
-// where every warp has 256 elements at most.
-// One code for all phases, in a loop: a phase's code is run once between barriers, so what it spends is instruction fetches (unrolled
-// six times as in gemv_kernel.cuh, with a copy per kind of input, the kernel was 137 KB and staging 288 elements took 2.3 us).
-template <class F, bool LN>
-__device__ __forceinline__ float stage_steps(const LayersParams& P, const float4* x4, int merge, const float* norm_w, const float* norm_b, int K, float eps, const Smem& S,
-                                             float* inv, float* stat) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    unsigned char* dig = reinterpret_cast<unsigned char*>(__cvta_shared_to_generic(S.dig));
-    unsigned char* sv = reinterpret_cast<unsigned char*>(__cvta_shared_to_generic(S.sv));
-    float sq = 0.f;
-    float4 nq[2], nw[2];
-#pragma unroll 1
-    for (int step = warp - WARPS;; step += WARPS) {  // (the loads of a round are ahead of its work, the first round only loads)
-        const int n4 = K >> 2, next = step + WARPS;
-        const bool more = 256 * next < K || (LN && norm_w && next == warp);
-        float4 q[2], w[2];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int j = 64 * next + 2 * lane + e;
-            q[e] = nq[e];
-            w[e] = nw[e];
-            nq[e] = more && j < n4 && merge <= 1 ? __ldcg(x4 + j) : zero4;
-            nw[e] = more && norm_w && j < n4 ? __ldg(reinterpret_cast<const float4*>(norm_w) + j) : zero4;
-        }
-        if (step < 0) {
-            if (!more) break;
-            continue;
-        }
-        const int i = 64 * step + 2 * lane;
+// The input of a phase's product for stage_steps: a vector, or the splits' partial outputs of the attention.
+struct PhaseInput {
+    const LayersParams& P;
+    const float4* x4;
+    int merge;  // splits to be merged (0, 1: none)
+    __device__ __forceinline__ float4 load(int j) const { return merge <= 1 ? __ldcg(x4 + j) : make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void finish(int i, int n4, float4 (&q)[2]) const {
         if (merge > 1 && i < n4) {
             merged(P, merge, i, q);
             if (blockIdx.x == 0) {  // (for slai_llama_read_state: nobody reads it inside the step)
@@ -247,80 +220,8 @@ __device__ __forceinline__ float stage_steps(const LayersParams& P, const float4
                 reinterpret_cast<float4*>(P.xb)[i + 1] = q[1];
             }
         }
-        if (norm_w) {
-            float mul = 1.f;
-            if (LN) {
-                float s = 0.f, none = 0.f;
-#pragma unroll
-                for (int e = 0; e < 2; e++) s += (q[e].x + q[e].y) + (q[e].z + q[e].w);
-                block_sum_max(s, none, stat);
-                const float mean = s / (float)K;
-                s = 0.f;
-#pragma unroll
-                for (int e = 0; e < 2; e++)
-                    if (i + e < n4) {
-                        q[e].x -= mean; q[e].y -= mean; q[e].z -= mean; q[e].w -= mean;
-                        s += q[e].x * q[e].x + q[e].y * q[e].y + q[e].z * q[e].z + q[e].w * q[e].w;
-                    }
-                block_sum_max(s, none, stat);
-                mul = 1.0f / sqrtf(s / (float)K + eps);
-            }
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                if (!LN) sq += q[e].x * q[e].x + q[e].y * q[e].y + q[e].z * q[e].z + q[e].w * q[e].w;
-                q[e].x = (q[e].x * mul) * w[e].x; q[e].y = (q[e].y * mul) * w[e].y; q[e].z = (q[e].z * mul) * w[e].z; q[e].w = (q[e].w * mul) * w[e].w;
-                if (LN && norm_b && i + e < n4) {
-                    const float4 b = __ldg(reinterpret_cast<const float4*>(norm_b) + i + e);
-                    q[e].x += b.x; q[e].y += b.y; q[e].z += b.z; q[e].w += b.w;
-                }
-            }
-        }
-        const float mx = warp_max(fmaxf(max4(q[0]), max4(q[1])));
-        float scale = 1.f, back = 1.f;
-        if (mx > 0.f && mx < 3.0e38f) {
-            const int e = max((int)(__float_as_uint(mx) >> 23) - 126, -90);  // mx = f * 2^e with f in [0.5, 1) (normal numbers)
-            scale = __uint_as_float((uint32_t)(127 + 26 - e) << 23);         // 2^(26 - e), and its inverse
-            back = __uint_as_float((uint32_t)(127 - 26 + e) << 23);
-        }
-        uint32_t pw[2][4];
-#pragma unroll
-        for (int e = 0; e < 2; e++)
-            digit_planes(digits_word(__float2int_rn(q[e].x * scale)), digits_word(__float2int_rn(q[e].y * scale)), digits_word(__float2int_rn(q[e].z * scale)),
-                         digits_word(__float2int_rn(q[e].w * scale)), pw[e]);
-        if (256 * step < K) {  // (a warp without elements took part in the LayerNorm's sums)
-#pragma unroll
-            for (int p = 0; p < 4; p++) *reinterpret_cast<uint2*>(dig + (size_t)p * S.plane + 256 * step + 8 * lane) = make_uint2(pw[0][p], pw[1][p]);
-            if (lane == 0) inv[step] = back;
-            if (F::SV_GRAN > 0) {
-                // digit sums of the sub-blocks, layouts of gemv_formats.cuh; two biased sums to a word, so that a shuffle serves two planes
-                constexpr int LANES = F::SV_GRAN > 0 ? F::SV_GRAN / 8 : 1, BIAS = 1024;  // (eight digits' sum lies in [-1024, 1016])
-                uint32_t s01 = (uint32_t)__dp4a((int)pw[0][0], 0x01010101, __dp4a((int)pw[1][0], 0x01010101, BIAS)) |
-                               ((uint32_t)__dp4a((int)pw[0][1], 0x01010101, __dp4a((int)pw[1][1], 0x01010101, BIAS)) << 16);
-                uint32_t s23 = (uint32_t)__dp4a((int)pw[0][2], 0x01010101, __dp4a((int)pw[1][2], 0x01010101, BIAS)) |
-                               ((uint32_t)__dp4a((int)pw[0][3], 0x01010101, __dp4a((int)pw[1][3], 0x01010101, BIAS)) << 16);
-#pragma unroll
-                for (int o = 1; o < LANES; o <<= 1) {
-                    s01 += __shfl_xor_sync(0xffffffffu, s01, o);
-                    s23 += __shfl_xor_sync(0xffffffffu, s23, o);
-                }
-                if (F::SV_GRAN == 32) {  // lane 4j + p: plane p of sub-block j
-                    const int p = lane & 3, j = lane >> 2;
-                    const uint32_t two = p & 2 ? s23 : s01;
-                    const int sd = (int)((p & 1) ? two >> 16 : two & 0xFFFFu) - BIAS * LANES, hi = (sd + 64) >> 7;
-                    unsigned char* tab = sv + step * 128;
-                    tab[(2 * p) * 16 + j] = (unsigned char)hi;
-                    tab[(2 * p + 1) * 16 + j] = (unsigned char)(sd - (hi << 7));
-                    if (lane < 8) *reinterpret_cast<uint2*>(tab + lane * 16 + 8) = make_uint2(0u, 0u);
-                } else if ((lane & (LANES - 1)) == 0) {
-                    reinterpret_cast<int4*>(sv)[16 * step + lane / LANES] =
-                        make_int4((int)(s01 & 0xFFFFu) - BIAS * LANES, (int)(s01 >> 16) - BIAS * LANES, (int)(s23 & 0xFFFFu) - BIAS * LANES, (int)(s23 >> 16) - BIAS * LANES);
-                }
-            }
-        }
-        if (!more) break;
     }
-    return sq;
-}
+};
 
 // The oldest stage's blocks are here.  A wait that runs out: nothing more is requested (Feed::run stays 0).
 template <class F>
@@ -702,8 +603,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
                 S.sv = S.dig + 4 * S.plane;
                 const bool norm = ph == PH_QKV || ph == PH_FF1;
                 const float* src = norm ? P.x : ph == PH_O ? P.xb : P.hb;
-                float sq = stage_steps<F, ARCH == ARCH_GPT2>(P, reinterpret_cast<const float4*>(src), ph == PH_O ? S_att : 0, norm ? W.norm_w[ph >> 1] : nullptr,
-                                                             W.norm_b[ph >> 1], K, P.eps, S, inv, stat);
+                float sq = stage_steps<F, ARCH == ARCH_GPT2>(PhaseInput{P, reinterpret_cast<const float4*>(src), ph == PH_O ? S_att : 0},
+                                                             norm ? W.norm_w[ph >> 1] : nullptr, W.norm_b[ph >> 1], K, P.eps, S, inv, stat);
                 if (ARCH == ARCH_LLAMA && norm) {
                     sq = warp_sum(sq);
                     if (lane == 0) stat[warp] = sq;

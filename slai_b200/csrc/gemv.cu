@@ -31,7 +31,8 @@ __global__ void __launch_bounds__(THREADS, SLAI_GEMV_MINB) gemv_kernel(const __g
     // Pull data the *next* kernel reads first (its norm weights) into L2 while this one runs.
     if (P.pf_lines > 0 && (int)blockIdx.x == (int)gridDim.x - 1)
         for (int i = threadIdx.x; i < P.pf_lines; i += THREADS) asm volatile("prefetch.global.L2 [%0];" ::"l"(P.pf_ptr + (size_t)i * 128));
-    // partial-sum buffer cleared while the predecessor drains
+    // partial-sum buffer and zero page cleared while the predecessor drains
+    if (threadIdx.x < ZERO_BYTES / 4) reinterpret_cast<uint32_t*>(smem_raw)[threadIdx.x] = 0u;
     for (int i = threadIdx.x; i < WAVE * WARPS * NMAT * 16; i += THREADS) reinterpret_cast<float*>(smem_raw + P.dig_region)[i] = 0.f;
     SLAI_TRACE_POINT(3)
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -132,7 +133,7 @@ size_t gemv_dig_region(int fmt, int K) {
     const int Kp = (K + 255) & ~255;
     const int sv_gran = (fmt == SLAI_FMT_Q4_K || fmt == SLAI_FMT_Q5_K) ? 32 : fmt == SLAI_FMT_Q6_K ? 16 : 0;
     const size_t sv_bytes = sv_gran ? (size_t)(Kp / sv_gran) * 16 : 0;
-    return ((size_t)gemvfmt::ZERO_BYTES + ((size_t)4 * (Kp + 32) + sv_bytes) + 127) & ~(size_t)127;
+    return ((size_t)gemvfmt::ZERO_BYTES + ((size_t)4 * (Kp + 32) + sv_bytes) + (size_t)Kp / 256 * 4 + 127) & ~(size_t)127;  // (and a scale per 256 elements)
 }
 
 // Validate a launch description and turn it into kernel parameters.  `dig_region` = 0: size it for this K.
