@@ -73,7 +73,7 @@ int tp_all_gather(slai_ctx* ctx, const float* d_in, float* d_out, int64_t n);
 // tp.cu: one more token decoded (sequence numbers of the peer exchange derive from it)
 int tp_tick(slai_ctx* ctx);
 
-// Map of slai_ctx::d_counters (unsigned words, all zero between launches).
+// Map of slai_ctx::d_counters (unsigned words, all zero between launches but the prompt flags).
 constexpr int CNT_ATTN_TICKETS = 0;    // one ticket per KV head (<= 1024): last split of a head merges the partials
 constexpr int CNT_ARGMAX = 1100;       // ticket, then per-block (value, index) pairs of the multi-block argmax
 constexpr int CNT_ATTN_POS = 2048;     // position scalar of the stand-alone slai_attention

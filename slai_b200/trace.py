@@ -30,6 +30,8 @@ EPI = {0: "store", 1: "resid", 2: "silu", 3: "gelu", 4: "qkv", 5: "xchg"}
 def kernel_name(kid: int) -> str:
     if kid == 999:
         return "attention"
+    if 2000 <= kid < 2004:  # phases of the one-launch layers (decode_layers.cuh); attention counts as o's wait
+        return "layers: " + ("q/k/v", "attention, o", "ff in", "ff out")[kid - 2000]
     k256, rest = divmod(kid, 1000)
     nmat, rest = divmod(rest, 100)
     pro, epi = divmod(rest, 10)
@@ -65,15 +67,20 @@ def summarise(rec: np.ndarray):
         if key not in rows:
             rows[key] = []
             order.append(key)
+        end = t[13]
         if kid == 999:
             parts = [0.0] * len(COLS)
             parts[3] = t[4] - t[0]
             parts[9] = t[13] - t[4]
+        elif kid >= 2000 and kid < 2004:  # stamps: 0 begin, 2 barrier passed, 3 staged, 4 loop done, 5 partial sums complete, 6 end
+            parts = [0.0] * len(COLS)
+            parts[3], parts[7], parts[9], parts[10], parts[11] = t[2] - t[0], t[3] - t[2], t[4] - t[3], t[5] - t[4], t[6] - t[5]
+            end = t[6]
         else:
             parts = [t[b] - t[a] for _, a, b in COLS]
         period = (rec[i + 1, 1] * 1e-3 - t[0]) if i + 1 < len(rec) else np.nan
-        handover = (rec[i + 1, 5] * 1e-3 - t[13]) if i + 1 < len(rec) else np.nan
-        rows[key].append(parts + [t[13] - t[0], period, handover])
+        after = i + 1 < len(rec) and not 2000 <= int(rec[i + 1, 0]) < 2004
+        rows[key].append(parts + [end - t[0], period, rec[i + 1, 5] * 1e-3 - end if after else np.nan])
     return [(key, len(rows[key]), *np.nanmean(np.array(rows[key]), axis=0)) for key in order]
 
 
