@@ -5,7 +5,10 @@
 // exact integers sc * q, so two products per 16 columns suffice (hi, lo); the super-block scale d multiplies the f32 sums
 // of each 256 columns, in registers, and the minimum term is one more product per super-block with its own sums and scale
 // dmin.  Q6_K (integers beyond fp16's 11 bits) and Q8_0 (a scale every 32 columns) carry the weights as pairs too: three
-// products (hi hi, hi lo, lo hi), about 2^-21 each.
+// products (hi hi, hi lo, lo hi), about 2^-21 each.  The tensor cores truncate a sum at every step, so whatever the format a sum ends with its
+// super-block (256 columns, Q8_0: 128) and the next one is added to it in registers: the error depends neither on K nor on how K is shared out.
+// (Q8_0 summed a CTA's whole share of K before.  One product against the sequential pass, before / now: 512 columns, 37 tokens 5.7e-7 / 1.9e-7; 4096
+// columns, 400 tokens 8.5e-6 / 3.5e-7.  4 layers of the 7B shape: 37 tokens 579 / 602 us, 511 tokens 2080 / 2360; sums of 256 columns: 603, 2210, 6.2e-7.)
 //
 // One CTA computes 128 weight rows x NT tokens (<= 128) over its share of K:
 //   warp 0      TMA: the activations' hi and lo planes, 64 columns per stage; the sums plane, 16 columns per super-block
@@ -392,14 +395,14 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         // ---- tensor cores: the whole warp walks the loop, so that descriptors live in uniform registers, one lane issues ----
         const uint32_t idesc = umma_idesc(PAIR ? 2 * PG_BM : PG_BM, NT), idesc2 = umma_idesc(PG_BM, 2 * NT);
         const uint64_t db0 = desc128(sb + L.b);
-        int slot = 0, u = 0;  // u: sums so far (of a super-block; Q8_0: of a tile's part), alternately in two buffers
+        int slot = 0, u = 0;  // u: super-blocks so far, their sums alternately in two buffers
         uint32_t ph = 0;
         for (int un = u_lo, nc; un < u_hi; un += nc) {
         nc = part_at(un).nc;
-        for (int c = 0; c < nc; c++) {
+        for (int c = 0; c < nc; c++, u++) {
             const int buf = u & 1;
             const uint32_t d = tmem + buf * DS;
-            if ((F::SCALED || c == 0) && u >= 2) mbar_wait<PAIR>(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
+            if (u >= 2) mbar_wait<PAIR>(dempty + 8 * buf, ((u >> 1) - 1) & 1, limit, P.err_flag);
             for (int st = 0; st < F::STAGES; st++) {
                 mbar_wait<PAIR>(full + 8 * slot, ph, limit, P.err_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -410,7 +413,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < PG_BK / 16; kk++) {
-                        const bool first = kk == 0 && st == 0 && (F::SCALED || c == 0);
+                        const bool first = kk == 0 && st == 0;
                         if (MERGED) {
                             umma_f16_ts<PAIR>(d, ah + 8 * kk, dbh + 2 * kk, idesc2, first ? 0u : 1u);
                         } else {
@@ -438,9 +441,8 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             if (elect_one()) {
                 if (F::MIN)
                     umma_f16<PAIR>(tmem + 2 * DS, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NB * 32), idesc, 0u);
-                if (F::SCALED || c == nc - 1) umma_commit<PAIR>(dfull + 8 * buf);
+                umma_commit<PAIR>(dfull + 8 * buf);
             }
-            if (F::SCALED || c == nc - 1) u++;
             __syncwarp();
         }
         }
@@ -568,7 +570,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             for (int i = 0; i < NG; i++)
 #pragma unroll
                 for (int j = 0; j < 16; j++) acc[i][j] = 0.f;
-            for (int c = F::SCALED ? 0 : nc - 1; c < nc; c++, u++) {
+            for (int c = 0; c < nc; c++, u++) {
                 const int buf = u & 1;
                 float d = 1.f, mn = 0.f;
                 if (F::SCALED) {
@@ -607,7 +609,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                         if (MERGED && F::MIN) tmem_ld16(tq + 2 * DS + col, z);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : __uint_as_float(v[j]);
+                        for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(v[j]), acc[i][j]) : acc[i][j] + __uint_as_float(v[j]);
                         if (MERGED) {
 #pragma unroll
                             for (int j = 0; j < 16; j++) acc[i][j] = F::SCALED ? fmaf(d, __uint_as_float(w[j]), acc[i][j]) : acc[i][j] + __uint_as_float(w[j]);

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from slai_b200 import synth, _lib
-from slai_b200.models import Gpt2Params, Llama2Config, llama_from_host, synthetic_gpt2_device, synthetic_llama_host
+from slai_b200.models import Gpt2Params, Llama2Config, llama_from_host, synthetic_gpt2_device, synthetic_llama_device, synthetic_llama_host
 from slai_b200.ops import BatchedMultiqueryAttentionParams
 from helpers import rel_l2
 
@@ -32,6 +32,24 @@ def test_prompt_pass_at_the_edges_of_its_tiles(backend, monkeypatch, fmt, T):
     for t in {0, T // 2, T - 1}:  # every token on its own, the last row of every head included
         assert rel_l2(kb[t], ks[t]) < 2e-5 and rel_l2(vb[t], vs[t]) < 2e-5
     assert rel_l2(got, want) < 1e-4  # one layer and the logits product
+
+
+# Q8_0 has no scale per super-block: its sums ended with a CTA's share of K, so their error depended on how K was shared out (512 columns, 37 tokens:
+# 1.7e-7 over a cluster of four, 5.7e-7 in one CTA; 4096 columns, 400 tokens: 9e-6).
+@pytest.mark.parametrize("dim,T", [(512, 16), (512, 37), (512, 300), (2048, 37), (4096, 16), (4096, 400)])
+def test_q8_0_sums_do_not_lose_bits_with_k(backend, monkeypatch, dim, T):
+    cfg = Llama2Config(dim=dim, hidden_dim=256, n_layers=1, n_q_heads=dim // 64, n_kv_heads=dim // 64, vocab_size=300, seq_len=T, kv_dtype=_lib.KV_F32)
+    batched, seq = (synthetic_llama_device(backend, cfg, synth.FMT_Q8_0, synth.FMT_Q8_0, seed=5, std=0.02) for _ in range(2))
+    ids = np.random.default_rng(T).integers(0, cfg.vocab_size, size=T).astype(np.int32)
+    batched.prefill(ids, 0)
+    monkeypatch.setenv("SLAI_PREFILL_SEQUENTIAL", "1")
+    seq.prefill(ids, 0)
+    # 128 columns are 24 products added up by the tensor core, each truncated by half of 2^-24 of a sum that is half of the last one on average: 3.6e-7;
+    # operands of 22 bits, f32 sums over the super-blocks
+    for got, want in zip(batched.read_kv(0, T), seq.read_kv(0, T)):
+        assert rel_l2(got, want) < 5e-7
+    batched.close()
+    seq.close()
 
 
 # The tensor-core attention (f16 cache, heads of 64 and 128): query tiles of 64, position tiles of 64, a first position inside a tile.

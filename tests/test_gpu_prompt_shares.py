@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 # 148 SMs: q/k/v are 96 tiles of 128 rows x 16 super-blocks (10.4 a CTA: a tile lies on up to three), gate and up 172; above 64 tokens pairs of CTAs
-# and several token tiles (400: 192 tiles over 74 pairs).  Q8_0 sums a part of a tile as a whole.
+# and several token tiles (400: 192 tiles over 74 pairs).
 @pytest.mark.parametrize("fmt", [synth.FMT_Q4_K, synth.FMT_Q6_K, synth.FMT_Q8_0])
 @pytest.mark.parametrize("T", [16, 40, 64, 400])
 def test_products_with_shared_tiles(backend, monkeypatch, fmt, T):
@@ -25,7 +25,7 @@ def test_products_with_shared_tiles(backend, monkeypatch, fmt, T):
     monkeypatch.setenv("SLAI_PREFILL_SEQUENTIAL", "1")
     want = seq.prefill(ids, 0, want_logits=True)
     ks, vs = seq.read_kv(0, T)
-    # operands of 22 bits, f32 sums of 16 blocks of 256 (Q8_0: of 4096 columns, truncated by the tensor core): below 2e-5
+    # operands of 22 bits, f32 sums of 16 blocks of 256 (Q8_0: 32 of 128): below 2e-5
     assert rel_l2(k, ks) < 2e-5 and rel_l2(v, vs) < 2e-5, (rel_l2(k, ks), rel_l2(v, vs))
     assert rel_l2(got, want) < 2e-4  # one layer and the logits product
     batched.close()
