@@ -82,6 +82,10 @@ constexpr int CNT_PROMPT_FLAGS = 3072;  // one word per CTA of a prompt GEMM: th
 constexpr int CNT_PROMPT_FLAG_WORDS = 512;
 constexpr int CNT_WORDS = 4096;
 
+// Polls of a wait for a block's own copies and products after those of slai_ctx::wait_limit, which only raise the error flag: they have to land before
+// the block ends, since its shared and tensor memory are another block's by then.
+constexpr unsigned int LAST_POLLS = (1u << 20) + 1;  // (odd, where wait_limit is even: a wait tells its parts apart by them)
+
 int slai_set_error(slai_ctx* ctx, int code, const char* fmt, ...);
 int slai_check_wait_flag(slai_ctx* ctx);  // ops.cu: SLAI_ERR_TIMEOUT if a bounded device-side wait ran out (stream must be idle)
 

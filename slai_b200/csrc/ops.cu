@@ -124,7 +124,7 @@ int slai_stats_mark(slai_ctx* ctx, int cls) {
 SLAI_API int slai_ctx_set_wait_limit(slai_ctx* ctx, uint32_t rounds) {
     if (!ctx) return SLAI_ERR_INVALID_ARG;
     SLAI_REQUIRE(ctx, rounds >= 16, SLAI_ERR_INVALID_ARG, "wait limit of %u rounds is too short for a healthy launch", rounds);
-    ctx->wait_limit = rounds;  // read when a launch is described: passes and graphs recorded earlier keep theirs
+    ctx->wait_limit = rounds - rounds % 2;  // (even: LAST_POLLS) read when a launch is described: passes and graphs recorded earlier keep theirs
     return SLAI_OK;
 }
 SLAI_API const char* slai_last_error_string(slai_ctx* ctx) { return ctx ? ctx->last_error.c_str() : g_noctx_error.c_str(); }

@@ -29,8 +29,10 @@
 // executed, where cuBLAS keeps 1375); with few tokens the chain of a stage through operand writer, product and commit (some 620 cycles for products of
 // 200), and 8 us of start and end a launch.  us per product of the 7B shape, weights' operands in shared memory and whole tiles / now: 511 tokens q/k/v 89.5 / 82, gate
 // and up 145 / 135, down 77 / 72; 37 tokens gate and up 57 / 34.
-// Every mbarrier wait is bounded: on expiry the error flag is raised, later waits of the thread give up at once and the
-// kernel runs to its end.
+// Every wait is bounded (mbar_wait): `wait_limit` polls, after which the error flag is raised, then LAST_POLLS more, because what it waits for is this CTA's
+// (pair's) own work and copies, which have to land before the CTA ends.  Only a thread whose last polls ran out too goes on without: it arrives on nothing and
+// requests nothing from then on, so that no barrier completes a phase it has not reached.  Whoever requested copies or products waits for
+// the last of them at its end.
 #include <math.h>
 
 #include <algorithm>
@@ -49,6 +51,7 @@ constexpr int PG_MAX_CTAS = CNT_PROMPT_FLAG_WORDS;
 constexpr int PG_MAX_STAGES = 6, PG_MAX_PACK = 3, PG_MAX_KS = 8;
 constexpr int PG_A_COLS = PG_BK / 2;            // tensor-memory columns of one operand plane of a stage
 constexpr int PG_SMEM_LIMIT = 227 * 1024 - 512; // the barriers are static
+constexpr unsigned int PART_POLLS = 1u << 14;   // fewest polls for another CTA's sums: some 10 ms, its whole work is a few
 
 struct PgSeg {
     const uint8_t* w;
@@ -87,33 +90,25 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(a), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// The same for a barrier that the other CTA of a pair arrives on too.
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(a), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// Bounded wait.  On expiry the error flag is raised and `limit` drops to one poll.
+// Bounded wait in two parts, see the top: `limit` polls, then (the error flag raised) LAST_POLLS, which `limit` is from then on; 0 once those have run out: that
+// wait and all later ones of the thread return false.  CLUSTER: on a barrier that the other CTA of a pair arrives on too.
+// (PTX, for its size: the waits are in loops whose time is a chain of waits, and unrolled; two loops in a wait cost 1 us a launch at 16 tokens.)
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
-    for (unsigned int i = 0; i < limit; i++) {
-        if (CLUSTER ? mbar_try_cluster(a, parity) : mbar_try(a, parity)) return true;
-        if (i > 64) __nanosleep(40);
-    }
-    atomicExch(err_flag, 5u);
-    limit = 1;
-    return false;
+#define PG_WAIT(SEM)                                                                                                                     \
+    asm volatile(                                                                                                                         \
+        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n"                                                                           \
+        "W:\n\tmbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t@p bra D;\n\tsetp.gt.u32 p, n, 64;\n\t"                     \
+        "@p nanosleep.u32 40;\n\tadd.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %0;\n\t@p bra W;\n\t"                                              \
+        "setp.eq.u32 p, %0, 0;\n\t@p bra D;\n\tst.volatile.global.u32 [%3], 5;\n\tsetp.eq.u32 p, %0, %4;\n\tselp.u32 %0, 0, %4, p;\n\t"  \
+        "mov.u32 n, 0;\n\tbra W;\nD:\n\t}"                                                                                               \
+        : "+r"(limit)                                                                                                                     \
+        : "r"(a), "r"(parity), "l"(err_flag), "n"(LAST_POLLS)                                                                             \
+        : "memory")
+    if (CLUSTER) PG_WAIT(".acquire.cluster");
+    else PG_WAIT("");
+#undef PG_WAIT
+    return limit != 0;
 }
 __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {  // the same shared-memory address in another CTA of the cluster
     uint32_t r;
@@ -195,6 +190,12 @@ __device__ __forceinline__ void umma_commit(uint32_t mbar) {
     else
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
+// ... on this CTA's barrier alone.
+template <bool PAIR>
+__device__ __forceinline__ void umma_commit_here(uint32_t mbar) {
+    if (PAIR) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+    else umma_commit<false>(mbar);
+}
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -259,12 +260,12 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
     const PgLayout L = pg_layout<FMT>(NB, P.stages, P.packs);
     const int NT = P.NT, S = P.stages, PK = P.packs;
     const uint32_t b_bytes = (uint32_t)NB * PG_BK * 2;  // one activation plane of a stage
-    __shared__ __align__(8) unsigned long long bars[2 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 11];
+    __shared__ __align__(8) unsigned long long bars[2 * PG_MAX_STAGES + 2 * PG_MAX_PACK + 12];
     __shared__ uint32_t tmem_slot;
     const uint32_t sb = smem_u32(smem);
     const uint32_t full = smem_u32(bars), empty = full + 8 * PG_MAX_STAGES,
                    pk_full = empty + 8 * PG_MAX_STAGES, pk_empty = pk_full + 8 * PG_MAX_PACK, dfull = pk_empty + 8 * PG_MAX_PACK,
-                   dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16, mempty = sc_full + 32;
+                   dempty = dfull + 16, bmin_full = dempty + 16, sc_full = bmin_full + 16, mempty = sc_full + 32, all_done = mempty + 8;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (warp: uniform for the compiler too)
     const int pr = PAIR ? (int)(blockIdx.x & 1) : 0;  // rank in the pair
@@ -311,6 +312,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         }
         for (int s = 0; s < 4; s++) mbar_init(sc_full + 8 * s, 8);
         mbar_init(mempty, PAIR ? 16 : 8);
+        mbar_init(all_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async();
     }
@@ -384,11 +386,11 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
             }
         }
-        if (!ok && pr == 0) {  // a wait ran out: the copies in flight land before the CTA (the pair) may end
-            for (int i = max(0, issued - S); i < issued; i++) {
-                limit = P.wait_limit;
-                mbar_wait(full + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
-            }
+        if (pr == 0) {  // the last copies land before the CTA (the pair) ends
+            limit = LAST_POLLS;
+            for (int i = max(0, issued - S); i < issued; i++) mbar_wait(full + 8 * (i % S), (i / S) & 1, limit, P.err_flag);
+            limit = LAST_POLLS;
+            for (int i = max(0, gc - 2); F::MIN && i < gc; i++) mbar_wait(bmin_full + 8 * (i & 1), (i >> 1) & 1, limit, P.err_flag);
         }
     } else if (warp == 1) {
         if (pr == 0) {
@@ -422,7 +424,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                         }
                         if (F::PLANES == 2) umma_f16_ts<PAIR>(d, ah + PG_A_COLS + 8 * kk, dbh + 2 * kk, idesc, 1u);
                     }
-                    umma_commit<PAIR>(empty + 8 * slot);
+                    if (limit) umma_commit<PAIR>(empty + 8 * slot);  // (behind the products: in front of them the test costs 20 cycles a stage)
                 }
                 __syncwarp();
                 if (++slot == S) {
@@ -441,11 +443,15 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             if (elect_one()) {
                 if (F::MIN)
                     umma_f16<PAIR>(tmem + 2 * DS, desc32(sb + L.amin + buf * PG_BM * 32), desc32(sb + L.bmin + buf * NB * 32), idesc, 0u);
-                umma_commit<PAIR>(dfull + 8 * buf);
+                if (limit) umma_commit<PAIR>(dfull + 8 * buf);
             }
             __syncwarp();
         }
         }
+        if (elect_one()) umma_commit_here<PAIR>(all_done);  // no product is under way when the CTA ends
+        limit = LAST_POLLS;
+        mbar_wait<PAIR>(all_done, 0, limit, P.err_flag);
+        __syncwarp();
         }
     } else if (warp == 2) {
         // ---- packed weights ----
@@ -478,12 +484,8 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
             }
         }
-        if (!ok) {
-            for (int i = max(0, issued - PK); i < issued; i++) {
-                limit = P.wait_limit;
-                mbar_wait(pk_full + 8 * (i % PK), (i / PK) & 1, limit, P.err_flag);
-            }
-        }
+        limit = LAST_POLLS;
+        for (int i = max(0, issued - PK); i < issued; i++) mbar_wait(pk_full + 8 * (i % PK), (i / PK) & 1, limit, P.err_flag);  // the last copies have landed
     } else if (warp >= 4 && warp < 12) {
         // ---- weights into operand rows in tensor memory ----
         // Thread = row: a warp reaches the 32 lanes of its quarter; the two warps of a quarter share the columns.  (In shared memory the rows cost, per
@@ -508,7 +510,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 // the readers)
                 if (part == 0) scales[(c & 3) * PG_BM + r] = pfq::row_scale<FMT>(blk, r16);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(sc_full + 8 * (c & 3));
+                if (lane == 0 && limit) mbar_arrive(sc_full + 8 * (c & 3));
             }
             // two stages at a time: a warp's way through one is a chain of latencies (load, arithmetic, store, arrive)
 #pragma unroll
@@ -547,7 +549,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 if (F::MIN && st == 0) fence_async();  // the minimum term's operand comes before the tensor core's reads
                 __syncwarp();
-                if (lane == 0) {
+                if (lane == 0 && limit) {
                     arrive_issuer<PAIR>(full + 8 * slot0);
                     arrive_issuer<PAIR>(full + 8 * slot1);
                     if (st == F::STAGES - 2) mbar_arrive(pk_empty + 8 * ps);
@@ -562,6 +564,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
         // ---- sums out of tensor memory ----
         const uint32_t* scales = reinterpret_cast<const uint32_t*>(smem + L.scale);
         int u = 0;
+        unsigned int part_polls = max(P.wait_limit, PART_POLLS);
         for (int un = u_lo; un < u_hi;) {
             const Part q = part_at(un);
             const int nc = q.nc;
@@ -597,7 +600,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) arrive_issuer<PAIR>(mempty);
+                    if (lane == 0 && limit) arrive_issuer<PAIR>(mempty);
                 }
 #pragma unroll
                 for (int i = 0; i < NG; i++) {
@@ -626,7 +629,7 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) arrive_issuer<PAIR>(dempty + 8 * buf);
+                if (lane == 0 && limit) arrive_issuer<PAIR>(dempty + 8 * buf);
             }
             if (!PAIR && P.ks > 1) break;  // one tile per cluster, stored below
             const size_t slot_floats = (size_t)NT * PG_BM;
@@ -646,15 +649,15 @@ prefill_gemm_kernel(const __grid_constant__ PgParams P, const __grid_constant__ 
             for (int p = me + 1; q.c0 + nc < P.nch && p < many && share(p) < (q.tile + 1) * P.nch; p++) {
                 const int cta = PAIR ? 2 * p + pr : p;
                 bool there = false;
-                for (unsigned int i = 0; i < limit && !there; i++) {
+                for (unsigned int i = 0; i < part_polls && !there; i++) {
                     unsigned int f;
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(P.flags + cta) : "memory");
                     there = f == P.seq;
                     if (!there && i > 64) __nanosleep(40);
                 }
-                if (!there) {
+                if (!there) {  // nothing of this CTA's own depends on it: on without those sums
                     atomicExch(P.err_flag, 5u);
-                    limit = 1;
+                    part_polls = 1;
                 }
                 __syncwarp();
                 const float* src = P.part + cta * slot_floats + 32 * quad + lane;

@@ -188,3 +188,37 @@ def test_prompt_products_do_not_count_the_time_of_the_kernel_before_them():
         assert np.array_equal(got, ref)
     m.close()
     backend.close()
+
+
+@pytest.mark.parametrize("fmt,T,pos", [(synth.FMT_Q4_K, 37, 300), (synth.FMT_Q6_K, 37, 300), (synth.FMT_Q8_0, 37, 300), (synth.FMT_Q4_K, 300, 0)])
+def test_prompt_pass_with_the_shortest_wait_limit(fmt, T, pos):
+    """16 rounds: the wait for another CTA's sums has a limit of its own (with 16 polls it ran out in 9 of 10 short turns, and the sums were missing); a wait
+    inside a CTA that takes longer is reported, but goes on until what it waits for is there, so that nothing lands in another block's memory."""
+    backend = Backend(0)
+    cfg = Llama2Config(dim=4096, hidden_dim=11008, n_layers=2, n_q_heads=32, n_kv_heads=32, vocab_size=512, seq_len=340, kv_dtype=_lib.KV_F16)
+    m = synthetic_llama_device(backend, cfg, fmt, fmt, seed=1, std=0.02)
+    ids = (np.arange(T + pos) % cfg.vocab_size).astype(np.int32)
+
+    def turn():
+        logits = m.prefill(ids[pos:], pos, want_logits=True)
+        backend.synchronize()
+        return logits
+
+    if pos:
+        m.prefill(ids[:pos], 0)
+    want = turn(), *m.read_kv(0, pos + T)
+    want1 = m.read_kv(1, pos + T)
+    backend.set_wait_limit(16)
+    for _ in range(12):
+        try:
+            turn()
+        except SlaiError as e:
+            assert e.code == _lib.ERR_TIMEOUT and "prompt product" in str(e)
+        for got, ref in zip(m.read_kv(0, pos + T), want[1:]):
+            assert np.array_equal(got, ref)
+        for got, ref in zip(m.read_kv(1, pos + T), want1):
+            assert np.array_equal(got, ref)
+    backend.set_wait_limit(1 << 20)
+    assert np.array_equal(turn(), want[0])
+    m.close()
+    backend.close()
