@@ -86,6 +86,32 @@ constexpr int CNT_WORDS = 4096;
 // the block ends, since its shared and tensor memory are another block's by then.
 constexpr unsigned int LAST_POLLS = (1u << 20) + 1;  // (odd, where wait_limit is even: a wait tells its parts apart by them)
 
+#ifdef __CUDACC__
+// Waits for the phase `parity` of the barrier at `a`: `limit` polls, then (the error flag set to CODE) LAST_POLLS, which `limit` is from then on; 0 once those
+// have run out: that wait and all later ones of the thread return false after one poll, so that the kernel still ends.
+// CLUSTER: on a barrier that another CTA arrives on too.  SLEEP: 40 ns between polls from the 64th on.
+// (PTX, for its size: the prompt GEMM's waits are in loops whose time is a chain of waits, and unrolled; two loops in a wait cost 1 us a launch at 16 tokens.)
+template <bool CLUSTER, bool SLEEP, int CODE>
+__device__ __forceinline__ bool bounded_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
+#define SLAI_BOUNDED_WAIT(SEM, NAP)                                                                                                      \
+    asm volatile(                                                                                                                         \
+        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n"                                                                           \
+        "W:\n\tmbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t@p bra D;\n\t" NAP                                            \
+        "add.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %0;\n\t@p bra W;\n\t"                                                                      \
+        "setp.eq.u32 p, %0, 0;\n\t@p bra D;\n\tst.volatile.global.u32 [%3], %5;\n\tsetp.eq.u32 p, %0, %4;\n\tselp.u32 %0, 0, %4, p;\n\t" \
+        "mov.u32 n, 0;\n\tbra W;\nD:\n\t}"                                                                                               \
+        : "+r"(limit)                                                                                                                     \
+        : "r"(a), "r"(parity), "l"(err_flag), "n"(LAST_POLLS), "n"(CODE)                                                                  \
+        : "memory")
+    if (CLUSTER && SLEEP) SLAI_BOUNDED_WAIT(".acquire.cluster", "setp.gt.u32 p, n, 64;\n\t@p nanosleep.u32 40;\n\t");
+    else if (CLUSTER) SLAI_BOUNDED_WAIT(".acquire.cluster", "");
+    else if (SLEEP) SLAI_BOUNDED_WAIT("", "setp.gt.u32 p, n, 64;\n\t@p nanosleep.u32 40;\n\t");
+    else SLAI_BOUNDED_WAIT("", "");
+#undef SLAI_BOUNDED_WAIT
+    return limit != 0;
+}
+#endif
+
 int slai_set_error(slai_ctx* ctx, int code, const char* fmt, ...);
 int slai_check_wait_flag(slai_ctx* ctx);  // ops.cu: SLAI_ERR_TIMEOUT if a bounded device-side wait ran out (stream must be idle)
 

@@ -20,8 +20,9 @@
 // contiguous run of the block's (tile, matrix, step) units; the partial sums of run (tile-matrix j, warp w) go to slot j + w, which no other
 // run of the phase has (the runs are ordered, each next one is a tile or a warp further).
 //
-// Every wait is bounded: on expiry the error flag is raised, nothing more is requested, later waits give up at once, and a warp waits for its own
-// copies in flight before the block ends.
+// Every wait on memory is bounded (bounded_wait, grid_barrier; the hardware's barrier of a cluster has no limit to give, and every block arrives on it as often
+// as the others): the error flag is raised and the step goes on.  A warp that has given up on its ring requests nothing more, and waits for its copies in
+// flight before the block ends.
 #pragma once
 #include "gemv_kernel.cuh"
 
@@ -223,7 +224,7 @@ struct PhaseInput {
     }
 };
 
-// The oldest stage's blocks are here.  A wait that runs out: nothing more is requested (Feed::run stays 0).
+// The oldest stage's blocks are here.  A wait that gives up: nothing more is requested (Feed::run stays 0).
 template <class F>
 __device__ __forceinline__ void feed_wait(Feed& R, const LayersParams& P) {
     uint32_t ok;
@@ -231,10 +232,7 @@ __device__ __forceinline__ void feed_wait(Feed& R, const LayersParams& P) {
                  : "=r"(ok)
                  : "r"(R.c_addr + Stage<F>::MBAR), "r"(R.c_phase)
                  : "memory");
-    if (!ok) {
-        ring_wait(R.c_addr + Stage<F>::MBAR, R.c_phase, R.limit, P.err_flag);
-        if (R.limit != P.wait_limit) R.run = 0;
-    }
+    if (!ok && !bounded_wait<false, false, 1>(R.c_addr + Stage<F>::MBAR, R.c_phase, R.limit, P.err_flag)) R.run = 0;
 }
 
 // ---- grid barrier ------------------------------------------------------------------------------------------------------------
@@ -731,12 +729,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
 #endif
         }
     }
-    if (R.limit != P.wait_limit) {  // a wait ran out: this warp's copies land before the block ends
+    if (R.limit == 0) {  // a wait gave up: this warp's copies land before the block ends
         const int nst = P.nstage;
-        unsigned int limit = P.wait_limit;
+        unsigned int limit = LAST_POLLS;
         for (int s = 0; s < nst; s++) {
             const int arms = ((int)R.issued - s + nst - 1) / nst;  // copies that went into stage s
-            if ((int)R.issued > s) ring_wait(R.base + s * Stage<F>::STRIDE + Stage<F>::MBAR, (uint32_t)(arms - 1) & 1u, limit, P.err_flag);
+            if ((int)R.issued > s) bounded_wait<false, false, 1>(R.base + s * Stage<F>::STRIDE + Stage<F>::MBAR, (uint32_t)(arms - 1) & 1u, limit, P.err_flag);
         }
     }
 }

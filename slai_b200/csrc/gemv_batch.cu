@@ -236,18 +236,7 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
     for (int unit = (int)blockIdx.x; unit < units; unit += stride, it++) {
         const int c = unit / P.ngroups, grp = unit - c * P.ngroups, slot = it & 1;
         const int nst = min(P.ch, P.nsteps - c * P.ch), tile = grp * BWARPS + warp;
-        {   // bounded wait for the unit's records; on expiry the error flag is raised and later waits give up at once
-            uint32_t ok = 0;
-            for (unsigned int i = 0; i < limit && !ok; i++)
-                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                             : "=r"(ok)
-                             : "r"(bar + 8 * slot), "r"((uint32_t)(it >> 1) & 1u)
-                             : "memory");
-            if (!ok) {
-                atomicExch(P.err_flag, 6u);
-                limit = 1;
-            }
-        }
+        bounded_wait<false, false, 6>(bar + 8 * slot, (uint32_t)(it >> 1) & 1u, limit, P.err_flag);  // the unit's records
         S.dig = sbase + ZERO_BYTES + slot * slot_bytes;
         // ---- this warp's tile: `nst` blocks against all vectors ----
         constexpr int NA = F::PAIRED ? NV / 2 : NV;
@@ -299,19 +288,9 @@ __global__ void __launch_bounds__(BTHREADS, 1) gemv_batch_kernel(const __grid_co
             }
         }
         __syncthreads();  // the unit's records have been read
-        if (tid == 0 && unit + 2 * stride < units) fetch_records(unit + 2 * stride, slot);
+        if (tid == 0 && limit && unit + 2 * stride < units) fetch_records(unit + 2 * stride, slot);  // (given up: what was requested has had its time to land)
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (limit != P.wait_limit && tid == 0) {  // a wait ran out: the records still on their way land before the block ends
-        for (int f = max(0, it - 1); f <= it; f++) {
-            uint32_t ok = 0;
-            for (unsigned int i = 0; i < P.wait_limit && !ok; i++)
-                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                             : "=r"(ok)
-                             : "r"(bar + 8 * ((f + 1) & 1)), "r"((uint32_t)((f - 1) >> 1) & 1u)
-                             : "memory");
-        }
-    }
 }
 
 // Sum of n values `stride` apart, in order; U loads in flight.

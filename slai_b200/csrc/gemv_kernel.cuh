@@ -606,7 +606,7 @@ struct Ring {
     uint32_t c_addr;          // stage consumed next
     uint32_t c_phase;
     uint32_t lane0;           // 1 in the lane that requests the copies
-    unsigned int limit;       // polls a wait may take; 1 after a wait has expired (later waits give up at once)
+    unsigned int limit;       // polls a wait may take before the error flag is raised; 0 once one has given up (bounded_wait)
     unsigned int* err_flag;
     // producer
     Cursor pc;
@@ -616,25 +616,6 @@ struct Ring {
 
 // Shared-memory layout: [staged vector: dig_region bytes = zero page, digit planes, digit sums][red RED_FLOATS f32][stat 64 f32][ring]
 __device__ __forceinline__ uint32_t smem_fixed_bytes(int dig_region) { return (uint32_t)dig_region + RED_FLOATS * 4 + 64 * 4; }
-
-// Bounded wait for the phase `parity` of the barrier at `a`.  On expiry the error flag is raised and `limit` drops to
-// one poll, so that the kernel still ends quickly.
-__device__ __forceinline__ void ring_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n"
-        "W:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra D;\n\tadd.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %3;\n\t@p bra W;\n\t"
-        "mov.u32 %0, 0;\n\tbra E;\n"
-        "D:\n\tmov.u32 %0, 1;\n"
-        "E:\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity), "r"(limit)
-        : "memory");
-    if (!ok) {
-        atomicExch(err_flag, 1u);
-        limit = 1;
-    }
-}
 
 template <class F>
 __device__ __forceinline__ void prod_run(Ring& R, const GemvParams& P, const Split& sp) {
@@ -782,7 +763,8 @@ __device__ __forceinline__ void gemv_body(const GemvParams& P, Ring& R, const Sp
             int step = c.step;
 #pragma unroll 1
             for (int i = run; i > 0; i--, step++) {
-                ring_wait(R.c_addr + RingGeom<F>::MBAR, R.c_phase, R.limit, R.err_flag);
+                // (given up: nothing more is requested, and what had been has had its time to land)
+                if (!bounded_wait<false, false, 1>(R.c_addr + RingGeom<F>::MBAR, R.c_phase, R.limit, R.err_flag)) R.p_run = 0;
                 if constexpr (STEPS) {
                     float a = 0.f, b = 0.f;
                     F::compute(R.c_addr, step, L, S, a, b);

@@ -29,7 +29,7 @@
 // executed, where cuBLAS keeps 1375); with few tokens the chain of a stage through operand writer, product and commit (some 620 cycles for products of
 // 200), and 8 us of start and end a launch.  us per product of the 7B shape, weights' operands in shared memory and whole tiles / now: 511 tokens q/k/v 89.5 / 82, gate
 // and up 145 / 135, down 77 / 72; 37 tokens gate and up 57 / 34.
-// Every wait is bounded (mbar_wait): `wait_limit` polls, after which the error flag is raised, then LAST_POLLS more, because what it waits for is this CTA's
+// Every wait is bounded (bounded_wait): `wait_limit` polls, after which the error flag is raised, then LAST_POLLS more, because what it waits for is this CTA's
 // (pair's) own work and copies, which have to land before the CTA ends.  Only a thread whose last polls ran out too goes on without: it arrives on nothing and
 // requests nothing from then on, so that no barrier completes a phase it has not reached.  Whoever requested copies or products waits for
 // the last of them at its end.
@@ -90,25 +90,9 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
-// Bounded wait in two parts, see the top: `limit` polls, then (the error flag raised) LAST_POLLS, which `limit` is from then on; 0 once those have run out: that
-// wait and all later ones of the thread return false.  CLUSTER: on a barrier that the other CTA of a pair arrives on too.
-// (PTX, for its size: the waits are in loops whose time is a chain of waits, and unrolled; two loops in a wait cost 1 us a launch at 16 tokens.)
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, unsigned int& limit, unsigned int* err_flag) {
-#define PG_WAIT(SEM)                                                                                                                     \
-    asm volatile(                                                                                                                         \
-        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\tmov.u32 n, 0;\n"                                                                           \
-        "W:\n\tmbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t@p bra D;\n\tsetp.gt.u32 p, n, 64;\n\t"                     \
-        "@p nanosleep.u32 40;\n\tadd.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %0;\n\t@p bra W;\n\t"                                              \
-        "setp.eq.u32 p, %0, 0;\n\t@p bra D;\n\tst.volatile.global.u32 [%3], 5;\n\tsetp.eq.u32 p, %0, %4;\n\tselp.u32 %0, 0, %4, p;\n\t"  \
-        "mov.u32 n, 0;\n\tbra W;\nD:\n\t}"                                                                                               \
-        : "+r"(limit)                                                                                                                     \
-        : "r"(a), "r"(parity), "l"(err_flag), "n"(LAST_POLLS)                                                                             \
-        : "memory")
-    if (CLUSTER) PG_WAIT(".acquire.cluster");
-    else PG_WAIT("");
-#undef PG_WAIT
-    return limit != 0;
+    return bounded_wait<CLUSTER, true, 5>(a, parity, limit, err_flag);
 }
 __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {  // the same shared-memory address in another CTA of the cluster
     uint32_t r;
