@@ -242,6 +242,7 @@ __device__ __forceinline__ void feed_wait(Feed& R, const LayersParams& P) {
 struct GridBar {
     unsigned int target, limit;
 };
+constexpr unsigned int BARRIER_POLLS = 1u << 14;  // fewest polls (some 10 ms): the wait is for the other blocks' phase, not for a copy (position 3900, 7B shape: more than 64)
 __device__ __forceinline__ void grid_barrier(const LayersParams& P, GridBar& B) {
     if (P.cluster) {  // the grid is one cluster: the hardware's barrier, 0.25 us
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_
     // The rows of x this thread updates, the same ones in both phases that do (PH_O, PH_FF2): kept here.
     const int x_row = ((int)blockIdx.x * P.ph[PH_O].base + min((int)blockIdx.x, P.ph[PH_O].rem)) * 16 + tid;
     float x_own = tid < (P.ph[PH_O].base + ((int)blockIdx.x < P.ph[PH_O].rem ? 1 : 0)) * 16 && x_row < P.ph[PH_O].rows ? __ldcg(P.x + x_row) : 0.f;
-    GridBar B{0u, P.wait_limit};
+    GridBar B{0u, max(P.wait_limit, BARRIER_POLLS)};
     auto barrier = [&] { grid_barrier(P, B); };
 
 #pragma unroll 1

@@ -96,3 +96,18 @@ def test_two_contexts_decode_at_the_same_time():
     for be, m in models:
         m.close()
         be.close()
+
+
+def test_short_wait_limit_at_a_long_context():
+    """A block's wait for the others takes as long as their phase: the attention over 3900 positions outlasts 64 polls, and is nobody's failure."""
+    be = Backend(0)
+    cfg = Llama2Config(dim=4096, hidden_dim=4096, n_layers=1, n_q_heads=32, n_kv_heads=32, vocab_size=500, seq_len=4096, kv_dtype=F16)
+    m = synthetic_llama_device(be, cfg, synth.FMT_Q4_K, synth.FMT_Q4_K, seed=1, std=0.02)
+    want = m.forward_logits(3900, 5)[0].copy()
+    be.set_wait_limit(16)
+    m2 = synthetic_llama_device(be, cfg, synth.FMT_Q4_K, synth.FMT_Q4_K, seed=1, std=0.02)
+    for _ in range(5):
+        assert np.array_equal(m2.forward_logits(3900, 5)[0], want)
+    m.close()
+    m2.close()
+    be.close()
