@@ -133,7 +133,7 @@ size_t gemv_dig_region(int fmt, int K) {
     const int Kp = (K + 255) & ~255;
     const int sv_gran = (fmt == SLAI_FMT_Q4_K || fmt == SLAI_FMT_Q5_K) ? 32 : fmt == SLAI_FMT_Q6_K ? 16 : 0;
     const size_t sv_bytes = sv_gran ? (size_t)(Kp / sv_gran) * 16 : 0;
-    return ((size_t)gemvfmt::ZERO_BYTES + ((size_t)4 * (Kp + 32) + sv_bytes) + (size_t)Kp / 256 * 4 + 127) & ~(size_t)127;  // (and a scale per 256 elements)
+    return ((size_t)gemvfmt::ZERO_BYTES + ((size_t)4 * (Kp + 32) + sv_bytes) + 127) & ~(size_t)127;
 }
 
 // Validate a launch description and turn it into kernel parameters.  `dig_region` = 0: size it for this K.
@@ -227,10 +227,10 @@ int gemv_fill_params(slai_ctx* ctx, const GemvLaunch& L, size_t dig_region, int 
     if (dig_region == 0) dig_region = need;
     SLAI_REQUIRE(ctx, dig_region >= need, SLAI_ERR_INVALID_ARG, "gemv: staging region too small");
     P.dig_region = (int)dig_region;
-    const size_t fixed = dig_region + (size_t)RED_FLOATS * 4 + 64 * 4 + 128;
+    const size_t fixed = dig_region + (size_t)RED_FLOATS * 4 + STAT_FLOATS * 4 + 128;
     const size_t per_stage = (size_t)WARPS * P.stage_stride;
     if (nstage <= 0) {
-        SLAI_REQUIRE(ctx, fixed + 2 * per_stage <= SMEM_LIMIT, SLAI_ERR_SHAPE, "gemv: K=%d does not fit in shared memory", K);
+        SLAI_REQUIRE(ctx, fixed + 2 * per_stage <= SMEM_LIMIT && (K + 255) / 256 <= MAX_STEPS, SLAI_ERR_SHAPE, "gemv: K=%d does not fit in shared memory", K);
         const int fit = (int)((SMEM_LIMIT - fixed) / per_stage);
         // Two stages in flight per warp for the K-quants (three otherwise) measured fastest: a deeper first fill asks for
         // most of the matrix at once and delays the activation loads of the staging pass behind it.

@@ -43,6 +43,8 @@ constexpr int THREADS = 32 * WARPS;
 constexpr int MAX_STAGES = 8;  // ring depth limit (host side)
 constexpr int WAVE = 8;  // tiles whose partial sums are held in shared memory at a time
 constexpr int SMEM_LIMIT = 227 * 1024;
+constexpr int STAT_FLOATS = 64;  // statistics of the staged vector: sums of the warps, then (vectors staged by steps) the exponents of its scales
+constexpr int MAX_STEPS = 4 * (STAT_FLOATS - WARPS);  // 256-element steps these have room for; shared memory ends at 138 (Q8_0, K = 35328)
 constexpr int STAGE_REGS = 6;  // float4 per thread kept in registers between the staging passes (K <= 12288)
 constexpr int RED_FLOATS = WAVE * WARPS * 2 * 16;  // partial sums (sized for the two-matrix gate/up phase)
 
@@ -398,11 +400,15 @@ __device__ __forceinline__ float stage_vector(const int PRO_ARG, const GemvParam
 // element; the product's sums of a step are multiplied by 1 / scale.  An RmsNorm needs no pass either: the digits are those of x * w, and
 // 1 / rms is a factor of the results (`sq`: this warp's sum of squares).  A LayerNorm does (its mean is subtracted first), for K <= 4096,
 // where every warp has 256 elements at most.
-// One code for all inputs (`In`: how elements are loaded), in a loop: it is run once per product, so what it spends is instruction fetches (as stage_vector,
+// `inv`: where the 1 / scale of the steps go.  One code for all inputs (`In`: how elements are loaded), in a loop: it is run once per product, so what it spends is instruction fetches (as stage_vector,
 // unrolled six times and with a copy per kind of input, it made decode_layers.cuh's kernel 137 KB, where staging 288 elements took 2.3 us).
-template <class F, bool LN, class In>
+__device__ __forceinline__ void put_inverse(float* p, float x) { *p = x; }
+// ... as the exponent alone, where shared memory is what limits K: x is a power of two.
+__device__ __forceinline__ void put_inverse(unsigned char* p, float x) { *p = (unsigned char)(__float_as_uint(x) >> 23); }
+__device__ __forceinline__ float inverse_at(const unsigned char* p) { return __uint_as_float((uint32_t)*p << 23); }
+template <class F, bool LN, class In, class Inv>
 __device__ __forceinline__ float stage_steps(const In& in, const float* norm_w, const float* norm_b, int K, float eps, const Smem& S,
-                                             float* inv, float* stat) {
+                                             Inv* inv, float* stat) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     unsigned char* dig = reinterpret_cast<unsigned char*>(__cvta_shared_to_generic(S.dig));
@@ -471,7 +477,7 @@ __device__ __forceinline__ float stage_steps(const In& in, const float* norm_w, 
         if (256 * step < K) {  // (a warp without elements took part in the LayerNorm's sums)
 #pragma unroll
             for (int p = 0; p < 4; p++) *reinterpret_cast<uint2*>(dig + (size_t)p * S.plane + 256 * step + 8 * lane) = make_uint2(pw[0][p], pw[1][p]);
-            if (lane == 0) inv[step] = back;
+            if (lane == 0) put_inverse(inv + step, back);
             if (F::SV_GRAN > 0) {
                 // digit sums of the sub-blocks, layouts of gemv_formats.cuh; two biased sums to a word, so that a shuffle serves two planes
                 constexpr int LANES = F::SV_GRAN > 0 ? F::SV_GRAN / 8 : 1, BIAS = 1024;  // (eight digits' sum lies in [-1024, 1016])
@@ -615,7 +621,7 @@ struct Ring {
 };
 
 // Shared-memory layout: [staged vector: dig_region bytes = zero page, digit planes, digit sums][red RED_FLOATS f32][stat 64 f32][ring]
-__device__ __forceinline__ uint32_t smem_fixed_bytes(int dig_region) { return (uint32_t)dig_region + RED_FLOATS * 4 + 64 * 4; }
+__device__ __forceinline__ uint32_t smem_fixed_bytes(int dig_region) { return (uint32_t)dig_region + RED_FLOATS * 4 + STAT_FLOATS * 4; }
 
 template <class F>
 __device__ __forceinline__ void prod_run(Ring& R, const GemvParams& P, const Split& sp) {
@@ -714,7 +720,7 @@ __device__ __forceinline__ void gemv_body(const GemvParams& P, Ring& R, const Sp
     SLAI_TRACE_POINT(5)
     // A LayerNorm, and a vector that arrives from peers, are staged with one scale; everything else with a scale per 256 elements.
     constexpr bool STEPS = PRO != PRO_LN && !XIN;
-    float* inv = reinterpret_cast<float*>(smem_raw + P.dig_region) - ((K + 255) >> 8);  // [K / 256] at the end of the region
+    unsigned char* inv = reinterpret_cast<unsigned char*>(stat + WARPS);  // [K / 256], behind the warps' sums of squares (MAX_STEPS)
     float inv_scale = 1.f;
     if constexpr (STEPS) {
         struct Plain {
@@ -768,7 +774,7 @@ __device__ __forceinline__ void gemv_body(const GemvParams& P, Ring& R, const Sp
                 if constexpr (STEPS) {
                     float a = 0.f, b = 0.f;
                     F::compute(R.c_addr, step, L, S, a, b);
-                    const float sc = inv[F::STEP == 256 ? step : step >> 1];
+                    const float sc = inverse_at(inv + (F::STEP == 256 ? step : step >> 1));
                     accA = fmaf(sc, a, accA);
                     accB = fmaf(sc, b, accB);
                 } else {

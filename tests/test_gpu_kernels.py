@@ -365,3 +365,22 @@ def test_kv_append(backend, ctx):
         a, b = kc.to_numpy().reshape(seq, kvd), vc.to_numpy().reshape(seq, kvd)
         assert np.array_equal(a[3], k.astype(npdt)) and np.array_equal(b[3], v.astype(npdt))
         assert not a[[0, 1, 2, 4, 5, 6, 7]].any()
+
+
+@pytest.mark.parametrize("fmt,K", [(synth.FMT_Q4_K, 30464), (synth.FMT_Q5_K, 26880), (synth.FMT_Q6_K, 20736), (synth.FMT_Q8_0, 35328), (synth.FMT_Q8_0, 35104)])
+def test_gemv_widest_vectors(backend, ctx, fmt, K):
+    """The largest K whose digits and two ring stages fit in shared memory; the next one is refused.  Elements of very different size from step to step."""
+    M = 40
+    rng = np.random.default_rng(K)
+    blocks = synth.quantize(fmt, synth.normal_matrix(K, M, K))
+    v = (rng.standard_normal(K) * 10.0 ** rng.integers(-6, 7, size=(K + 255) // 256).repeat(256)[:K]).astype(np.float32)
+    m, out = GpuQuantMatrix(backend, fmt, M, K, blocks), backend.zeros(M)
+    ctx.matmul_quant_assign(out, m, backend.vector(v))
+    want = O.dequantize(fmt, blocks).reshape(M, K).astype(np.float64) @ v.astype(np.float64)
+    assert rel_l2(out.to_numpy(), want) < 1e-6  # digits of 26 bits, f32 sums of 138 steps at most
+    more = K + (32 if fmt == synth.FMT_Q8_0 else 256)
+    if K == 35104:
+        return
+    wide = GpuQuantMatrix(backend, fmt, M, more, synth.quantize(fmt, synth.normal_matrix(K, M, more)))
+    with pytest.raises(SlaiError):
+        ctx.matmul_quant_assign(out, wide, backend.zeros(more))
