@@ -462,3 +462,4 @@ int prefill_rope_kv_launch(slai_ctx* ctx, const float* qkv, int ld, int q_dim, i
                            const float* theta, int neox, float* q_out, void* kcache, void* vcache, int kv_f16, long long kv_head_stride);
 
 size_t gemv_dig_region(int fmt, int K);
+bool gemv_width_fits(int fmt, int K);  // ... and two stages of every warp's ring beside it

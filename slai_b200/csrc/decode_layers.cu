@@ -55,7 +55,10 @@ bool plan(slai_ctx* ctx, const DecodeLayers& D, bool cluster, LayersParams& P, P
     P.kvq = D.kv_mul / share;
     P.n_heads = D.n_heads;
     P.n_items = D.n_heads / P.kvq;
-    if (P.kvq > 2) return false;
+    // What the kernels one by one refuse (attention.cu, gemv.cu) is theirs to refuse: they are what the statistics run too.
+    if (D.kv_mul > 8 || P.kvq > 2 || D.n_heads / D.kv_mul * share > 1024) return false;
+    for (int k : K)
+        if (!gemv_width_fits(D.fmt, k)) return false;
     // No more blocks than some phase has tiles: a barrier of fewer blocks is quicker.
     pl.grid = std::min(ctx->sm_count, *std::max_element(items, items + PH_COUNT));
     P.cluster = cluster && one_cluster(D) ? 1 : 0;

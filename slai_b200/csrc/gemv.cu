@@ -136,6 +136,12 @@ size_t gemv_dig_region(int fmt, int K) {
     return ((size_t)gemvfmt::ZERO_BYTES + ((size_t)4 * (Kp + 32) + sv_bytes) + 127) & ~(size_t)127;
 }
 
+static size_t smem_fixed(size_t dig_region) { return dig_region + (size_t)RED_FLOATS * 4 + STAT_FLOATS * 4 + 128; }
+bool gemv_width_fits(int fmt, int K) {
+    const size_t stage = (layout::step_bytes(fmt) + 8 + 127) & ~127;  // block + its mbarrier (RingGeom)
+    return smem_fixed(gemv_dig_region(fmt, K)) + 2 * WARPS * stage <= SMEM_LIMIT && (K + 255) / 256 <= MAX_STEPS;
+}
+
 // Validate a launch description and turn it into kernel parameters.  `dig_region` = 0: size it for this K.
 int gemv_fill_params(slai_ctx* ctx, const GemvLaunch& L, size_t dig_region, int nstage, GemvParams& P, size_t* smem_out,
                      int* grid_out) {
@@ -227,7 +233,7 @@ int gemv_fill_params(slai_ctx* ctx, const GemvLaunch& L, size_t dig_region, int 
     if (dig_region == 0) dig_region = need;
     SLAI_REQUIRE(ctx, dig_region >= need, SLAI_ERR_INVALID_ARG, "gemv: staging region too small");
     P.dig_region = (int)dig_region;
-    const size_t fixed = dig_region + (size_t)RED_FLOATS * 4 + STAT_FLOATS * 4 + 128;
+    const size_t fixed = smem_fixed(dig_region);
     const size_t per_stage = (size_t)WARPS * P.stage_stride;
     if (nstage <= 0) {
         SLAI_REQUIRE(ctx, fixed + 2 * per_stage <= SMEM_LIMIT && (K + 255) / 256 <= MAX_STEPS, SLAI_ERR_SHAPE, "gemv: K=%d does not fit in shared memory", K);

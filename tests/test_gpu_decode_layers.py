@@ -8,6 +8,7 @@ import pytest
 
 from oracle import oracle as O
 from slai_b200 import _lib, synth
+from slai_b200._lib import SlaiError
 from slai_b200.models import Gpt2Params, Llama2Config, gpt2_from_host, llama_from_host, synthetic_gpt2_host, synthetic_llama_device, synthetic_llama_host
 from slai_b200.ops import Backend
 from helpers import oracle_gpt2, oracle_llama, rel_l2
@@ -111,3 +112,15 @@ def test_short_wait_limit_at_a_long_context():
     m.close()
     m2.close()
     be.close()
+
+
+def test_what_the_separate_kernels_refuse_is_refused(backend):
+    """More than eight query heads to a key head, and a feed-forward part wider than a product takes (28672 fits, its down product's 30720 does not)."""
+    for sh in (dict(dim=512, hidden_dim=1024, n_q_heads=16, n_kv_heads=1), dict(dim=256, hidden_dim=30720, n_q_heads=4, n_kv_heads=4)):
+        cfg = Llama2Config(n_layers=1, vocab_size=100, seq_len=32, kv_dtype=F16, **sh)
+        m = synthetic_llama_device(backend, cfg, synth.FMT_Q4_K, synth.FMT_Q4_K, seed=1, std=0.05)
+        for call in (lambda: m.forward_logits(0, 3), lambda: m.generate(3, 0, 4), lambda: m.stats(3, 0)):
+            with pytest.raises(SlaiError) as e:
+                call()
+            assert e.value.code == _lib.ERR_SHAPE
+        m.close()
