@@ -1,4 +1,5 @@
 // Host side of the layers of a decode step in one launch (decode_layers.cuh): which models take it, and its parameters.
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -17,14 +18,17 @@ constexpr int MAX_PART = 32768;
 // Layers of few bytes go to one cluster of 16 blocks instead of the whole chip: the cluster's hardware barrier takes 0.25 us, the grid's 1.0 to 1.2, five times a
 // layer, which is more than 16 SMs lose on few bytes.  us a token, whole chip / one cluster: tiny story model (1.1 MB a layer, Q8_0) 125.7 / 111.1,
 // 256 wide Q4_K (0.5 MB) 171 / 149, 512 wide Q4_K (1.8 MB) 171 / 161, 512 wide Q6_K (2.2 MB) 202 / 195; but 768 wide Q5_K (5.1 MB) 182 / 200 and
-// 1024 wide Q6_K (9.4 MB) 226 / 277.
+// 1024 wide Q6_K (9.4 MB) 226 / 277.  Keys and values count half, since their loads are ahead of the barrier: 16 SMs read them in all (at most 16 / items splits).
+// us a token at positions 500, 2000, 8000 of 8 layers 512 wide, f32 cache, whole chip 176, 198, 264, one cluster 174, 241, 558 (kernel by kernel 221, 246, 317);
+// f16 173, 182, 228 and 171, 200, 390; 256 wide, f16 170, 178, 202 and 147, 161, 237.
 constexpr int CLUSTER = 16;
 constexpr long long CLUSTER_BYTES = 3000000;
-bool one_cluster(const DecodeLayers& D) {
+long long weight_bytes(const DecodeLayers& D) {  // of a layer
     const long long rows_dim = (long long)D.q_dim + 2 * D.kv_dim + (D.arch == ARCH_LLAMA ? 2 : 1) * (long long)D.hidden;  // matrices of width `dim`
     auto bytes = [&](long long rows, int K) { return rows * layout::num_steps(D.fmt, K) * layout::step_bytes(D.fmt) / 16; };
-    return bytes(rows_dim, D.dim) + bytes(D.dim, D.q_dim) + bytes(D.dim, D.hidden) < CLUSTER_BYTES;
+    return bytes(rows_dim, D.dim) + bytes(D.dim, D.q_dim) + bytes(D.dim, D.hidden);
 }
+bool one_cluster(const DecodeLayers& D) { return !D.whole_chip && weight_bytes(D) < CLUSTER_BYTES; }
 
 struct Plan {
     int grid = 0;
@@ -106,6 +110,11 @@ bool decode_layers_supported(slai_ctx* ctx, const DecodeLayers& D) {
     static thread_local LayersParams P;  // (some 20 KB: not on the caller's stack)
     Plan pl;
     return plan(ctx, D, false, P, pl);  // (one cluster is only ever taken instead)
+}
+
+int decode_layers_cluster_positions(const DecodeLayers& D) {
+    const long long left = CLUSTER_BYTES - weight_bytes(D), row = 2ll * D.kv_dim * (D.kv_f16 ? 2 : 4);  // keys and values of a position
+    return left <= 0 || 2 * left / row >= D.seq_len ? INT_MAX : (int)(2 * left / row);
 }
 
 size_t decode_layers_scratch_bytes(const DecodeLayers& D) {

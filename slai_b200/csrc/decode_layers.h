@@ -19,8 +19,10 @@ struct DecodeLayers {
     const int* d_pos = nullptr;
     void *kcache = nullptr, *vcache = nullptr;  // [layer][head][position][head size]
     size_t layer_bytes = 0;
+    bool whole_chip = false;      // not one cluster, see decode_layers_cluster_positions
 };
 bool decode_layers_supported(slai_ctx* ctx, const DecodeLayers& D);
+int decode_layers_cluster_positions(const DecodeLayers& D);  // first position from which the whole chip is the quicker choice (INT_MAX: no choice)
 size_t decode_layers_scratch_bytes(const DecodeLayers& D);
 unsigned int* decode_layers_counter(void* scratch);  // the kernel's barrier counter: zero before every launch
 int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch);

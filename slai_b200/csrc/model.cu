@@ -7,6 +7,8 @@
 // down+residual), chained with programmatic dependent launch and captured once into a CUDA graph that is
 // replayed per token; token id and position live in device scalars, and greedy decoding / prompt
 // processing advance them on the device so the host only launches graphs.
+#include <limits.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -21,9 +23,11 @@ struct Scalars {  // device ints: [0] token, [1] pos, [2] step, [3] next
 enum GraphKind { G_DECODE = 0, G_GENERATE = 1, G_FORCED = 2, G_SAMPLED = 3, G_COUNT = 4 };
 
 struct GraphSet {
-    cudaGraphExec_t exec[G_COUNT] = {};
-    bool warmed[G_COUNT] = {};  // first token of a kind runs eagerly (sets kernel attributes)
+    cudaGraphExec_t exec[2][G_COUNT] = {};  // [`wide`]
+    bool warmed[2][G_COUNT] = {};           // first token of a kind runs eagerly (sets kernel attributes)
     bool use_graph = true;
+    int wide = 0;                 // this step's layers on the whole chip rather than on one cluster of blocks
+    int wide_from = INT_MAX;      // ... from this position on (decode_layers_cluster_positions)
 };
 
 int copy_f32(slai_ctx* ctx, float** dst, const float* src, int64_t n, bool from_device) {
@@ -40,12 +44,15 @@ int copy_f32(slai_ctx* ctx, float** dst, const float* src, int64_t n, bool from_
 }
 
 void destroy_graphs(GraphSet& g) {
-    for (int i = 0; i < G_COUNT; i++)
-        if (g.exec[i]) {
-            cudaGraphExecDestroy(g.exec[i]);
-            g.exec[i] = nullptr;
-        }
-    for (int i = 0; i < G_COUNT; i++) g.warmed[i] = false;
+    for (auto& set : g.exec)
+        for (auto& e : set)
+            if (e) {
+                cudaGraphExecDestroy(e);
+                e = nullptr;
+            }
+    for (auto& set : g.warmed)
+        for (bool& w : set) w = false;
+    g.wide_from = INT_MAX;
 }
 
 // Bytes of later weights one kernel asks for ahead of time (PrefetchPlan).  Off unless SLAI_AHEAD_MB is set: the main
@@ -216,6 +223,8 @@ static bool llama_one_launch(slai_llama* m, bool table, DecodeLayers& D, std::ve
     D.head_size = m->head_size; D.n_heads = m->n_q_local; D.kv_mul = m->kv_mul; D.seq_len = c.seq_len; D.eps = c.rms_norm_eps;
     D.x = m->x; D.q = m->q; D.xb = m->xb; D.hb = m->hb; D.rope_cs = m->rope_cs; D.d_pos = m->sc.d + 1;
     D.kcache = m->kcache; D.vcache = m->vcache; D.layer_bytes = m->kv_layer_elems * (D.kv_f16 ? 2 : 4);
+    D.whole_chip = m->graphs.wide;
+    m->graphs.wide_from = decode_layers_cluster_positions(D);
     return decode_layers_supported(m->ctx, D);
 }
 
@@ -505,21 +514,23 @@ static int llama_record(slai_llama* m, int kind) {
 
 
 template <class M, class RecordFn>
-static int run_graph(M* m, int kind, RecordFn record) {
+static int run_graph(M* m, int kind, int pos, RecordFn record) {
     slai_ctx* ctx = m->ctx;
+    const int wide = m->graphs.wide = pos >= m->graphs.wide_from ? 1 : 0;
     if (!m->graphs.use_graph) return record(m, kind);
-    if (!m->graphs.warmed[kind]) {
-        m->graphs.warmed[kind] = true;
+    if (!m->graphs.warmed[wide][kind]) {
+        m->graphs.warmed[wide][kind] = true;
         return record(m, kind);
     }
-    if (!m->graphs.exec[kind]) {
+    cudaGraphExec_t& exec = m->graphs.exec[wide][kind];
+    if (!exec) {
         cudaGraph_t graph = nullptr;
         SLAI_CHECK_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = record(m, kind);
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
         if (rc == SLAI_OK && e == cudaSuccess) {
-            e = cudaGraphInstantiate(&m->graphs.exec[kind], graph, 0);
-            if (e != cudaSuccess) m->graphs.exec[kind] = nullptr;
+            e = cudaGraphInstantiate(&exec, graph, 0);
+            if (e != cudaSuccess) exec = nullptr;
         }
         if (graph) cudaGraphDestroy(graph);
         if (rc != SLAI_OK || e != cudaSuccess) {
@@ -531,7 +542,7 @@ static int run_graph(M* m, int kind, RecordFn record) {
             return record(m, kind);
         }
     }
-    SLAI_CHECK_CUDA(ctx, cudaGraphLaunch(m->graphs.exec[kind], ctx->stream));
+    SLAI_CHECK_CUDA(ctx, cudaGraphLaunch(exec, ctx->stream));
     return SLAI_OK;
 }
 
@@ -907,7 +918,7 @@ static int decode_impl(M* m, RecordFn record, int vocab, int seq_len, int32_t to
     SLAI_REQUIRE(ctx, pos >= 0 && pos < seq_len, SLAI_ERR_INVALID_ARG, "decode: pos %d out of range", pos);
     int rc = set_scalars(m, token, pos, 0);
     if (rc) return rc;
-    if ((rc = run_graph(m, G_DECODE, record))) return rc;
+    if ((rc = run_graph(m, G_DECODE, pos, record))) return rc;
     if (h_logits) SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(h_logits, m->logits, (size_t)vocab * 4, cudaMemcpyDeviceToHost, ctx->stream));
     if (next_token) SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(next_token, m->sc.d + 3, 4, cudaMemcpyDeviceToHost, ctx->stream));
     if (h_logits || next_token) {
@@ -927,7 +938,7 @@ static int generate_impl(M* m, RecordFn record, int vocab, int seq_len, int32_t 
     int rc = set_scalars(m, token, pos, 0);
     if (rc) return rc;
     for (int i = 0; i < n; i++)
-        if ((rc = run_graph(m, kind, record))) return rc;
+        if ((rc = run_graph(m, kind, pos + i, record))) return rc;
     if (h_tokens) SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(h_tokens, m->d_history, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return slai_check_wait_flag(ctx);
@@ -949,7 +960,7 @@ static int prefill_impl(M* m, RecordFn record, int vocab, int seq_len, const int
     if (rc) return rc;
     SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // `next` leaves scope
     for (int i = 0; i < n; i++)
-        if ((rc = run_graph(m, G_FORCED, record))) return rc;
+        if ((rc = run_graph(m, G_FORCED, pos0 + i, record))) return rc;
     if (h_last_logits) SLAI_CHECK_CUDA(ctx, cudaMemcpyAsync(h_last_logits, m->logits, (size_t)vocab * 4, cudaMemcpyDeviceToHost, ctx->stream));
     SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return slai_check_wait_flag(ctx);
@@ -1330,6 +1341,8 @@ static bool gpt2_one_launch(slai_gpt2* m, DecodeLayers& D, std::vector<DecodeLay
     D.head_size = m->head_size; D.n_heads = c.n_head; D.kv_mul = 1; D.seq_len = c.n_seq; D.eps = c.layernorm_eps;
     D.x = m->x; D.q = m->q; D.xb = m->xb; D.hb = m->ff; D.d_pos = m->sc.d + 1;
     D.kcache = m->kcache; D.vcache = m->vcache; D.layer_bytes = m->kv_layer_elems * (D.kv_f16 ? 2 : 4);
+    D.whole_chip = m->graphs.wide;
+    m->graphs.wide_from = decode_layers_cluster_positions(D);
     return decode_layers_supported(m->ctx, D);
 }
 

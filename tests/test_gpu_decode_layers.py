@@ -124,3 +124,31 @@ def test_what_the_separate_kernels_refuse_is_refused(backend):
                 call()
             assert e.value.code == _lib.ERR_SHAPE
         m.close()
+
+
+@pytest.mark.parametrize("arch", ["llama", "gpt2"])
+def test_small_layers_leave_the_cluster_at_a_long_context(backend, arch):
+    """256 wide: one cluster of blocks while the weights of a layer and half of its keys and values are below 3 MB, the whole chip behind that position (for
+    these f32 caches 2045 and 1187 positions), in the device loop as in single steps, and back again."""
+    n, first = (1300, 1150) if arch == "gpt2" else (2160, 2010)
+    if arch == "llama":
+        cfg = Llama2Config(dim=256, hidden_dim=768, n_layers=1, n_q_heads=4, n_kv_heads=4, vocab_size=300, seq_len=n, kv_dtype=F32)
+        w = synthetic_llama_host(cfg, synth.FMT_Q8_0, seed=21, std=0.05, embd_std=1.0)
+        m, ref = llama_from_host(backend, cfg, w, synth.FMT_Q8_0), oracle_llama(cfg, w, synth.FMT_Q8_0)
+    else:
+        p = Gpt2Params(n_vocab=300, n_seq=n, n_embd=320, n_head=5, n_layer=1, ff_len=1280, kv_dtype=F32)
+        w = synthetic_gpt2_host(p, synth.FMT_Q8_0, seed=22, std=0.05)
+        m, ref = gpt2_from_host(backend, p, w, synth.FMT_Q8_0), oracle_gpt2(p, w)
+    one = (lambda pos, t: m.forward_logits(pos, t)[0]) if arch == "llama" else (lambda pos, t: m.forward(t, pos)[0])
+    toks = np.random.default_rng(4).integers(0, 300, size=n)
+    m.prefill(toks[:first].astype(np.int32), 0)
+    early = one(3, int(toks[3])).copy()
+    for pos in range(n):
+        want = ref.forward(int(toks[pos]), pos)
+        if pos >= first:
+            got = one(pos, int(toks[pos]))
+            if pos % 8 == 0 or pos == n - 1:
+                assert rel_l2(got, want) < 2e-5, pos
+    assert np.array_equal(one(3, int(toks[3])), early)
+    assert np.array_equal(m.generate(int(toks[first]), first, 100), m.generate(int(toks[first]), first, 100))
+    m.close()
