@@ -55,6 +55,17 @@ def read_timeline(backend, cap=CAP):
     return buf[: SLOTS * n].reshape(n, SLOTS).astype(np.int64)
 
 
+def staged_stamps(t: np.ndarray) -> np.ndarray:
+    """The stamps (last axis) of a GEMV launch with points 6 and 7 (vector loaded, statistics known) at point 5 and point 8 (digits stored) at point 9 where the
+    kernel has no such points: a vector that is staged step by step is loaded, converted and stored in one pass, which then counts as `digits`.  The
+    places keep what an earlier launch left there, or zero."""
+    t = np.array(t, dtype=np.float64)
+    stale = ~((t[..., 5] <= t[..., 6]) & (t[..., 6] <= t[..., 7]) & (t[..., 7] <= t[..., 8]) & (t[..., 8] <= t[..., 9]))
+    for point, instead in ((6, 5), (7, 5), (8, 9)):
+        t[..., point] = np.where(stale, t[..., instead], t[..., point])
+    return t
+
+
 def summarise(rec: np.ndarray):
     """rec: one token's records [id, stamp 0..14] in execution order.  Per kernel (in order of first appearance): mean
     microseconds of every phase of block 0, the whole kernel, the period (start to the next kernel's start) and the
@@ -77,7 +88,8 @@ def summarise(rec: np.ndarray):
             parts[3], parts[7], parts[9], parts[10], parts[11] = t[2] - t[0], t[3] - t[2], t[4] - t[3], t[5] - t[4], t[6] - t[5]
             end = t[6]
         else:
-            parts = [t[b] - t[a] for _, a, b in COLS]
+            s = staged_stamps(t)
+            parts = [s[b] - s[a] for _, a, b in COLS]
         period = (rec[i + 1, 1] * 1e-3 - t[0]) if i + 1 < len(rec) else np.nan
         after = i + 1 < len(rec) and not 2000 <= int(rec[i + 1, 0]) < 2004
         rows[key].append(parts + [end - t[0], period, rec[i + 1, 5] * 1e-3 - end if after else np.nan])
@@ -105,7 +117,7 @@ def block_report(backend, nblocks):
             continue
         t = t[used]
         t0 = t[:, 0].min()
-        out.append((t0, slot, int(used.sum()), t - t0))
+        out.append((t0, slot, int(used.sum()), staged_stamps(t) - t0))
     out.sort()
     for t0, slot, nb, t in out[-6:]:
         print(f"slot {slot}: {nb} blocks; microseconds after the earliest block start: min / median / max over blocks")
