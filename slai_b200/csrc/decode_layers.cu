@@ -6,7 +6,6 @@
 
 #include "attention.cuh"
 #include "decode_layers.cuh"
-#include "decode_layers.h"
 
 using namespace declayers;
 
@@ -128,7 +127,7 @@ static int launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* l
     P = LayersParams{};
     Plan pl;
     if (!plan(ctx, D, cluster, P, pl)) {
-        if (cluster) return NO_CLUSTER;  // (a few tall matrices: more rows than 16 blocks' epilogues take)
+        if (cluster) return DECODE_LAYERS_NO_FIT;  // (a few tall matrices: more rows than 16 blocks' epilogues take)
         return slai_set_error(ctx, SLAI_ERR_SHAPE, "decode: these layers do not fit one launch");
     }
     P.n_layers = D.n_layers;
@@ -170,5 +169,5 @@ static int launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* l
 
 int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch) {
     const int rc = launch(ctx, D, layers, scratch, true);
-    return rc == NO_CLUSTER ? launch(ctx, D, layers, scratch, false) : rc;
+    return rc == DECODE_LAYERS_NO_FIT ? launch(ctx, D, layers, scratch, false) : rc;
 }

@@ -24,6 +24,7 @@
 // as the others): the error flag is raised and the step goes on.  A warp that has given up on its ring requests nothing more, and waits for its copies in
 // flight before the block ends.
 #pragma once
+#include "decode_layers.h"
 #include "gemv_kernel.cuh"
 
 namespace declayers {
@@ -34,7 +35,6 @@ enum Phase { PH_QKV = 0, PH_O = 1, PH_FF1 = 2, PH_FF2 = 3, PH_COUNT = 4 };
 enum Arch { ARCH_LLAMA = 0, ARCH_GPT2 = 1 };
 constexpr int MAX_LAYERS = 128;
 constexpr int MAX_SPLITS = 16;
-constexpr int NO_CLUSTER = -1000;  // launch_inst: the cluster does not fit, nothing was launched
 constexpr int MAX_TILES = THREADS / 16;  // row tiles of a block in a phase: its rows are the epilogue's threads
 
 struct LayerPtrs {
@@ -765,13 +765,18 @@ int launch_inst(slai_ctx* ctx, const LayersParams& P, int grid, size_t smem) {
         int clusters = 0;  // (none on a part of a chip without that many neighbouring SMs)
         if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
             cudaGetLastError();
-            return NO_CLUSTER;
+            return DECODE_LAYERS_NO_FIT;
         }
     } else {
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
     }
-    SLAI_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, P));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // the process has a part of the chip that its properties do not tell of
+        cudaGetLastError();
+        return DECODE_LAYERS_NO_FIT;
+    }
+    SLAI_CHECK_CUDA(ctx, e);
     return SLAI_OK;
 }
 template <class F, typename T>

@@ -25,4 +25,5 @@ bool decode_layers_supported(slai_ctx* ctx, const DecodeLayers& D);
 int decode_layers_cluster_positions(const DecodeLayers& D);  // first position from which the whole chip is the quicker choice (INT_MAX: no choice)
 size_t decode_layers_scratch_bytes(const DecodeLayers& D);
 unsigned int* decode_layers_counter(void* scratch);  // the kernel's barrier counter: zero before every launch
+constexpr int DECODE_LAYERS_NO_FIT = -1000;  // decode_layers_launch: the blocks cannot all run at once here; nothing was launched
 int decode_layers_launch(slai_ctx* ctx, const DecodeLayers& D, const DecodeLayerPtrs* layers, void* scratch);

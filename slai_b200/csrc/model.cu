@@ -28,6 +28,7 @@ struct GraphSet {
     bool use_graph = true;
     int wide = 0;                 // this step's layers on the whole chip rather than on one cluster of blocks
     int wide_from = INT_MAX;      // ... from this position on (decode_layers_cluster_positions)
+    bool separate = false;        // the layers' launch does not fit the SMs this process has: kernel by kernel
 };
 
 int copy_f32(slai_ctx* ctx, float** dst, const float* src, int64_t n, bool from_device) {
@@ -198,11 +199,17 @@ static void llama_drop_prefill(slai_llama* m) {
     m->pf_cap = 0;
 }
 
+// SLAI_SEPARATE_LAYERS=1: a step's layers kernel by kernel (a launch that takes all SMs at once waits for other streams' kernels to leave them).
+static bool separate_layers(const GraphSet& g) {
+    const char* e = getenv("SLAI_SEPARATE_LAYERS");
+    return g.separate || (e && e[0] == '1');
+}
+
 // The step's layers as one launch (decode_layers.cuh), if these are layers it takes: one format for all their matrices, adjacent-pair
 // RoPE from the table, not sharded, not being timed kernel by kernel.
 static bool llama_one_launch(slai_llama* m, bool table, DecodeLayers& D, std::vector<DecodeLayerPtrs>& layers) {
     const slai_llama_config& c = m->cfg;
-    if (m->tp != 1 || m->ctx->stats_on || !table) return false;
+    if (m->tp != 1 || m->ctx->stats_on || !table || separate_layers(m->graphs)) return false;
     layers.resize(c.n_layers);
     const int fmt = m->layers[0].wq ? m->layers[0].wq->fmt : -1;
     for (int l = 0; l < c.n_layers; l++) {
@@ -246,7 +253,7 @@ static int llama_record(slai_llama* m, int kind) {
     const bool table = c.rope_variant == 0 && m->head_size / 2 <= 256;
     DecodeLayers D;
     std::vector<DecodeLayerPtrs> dl;
-    const bool one_launch = llama_one_launch(m, table, D, dl);
+    bool one_launch = llama_one_launch(m, table, D, dl);
     if (one_launch && (rc = layers_scratch_reserve(ctx, D, &m->layers_scratch))) return rc;
     unsigned int* zero = one_launch ? decode_layers_counter(m->layers_scratch) : nullptr;
     if (m->embd_q) rc = launch_embed_q8(ctx, m->x, m->embd_q, d_token, nullptr, d_pos, false, m->rope_theta, table ? m->rope_cs : nullptr, m->head_size / 2, zero);
@@ -254,8 +261,15 @@ static int llama_record(slai_llama* m, int kind) {
     if (rc) return rc;
     n++;
     if (one_launch) {
-        if ((rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch))) return rc;
-        n++;
+        rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch);
+        if (rc == DECODE_LAYERS_NO_FIT) {
+            one_launch = false;
+            m->graphs.separate = true;
+        } else if (rc) {
+            return rc;
+        } else {
+            n++;
+        }
     }
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     // A row-parallel GEMV (each rank holds a K range of every row): x += W v.  Sharded: the partial goes to xpart
@@ -1315,7 +1329,7 @@ static void gpt2_drop_prefill(slai_gpt2* m) {
 
 static bool gpt2_one_launch(slai_gpt2* m, DecodeLayers& D, std::vector<DecodeLayerPtrs>& layers) {
     const slai_gpt2_config& c = m->cfg;
-    if (m->ctx->stats_on || c.n_embd % 16) return false;
+    if (m->ctx->stats_on || c.n_embd % 16 || separate_layers(m->graphs)) return false;
     layers.resize(c.n_layer);
     const int fmt = m->layers[0].w_qkv ? m->layers[0].w_qkv->fmt : -1;
     if (fmt == SLAI_FMT_F32) return false;
@@ -1358,15 +1372,22 @@ static int gpt2_record(slai_gpt2* m, int kind) {
     // x = wte[:,tok] + wpe[:,pos]                                              gpt2/cpu.rs:227-228
     DecodeLayers D;
     std::vector<DecodeLayerPtrs> dl;
-    const bool one_launch = gpt2_one_launch(m, D, dl);
+    bool one_launch = gpt2_one_launch(m, D, dl);
     if (one_launch && (rc = layers_scratch_reserve(ctx, D, &m->layers_scratch))) return rc;
     if ((rc = launch_embed_q8(ctx, m->x, m->wte, d_token, m->wpe, d_pos, false, nullptr, nullptr, 0,
                               one_launch ? decode_layers_counter(m->layers_scratch) : nullptr)))
         return rc;
     n++;
     if (one_launch) {
-        if ((rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch))) return rc;
-        n++;
+        rc = decode_layers_launch(ctx, D, dl.data(), m->layers_scratch);
+        if (rc == DECODE_LAYERS_NO_FIT) {
+            one_launch = false;
+            m->graphs.separate = true;
+        } else if (rc) {
+            return rc;
+        } else {
+            n++;
+        }
     }
     const size_t esz = c.kv_dtype == SLAI_KV_F16 ? 2 : 4;
     for (int l = one_launch ? c.n_layer : 0; l < c.n_layer; l++) {
