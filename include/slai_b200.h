@@ -322,9 +322,10 @@ int slai_llama_read_kv(slai_llama* m, int layer, int n_pos, float* h_keys, float
 /* Where a decode step spends its device time.  Classes (index of `us` / `launches`): 0 everything else (embedding,
  * rotation, sampling, collectives, gaps between kernels), 1 norm + q/k/v GEMV + RoPE + cache append, 2 attention,
  * 3 output projection + residual, 4 norm + gate/up GEMV + SiLU, 5 down projection + residual, 6 final norm + logits
- * GEMV.  The step runs once outside the replayed graph, kernel after kernel (no overlap between launches), with events
- * around each launch: the sum is therefore larger than the time of a replayed step; the split is what it is for.  It
- * is a real step: position `pos` of the KV cache is written.  Replaces reading the reference's per-dispatch GPU
+ * GEMV.  The step's operators run once outside the replayed graph, kernel after kernel (no overlap between launches), with events
+ * around each launch: the sum is therefore larger than the time of a replayed step, most of all where a step's layers are one launch
+ * (matrices of one format, adjacent-pair RoPE, not sharded); the split is what it is for.  Afterwards cache row `pos`, state and
+ * logits are those of a step.  Replaces reading the reference's per-dispatch GPU
  * timestamps (crates/slai/src/models/llama2/transformer.rs:316-381 runs each operator as its own dispatch). */
 typedef struct slai_llama_stats_t {
     float us_total;

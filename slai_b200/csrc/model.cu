@@ -1198,8 +1198,8 @@ SLAI_API int slai_llama_prefill(slai_llama* m, const int32_t* h_tokens, int32_t 
     }
     return prefill_impl(m, llama_record, m->cfg.vocab_size, m->cfg.seq_len, h_tokens, n, pos0, h_last_logits);
 }
-// One decode step outside the graph and without programmatic dependent launch, with events around every GEMV and
-// attention launch: device time per kernel class.  The step is a real one (the KV cache is written at `pos`).
+// One decode step kernel by kernel, outside the graph and without programmatic dependent launch, with events around every GEMV and
+// attention launch: device time per kernel class.  What it leaves behind is what a step does (the KV cache is written at `pos`).
 SLAI_API int slai_llama_stats(slai_llama* m, int32_t token, int32_t pos, slai_llama_stats_t* out) {
     if (!m || !out) return SLAI_ERR_INVALID_ARG;
     SLAI_ENTER(m->ctx);
@@ -1236,10 +1236,14 @@ SLAI_API int slai_llama_stats(slai_llama* m, int32_t token, int32_t pos, slai_ll
     ctx->stats_cls.clear();
     if (rc) return rc;
     if (e != cudaSuccess) return slai_set_error(ctx, SLAI_ERR_CUDA, "stats: %s", cudaGetErrorString(e));
-    // What is left behind (cache row, logits) is a plain step's, whose layers may be one launch with sums in another order.
-    if ((rc = set_scalars(m, token, pos, 0))) return rc;
-    if ((rc = llama_record(m, G_DECODE))) return rc;
-    SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    // A model whose step is not these kernels (its layers are one launch, with sums in another order): what is left behind, cache row and logits, is the step's.
+    DecodeLayers D;
+    std::vector<DecodeLayerPtrs> dl;
+    if (llama_one_launch(m, m->cfg.rope_variant == 0 && m->head_size / 2 <= 256, D, dl)) {
+        if ((rc = set_scalars(m, token, pos, 0))) return rc;
+        if ((rc = llama_record(m, G_DECODE))) return rc;
+        SLAI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     return slai_check_wait_flag(ctx);
 }
 
