@@ -465,7 +465,9 @@ __device__ __forceinline__ float stage_steps(const In& in, const float* norm_w, 
         const float mx = warp_max(fmaxf(max4(q[0]), max4(q[1])));
         float scale = 1.f, back = 1.f;
         if (mx > 0.f && mx < 3.0e38f) {
-            const int e = max((int)(__float_as_uint(mx) >> 23) - 126, -90);  // mx = f * 2^e with f in [0.5, 1) (normal numbers)
+            // mx = f * 2^e with f in [0.5, 1) (normal numbers); -100 is where the inverse is the smallest one.  (An RmsNorm's digits are those of x * w, which
+            // may be 1 / sqrt(eps) times smaller than what comes out of the norm: held at -90, x of 1e-32 kept 10 bits.)
+            const int e = max((int)(__float_as_uint(mx) >> 23) - 126, -100);
             scale = __uint_as_float((uint32_t)(127 + 26 - e) << 23);         // 2^(26 - e), and its inverse
             back = __uint_as_float((uint32_t)(127 - 26 + e) << 23);
         }

@@ -152,3 +152,16 @@ def test_small_layers_leave_the_cluster_at_a_long_context(backend, arch):
     assert np.array_equal(one(3, int(toks[3])), early)
     assert np.array_equal(m.generate(int(toks[first]), first, 100), m.generate(int(toks[first]), first, 100))
     m.close()
+
+
+@pytest.mark.parametrize("separate", [False, True])
+def test_norms_of_tiny_values_keep_their_bits(backend, monkeypatch, separate):
+    """x of 1e-32: what comes out of the norms is 1 / sqrt(eps) = 316 times that, still far below one, and has 20 bits of each step's largest element at least."""
+    if separate:
+        monkeypatch.setenv("SLAI_SEPARATE_LAYERS", "1")
+    cfg = Llama2Config(dim=512, hidden_dim=1024, n_layers=2, n_q_heads=4, n_kv_heads=4, vocab_size=300, seq_len=8, kv_dtype=F32)
+    w = synthetic_llama_host(cfg, synth.FMT_Q6_K, seed=31, std=0.05, embd_std=1e-32)
+    m, ref = llama_from_host(backend, cfg, w, synth.FMT_Q6_K), oracle_llama(cfg, w, synth.FMT_Q6_K)
+    for pos, tok in enumerate((5, 17, 200)):
+        assert rel_l2(m.forward_logits(pos, tok)[0] * 1e30, ref.forward(tok, pos).astype(np.float64) * 1e30) < 1e-5
+    m.close()
