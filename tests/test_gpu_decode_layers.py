@@ -1,6 +1,7 @@
 """The layers of a decode step in one launch (decode_layers.cuh) against the oracle, at the edges of its dispatch: one cluster of blocks or the whole chip,
 splits of the positions (more positions than a round of lane groups holds), one or two query heads an item, widths that are not multiples of a digit step,
-both cache types, every format.  Bars as in test_gpu_models.py: 1e-3 relative L2 of the logits, two orders above what is measured."""
+both cache types, every format.  Bars, relative L2 of the logits: 1e-3 with f16 caches, where a key may round to the other of two halves (test_gpu_models.py's bar);
+1e-5 with f32 caches, whose steps keep 26 bits: both sides' f32 sums are what is left (measured 2e-7 to 2e-6; the lowest digit of the input alone is 4e-6 of it)."""
 import threading
 
 import numpy as np
@@ -35,8 +36,9 @@ def test_decode_against_the_oracle(backend, dim, hidden, hq, hkv, fmt, kv, n):
         got = m.forward_logits(pos, int(tok))[0]
         want = ref.forward(int(tok), pos)
         if pos < 3 or pos % 16 < 2 or pos == n - 1:
-            assert rel_l2(got, want) < 1e-3, pos
-            assert rel_l2(m.read_state("x"), ref.x()) < 1e-3, pos
+            bar = 1e-3 if kv == F16 else 1e-5
+            assert rel_l2(got, want) < bar, (pos, rel_l2(got, want))
+            assert rel_l2(m.read_state("x"), ref.x()) < bar, (pos, rel_l2(m.read_state("x"), ref.x()))
     assert m.launches_per_token() == 4  # embedding, layers, logits, greedy choice
     m.close()
 
@@ -54,9 +56,38 @@ def test_biases_and_a_tall_feed_forward_part(backend):
     ref = oracle_llama(cfg, w, fmt)
     for pos in range(cfg.seq_len):
         tok = int(rng.integers(cfg.vocab_size))
-        assert rel_l2(m.forward_logits(pos, tok)[0], ref.forward(tok, pos)) < 1e-3, pos
+        assert rel_l2(m.forward_logits(pos, tok)[0], ref.forward(tok, pos)) < 1e-5, pos
     assert m.launches_per_token() == 4
     m.close()
+
+
+@pytest.mark.parametrize("fmt", [synth.FMT_Q4_K, synth.FMT_Q5_K, synth.FMT_Q6_K, synth.FMT_Q8_0])
+@pytest.mark.parametrize("dim,hidden,hq,hkv", [(512, 1280, 8, 4), (2048, 5632, 16, 16)])  # one cluster, the whole chip
+def test_one_launch_against_the_separate_kernels(backend, monkeypatch, fmt, dim, hidden, hq, hkv):
+    """The same model both ways, f32 caches, where the 256-element steps of every norm's output differ by up to 2^12 and the matrices' columns make up for it: each
+    step's scale counts, and every digit of it."""
+    cfg = Llama2Config(dim=dim, hidden_dim=hidden, n_layers=2, n_q_heads=hq, n_kv_heads=hkv, vocab_size=300, seq_len=24, kv_dtype=F32)
+    w = synthetic_llama_host(cfg, fmt, seed=17, std=0.05, embd_std=1.0)
+    rng = np.random.default_rng(3)
+    for l in range(cfg.n_layers):
+        for norm, names in (("attn_norm", ("wq", "wk", "wv")), ("ffn_norm", ("w_gate", "w_up"))):
+            p2 = 2.0 ** rng.integers(-6, 7, size=dim // 256).repeat(256)  # (an f16 scale has to hold the inverse)
+            w[(norm, l)] = p2.astype(np.float32)
+            for name in names:
+                r, c = cfg.matrix_shapes()[name]
+                w[(name, l)] = synth.quantize(fmt, (synth.normal_matrix([l, r, len(name)], r, c, 0.05) / p2).astype(np.float32))
+    one = llama_from_host(backend, cfg, w, fmt)
+    many = llama_from_host(backend, cfg, w, fmt)
+    toks = rng.integers(0, cfg.vocab_size, size=cfg.seq_len)
+    got = [(one.forward_logits(pos, int(t))[0].copy(), one.read_state("x")) for pos, t in enumerate(toks)]
+    monkeypatch.setenv("SLAI_SEPARATE_LAYERS", "1")
+    for pos, t in enumerate(toks):
+        logits = many.forward_logits(pos, int(t))[0]
+        # the same digits and integer sums; f32 sums over the steps and warps in another order, a few 2^-24 of the largest terms, over two layers
+        assert rel_l2(got[pos][0], logits) < 2e-6 and rel_l2(got[pos][1], many.read_state("x")) < 2e-6, (pos, rel_l2(got[pos][0], logits))
+    assert one.launches_per_token() == 4 and many.launches_per_token() == 3 + 5 * cfg.n_layers
+    one.close()
+    many.close()
 
 
 def test_gpt2_decode_against_the_oracle(backend):
