@@ -79,10 +79,6 @@ SLAI_HD void fetch(const unsigned char* blk, int r16, int part, int st, Packed& 
     }
 }
 
-SLAI_HD void put(unsigned char* plane, int r, int c, const uint32_t (&v)[4]) {
-    *reinterpret_cast<uint4*>(plane + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
-}
-
 // A row's 32 of the 64 columns of a stage as pairs of halves, hi (and lo) plane: words 0-7 and 8-15 are columns 16 part .. and 32 + 16 part ..
 // (Q8_0: all sixteen are columns 32 part ..).
 template <int FMT>
@@ -132,22 +128,6 @@ SLAI_HD void make(const Packed& P, int st, uint32_t (&hi)[16], uint32_t (&lo)[16
             const __half2 v = __hmul2(q, d);
             hi[i] = bits(v);
             lo[i] = bits(fma2(q, d, __hneg2(v)));
-        }
-    }
-}
-
-// The same words as row r of operand planes in memory, in 128-byte swizzled chunks (what the CPU test looks at).
-template <int FMT>
-SLAI_HD void emit(const Packed& P, int r, int part, int st, unsigned char* hi, unsigned char* lo) {
-    uint32_t h[16], l[16];
-    make<FMT>(P, st, h, l);
-    for (int c = 0; c < 4; c++) {
-        const int chunk = FMT == 8 ? 4 * part + c : 4 * (c >> 1) + 2 * part + (c & 1);
-        const uint32_t vh[4] = {h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]};
-        put(hi, r, chunk, vh);
-        if (Fmt<FMT>::PLANES == 2) {
-            const uint32_t vl[4] = {l[4 * c], l[4 * c + 1], l[4 * c + 2], l[4 * c + 3]};
-            put(lo, r, chunk, vl);
         }
     }
 }

@@ -1,7 +1,7 @@
 // The prompt GEMM's operand staging (slai_b200/csrc/prefill_dequant.cuh) on the host: one 16-row tile, every thread of the warp
 // that serves it in turn.  Usage: host_prefill <fmt> <K> <blocks.bin (16 rows, GGUF order)>  -> 16 x K doubles (binary, stdout):
-// the weights as the kernel's products see them (operand planes un-swizzled and added, times the row scale, minus the
-// minimum term).
+// the weights as the kernel's products see them (the words that go to tensor memory, both planes added, times the row scale, minus
+// the minimum term).
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -31,16 +31,21 @@ static void run(const std::vector<uint8_t>& tile, int K, std::vector<double>& ou
     const int elems = layout::step_elems(FMT), steps = (int)layout::num_steps(FMT, K);
     for (int tile_row = 0; tile_row < 128; tile_row += 112)  // first and last 16 rows of a CTA's 128
         for (int c = 0; c < steps; c++) {
-            alignas(16) unsigned char hi[128 * 128], lo[128 * 128], mn[128 * 32];
+            alignas(16) unsigned char mn[128 * 32];
             const unsigned char* blk = tile.data() + (size_t)c * F::STEP;
             for (int lane = 0; lane < 32 && F::MIN; lane++) pfq::min_row(blk, lane & 15, tile_row + (lane & 15), lane >> 4, mn);
             for (int st = 0; st < F::STAGES; st++) {
-                memset(hi, 0xFF, sizeof hi);
-                memset(lo, 0, sizeof lo);
+                double sum[16][64];  // 16 rows, the stage's 64 columns
                 for (int lane = 0; lane < 32; lane++) {
+                    const int r16 = lane & 15, part = lane >> 4;
                     pfq::Packed p = {};
-                    pfq::fetch<FMT>(blk, lane & 15, lane >> 4, st, p);
-                    pfq::emit<FMT>(p, tile_row + (lane & 15), lane >> 4, st, hi, lo);
+                    pfq::fetch<FMT>(blk, r16, part, st, p);
+                    uint32_t hi[16], lo[16] = {};
+                    pfq::make<FMT>(p, st, hi, lo);
+                    for (int i = 0; i < 32; i++) {  // the words' halves
+                        const int col = FMT == 8 ? 32 * part + i : 32 * (i >> 4) + 16 * part + (i & 15), sh = 16 * (i & 1);
+                        sum[r16][col] = half_bits((hi[i >> 1] >> sh) & 0xFFFF) + (F::PLANES == 2 ? half_bits((lo[i >> 1] >> sh) & 0xFFFF) : 0.0);
+                    }
                 }
                 for (int r16 = 0; r16 < 16; r16++) {
                     const int r = tile_row + r16;
@@ -48,7 +53,7 @@ static void run(const std::vector<uint8_t>& tile, int K, std::vector<double>& ou
                     for (int k = 0; k < 64; k++) {
                         const int col = c * elems + 64 * st + k;
                         if (col >= K) continue;
-                        double w = at(hi, 128, r & 7, r, k) + at(lo, 128, r & 7, r, k);
+                        double w = sum[r16][k];
                         if (F::SCALED) w *= half_bits(dd & 0xFFFF);
                         if (F::MIN) {
                             const int j = 2 * st + (k >> 5), sw = (r >> 2) & 1;

@@ -1,4 +1,4 @@
-"""The prompt GEMM's operand staging (packed quants -> swizzled fp16 rows, row scales, minimum term) executed on the CPU
+"""The prompt GEMM's operand staging (packed quants -> fp16 pairs of columns, row scales, minimum term) executed on the CPU
 (tests/host_prefill.cpp) against the oracle's dequantised weights.  Q4_K, Q5_K and Q6_K operands are exact integers times the
 block scales: they differ from the oracle's f32 weights by the oracle's own two roundings, 2^-24 each of the two terms
 (minimum and product) at most.  Q8_0: pairs of halves carry q * d to 2^-22, plus half a step of the smallest fp16 number."""
