@@ -153,15 +153,36 @@ def build_model(backend, seed=0):
     return cfg, m, mats, raw
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of the gate/up kernel on 2 x 11008 x 4096 Q4_K, from an ncu capture
+# dram__bytes_read.sum + dram__bytes_write.sum of the step's layers (one launch, decode_layers_kernel) per layer of the model, from an ncu capture of a
+# two-layer model of this shape at position 501 (summary under profiles/)
+LAYERS_DRAM_BYTES = 127_440_000
+# The same per launch of the gate/up operator on 2 x 11008 x 4096 Q4_K, from an ncu capture
 # of `python -m slai_b200.microbench --fmt q4_k --M 11008 --K 4096 --pair` (summary under profiles/): 2 x 688 tiles x 16 steps x 2368-byte blocks = 52 137 984 bytes of weights (the 2.8 % above the
 # GGUF byte count being the unpacked scales) plus the vectors
-DOMINANT_KERNEL_DRAM_BYTES = 52_230_000
+GATE_UP_DRAM_BYTES = 52_230_000
 
 
-def time_dominant_kernel(backend, ctx, cfg, mats, rounds=8):
-    """Average duration of the decode step's dominant kernel: RmsNorm + gate/up GEMV pair + SiLU (2 x 11008 x 4096 Q4_K, the
-    largest share of the step), run on the gate / up matrices of all 32 layers in turn (1.6 GB, larger than L2) as one
+def time_logits_product(backend, ctx, cfg, out_matrix, rounds=50):
+    """Seconds of the logits product as an operator of its own, in a recorded pass: the part of a step that is not its layers, but for the embedding row and the
+    greedy choice (its 107 MB stay in L2 here: no longer than in the step)."""
+    x = backend.vector(np.random.default_rng(0).standard_normal(cfg.dim).astype(np.float32))
+    out = backend.zeros(cfg.vocab_size)
+    ctx.matmul_quant_assign(out, out_matrix, x)
+    backend.synchronize()
+    with backend.record() as rec:
+        ctx.matmul_quant_assign(out, out_matrix, x)
+    rec.launch(3)
+    backend.synchronize()
+    backend.timer_start()
+    rec.launch(rounds)
+    ms = backend.timer_stop()
+    rec.close()
+    return ms / rounds * 1e-3
+
+
+def time_gate_up_operator(backend, ctx, cfg, mats, rounds=8):
+    """Average duration of the largest operator a host engine calls itself: RmsNorm + gate/up GEMV pair + SiLU (2 x 11008 x 4096 Q4_K; the timed step's layers
+    are one launch and do not contain it as a kernel), run on the gate / up matrices of all 32 layers in turn (1.6 GB, larger than L2) as one
     recorded pass, CUDA events on the launching stream.  Algorithmic bytes: both matrices' GGUF bytes + input + output."""
     from slai_b200 import synth
     x = backend.vector(np.random.default_rng(0).standard_normal(cfg.dim).astype(np.float32))
@@ -604,7 +625,8 @@ def main():
             batch = measure_batch(m, cfg, 8, PROMPT_LEN, 32, 3, ms / K)
         except Exception as e:  # the headline line is still reported
             batch = {"error": f"{type(e).__name__}: {e}"}
-    algo, per, nl = time_dominant_kernel(backend, ctx, cfg, mats) if rank == 0 else (0, 1.0, 0)
+    algo, per, nl = time_gate_up_operator(backend, ctx, cfg, mats) if rank == 0 else (0, 1.0, 0)
+    logits_s = time_logits_product(backend, ctx, cfg, raw["output"]) if rank == 0 else 0.0
     launches_per_token = m.launches_per_token()
     backend.lib.slai_free_host(backend.h, pinned)
     cpu = None
@@ -636,6 +658,8 @@ def main():
         kv_mean = float(np.mean([cfg.kv_bytes_at(p) for p in range(pos_first, pos_last + 1)]))
         small = (2 * cfg.n_layers + 1) * cfg.dim * 4 + cfg.dim * 4
         token_bytes = wbytes + kv_mean + small
+        layers_bytes = wbytes - cfg.vocab_size * cfg.dim * synth.BITS_PER_WEIGHT[synth.FMT_Q6_K] / 8 + kv_mean + 2 * cfg.n_layers * cfg.dim * 4
+        layers_s = ms / K * 1e-3 - logits_s
         line = {
             "metric": "decode tok/s bs1 (Llama-2-7B Q4_K)", "value": value, "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": W,
             "ms_per_step": ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -647,12 +671,19 @@ def main():
             "launches_per_token": launches_per_token,
             "token_roofline": {"bytes_per_token": token_bytes, "roofline_tok_s": peak * 1e9 / token_bytes,
                                "frac": (value / world) / (peak * 1e9 / token_bytes), "peak_source": peak_src},
-            "roofline": {"bound": "hbm", "kernel": "gemv_kernel<Q4_K, gate/up pair, rmsnorm, silu> 2 x 11008x4096: the decode step's dominant kernel "
-                                                   "(all 32 layers' pairs in turn, 1.6 GB > L2)",
-                         "achieved": algo / per / 1e9, "peak": peak, "unit": "GB/s", "frac": algo / per / 1e9 / peak,
-                         "traffic": DOMINANT_KERNEL_DRAM_BYTES, "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of this "
-                         "kernel on this shape (captured launches of slai_b200.microbench --pair); algorithmic bytes %d" % algo,
-                         "launches_timed": nl, "us_per_launch": per * 1e6, "peak_source": peak_src},
+            "roofline": {"bound": "hbm", "kernel": "decode_layers_kernel<Q4_K, llama, one query head an item, f16 cache>: the %d layers of a step in one launch" % cfg.n_layers,
+                         "achieved": layers_bytes / layers_s / 1e9, "peak": peak, "unit": "GB/s", "frac": layers_bytes / layers_s / 1e9 / peak,
+                         "bytes": layers_bytes, "traffic": LAYERS_DRAM_BYTES * cfg.n_layers,
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel on two layers of this shape, times the layers",
+                         "launches_timed": K, "us_per_launch": layers_s * 1e6,
+                         "time_source": "the timed step less the logits product (%.1f us as an operator): embedding row and greedy choice still in it" % (logits_s * 1e6),
+                         "peak_source": peak_src},
+            "operator_roofline": {"bound": "hbm", "kernel": "gemv_kernel<Q4_K, gate/up pair, rmsnorm, silu> 2 x 11008x4096, an operator of its own, not a kernel of the timed "
+                                                            "step (all 32 layers' pairs in turn, 1.6 GB > L2)",
+                                  "achieved": algo / per / 1e9, "peak": peak, "unit": "GB/s", "frac": algo / per / 1e9 / peak,
+                                  "traffic": GATE_UP_DRAM_BYTES, "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of this "
+                                  "kernel on this shape (captured launches of slai_b200.microbench --pair); algorithmic bytes %d" % algo,
+                                  "launches_timed": nl, "us_per_launch": per * 1e6, "peak_source": peak_src},
         }
         if gemv_table is not None:
             line["gemv_microbench"] = gemv_table
