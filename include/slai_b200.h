@@ -72,9 +72,11 @@ int slai_ctx_destroy(slai_ctx* ctx);
  * inside a kernel (weight ring, grid barrier) ran out since the last call: every device-side wait has an
  * iteration limit and raises a flag instead of hanging. */
 int slai_ctx_sync(slai_ctx* ctx);
-/* Rounds a device-side wait polls before it gives up (default 2^20, about a second).  No counterpart in the
- * reference, whose dispatches never wait on one another.  Applies to launches described after the call; a host
- * that supervises its ranks itself can shorten it to detect a missing peer sooner.  rounds >= 16. */
+/* Rounds a device-side wait polls before it raises the error (default 2^20, about a second; rounded down to even).  No
+ * counterpart in the reference, whose dispatches never wait on one another.  A wait for another rank then goes on without it; a
+ * wait for a block's own copies and products goes on until they are there (they must not land later); waits of blocks for one
+ * another have at least 2^14 rounds.  Applies to launches described after the call; a host that supervises its ranks itself can
+ * shorten it to detect a missing peer sooner.  rounds >= 16. */
 int slai_ctx_set_wait_limit(slai_ctx* ctx, uint32_t rounds);
 const char* slai_last_error_string(slai_ctx* ctx);
 void* slai_ctx_stream(slai_ctx* ctx); /* the cudaStream_t all work of this context is enqueued on */

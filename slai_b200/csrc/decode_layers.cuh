@@ -483,6 +483,8 @@ __device__ __forceinline__ void attention_phase(const LayersParams& P, int layer
 #define DL_STAMP(k)
 #endif
 
+// 16 warps leave 128 registers a thread.  Two query heads an item with an f16 cache (most grouped-query models) is the one instance that does not fit: it spills
+// 60 bytes (120 bytes of loads) in every format, in the attention phase.
 template <class F, int ARCH, int MAXQ, typename T>
 __global__ void __launch_bounds__(THREADS, 1) decode_layers_kernel(const __grid_constant__ LayersParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -27,8 +27,8 @@
 //
 // What bounds it: from some 200 tokens on power (the clock falls to 1.6 GHz with the tensor cores 63 % busy; 511 tokens, gate and up: 1180 TFLOP/s
 // executed, where cuBLAS keeps 1375); with few tokens the chain of a stage through operand writer, product and commit (some 620 cycles for products of
-// 200), and 8 us of start and end a launch.  us per product of the 7B shape, weights' operands in shared memory and whole tiles / now: 511 tokens q/k/v 89.5 / 82, gate
-// and up 145 / 135, down 77 / 72; 37 tokens gate and up 57 / 34.
+// 200), and 8 us of start and end a launch.  us per product of the 7B shape, Q4_K (ncu, serialised: the power limit is not reached): 37 tokens q/k/v 26, o 16, gate and
+// up 35, down 25; 511 tokens 91, 40, 151, 80.
 // Every wait is bounded (bounded_wait): `wait_limit` polls, after which the error flag is raised, then LAST_POLLS more, because what it waits for is this CTA's
 // (pair's) own work and copies, which have to land before the CTA ends.  Only a thread whose last polls ran out too goes on without: it arrives on nothing and
 // requests nothing from then on, so that no barrier completes a phase it has not reached.  Whoever requested copies or products waits for
@@ -810,8 +810,9 @@ int launch_fmt(slai_ctx* ctx, PgParams& P, const PrefillGemm& G) {
     // What the longest SM has to do, in units of a plain super-block (some 2400 cycles): whole tiles one after the other; an equal share of all super-blocks,
     // where every CTA that a tile is spread over beyond its first costs the one that adds the sums about two; or a share of K of one tile in a
     // cluster, about three and a half for its start and end in every round.  A pair's super-block takes about two thirds of the time (half the
-    // activations' L2 and shared-memory traffic per SM).  us per product, 7B shape, whole tiles or cluster / equal shares: 37 tokens q/k/v 30.1 / 27.7, o
-    // 17 (cluster of 4) / 21, gate and up 57 (2) / 38.6, down 27 (4) / 31; 200 tokens q/k/v 64 / 56, gate and up 95 / 88; 511 tokens (pairs) o 41 / 47.
+    // activations' L2 and shared-memory traffic per SM).  us per product, 7B shape, without equal shares / as chosen (ncu, serialised; the same
+    // build with the rule off): 37 tokens q/k/v 27.2 / 25.7, gate and up 47.6 / 35.1 (o and down stay clusters of 4: 16.0, 24.9); 200 tokens q/k/v 59.5 / 50.4, gate and
+    // up 86.0 / 78.0, down 53.4 / 50.9; 511 tokens (pairs) q/k/v 92.9 / 91.3, gate and up 149.5 / 151.4.
     const int sms = std::min(ctx->sm_count > 0 ? ctx->sm_count : 148, PG_MAX_CTAS);
     auto m_tiles = [&](int rows) {
         int t = 0;
