@@ -6,8 +6,10 @@
 // for the load of the input behind it), and the rings of weight blocks run on across the barriers.  What is left of the 43 us a layer now takes are chains of latencies: four
 // warps a scheduler issue one of their instructions every 8 cycles, so what counts is the number of instructions between two barriers, and
 // the size of the code (all of it is run once a layer; 137 KB of it took 24 % longer than 60 KB).
-// us a token, kernel by kernel / here: Llama-2 7B Q4_K at position 515 1579 / 1457, 8 layers of the 70B shape at 3500 1301 / 1140, GPT-2 XL 1511 / 1348,
-// the tiny story model 122 / 111.
+// us a token, kernel by kernel (whose vectors are staged the same way by now) / here: Llama-2 7B Q4_K at position 515 1484 / 1458, with an f32 cache 1471 / 1500; 8
+// layers of the 70B shape at 3500 1239 / 1136; GPT-2 XL 1476 / 1353; the tiny story model 107.5 / 110.8: what is left is the gain of LayerNorm models and of
+// grouped queries.  All SMs are taken at once: two contexts that decode at the same time take turns (8 layers 1024 wide: 5381 tokens/s together, kernel by kernel
+// 8032; 512 wide 6790 and 10582; 4096 wide 2989 and 3590), and a step waits for other streams' kernels (SLAI_SEPARATE_LAYERS).
 //
 // A layer is five phases, as many as the separate path has launches:
 //   q/k/v    norm of x, product, RoPE, q to its buffer, k and v to the cache (PH_QKV)
